@@ -953,21 +953,18 @@ int wb200_quantize_mxfp4(const void* x, int x_dtype, long long ldx, int rows, in
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int k_atoms = wb::sf_k_atoms(K);
-  if (scale_packed && (rows % 128 != 0 || (K / 32) % 8 != 0)) {
-    const int rbs = wb::sf_row_blocks(rows);
-    const long long total = (long long)rbs * k_atoms * 512;
-    wb::fill_scale_padding_kernel<<<unsigned((total + 255) / 256), 256, 0, s>>>(static_cast<uint8_t*>(scale_packed), rows,
-                                                                                  K / 32, k_atoms, rbs);
-  }
-  const dim3 blocks(rows, (K / 32 + 63) / 64);
+  const int total_rows = scale_packed ? wb::sf_row_blocks(rows) * 128 : rows;
+  const int q_vec = (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+  const long long warps = (long long)total_rows * ((k_atoms + 7) / 8);
+  const unsigned blocks = unsigned((warps + 7) / 8);
   if (x_dtype == WB200_F32)
-    wb::quantize_mxfp4_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), ldx, rows, K, static_cast<uint8_t*>(q),
-                                                            static_cast<uint8_t*>(scale_rowmajor),
+    wb::quantize_mxfp4_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), ldx, rows, total_rows, K,
+                                                            static_cast<uint8_t*>(q), q_vec, static_cast<uint8_t*>(scale_rowmajor),
                                                             static_cast<uint8_t*>(scale_packed), k_atoms);
   else
     wb::quantize_mxfp4_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(x), ldx, rows, K, static_cast<uint8_t*>(q), static_cast<uint8_t*>(scale_rowmajor),
-        static_cast<uint8_t*>(scale_packed), k_atoms);
+        static_cast<const __nv_bfloat16*>(x), ldx, rows, total_rows, K, static_cast<uint8_t*>(q), q_vec,
+        static_cast<uint8_t*>(scale_rowmajor), static_cast<uint8_t*>(scale_packed), k_atoms);
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
 }
@@ -1143,14 +1140,18 @@ int wb200_moe_quantize_scatter(const void* x, int x_dtype, long long ldx, int to
   int rc = get_device(&dev);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const dim3 blocks(tokens, (K / 32 + 63) / 64);
+  const int k_atoms = wb::sf_k_atoms(K);
+  const int q_vec = (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+  const long long warps = (long long)tokens * ((k_atoms + 7) / 8);
+  const unsigned blocks = unsigned((warps + 7) / 8);
   if (x_dtype == WB200_F32)
     wb::quantize_scatter_mxfp4_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), ldx, tokens, K, top_k, dst_rows,
-                                                                    static_cast<uint8_t*>(q), static_cast<uint8_t*>(scale_rowmajor));
+                                                                    static_cast<uint8_t*>(q), q_vec,
+                                                                    static_cast<uint8_t*>(scale_rowmajor), nullptr, k_atoms, 0);
   else
     wb::quantize_scatter_mxfp4_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), ldx, tokens, K,
-                                                                            top_k, dst_rows, static_cast<uint8_t*>(q),
-                                                                            static_cast<uint8_t*>(scale_rowmajor));
+                                                                            top_k, dst_rows, static_cast<uint8_t*>(q), q_vec,
+                                                                            static_cast<uint8_t*>(scale_rowmajor), nullptr, k_atoms, 0);
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
 }
