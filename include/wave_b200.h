@@ -203,6 +203,23 @@ int wb200_moe_gather_rows(const void* src, long long src_pitch, int row_bytes, c
 int wb200_silu_and_mul(const void* x1, const void* x2, long long ld1, long long ld2, int dtype, int rows, int n, void* out,
                        long long ldo, void* q, void* scale_rowmajor, void* scale_packed, const int* num_rows, void* stream);
 
+/* The whole expert MLP on device-side routing: out[t] = sum_j w_j * down_e(silu(gate_e(x_t)) * up_e(x_t)) over the top_k
+ * experts of token t, w = softmax(logits) in f32 (tests/kernel/moe_test.py:105-127). Six launches on `stream`, each the
+ * programmatic dependent of the one before; nothing is read on the host. x [T, K] and logits [T, E] are f32 or bf16
+ * (pitches in elements, x rows 16-byte aligned), out [T, N] bf16. w1[e]: packed E2M1 [2 inter, K/2], gate rows then up
+ * rows; w2[e]: [N, inter/2]; w1_scale / w2_scale: their scales from wb200_repack_scales (HOST arrays of device
+ * pointers). The gate|up GEMM rounds its sums to bf16 and writes silu(gate) * up already quantised, the codes of
+ * wb200_mxfp4_moe_gemm + wb200_silu_and_mul.
+ * w1_scale_decode (may be NULL; used for T <= 128): w1's scales packed in the row order of 128-row tiles of 64 gate rows
+ * and the 64 up rows of the same hidden columns. Limits: E <= 32, inter % 128 == 0, K % 32 == 0, N % 32 == 0.
+ * workspace: 16-byte aligned, of the size the first function returns (0 for arguments outside the limits). */
+size_t wb200_mxfp4_expert_mlp_workspace_bytes(int T, int E, int K, int inter, int N, int top_k);
+int wb200_mxfp4_expert_mlp(int T, int E, int K, int inter, int N, int top_k, const void* x, int x_dtype, long long ldx,
+                           const void* logits, int logits_dtype, long long ld_logits, const void* const* w1,
+                           const void* const* w1_scale, const void* const* w1_scale_decode, const void* const* w2,
+                           const void* const* w2_scale, void* out, long long ldo, void* workspace, size_t workspace_bytes,
+                           void* stream);
+
 /* Quantise routed tokens straight to their expert-sorted rows: row t of x [tokens, K] (f32 or bf16) is quantised
  * once (as wb200_quantize_mxfp4) and its codes and row-major scales are written to the rows dst_rows[t * top_k + j]
  * of q / scale_rowmajor for j < top_k (DEVICE array, the `inverse` output of wb200_moe_align_block_size; negative

@@ -269,3 +269,80 @@ def test_silu_and_mul_row_limit_from_device():
     ref = moe_oracle.silu_and_mul(h[:384, :n].cpu(), h[:384, n:].cpu())
     assert int(orc.bf16_ulp_distance(out[:384], ref).max()) <= 1
     assert bool((out[384:] == -3.0).all())
+
+
+def _poison(nbytes=1 << 28):
+    """Leave freed blocks full of 0xFF in the allocator: workspaces then start as NaN scales and saturated codes."""
+    blocks = [torch.full((n,), 255, dtype=torch.uint8, device=DEV) for n in (nbytes, 1 << 22, 1 << 20, 1 << 18)]
+    torch.cuda.synchronize()
+    del blocks
+
+
+@pytest.mark.parametrize("T,E,K,inter,N,k,x_dtype,l_dtype", [
+    (1, 4, 256, 128, 256, 1, torch.bfloat16, torch.float32),      # one token, one atom pair, one block
+    (16, 8, 416, 384, 160, 2, torch.float32, torch.bfloat16),     # K, N ragged, odd atom count of the hidden columns
+    (17, 3, 1024, 128, 96, 3, torch.bfloat16, torch.float16),     # every expert gets every token
+    (64, 32, 512, 256, 512, 8, torch.bfloat16, torch.float32),    # the large table of experts
+    (128, 9, 288, 640, 256, 2, torch.bfloat16, torch.float32),    # the largest batch of the decode form
+    (129, 9, 288, 640, 256, 2, torch.bfloat16, torch.float32),    # the smallest of the tile form
+    (700, 2, 512, 384, 160, 1, torch.float32, torch.float32),
+    (513, 17, 1056, 128, 4096, 4, torch.bfloat16, torch.bfloat16),
+])
+def test_expert_mlp_single_call_form(T, E, K, inter, N, k, x_dtype, l_dtype):
+    """The single native call against the oracle and against the step-by-step form, over both row layouts. The hidden codes
+    of the two forms are the same; the routing weights may differ in their last bits (another order of the softmax's sum),
+    so an output by one rounding to bf16, 2^-8 of itself. Against the oracle the f32 sums in front of the bf16 rounding
+    differ in their last bits: a value next to a rounding boundary moves by 2^-8, and about 2^-8 * 8 of those cross one of
+    the 4-bit quantiser, by a third of the value. With one in a hundred next to a boundary that is a share of 3e-4,
+    a relative 2-norm of sqrt(3e-4) / 3 ~ 6e-3, and 2^-8 / sqrt(3) of bf16 rounding in y and the output: 1.5e-2 in all."""
+    g = torch.Generator().manual_seed(T * 31 + E)
+    x = torch.randn(T, K, generator=g).to(x_dtype)
+    logits = torch.randn(T, E, generator=g).to(l_dtype)
+    w1, w1s, w2, w2s = [], [], [], []
+    for e in range(E):
+        q, s = orc.quantize_mxfp4(torch.randn(2 * inter, K, generator=g) * 0.05)
+        w1.append(q); w1s.append(s)
+        q, s = orc.quantize_mxfp4(torch.randn(N, inter, generator=g) * 0.05)
+        w2.append(q); w2s.append(s)
+    mlp = wb.MXFP4ExpertMLP([t.to(DEV) for t in w1], [t.to(DEV) for t in w1s], [t.to(DEV) for t in w2],
+                            [t.to(DEV) for t in w2s], top_k=k)
+    xd, ld = x.to(DEV), logits.to(DEV)
+    assert mlp._takes_fused(xd, ld)
+    _poison()
+    out = mlp(xd, ld)
+    ref = moe_oracle.expert_mlp(x, w1, w1s, w2, w2s, logits.float(), k)
+    assert float((out.cpu().float() - ref).norm() / ref.norm()) < 1.5e-2
+    steps = mlp._forward_steps(xd, ld).float()
+    assert bool(((out.float() - steps).abs() <= 2 ** -7 * steps.abs() + 1e-6 * steps.abs().max()).all())
+    assert torch.equal(mlp(xd, ld), out)  # whichever CTA takes a tile
+    wide = torch.zeros(T, K + 64, dtype=x_dtype, device=DEV)
+    wide[:, 32:K + 32] = xd
+    assert torch.equal(mlp(wide[:, 32:K + 32], ld.t().contiguous().t()), out)  # row pitch of x, column-major logits
+    ops.check_device_status()
+
+
+@pytest.mark.parametrize("T", [40, 200])
+def test_expert_mlp_single_call_form_special_logits(T):
+    """Masked experts (-inf), ties and a NaN row: the same tokens through the library router and the step-by-step form."""
+    E, K, inter, N, k = 6, 256, 128, 128, 2
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16).to(DEV)
+    logits = torch.randn(T, E, generator=g)
+    logits[3, 1:] = float("-inf")
+    logits[4, ::2] = float("-inf")
+    logits[5, 2] = float("nan")
+    w1 = [orc.quantize_mxfp4(torch.randn(2 * inter, K, generator=g) * 0.05) for _ in range(E)]
+    w2 = [orc.quantize_mxfp4(torch.randn(N, inter, generator=g) * 0.05) for _ in range(E)]
+    mlp = wb.MXFP4ExpertMLP([q.to(DEV) for q, _ in w1], [s.to(DEV) for _, s in w1], [q.to(DEV) for q, _ in w2],
+                            [s.to(DEV) for _, s in w2], top_k=k)
+    out = mlp(x, logits.to(DEV)).float()
+    steps = mlp._forward_steps(x, logits.to(DEV)).float()
+    assert bool(out[5].isnan().all()) and bool(steps[5].isnan().all())
+    rows = torch.arange(T, device=DEV) != 5
+    assert bool(((out[rows] - steps[rows]).abs() <= 2 ** -7 * steps[rows].abs() + 1e-6 * steps[rows].abs().max()).all())
+    # a tie between all experts: any of them is a correct choice; the lower ones are taken
+    tied = torch.zeros(T, E, device=DEV)
+    first = torch.full((T, E), -30.0, device=DEV)
+    first[:, :k] = 0.0
+    torch.testing.assert_close(mlp(x, tied).float() * 3.0, mlp(x, first).float(), rtol=2 ** -7, atol=1e-6)
+    ops.check_device_status()

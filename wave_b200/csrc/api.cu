@@ -356,7 +356,6 @@ int launch_grouped(const DeviceInfo& dev, int num_groups, const int* row_offsets
   const int tiles_n = (N + BN - 1) / BN;
   maps.num_groups = num_groups;
   maps.interleave = (c_ptrs != nullptr) ? 1 : 0;
-  maps.aligned = 0;
   maps.tiles_max = 0;
   maps.tile_start[0] = 0;
   for (int g = 0; g < num_groups; ++g) {
@@ -413,69 +412,121 @@ int launch_grouped(const DeviceInfo& dev, int num_groups, const int* row_offsets
   return WB200_OK;
 }
 
-// Grouped GEMM over a block-aligned row layout described by DEVICE arrays (see GroupedMaps::aligned).
-template <typename OutT, int BN = 256>
-int launch_aligned(const DeviceInfo& dev, int num_groups, int max_rows, const int* expert_ids, const int* num_rows, int N, int K,
-                   const void* a, const void* a_sf, const void* const* b_ptrs, const void* const* b_sf_ptrs, void* c,
-                   long long ldc, cudaStream_t stream) {
-  constexpr int CG = 2;
-  using Cfg = wb::GemmCfg<CG, BN, int(sizeof(OutT))>;
-  static wb::GroupedMaps maps;
-  static std::mutex mu;
-  std::lock_guard<std::mutex> lk(mu);
-  const int esz = int(sizeof(OutT));
-  const int k_atoms = wb::sf_k_atoms(K);
-  maps.num_groups = num_groups;
-  maps.interleave = 0;
-  maps.aligned = 1;
-  maps.tile_rows = Cfg::BM * CG;
-  maps.tiles_m_cap = max_rows / (Cfg::BM * CG);
-  maps.tiles_max = 0;
-  maps.expert_ids = expert_ids;
-  maps.num_rows = num_rows;
-  maps.c_base[0] = c;
-  for (int g = 0; g < num_groups; ++g) {
-    int rc = check_common(max_rows, N, K, a, a_sf, b_ptrs[g], b_sf_ptrs[g], c, esz == 4 ? WB200_F32 : WB200_BF16, ldc);
-    if (rc) return rc;
-    CUtensorMap* m = &maps.m[g * 5];
-    if ((rc = make_operand_map(m + 0, a, max_rows, K / 2, Cfg::BM))) return rc;
-    if ((rc = make_operand_map(m + 1, b_ptrs[g], N, K / 2, Cfg::B_ROWS))) return rc;
-    if ((rc = make_scale_map(m + 2, a_sf, wb::sf_row_blocks(max_rows), k_atoms, 1))) return rc;
-    if ((rc = make_scale_map(m + 3, b_sf_ptrs[g], wb::sf_row_blocks(N), k_atoms, Cfg::SFB_BLOCKS))) return rc;
-    if ((rc = make_output_map(m + 4, c, max_rows, N, ldc, esz))) return rc;
+// Launch attributes of a CTA-pair persistent kernel, optionally a programmatic dependent of the kernel before it.
+struct PairLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  PairLaunch(unsigned grid, int threads, int smem, cudaStream_t stream) {
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = tl_dependent_launch ? 2 : 1;
   }
+};
+
+// An ordinary kernel, optionally a programmatic dependent of the one before it in the stream.
+template <typename... P, typename... A>
+cudaError_t launch_kernel(bool dependent, void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+// Operands of a GEMM over routed rows: the weights of every expert, and which expert a row block belongs to (DEVICE arrays).
+struct RoutedGemm {
+  int num_groups, max_rows;
+  const int *expert_ids, *num_rows;
+  int N, K;
+  const void *a, *a_sf;
+  const void* const* b_ptrs;
+  const void* const* b_sf_ptrs;
+};
+// Where the gate|up projection leaves the quantised hidden activations.
+struct HiddenOut {
+  int inter;
+  void *q, *scale_packed;
+};
+
+// Grouped GEMM over a block-aligned row layout described by DEVICE arrays (see AlignedMaps); with `hidden` the gate|up
+// form (SiluMaps): N = 2 inter, nothing is written to c.
+template <typename OutT, typename Maps>
+int launch_aligned_maps(const DeviceInfo& dev, const RoutedGemm& g, void* c, long long ldc, const HiddenOut* hidden, cudaStream_t stream) {
+  constexpr int CG = 2, BN = 256;
+  using Cfg = wb::GemmCfg<CG, BN, int(sizeof(OutT))>;
+  Maps maps;
+  const int esz = int(sizeof(OutT));
+  const int k_atoms = wb::sf_k_atoms(g.K);
+  maps.num_groups = g.num_groups;
+  maps.tile_rows = Cfg::BM * CG;
+  maps.tiles_m_cap = g.max_rows / (Cfg::BM * CG);
+  maps.expert_ids = g.expert_ids;
+  maps.num_rows = g.num_rows;
+  maps.c_base = c;
+  int rc;
+  for (int e = 0; e < g.num_groups; ++e) {
+    rc = check_common(g.max_rows, g.N, g.K, g.a, g.a_sf, g.b_ptrs[e], g.b_sf_ptrs[e], Maps::kSilu ? hidden->q : c,
+                      esz == 4 ? WB200_F32 : WB200_BF16, Maps::kSilu ? g.N : ldc);
+    if (rc) return rc;
+    if ((rc = make_operand_map(&maps.w_map[2 * e], g.b_ptrs[e], g.N, g.K / 2, Cfg::B_ROWS))) return rc;
+    if ((rc = make_scale_map(&maps.w_map[2 * e + 1], g.b_sf_ptrs[e], wb::sf_row_blocks(g.N), k_atoms, Maps::kSilu ? 1 : Cfg::SFB_BLOCKS))) return rc;
+  }
+  if ((rc = make_operand_map(&maps.rows_map[0], g.a, g.max_rows, g.K / 2, Cfg::BM))) return rc;
+  if ((rc = make_scale_map(&maps.rows_map[1], g.a_sf, wb::sf_row_blocks(g.max_rows), k_atoms, 1))) return rc;
+  if constexpr (Maps::kSilu) maps.rows_map[2] = maps.rows_map[0];  // not used
+  else if ((rc = make_output_map(&maps.rows_map[2], c, g.max_rows, g.N, ldc, esz))) return rc;
   wb::GemmParams p = {};
   p.c = c;
-  p.M = max_rows; p.N = N; p.K = K;
+  p.M = g.max_rows; p.N = g.N; p.K = g.K;
   p.ldc = int(ldc);
   p.tiles_m = maps.tiles_m_cap;
-  p.tiles_n = (N + BN - 1) / BN;
+  p.tiles_n = (g.N + BN - 1) / BN;
+  if constexpr (Maps::kSilu) {
+    maps.q = static_cast<uint8_t*>(hidden->q);
+    maps.scale_packed = static_cast<uint8_t*>(hidden->scale_packed);
+    maps.inter = hidden->inter;
+    maps.k_atoms = wb::sf_k_atoms(hidden->inter);
+    p.tiles_n = hidden->inter / 128;
+  }
   p.group_n = std::max(1, std::min(tl_group_n, p.tiles_n));
   p.vec_ok = 1;
   p.tma_store = 1;
   p.accumulate = 0;
   p.status = dev.status_ptr;
-  auto kernel = wb::mxfp4_gemm_kernel<CG, BN, OutT, wb::GroupedMaps>;
+  auto kernel = wb::mxfp4_gemm_kernel<CG, BN, OutT, Maps>;
   static bool smem_set[kMaxDevices] = {};
-  int rc = set_smem(kernel, Cfg::SMEM_BYTES, smem_set);
-  if (rc) return rc;
+  if ((rc = set_smem(kernel, Cfg::SMEM_BYTES, smem_set))) return rc;
   const long long tiles = (long long)maps.tiles_m_cap * p.tiles_n;
   if (tiles == 0) return WB200_OK;
   const int units = dev.sm_count / CG;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(int(tiles < units ? tiles : units) * CG, 1, 1);
-  cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
-  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CG;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
+  PairLaunch l(unsigned(tiles < units ? tiles : units) * CG, Cfg::THREADS, Cfg::SMEM_BYTES, stream);
+  WB_CUDA(cudaLaunchKernelEx(&l.cfg, kernel, maps, p));
   return WB200_OK;
+}
+
+template <typename OutT>
+int launch_aligned(const DeviceInfo& dev, const RoutedGemm& g, void* c, long long ldc, cudaStream_t stream) {
+  if (g.num_groups <= 8) return launch_aligned_maps<OutT, wb::AlignedMaps<8>>(dev, g, c, ldc, nullptr, stream);
+  return launch_aligned_maps<OutT, wb::AlignedMaps<wb::kMaxGroups>>(dev, g, c, ldc, nullptr, stream);
+}
+
+int launch_aligned_silu(const DeviceInfo& dev, const RoutedGemm& g, const HiddenOut& hidden, cudaStream_t stream) {
+  if (g.num_groups <= 8) return launch_aligned_maps<__nv_bfloat16, wb::SiluMaps<8>>(dev, g, nullptr, 0, &hidden, stream);
+  return launch_aligned_maps<__nv_bfloat16, wb::SiluMaps<wb::kMaxGroups>>(dev, g, nullptr, 0, &hidden, stream);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -526,7 +577,6 @@ int launch_splitk(const DeviceInfo& dev, int slices, int M, int N, int K, const 
   last_valid = false;
   maps.num_groups = slices;
   maps.interleave = 1;
-  maps.aligned = 0;
   maps.tiles_max = tiles_m * tiles_n;
   maps.tile_start[0] = 0;
   for (int g = 0; g < slices; ++g) {
@@ -684,17 +734,17 @@ int launch_skinny_whole(const DeviceInfo& dev, int M, int N, int K, const void* 
                         int elem_format = 0) {
   using Base = wb::SkinnyCfg<NP, STAGES, EB, WR>;
   using Cfg = wb::SkinnyWholeCfg<NP, STAGES, EB, WR, SBUFS>;
-  CUtensorMap tmW, tmX, tmSFW, tmSFX;
+  wb::SkinnyMaps maps = {};
   const long long row_bytes = (long long)K * EB / 8;
   const int tile_rows = tl_b_tile_rows;  // 128 with the usual packing of the weight scales
   const int tiles_n = (N + tile_rows - 1) / tile_rows;
-  int rc = weights_are_fp4(EB, elem_format) ? make_operand_map_u4(&tmW, b, N, K, tile_rows) : make_operand_map(&tmW, b, N, row_bytes, tile_rows);
+  int rc = weights_are_fp4(EB, elem_format) ? make_operand_map_u4(&maps.w, b, N, K, tile_rows) : make_operand_map(&maps.w, b, N, row_bytes, tile_rows);
   if (rc) return rc;
-  rc = make_operand_map(&tmX, a, M, row_bytes, NP);
+  rc = make_operand_map(&maps.x, a, M, row_bytes, NP);
   if (rc) return rc;
-  rc = make_scale_map(&tmSFW, bs, tiles_n, wb::sf_k_atoms(K), 1, Base::SF_ATOMS);
+  rc = make_scale_map(&maps.sfw, bs, tiles_n, wb::sf_k_atoms(K), 1, Base::SF_ATOMS);
   if (rc) return rc;
-  rc = make_scale_map(&tmSFX, as, 1, wb::sf_k_atoms(K), 1, Base::SF_ATOMS);
+  rc = make_scale_map(&maps.sfx, as, 1, wb::sf_k_atoms(K), 1, Base::SF_ATOMS);
   if (rc) return rc;
   wb::SkinnyWholeParams p;
   p.c = c;
@@ -711,9 +761,8 @@ int launch_skinny_whole(const DeviceInfo& dev, int M, int N, int K, const void* 
   // TMA stores of the staged chunks: 16-byte aligned C, no accumulation, and two staging halves that each hold a chunk
   // in the output type (the single-buffer variant has room for bf16 chunks only)
   p.tma_store = (p.c_vec && !accumulate && (sizeof(OutT) == 2 || SBUFS == 2)) ? 1 : 0;
-  CUtensorMap tmC = {};
   if (p.tma_store) {
-    rc = make_output_map_dense(&tmC, c, M, N, ldc, int(sizeof(OutT)), tile_rows, 16);
+    rc = make_output_map_dense(&maps.c, c, M, N, ldc, int(sizeof(OutT)), tile_rows, 16);
     if (rc) return rc;
   }
   p.status = dev.status_ptr;
@@ -731,9 +780,80 @@ int launch_skinny_whole(const DeviceInfo& dev, int M, int N, int K, const void* 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = tl_dependent_launch ? 1 : 0;
-  WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, tmW, tmX, tmSFW, tmSFX, tmC, p));
+  WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
+}
+
+// The tiles of all experts of a decode step in one launch (SkinnyExpertMaps). T: tokens = rows of a block that can be real.
+template <int NP, int STAGES, typename Maps>
+int launch_skinny_experts(const DeviceInfo& dev, const RoutedGemm& g, int T, void* c, long long ldc, const HiddenOut* hidden, void* counters,
+                          cudaStream_t stream) {
+  using Base = wb::SkinnyCfg<NP, STAGES, 4>;
+  using Cfg = wb::SkinnyWholeCfg<NP, STAGES, 4>;
+  Maps maps;
+  const int k_atoms = wb::sf_k_atoms(g.K);
+  int rc;
+  const int tiles_n = Maps::kSilu ? hidden->inter / 64 : (g.N + 127) / 128;
+  for (int e = 0; e < g.num_groups; ++e) {
+    if ((rc = check_common(g.max_rows, g.N, g.K, g.a, g.a_sf, g.b_ptrs[e], g.b_sf_ptrs[e], Maps::kSilu ? hidden->q : c, WB200_BF16,
+                           Maps::kSilu ? g.N : ldc)))
+      return rc;
+    if ((rc = make_operand_map(&maps.w[e], g.b_ptrs[e], g.N, g.K / 2, Maps::kSilu ? 64 : 128))) return rc;
+    if ((rc = make_scale_map(&maps.sfw[e], g.b_sf_ptrs[e], tiles_n, k_atoms, 1, Base::SF_ATOMS))) return rc;
+  }
+  if ((rc = make_operand_map(&maps.x, g.a, g.max_rows, g.K / 2, NP))) return rc;
+  if ((rc = make_scale_map(&maps.sfx, g.a_sf, wb::sf_row_blocks(g.max_rows), k_atoms, 1, Base::SF_ATOMS))) return rc;
+  maps.num_groups = g.num_groups;
+  maps.max_blocks = g.max_rows / wb::kExpertBlockRows;
+  maps.expert_ids = g.expert_ids;
+  maps.num_rows = g.num_rows;
+  wb::SkinnyWholeParams p = {};
+  if constexpr (Maps::kSilu) {
+    maps.inter = hidden->inter;
+    maps.k_atoms = wb::sf_k_atoms(hidden->inter);
+    maps.q = static_cast<uint8_t*>(hidden->q);
+    maps.scale_packed = static_cast<uint8_t*>(hidden->scale_packed);
+    maps.c = maps.x;  // not used
+  } else {
+    if ((rc = make_output_map_dense(&maps.c, c, g.max_rows, g.N, ldc, 2, 128, 16))) return rc;
+    p.tma_store = 1;
+  }
+  p.c = c;
+  p.counters = static_cast<unsigned int*>(counters);
+  p.M = T; p.N = g.N; p.K = g.K;
+  p.ldc = int(ldc);
+  p.tiles_n = tiles_n;
+  p.tile_rows = 128;
+  p.num_kb = (g.K + Base::BK - 1) / Base::BK;
+  p.dependent = tl_dependent_launch ? 1 : 0;
+  p.c_vec = 1;
+  p.status = dev.status_ptr;
+  auto kernel = wb::mxfp4_skinny_whole_kernel<NP, STAGES, __nv_bfloat16, 4, 128, 2, Maps>;
+  static bool smem_set[kMaxDevices] = {};
+  if ((rc = set_smem(kernel, Cfg::SMEM_BYTES, smem_set))) return rc;
+  const long long items = (long long)maps.max_blocks * tiles_n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(items < dev.sm_count ? items : dev.sm_count), 1, 1);
+  cfg.blockDim = dim3(192, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = tl_dependent_launch ? 1 : 0;
+  WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
+  return WB200_OK;
+}
+
+template <typename Maps>
+int dispatch_skinny_experts(const DeviceInfo& dev, const RoutedGemm& g, int T, void* c, long long ldc, const HiddenOut* hidden, void* counters,
+                            cudaStream_t stream) {
+  if (T <= 16) return launch_skinny_experts<16, 10, Maps>(dev, g, T, c, ldc, hidden, counters, stream);
+  if (T <= 32) return launch_skinny_experts<32, 9, Maps>(dev, g, T, c, ldc, hidden, counters, stream);
+  if (T <= 64) return launch_skinny_experts<64, 8, Maps>(dev, g, T, c, ldc, hidden, counters, stream);
+  return launch_skinny_experts<128, 6, Maps>(dev, g, T, c, ldc, hidden, counters, stream);
 }
 
 template <typename OutT, int EB = 4>
@@ -991,11 +1111,11 @@ int wb200_moe_align_block_size(const void* topk_ids, int ids_are_int64, int num_
   if (ids_are_int64)
     wb::moe_align_block_size_kernel<long long><<<1, 1024, 0, s>>>(static_cast<const long long*>(topk_ids), num_ids, num_experts,
                                                                   block_size, sorted_capacity, sorted_ids, expert_ids,
-                                                                  num_tokens_post_pad, inverse);
+                                                                  num_tokens_post_pad, inverse, 0, nullptr);
   else
     wb::moe_align_block_size_kernel<int><<<1, 1024, 0, s>>>(static_cast<const int*>(topk_ids), num_ids, num_experts, block_size,
                                                             sorted_capacity, sorted_ids, expert_ids, num_tokens_post_pad,
-                                                            inverse);
+                                                            inverse, 0, nullptr);
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
 }
@@ -1068,6 +1188,19 @@ int wb200_silu_and_mul(const void* x1, const void* x2, long long ld1, long long 
   return launch_silu<__nv_bfloat16>(x1, x2, ld1, ld2, rows, n, out, ldo, q, scale_rowmajor, scale_packed, k_atoms, num_rows, s);
 }
 
+extern "C++" {
+template <typename T>
+static int launch_combine(const void* y, long long ldy, const int* row_of, const float* weight, int tokens, int top_k, int cols, void* out,
+                          long long ldo, bool dependent, cudaStream_t s) {
+  auto ok = [&](const void* p, long long ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (ld * sizeof(T)) % 16 == 0; };
+  auto kernel = (cols % 8 == 0 && ok(y, ldy) && ok(out, ldo)) ? wb::moe_combine_kernel<T, true> : wb::moe_combine_kernel<T, false>;
+  const long long threads = (long long)tokens * ((cols + 7) / 8);
+  WB_CUDA(launch_kernel(dependent, kernel, unsigned((threads + 255) / 256), 256, s, static_cast<const T*>(y), ldy, row_of, weight, tokens,
+                        top_k, cols, static_cast<T*>(out), ldo, int(dependent)));
+  return WB200_OK;
+}
+}  // extern "C++"
+
 int wb200_moe_combine(const void* y, long long ldy, int dtype, const int* row_of, const float* weight, int tokens, int top_k,
                       int cols, void* out, long long ldo, void* stream) {
   if (tokens <= 0 || top_k <= 0 || cols <= 0)
@@ -1079,16 +1212,8 @@ int wb200_moe_combine(const void* y, long long ldy, int dtype, const int* row_of
   int rc = get_device(&dev);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const long long threads = (long long)tokens * ((cols + 3) / 4);
-  const unsigned blocks = unsigned((threads + 255) / 256);
-  if (dtype == WB200_F32)
-    wb::moe_combine_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(y), ldy, row_of, weight, tokens, top_k, cols,
-                                                         static_cast<float*>(out), ldo);
-  else
-    wb::moe_combine_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(y), ldy, row_of, weight,
-                                                                 tokens, top_k, cols, static_cast<__nv_bfloat16*>(out), ldo);
-  WB_CUDA(cudaGetLastError());
-  return WB200_OK;
+  return dtype == WB200_F32 ? launch_combine<float>(y, ldy, row_of, weight, tokens, top_k, cols, out, ldo, false, s)
+                            : launch_combine<__nv_bfloat16>(y, ldy, row_of, weight, tokens, top_k, cols, out, ldo, false, s);
 }
 
 int wb200_quantize_mxfp8(const void* x, int x_dtype, long long ldx, int rows, int K, int elem_format, void* q,
@@ -1429,11 +1554,124 @@ int wb200_mxfp4_moe_gemm(int num_experts, int max_rows, const int* expert_ids, c
   DeviceInfo* dev;
   int rc = get_device(&dev);
   if (rc) return rc;
-  if (c_dtype == WB200_F32)
-    return launch_aligned<float>(*dev, num_experts, max_rows, expert_ids, num_rows, N, K, a, a_scale_packed, b_ptrs, b_scale_ptrs,
-                                 c, ldc, static_cast<cudaStream_t>(stream));
-  return launch_aligned<__nv_bfloat16>(*dev, num_experts, max_rows, expert_ids, num_rows, N, K, a, a_scale_packed, b_ptrs,
-                                       b_scale_ptrs, c, ldc, static_cast<cudaStream_t>(stream));
+  const RoutedGemm g{num_experts, max_rows, expert_ids, num_rows, N, K, a, a_scale_packed, b_ptrs, b_scale_ptrs};
+  if (c_dtype == WB200_F32) return launch_aligned<float>(*dev, g, c, ldc, static_cast<cudaStream_t>(stream));
+  return launch_aligned<__nv_bfloat16>(*dev, g, c, ldc, static_cast<cudaStream_t>(stream));
+}
+
+// Buffers of one expert-MLP forward pass inside the caller's workspace.
+struct ExpertMlpPlan {
+  bool decode;
+  int block, cap;  // rows per routing block, rows of the routed matrices (the worst case of the routing)
+  size_t counters, weight, ids, inverse, expert_ids, num_rows, a, a_sf, q, q_sf, y, total;
+};
+static ExpertMlpPlan plan_expert_mlp(int T, int E, int K, int inter, int N, int top_k, bool decode_packing) {
+  ExpertMlpPlan p;
+  const long long n = (long long)T * top_k;
+  // At most 128 tokens: no expert can get more than one 128-row block, and the decode kernel streams the weights once.
+  p.decode = decode_packing && T <= wb::kExpertBlockRows;
+  p.block = p.decode ? wb::kExpertBlockRows : 256;
+  const long long blocks = p.decode ? (n < E ? n : E) : (n + (long long)E * 255 + 255) / 256;
+  p.cap = int(blocks * p.block);
+  size_t at = 0;
+  auto take = [&](size_t bytes) { const size_t here = at; at += (bytes + 255) / 256 * 256; return here; };
+  p.counters = take((wb::kWholeWorkCounter + 1) * 4);
+  p.weight = take(n * 4);
+  p.ids = take(n * 4);
+  p.inverse = take(n * 4);
+  p.expert_ids = take(blocks * 4);
+  p.num_rows = take(4);
+  p.a = take(size_t(p.cap) * (K / 2));
+  p.a_sf = take(wb::sf_packed_bytes(p.cap, K));
+  p.q = take(size_t(p.cap) * (inter / 2));
+  p.q_sf = take(wb::sf_packed_bytes(p.cap, inter));
+  p.y = take(size_t(p.cap) * N * 2);
+  p.total = at;
+  return p;
+}
+
+static int check_expert_mlp(int T, int E, int K, int inter, int N, int top_k) {
+  if (T <= 0 || E <= 0 || E > wb::kMaxGroups || top_k <= 0 || top_k > E)
+    return fail(WB200_ERR_INVALID_ARG, "expert_mlp: %d tokens, %d experts (1..%d), top_k = %d", T, E, wb::kMaxGroups, top_k);
+  if (K <= 0 || K % 32 || inter <= 0 || inter % 128 || N <= 0 || N % 32)
+    return fail(WB200_ERR_UNSUPPORTED, "expert_mlp: K = %d and N = %d must be multiples of 32, inter = %d of 128", K, N, inter);
+  if ((long long)T * top_k + 256ll * E > 0x7fffffffll / 2) return fail(WB200_ERR_UNSUPPORTED, "expert_mlp: too many routed rows");
+  return WB200_OK;
+}
+
+size_t wb200_mxfp4_expert_mlp_workspace_bytes(int T, int E, int K, int inter, int N, int top_k) {
+  if (check_expert_mlp(T, E, K, inter, N, top_k)) return 0;
+  return std::max(plan_expert_mlp(T, E, K, inter, N, top_k, true).total, plan_expert_mlp(T, E, K, inter, N, top_k, false).total);
+}
+
+int wb200_mxfp4_expert_mlp(int T, int E, int K, int inter, int N, int top_k, const void* x, int x_dtype, long long ldx,
+                           const void* logits, int logits_dtype, long long ld_logits, const void* const* w1,
+                           const void* const* w1_scale, const void* const* w1_scale_decode, const void* const* w2,
+                           const void* const* w2_scale, void* out, long long ldo, void* workspace, size_t workspace_bytes,
+                           void* stream) {
+  int rc = check_expert_mlp(T, E, K, inter, N, top_k);
+  if (rc) return rc;
+  if (!x || !logits || !w1 || !w1_scale || !w2 || !w2_scale || !out || !workspace) return fail(WB200_ERR_INVALID_ARG, "expert_mlp: null pointer");
+  if ((x_dtype != WB200_F32 && x_dtype != WB200_BF16) || (logits_dtype != WB200_F32 && logits_dtype != WB200_BF16))
+    return fail(WB200_ERR_INVALID_ARG, "expert_mlp: unknown input dtype");
+  if (ldx < K || ld_logits < E || ldo < N) return fail(WB200_ERR_INVALID_ARG, "expert_mlp: a row pitch is smaller than a row");
+  if ((reinterpret_cast<uintptr_t>(x) & 15) || (ldx * (x_dtype == WB200_F32 ? 4 : 2)) % 16 != 0)
+    return fail(WB200_ERR_ALIGNMENT, "expert_mlp: x rows must be 16-byte aligned");
+  if (reinterpret_cast<uintptr_t>(workspace) & 15) return fail(WB200_ERR_ALIGNMENT, "expert_mlp: the workspace must be 16-byte aligned");
+  const ExpertMlpPlan plan = plan_expert_mlp(T, E, K, inter, N, top_k, w1_scale_decode != nullptr);
+  if (workspace_bytes < plan.total) return fail(WB200_ERR_WORKSPACE, "expert_mlp: workspace of %zu bytes needed (got %zu)", plan.total, workspace_bytes);
+  DeviceInfo* dev;
+  if ((rc = get_device(&dev))) return rc;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  float* weight = reinterpret_cast<float*>(ws + plan.weight);
+  int *ids = reinterpret_cast<int*>(ws + plan.ids), *inverse = reinterpret_cast<int*>(ws + plan.inverse);
+  int *expert_ids = reinterpret_cast<int*>(ws + plan.expert_ids), *num_rows = reinterpret_cast<int*>(ws + plan.num_rows);
+  unsigned int* counters = reinterpret_cast<unsigned int*>(ws + plan.counters);
+  const int n = T * top_k;
+  // Every launch after the first is the programmatic dependent of the one before it. The first one is an ordinary launch,
+  // so what the kernels before this call wrote (x, the logits) is complete for all of them.
+  const unsigned topk_blocks = unsigned((T + 127) / 128);
+  if (logits_dtype == WB200_F32)
+    WB_CUDA(launch_kernel(false, wb::moe_topk_kernel<float>, topk_blocks, 128, s, static_cast<const float*>(logits), ld_logits, T, E, top_k, weight, ids));
+  else
+    WB_CUDA(launch_kernel(false, wb::moe_topk_kernel<__nv_bfloat16>, topk_blocks, 128, s, static_cast<const __nv_bfloat16*>(logits), ld_logits, T, E,
+                          top_k, weight, ids));
+  WB_CUDA(launch_kernel(true, wb::moe_align_block_size_kernel<int>, 1, 1024, s, ids, n, E, plan.block, 0, static_cast<int*>(nullptr), expert_ids,
+                        num_rows, inverse, 1, counters + wb::kWholeWorkCounter));
+  const int k_atoms = wb::sf_k_atoms(K);
+  const unsigned q_blocks = unsigned(((long long)T * ((k_atoms + 7) / 8) + 7) / 8);
+  // Tokens are quantised once and written straight to their sorted rows, scales in the packed layout. Rows that pad an
+  // expert to whole blocks are never written: an output row depends on its own input row only, and the combination
+  // reads routed rows only.
+  if (x_dtype == WB200_F32)
+    WB_CUDA(launch_kernel(true, wb::quantize_scatter_mxfp4_kernel<float>, q_blocks, 256, s, static_cast<const float*>(x), ldx, T, K, top_k, inverse,
+                          ws + plan.a, 1, static_cast<uint8_t*>(nullptr), ws + plan.a_sf, k_atoms, 1));
+  else
+    WB_CUDA(launch_kernel(true, wb::quantize_scatter_mxfp4_kernel<__nv_bfloat16>, q_blocks, 256, s, static_cast<const __nv_bfloat16*>(x), ldx, T, K,
+                          top_k, inverse, ws + plan.a, 1, static_cast<uint8_t*>(nullptr), ws + plan.a_sf, k_atoms, 1));
+  struct DependentScope {  // restores the previous value on every return path
+    bool saved = tl_dependent_launch;
+    DependentScope() { tl_dependent_launch = true; }
+    ~DependentScope() { tl_dependent_launch = saved; }
+  } dependent_scope;
+  const RoutedGemm up{E, plan.cap, expert_ids, num_rows, 2 * inter, K, ws + plan.a, ws + plan.a_sf, w1, plan.decode ? w1_scale_decode : w1_scale};
+  const RoutedGemm down{E, plan.cap, expert_ids, num_rows, N, inter, ws + plan.q, ws + plan.q_sf, w2, w2_scale};
+  const HiddenOut hidden{inter, ws + plan.q, ws + plan.q_sf};
+  void* y = ws + plan.y;
+  if (plan.decode) {
+    if (E <= 8) {
+      if ((rc = dispatch_skinny_experts<wb::SkinnyExpertMaps<8, true>>(*dev, up, T, nullptr, 0, &hidden, counters, s))) return rc;
+      if ((rc = dispatch_skinny_experts<wb::SkinnyExpertMaps<8, false>>(*dev, down, T, y, N, nullptr, counters, s))) return rc;
+    } else {
+      if ((rc = dispatch_skinny_experts<wb::SkinnyExpertMaps<wb::kMaxGroups, true>>(*dev, up, T, nullptr, 0, &hidden, counters, s))) return rc;
+      if ((rc = dispatch_skinny_experts<wb::SkinnyExpertMaps<wb::kMaxGroups, false>>(*dev, down, T, y, N, nullptr, counters, s))) return rc;
+    }
+  } else {
+    if ((rc = launch_aligned_silu(*dev, up, hidden, s))) return rc;
+    if ((rc = launch_aligned<__nv_bfloat16>(*dev, down, y, N, s))) return rc;
+  }
+  return launch_combine<__nv_bfloat16>(y, N, inverse, weight, T, top_k, N, out, ldo, true, s);
 }
 
 int wb200_mxfp4_gemm_scatter_rows(int num_parts, const int* row_offsets, int N, int K, const void* a,

@@ -24,6 +24,7 @@
 //     of both CTAs complete on the leader CTA's barrier, and the leader issues the MMAs.
 #pragma once
 #include "ptx.cuh"
+#include "quantize.cuh"
 #include <cuda_bf16.h>
 
 namespace wb {
@@ -103,17 +104,18 @@ struct GemmParams {
 };
 
 // The tensor maps of one launch, passed by value as a kernel parameter. Index: 0 = a, 1 = b,
-// 2 = packed a scales, 3 = packed b scales, 4 = c.
+// 2 = packed a scales, 3 = packed b scales, 4 = c. map(g, i): map i of group g.
 struct PlainMaps {
-  static constexpr bool kGrouped = false;
+  static constexpr bool kGrouped = false, kAligned = false, kSilu = false;
   CUtensorMap m[5];
+  __device__ __forceinline__ const CUtensorMap* map(int, int i) const { return &m[i]; }
 };
 // Grouped (per-expert) launch: five maps per group, each describing only that group's rows, so that
 // TMA zero-fills loads and clips stores at the group's end; tile_start is the running count of
 // tiles over the groups, rows the row count of each group.
 constexpr int kMaxGroups = 32;
 struct GroupedMaps {
-  static constexpr bool kGrouped = true;
+  static constexpr bool kGrouped = true, kAligned = false, kSilu = false;
   CUtensorMap m[kMaxGroups * 5];
   void* c_base[kMaxGroups];  // first output row of each group, for the stores that do not go through its tensor map
   int tile_start[kMaxGroups + 1];
@@ -124,17 +126,71 @@ struct GroupedMaps {
   // groups differ in WHERE their output goes (another GPU): the remote stores then spread over the whole launch.
   int interleave;
   int tiles_max;
-  // aligned != 0: the rows of all groups sit in ONE matrix, every group padded to whole tile_rows-row tiles, and
-  // which group a row tile belongs to is read from device memory (expert_ids[M tile], as written by
-  // moe_align_block_size with block_size = tile_rows); row tiles at or past *num_rows are skipped. Slots 0, 2, 4
-  // of every group's maps describe that one matrix; slots 1, 3 are the group's own weights. The host needs
-  // no knowledge of the routing: no read-back, and the launch can be captured in a CUDA graph.
-  int aligned;
+  __device__ __forceinline__ const CUtensorMap* map(int g, int i) const { return &m[g * 5 + i]; }
+};
+// Routed (mixture-of-experts) launch: the rows of all experts sit in ONE matrix, every expert padded to whole
+// tile_rows-row tiles, and which expert a row tile belongs to is read from device memory (expert_ids[M tile], as
+// written by moe_align_block_size with block_size = tile_rows); only the row tiles below *num_rows are walked. The
+// host needs no knowledge of the routing: no read-back, and the launch can be captured in a CUDA graph. Three maps
+// describe the common matrices (a, packed a scales, c) and two each expert's weights, in a table of G experts: the
+// parameter block, which the host copies on every launch, is 2.5 KB for up to 8 experts and 8.7 KB for up to 32.
+template <int G>
+struct AlignedMaps {
+  static constexpr bool kGrouped = true, kAligned = true, kSilu = false;
+  CUtensorMap rows_map[3];   // a, packed a scales, c
+  CUtensorMap w_map[2 * G];  // b, packed b scales of every expert
+  void* c_base;
+  int num_groups;
   int tile_rows;
   int tiles_m_cap;
   const int* expert_ids;
   const int* num_rows;
+  __device__ __forceinline__ const CUtensorMap* map(int g, int i) const {
+    return (i & 1) ? &w_map[g * 2 + (i >> 1)] : &rows_map[i >> 1];
+  }
 };
+// The gate|up projection of an expert MLP with silu(gate) * up and its quantisation in the epilogue (aligned layout).
+// b holds `inter` gate rows and then `inter` up rows per expert; tile nt takes gate rows nt * 128 .. + 127 (loaded by the
+// first CTA of the pair) and up rows inter + nt * 128 .. (the second CTA), so that accumulator columns c and 128 + c are
+// the two halves of hidden column nt * 128 + c and no weight has to be laid out anew. One thread holds the 32 columns of
+// a scale block of its row: the block maximum needs no shuffle, the codes of a block are one 16-byte store and the four
+// blocks of a tile are one word of a packed scale atom. inter % 128 == 0 (a scale atom and both row blocks then belong
+// to one tile).
+// Instead of [rows, 2 inter] bf16 written here and read back by a second kernel, [rows, inter / 2] bytes leave.
+template <int G>
+struct SiluMaps : AlignedMaps<G> {
+  static constexpr bool kSilu = true;
+  uint8_t* q;             // [rows, inter / 2] codes
+  uint8_t* scale_packed;  // packed scales of [rows, inter]
+  int inter;
+  int k_atoms;            // atoms per 128-row block of scale_packed
+};
+
+// Codes and scale byte of silu(g) * u for one block of 32 columns held by one thread (accumulator bits). The projections
+// are rounded to bf16 first, the type they have where they are written to memory (`wb200_mxfp4_moe_gemm` followed by
+// `wb200_silu_and_mul`): the codes are those of that form.
+__device__ __forceinline__ uint32_t silu_quantize_block(const uint32_t (&g)[32], const uint32_t (&u)[32], uint4& codes) {
+  float y[32];
+  uint32_t m = 0;
+#pragma unroll
+  for (int j = 0; j < 32; j += 2) {
+    silu_mul_bf16x2(pack_bf16x2(__uint_as_float(g[j]), __uint_as_float(g[j + 1])), pack_bf16x2(__uint_as_float(u[j]), __uint_as_float(u[j + 1])),
+                    y[j], y[j + 1]);
+    m = max(m, max(__float_as_uint(y[j]) & 0x7fffffffu, __float_as_uint(y[j + 1]) & 0x7fffffffu));
+  }
+  const int sb = mxfp4_scale_byte(m);
+  const float f = mxfp4_code_factor(sb);
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    w[i] = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[i] |= e2m1x2_code(y[8 * i + 2 * j] * f, y[8 * i + 2 * j + 1] * f) << (8 * j);
+    if (sb == 255) w[i] = 0u;  // a NaN or an infinity in the block
+  }
+  codes = make_uint4(w[0], w[1], w[2], w[3]);
+  return uint32_t(sb);
+}
 
 // Tile order: groups of `group_n` N tiles, each group swept down M with N fastest.
 __device__ __forceinline__ void raster_tile(int t, int tiles_m, int tiles_n, int group_n, int& mt,
@@ -148,32 +204,43 @@ __device__ __forceinline__ void raster_tile(int t, int tiles_m, int tiles_n, int
   nt = n0 + (r - mt * gw);
 }
 
-// Tile id -> (group, M tile, N tile, rows of the group) and the group's first tensor map; nullptr for an
-// id that names no tile (interleaved walk over groups of unequal size).
+// Number of tile ids of this launch. Aligned form: from what the routing kernels wrote.
 template <typename Maps>
-__device__ __forceinline__ const CUtensorMap* decode_tile(const Maps& maps, const GemmParams& p, int t, int& mt, int& nt,
-                                                          int& rows, void** c_base = nullptr) {
+__device__ __forceinline__ int count_tiles(const Maps& maps, const GemmParams& p, int& tiles_m) {
+  tiles_m = p.tiles_m;
+  if constexpr (Maps::kAligned) {
+    tiles_m = min(maps.tiles_m_cap, __ldcg(maps.num_rows) / maps.tile_rows);
+    return tiles_m * p.tiles_n;
+  } else if constexpr (Maps::kGrouped) {
+    return maps.interleave ? maps.num_groups * maps.tiles_max : maps.tile_start[maps.num_groups];
+  } else {
+    return p.tiles_m * p.tiles_n;
+  }
+}
+
+// Tile id -> M tile, N tile, rows of its group; returns the group, or -1 for an id that names no tile (interleaved walk
+// over groups of unequal size). tiles_m: from count_tiles.
+template <typename Maps>
+__device__ __forceinline__ int decode_tile(const Maps& maps, const GemmParams& p, int t, int tiles_m, int& mt, int& nt,
+                                           int& rows, void** c_base = nullptr) {
   if constexpr (!Maps::kGrouped) {
     raster_tile(t, p.tiles_m, p.tiles_n, p.group_n, mt, nt);
     rows = p.M;
     if (c_base) *c_base = p.c;
-    return &maps.m[0];
+    return 0;
+  } else if constexpr (Maps::kAligned) {
+    raster_tile(t, tiles_m, p.tiles_n, p.group_n, mt, nt);
+    const int e = __ldcg(maps.expert_ids + mt);
+    if (e < 0 || e >= maps.num_groups) return -1;  // never written by a correct router; do not index out of the table
+    rows = tiles_m * maps.tile_rows;
+    if (c_base) *c_base = maps.c_base;
+    return e;
   } else {
-    if (maps.aligned) {
-      raster_tile(t, maps.tiles_m_cap, p.tiles_n, p.group_n, mt, nt);
-      const int total = __ldg(maps.num_rows);
-      if (mt * maps.tile_rows >= total) return nullptr;
-      int e = __ldg(maps.expert_ids + mt);
-      if (e < 0 || e >= maps.num_groups) return nullptr;  // never written by a correct router; do not index out of the table
-      rows = total;
-      if (c_base) *c_base = maps.c_base[0];
-      return &maps.m[e * 5];
-    }
     int g = 0, local;
     if (maps.interleave) {
       g = t % maps.num_groups;
       local = t / maps.num_groups;
-      if (local >= maps.tile_start[g + 1] - maps.tile_start[g]) return nullptr;
+      if (local >= maps.tile_start[g + 1] - maps.tile_start[g]) return -1;
     } else {
       while (g + 1 < maps.num_groups && t >= maps.tile_start[g + 1]) ++g;
       local = t - maps.tile_start[g];
@@ -181,7 +248,7 @@ __device__ __forceinline__ const CUtensorMap* decode_tile(const Maps& maps, cons
     raster_tile(local, (maps.tile_start[g + 1] - maps.tile_start[g]) / p.tiles_n, p.tiles_n, p.group_n, mt, nt);
     rows = maps.rows[g];
     if (c_base) *c_base = maps.c_base[g];
-    return &maps.m[g * 5];
+    return g;
   }
 }
 
@@ -326,7 +393,7 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
   }
   if (warp == 0 && lane == 0) {
 #pragma unroll
-    for (int i = 0; i < 5; ++i) prefetch_tensormap(&maps.m[i]);
+    for (int i = 0; i < (Maps::kSilu ? 4 : 5); ++i) prefetch_tensormap(maps.map(0, i));
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -337,10 +404,10 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  int num_tiles = p.tiles_m * p.tiles_n;
-  if constexpr (Maps::kGrouped)
-    num_tiles = maps.aligned ? maps.tiles_m_cap * p.tiles_n
-                             : (maps.interleave ? maps.num_groups * maps.tiles_max : maps.tile_start[maps.num_groups]);
+  // The routing arrays of an aligned launch are written by the kernels before this one: every role waits for them.
+  if constexpr (Maps::kAligned) pdl_wait();
+  int tiles_m;
+  const int num_tiles = count_tiles(maps, p, tiles_m);
   const int first_tile = (CG == 2) ? (blockIdx.x >> 1) : blockIdx.x;
   const int tile_step = (CG == 2) ? (gridDim.x >> 1) : gridDim.x;
   const int num_kb = (p.K + Cfg::BK - 1) / Cfg::BK;
@@ -355,10 +422,12 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
     pdl_wait();  // the packed activation scales may be written by the kernel launched just before this one
     for (int t = first_tile; t < num_tiles; t += tile_step) {
       int mt, nt, rows;
-      const CUtensorMap* tm = decode_tile(maps, p, t, mt, nt, rows);
-      if (Maps::kGrouped && tm == nullptr) continue;
+      const int group = decode_tile(maps, p, t, tiles_m, mt, nt, rows);
+      if (Maps::kGrouped && group < 0) continue;
+      const CUtensorMap *tm_a = maps.map(group, 0), *tm_b = maps.map(group, 1), *tm_sfa = maps.map(group, 2), *tm_sfb = maps.map(group, 3);
       const int a_row = (mt * CG + int(rank)) * Cfg::BM;
-      const int b_row = nt * BN + int(rank) * Cfg::B_ROWS;
+      int b_row = nt * BN + int(rank) * Cfg::B_ROWS;
+      if constexpr (Maps::kSilu) b_row = nt * Cfg::B_ROWS + int(rank) * maps.inter;
       const int sfa_rb = mt * CG + int(rank);
       const int sfb_rb = Cfg::TILED_SFB ? nt * Cfg::SFB_BLOCKS : (nt * BN) / 128;
       for (int kb = 0; kb < num_kb; ++kb) {
@@ -382,11 +451,16 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
         if (elect_one()) {
           // 4-bit weights expanded by the copy engine (EB == 8 kernels only): the transaction count is the packed size
           if (leader) mbar_expect_tx(full_bar(stage), (Cfg::LOAD_BYTES - ((EB == 8 && (p.elem_format & 0x10)) ? Cfg::B_BYTES / 2 : 0)) * CG);
-          tma_load_2d<CG>(sA, tm + 0, kb * 128, a_row, fb);
-          tma_load_2d<CG>(sB, tm + 1, kb * 128, b_row, fb);
+          tma_load_2d<CG>(sA, tm_a, kb * 128, a_row, fb);
+          tma_load_2d<CG>(sB, tm_b, kb * 128, b_row, fb);
           // scale factors: SF_ATOMS atoms of 512 bytes (128 32-bit words) per 128-row block and stage
-          tma_load_2d<CG>(sSFA, tm + 2, kb * (Cfg::SF_ATOMS * 128), sfa_rb, fb);
-          tma_load_2d<CG>(sSFB, tm + 3, kb * (Cfg::SF_ATOMS * 128), sfb_rb, fb);
+          tma_load_2d<CG>(sSFA, tm_sfa, kb * (Cfg::SF_ATOMS * 128), sfa_rb, fb);
+          if constexpr (Maps::kSilu) {  // the gate rows' block, then the up rows'
+            tma_load_2d<CG>(sSFB, tm_sfb, kb * (Cfg::SF_ATOMS * 128), nt, fb);
+            tma_load_2d<CG>(sSFB + Cfg::SF_ATOMS * 512, tm_sfb, kb * (Cfg::SF_ATOMS * 128), maps.inter / 128 + nt, fb);
+          } else {
+            tma_load_2d<CG>(sSFB, tm_sfb, kb * (Cfg::SF_ATOMS * 128), sfb_rb, fb);
+          }
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -406,7 +480,7 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
         uint32_t sfb_group = 0;
         if constexpr ((BN % 128 != 0 && !Cfg::TILED_SFB) || Maps::kGrouped) {
           int mt, nt, rows;
-          if (decode_tile(maps, p, t, mt, nt, rows) == nullptr) continue;
+          if (decode_tile(maps, p, t, tiles_m, mt, nt, rows) < 0) continue;
           sfb_group = uint32_t((nt * BN) % 128) / 32u;
         }
         const int as = it & 1;
@@ -493,8 +567,8 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
     for (int t = first_tile; t < num_tiles; t += tile_step) {
       int mt, nt, rows;
       void* c_group = nullptr;
-      const CUtensorMap* tm = decode_tile(maps, p, t, mt, nt, rows, &c_group);
-      if (Maps::kGrouped && tm == nullptr) continue;
+      const int group = decode_tile(maps, p, t, tiles_m, mt, nt, rows, &c_group);
+      if (Maps::kGrouped && group < 0) continue;
       const int as = it & 1;
       mbar_wait(acc_full_bar(as), uint32_t(it >> 1) & 1u, ctx, WB_DEV_TIMEOUT_EPILOGUE);
       tc_fence_after_sync();
@@ -516,6 +590,44 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
       ++it;
       continue;
 #endif
+      if constexpr (Maps::kSilu) {
+        static_assert(CG == 2 && BN == 256 && EB == 4 && Cfg::OVERLAP_CHUNKS == 2, "gate and up share a 256-column tile");
+        // Columns shared with the other accumulator first: up chunks 2, 3 of accumulator 0, gate chunks 0, 1 of
+        // accumulator 1. They wait in registers for their partners.
+        uint32_t h0[32], h1[32];
+        tmem_ld_32x32(t_acc + (as ? 0 : 6) * 32, h0);
+        tmem_ld_32x32(t_acc + (as ? 1 : 7) * 32, h1);
+        tmem_ld_wait();
+        release();
+        uint32_t sf_word = 0;
+        uint8_t* q_row = maps.q + size_t(row) * (maps.inter / 2) + nt * 64;
+#pragma unroll 1
+        for (int ci = 0; ci < 4; ++ci) {
+          const int chunk = as ? ci : (ci + 2) & 3;  // 32 hidden columns nt * 128 + chunk * 32 ..
+          uint32_t x[32];
+          tmem_ld_32x32(t_acc + (as ? 4 + chunk : chunk) * 32, x);
+          if (ci == 1) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) h0[j] = h1[j];
+          } else if (ci > 1) {
+            tmem_ld_32x32(t_acc + (as ? chunk : 4 + chunk) * 32, h0);
+          }
+          tmem_ld_wait();
+          uint4 codes;
+          const uint32_t sb = as ? silu_quantize_block(h0, x, codes) : silu_quantize_block(x, h0, codes);
+          sf_word |= sb << (8 * chunk);
+          if (row < rows && WB_CHECK(row >= 0 && row < p.M && nt < p.tiles_n, kCheckOutputIndex, (long long)row << 32 | unsigned(nt)))
+            *reinterpret_cast<uint4*>(q_row + chunk * 16) = codes;
+        }
+        if (row < rows) {
+          *packed_scale_word(maps.scale_packed, maps.k_atoms, row, nt) = sf_word;
+          // an odd atom count is padded to whole pipeline stages
+          if (nt == p.tiles_n - 1 && nt + 1 < maps.k_atoms)
+            *packed_scale_word(maps.scale_packed, maps.k_atoms, row, nt + 1) = 0x01010101u * WB_SF_PAD;
+        }
+        ++it;
+        continue;
+      }
       constexpr int NCHUNK = BN / 32;
       // Overlapping accumulators: the MMA warp cannot start the next tile before the shared columns are read. Both
       // shared chunks are therefore fetched at once, ahead of any staging, and the accumulator is handed back as soon
@@ -599,7 +711,7 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
               // altogether still commits an (empty) group, because the buffer hand-over above counts
               // groups: one group per store, whether or not it wrote anything.
               const int scol = col - (PER_STORE - 1) * 32;
-              if (row0 < rows && scol < p.N) tma_store_2d_hint(tm + 4, buf, scol, row0, store_policy);
+              if (row0 < rows && scol < p.N) tma_store_2d_hint(maps.map(group, 4), buf, scol, row0, store_policy);
               bulk_commit_group();
             }
             ++store_count;  // the buffers alternate store by store, across tiles too

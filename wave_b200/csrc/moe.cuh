@@ -21,26 +21,45 @@ namespace wb {
 
 constexpr int kMoeMaxExperts = 256;
 
+template <typename T>
+__device__ __forceinline__ float to_f32(T v);
+template <>
+__device__ __forceinline__ float to_f32<float>(float v) { return v; }
+template <>
+__device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+template <typename T>
+__device__ __forceinline__ T from_f32(float v);
+template <>
+__device__ __forceinline__ float from_f32<float>(float v) { return v; }
+template <>
+__device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+
 // One CTA of 1024 threads. ids: [n] expert of every routed (token, slot) pair in flat order.
 // sorted_ids [sorted_cap]: flat indices grouped by expert, ascending inside an expert, each expert's
 // run padded with the value n to a multiple of block_size; the rest of the array is n as well.
 // expert_ids [total / block_size]: expert of every block. inverse [n] (may be null): position of
-// flat index i in sorted_ids. Ids outside [0, E) are skipped.
+// flat index i in sorted_ids. Ids outside [0, E) are skipped. sorted_ids may be null (only the inverse is wanted).
+// dependent: launched as the programmatic dependent of the kernel that writes ids. zero_word (may be null): a word to clear
+// for the kernels that follow (the decode GEMM's tile counter).
 template <typename IdT>
 __global__ void __launch_bounds__(1024)
 moe_align_block_size_kernel(const IdT* __restrict__ ids, int n, int E, int block_size, int sorted_cap,
                             int* __restrict__ sorted_ids, int* __restrict__ expert_ids,
-                            int* __restrict__ num_tokens_post_pad, int* __restrict__ inverse) {
+                            int* __restrict__ num_tokens_post_pad, int* __restrict__ inverse, int dependent, unsigned int* zero_word) {
   __shared__ int counts[kMoeMaxExperts];
   __shared__ int running[kMoeMaxExperts];
   __shared__ int warp_counts[32][kMoeMaxExperts];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < sorted_cap; i += blockDim.x) sorted_ids[i] = n;
+  pdl_launch_dependents();
+  if (sorted_ids)
+    for (int i = tid; i < sorted_cap; i += blockDim.x) sorted_ids[i] = n;
   for (int e = tid; e < E; e += blockDim.x) counts[e] = 0;
   for (int i = tid; i < 32 * kMoeMaxExperts; i += blockDim.x) (&warp_counts[0][0])[i] = 0;
+  if (tid == 0 && zero_word) *zero_word = 0u;
+  if (dependent) pdl_wait();
   __syncthreads();
   for (int i = tid; i < n; i += blockDim.x) {
-    const long long e = (long long)ids[i];
+    const long long e = (long long)__ldcg(ids + i);
     if (e >= 0 && e < E) atomicAdd(&counts[int(e)], 1);
   }
   __syncthreads();
@@ -61,7 +80,7 @@ moe_align_block_size_kernel(const IdT* __restrict__ ids, int n, int E, int block
   // elements of that expert in earlier chunks + in lower warps of this chunk + in lower lanes.
   for (int base = 0; base < n; base += blockDim.x) {
     const int i = base + tid;
-    long long e64 = (i < n) ? (long long)ids[i] : -1;
+    long long e64 = (i < n) ? (long long)__ldcg(ids + i) : -1;
     const int e = (e64 >= 0 && e64 < E) ? int(e64) : -1;
     const unsigned same = __match_any_sync(0xffffffffu, e);
     const int rank = __popc(same & ((1u << lane) - 1u));
@@ -70,7 +89,7 @@ moe_align_block_size_kernel(const IdT* __restrict__ ids, int n, int E, int block
     if (e >= 0) {
       int at = running[e] + rank;
       for (int w = 0; w < warp; ++w) at += warp_counts[w][e];
-      sorted_ids[at] = i;
+      if (sorted_ids) sorted_ids[at] = i;
       if (inverse) inverse[i] = at;
     } else if (i < n && inverse) {
       inverse[i] = -1;
@@ -85,6 +104,48 @@ moe_align_block_size_kernel(const IdT* __restrict__ ids, int n, int E, int block
       running[x] += s;
     }
     __syncthreads();
+  }
+}
+
+// Order-preserving integer of an f32, every NaN above the infinity.
+__device__ __forceinline__ uint32_t order_key(float v) {
+  if (v != v) return 0xffffffffu;
+  const uint32_t b = __float_as_uint(v);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+
+// Router: softmax over the experts in f32 and the top_k largest, one thread per token. weight / ids [tokens, top_k] in
+// descending order of the logit, the lower expert first among equals. Latency-bound (a few hundred bytes per token):
+// one launch where softmax and top-k are three library kernels.
+template <typename T>
+__global__ void __launch_bounds__(128)
+moe_topk_kernel(const T* __restrict__ logits, long long ld, int tokens, int E, int top_k, float* __restrict__ weight,
+                int* __restrict__ ids) {
+  pdl_launch_dependents();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= tokens) return;
+  const T* row = logits + (long long)t * ld;
+  float mx = -INFINITY;
+  for (int e = 0; e < E; ++e) mx = fmaxf(mx, to_f32<T>(row[e]));
+  float sum = 0.f;
+  for (int e = 0; e < E; ++e) sum += expf(to_f32<T>(row[e]) - mx);
+  uint32_t last_key = 0xffffffffu;
+  int last = -1;
+  for (int j = 0; j < top_k; ++j) {
+    // the next one in (key descending, index ascending) order after (last_key, last)
+    uint32_t best_key = 0;
+    int best = -1;
+    float best_v = 0.f;
+    for (int e = 0; e < E; ++e) {
+      const float v = to_f32<T>(row[e]);
+      const uint32_t key = order_key(v);
+      const bool after = key < last_key || (key == last_key && e > last);
+      if (after && (best < 0 || key > best_key)) { best = e; best_key = key; best_v = v; }
+    }
+    weight[(long long)t * top_k + j] = expf(best_v - mx) / sum;
+    ids[(long long)t * top_k + j] = best;
+    last_key = best_key;
+    last = best;
   }
 }
 
@@ -110,19 +171,12 @@ moe_gather_rows_kernel(const uint8_t* __restrict__ src, long long src_pitch, int
   }
 }
 
-template <typename T>
-__device__ __forceinline__ float to_f32(T v);
-template <>
-__device__ __forceinline__ float to_f32<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <typename T>
-__device__ __forceinline__ T from_f32(float v);
-template <>
-__device__ __forceinline__ float from_f32<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-
+// 8 consecutive values from 16-byte aligned memory that an overlapping earlier kernel wrote (through L2).
+__device__ __forceinline__ void load8_cg(const float* p, float (&v)[8]) {
+  const float4 a = __ldcg(reinterpret_cast<const float4*>(p)), b = __ldcg(reinterpret_cast<const float4*>(p) + 1);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void load8_cg(const __nv_bfloat16* p, float (&v)[8]) { raw8_values(__ldcg(reinterpret_cast<const uint4*>(p)), v); }
 __device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
   reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
   reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
@@ -180,7 +234,7 @@ silu_and_mul_kernel(const T* __restrict__ x1, const T* __restrict__ x2, long lon
     const int c0 = kb * 32 + sub * 8;
     float y[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) y[j] = __fdividef(g[i][j], 1.0f + __expf(-g[i][j])) * u[i][j];  // ~1e-6 relative
+    for (int j = 0; j < 8; ++j) y[j] = silu_mul(g[i][j], u[i][j]);
     if (out && active[i]) {
       T* po = out + (long long)r * ldo + c0;
       if (full[i]) {
@@ -196,29 +250,44 @@ silu_and_mul_kernel(const T* __restrict__ x1, const T* __restrict__ x2, long lon
 }
 
 // out[t, c] = sum_j weight[t * top_k + j] * y[row_of[t * top_k + j], c], accumulated in f32 in slot
-// order; pairs with row_of < 0 are skipped. One thread per (token, 4 columns).
-template <typename T>
+// order; pairs with row_of < 0 are skipped. One thread per (token, 8 columns); VEC: cols % 8 == 0 and 16-byte aligned
+// rows of both matrices, so that a thread's columns move as 16-byte accesses.
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const T* __restrict__ y, long long ldy, const int* __restrict__ row_of,
                    const float* __restrict__ weight, int tokens, int top_k, int cols, T* __restrict__ out,
-                   long long ldo) {
+                   long long ldo, int dependent) {
+  pdl_launch_dependents();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int cvec = (cols + 3) >> 2;
+  const int cvec = (cols + 7) >> 3;
+  if (dependent) pdl_wait();
   if (idx >= (long long)tokens * cvec) return;
   const int t = int(idx / cvec);
-  const int c0 = int(idx - (long long)t * cvec) * 4;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  const int c0 = int(idx - (long long)t * cvec) * 8;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int j = 0; j < top_k; ++j) {
-    const int row = row_of[t * top_k + j];
+    const int row = __ldcg(row_of + (long long)t * top_k + j);
     if (row < 0) continue;
-    const float w = weight[t * top_k + j];
+    const float w = __ldcg(weight + (long long)t * top_k + j);
+    const T* src = y + (long long)row * ldy + c0;
+    float v[8];
+    if constexpr (VEC) {
+      load8_cg(src, v);
+    } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (c0 + i < cols) acc[i] += w * to_f32<T>(y[(long long)row * ldy + c0 + i]);
+      for (int i = 0; i < 8; ++i) v[i] = (c0 + i < cols) ? to_f32<T>(src[i]) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] += w * v[i];
   }
+  T* dst = out + (long long)t * ldo + c0;
+  if constexpr (VEC) {
+    store8(dst, acc);
+  } else {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (c0 + i < cols) out[(long long)t * ldo + c0 + i] = from_f32<T>(acc[i]);
+    for (int i = 0; i < 8; ++i)
+      if (c0 + i < cols) dst[i] = from_f32<T>(acc[i]);
+  }
 }
 
 // out[i] = slots[0][i] + slots[1][i] + ... in slot order (f32), rounded once to the output type: the

@@ -38,6 +38,14 @@ __device__ __forceinline__ uint32_t e2m1x2_code(float lo, float hi) {
   return uint32_t(r);
 }
 
+// silu(g) * u = g / (1 + exp(-g)) * u in f32 with the fast exponential and division (~1e-6 relative).
+__device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
+// The same for two packed bf16 pairs.
+__device__ __forceinline__ void silu_mul_bf16x2(uint32_t g, uint32_t u, float& lo, float& hi) {
+  lo = silu_mul(__uint_as_float(g << 16), __uint_as_float(u << 16));
+  hi = silu_mul(__uint_as_float(g & 0xffff0000u), __uint_as_float(u & 0xffff0000u));
+}
+
 // Bit pattern of the largest |v| over the 32 values held by a group of 32 / VPL neighbouring lanes. For
 // non-negative floats the unsigned order of the bit patterns is the numeric order, with the infinity above
 // every finite value and every NaN above the infinity: an integer maximum keeps a NaN that fmaxf would drop.
@@ -322,7 +330,7 @@ quantize_scatter_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows
   if (dependent) pdl_wait();  // the destination rows are the previous kernel's; the outputs may still be read before it
   const int g = lane >> 2, sub = lane & 3;
   for (int j = 0; j < copies; ++j) {
-    const int dst = dst_rows[r * copies + j];
+    const int dst = __ldcg(dst_rows + r * copies + j);
     if (dst < 0) continue;
     if (kb0 + lane < kblocks) {
       uint8_t* d = q + (long long)dst * (K / 2) + (kb0 + lane) * 16;

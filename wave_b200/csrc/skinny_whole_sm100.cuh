@@ -20,6 +20,7 @@
 // memory (mbarrier-guarded), since only it talks to the counter.
 #pragma once
 #include "ptx.cuh"
+#include "quantize.cuh"
 #include "skinny_sm100.cuh"
 #include <cuda_bf16.h>
 
@@ -61,11 +62,41 @@ struct SkinnyWholeParams {
   int* status;
 };
 
-template <int NP, int STAGES, typename OutT, int EB = 4, int WR = 128, int SBUFS = 2>
+// The tensor maps of a launch over one weight.
+struct SkinnyMaps {
+  static constexpr bool kExperts = false, kSilu = false;
+  CUtensorMap w, sfw;  // weights and their packed scales
+  CUtensorMap x, sfx;  // activations and their packed scales
+  CUtensorMap c;
+};
+// A decode step of a mixture-of-experts layer (at most 128 tokens, so at most 128 rows per expert): the tiles of every
+// expert that received tokens, in one launch. x holds one block of 128 rows per such expert (moe_align_block_size with
+// block_size = 128), expert_ids the expert of each block and *num_rows 128 times their number, both in device memory; an
+// item of the dispenser is (block, weight tile). The 256-row tile kernel would multiply 256 rows for the few that are
+// real, in whole waves of 74 CTA pairs; here the weights are streamed once at the decode kernel's rate.
+// Silu form: w holds `inter` gate rows and then `inter` up rows; a tile is 64 gate rows (lanes 0 .. 63) and the 64 up rows
+// of the same hidden columns (lanes 64 .. 127), its scales packed in that row order, and what leaves is silu(gate) * up
+// quantised: codes q [rows, inter / 2] and packed scales. inter % 64 == 0.
+template <int G, bool SILU>
+struct SkinnyExpertMaps {
+  static constexpr bool kExperts = true, kSilu = SILU;
+  CUtensorMap w[G], sfw[G];
+  CUtensorMap x, sfx;
+  CUtensorMap c;
+  int num_groups;
+  int max_blocks;
+  const int* expert_ids;
+  const int* num_rows;
+  int inter;    // silu form
+  int k_atoms;  // atoms per 128-row block of scale_packed
+  uint8_t* q;
+  uint8_t* scale_packed;
+};
+constexpr int kExpertBlockRows = 128;
+
+template <int NP, int STAGES, typename OutT, int EB = 4, int WR = 128, int SBUFS = 2, typename Maps = SkinnyMaps>
 __global__ void __launch_bounds__(192, 1)
-mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
-                          const __grid_constant__ CUtensorMap tmSFW, const __grid_constant__ CUtensorMap tmSFX,
-                          const __grid_constant__ CUtensorMap tmC, const SkinnyWholeParams p) {
+mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholeParams p) {
   using Base = SkinnyCfg<NP, STAGES, EB, WR>;
   using Cfg = SkinnyWholeCfg<NP, STAGES, EB, WR, SBUFS>;
   constexpr int IQ = kWholeItemQueue;
@@ -78,9 +109,11 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
 #ifdef WB200_TRACE
   if (threadIdx.x == 0) WB_TRACE_SET(0, trace_now());  // timeline marks as in skinny_sm100.cuh; a "segment" is a tile here
 #endif
-  if (warp == 0 && lane < 4)  // the copy engine fetches a descriptor on first use: start that now
-    prefetch_tensormap(lane == 0 ? &tmW : lane == 1 ? &tmSFW : lane == 2 ? &tmX : &tmSFX);
-  if (warp == 2 && lane == 0 && p.tma_store) prefetch_tensormap(&tmC);
+  if (warp == 0 && lane < 4) {  // the copy engine fetches a descriptor on first use: start that now
+    if constexpr (Maps::kExperts) prefetch_tensormap((lane & 1) ? &maps.sfx : &maps.x);
+    else prefetch_tensormap(lane == 0 ? &maps.w : lane == 1 ? &maps.sfw : lane == 2 ? &maps.x : &maps.sfx);
+  }
+  if (!Maps::kSilu && warp == 2 && lane == 0 && p.tma_store) prefetch_tensormap(&maps.c);
 
   const uint32_t staging_base = smem_base + STAGES * Cfg::STAGE_BYTES;
   const uint32_t bar_base = staging_base + Cfg::STAGING_BYTES;
@@ -123,9 +156,27 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
   // ---------------------------------------------------------------------------------- producer state
   uint32_t p_stage = 0, p_phase = 0;
   uint64_t stream_policy = 0, keep_policy = 0;
+  // Tensor maps, weight tile and block of activation rows of an item (one weight: block 0).
+  const CUtensorMap *tm_w = nullptr, *tm_sfw = nullptr;
+  int w_tile = 0, block = 0;
+  auto locate = [&](int item) -> bool {
+    if constexpr (Maps::kExperts) {
+      block = item / p.tiles_n;
+      w_tile = item - block * p.tiles_n;
+      const int e = __ldcg(maps.expert_ids + block);
+      if (e < 0 || e >= maps.num_groups) return false;  // never written by a correct router; do not index out of the table
+      tm_w = &maps.w[e];
+      tm_sfw = &maps.sfw[e];
+    } else {
+      w_tile = item;
+      tm_w = &maps.w;
+      tm_sfw = &maps.sfw;
+    }
+    return true;
+  };
   // part 0: all four loads of a stage; part 1: only the weights and their scales (no arrival on the barrier
   // yet); part 2: the arrival with the stage's byte count plus the activations and their scales.
-  auto load_stage = [&](int tile, int kb, uint32_t stage, int part) {
+  auto load_stage = [&](int kb, uint32_t stage, int part) {
     const uint32_t sW = smem_base + stage * Cfg::STAGE_BYTES;
     const uint32_t sX = sW + Base::W_BYTES;
     const uint32_t sSFW = sX + Base::X_BYTES;
@@ -139,12 +190,17 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
       if (part != 1)
         mbar_expect_tx(fb, Cfg::STAGE_BYTES - Base::W_BYTES + uint32_t(p.tile_rows) * ((EB == 8 && (p.elem_format & 0x10)) ? 64u : 128u));
       if (part != 2) {
-        tma_load_2d_hint(sW, &tmW, kb * 128, tile * p.tile_rows, fb, stream_policy);
-        tma_load_2d(sSFW, &tmSFW, kb * (Base::SF_ATOMS * 128), tile, fb);
+        if constexpr (Maps::kSilu) {
+          tma_load_2d_hint(sW, tm_w, kb * 128, w_tile * 64, fb, stream_policy);
+          tma_load_2d_hint(sW + 64 * 128, tm_w, kb * 128, maps.inter + w_tile * 64, fb, stream_policy);
+        } else {
+          tma_load_2d_hint(sW, tm_w, kb * 128, w_tile * p.tile_rows, fb, stream_policy);
+        }
+        tma_load_2d(sSFW, tm_sfw, kb * (Base::SF_ATOMS * 128), w_tile, fb);
       }
       if (part != 1) {
-        tma_load_2d_hint(sX, &tmX, kb * 128, 0, fb, keep_policy);
-        tma_load_2d(sSFX, &tmSFX, kb * (Base::SF_ATOMS * 128), 0, fb);
+        tma_load_2d_hint(sX, &maps.x, kb * 128, block * kExpertBlockRows, fb, keep_policy);
+        tma_load_2d(sSFX, &maps.sfx, kb * (Base::SF_ATOMS * 128), block, fb);
       }
     }
     __syncwarp();
@@ -157,8 +213,11 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
   if (warp == 0) {
     stream_policy = l2_policy_evict_first();  // weights are read once
     keep_policy = l2_policy_evict_last();     // activations are re-read by every CTA
-    head = min(STAGES, p.num_kb);
-    for (int i = 0; i < head; ++i) load_stage(int(blockIdx.x), i, uint32_t(i), p.dependent ? 1 : 0);
+    if constexpr (!Maps::kExperts) {  // (which expert a tile belongs to is known after the dependency wait only)
+      locate(int(blockIdx.x));
+      head = min(STAGES, p.num_kb);
+      for (int i = 0; i < head; ++i) load_stage(i, uint32_t(i), p.dependent ? 1 : 0);
+    }
 #ifdef WB200_TRACE
     if (lane == 0) WB_TRACE_SET(4, trace_now());
 #endif
@@ -176,6 +235,8 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
     // ------------------------------------------------------------------ TMA producer
     // The whole warp walks the loop; one elected lane issues the copies.
     if (p.dependent) pdl_wait();  // the activations' scales, and the counter, belong to the kernels before this one until now
+    int items = p.tiles_n;
+    if constexpr (Maps::kExperts) items = min(maps.max_blocks, __ldcg(maps.num_rows) / kExpertBlockRows) * p.tiles_n;
     int seq = 0;
     auto emit = [&](int tile) {
       const int s = seq & (IQ - 1);
@@ -188,22 +249,23 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
       ++seq;
     };
     auto run_tile = [&](int tile) {
+      if (!locate(tile)) return;
       emit(tile);
       for (int kb = 0; kb < p.num_kb; ++kb) {
         if (head > 0) {  // this stage's weights are already on their way
           --head;
-          if (p.dependent) load_stage(tile, kb, p_stage, 2);
+          if (p.dependent) load_stage(kb, p_stage, 2);
         } else {
           mbar_wait(empty_bar(p_stage), p_phase ^ 1u, ctx, WB_DEV_TIMEOUT_PRODUCER);
-          load_stage(tile, kb, p_stage, 0);
+          load_stage(kb, p_stage, 0);
         }
         if (++p_stage == STAGES) { p_stage = 0; p_phase ^= 1u; }
       }
     };
-    run_tile(int(blockIdx.x));
+    if (!Maps::kExperts || int(blockIdx.x) < items) run_tile(int(blockIdx.x));
     // Further tiles: one atomic per tile, drawn only when the loads of the previous tile are all issued (drawing
     // ahead would commit this CTA to a tile that a faster CTA could take); the loads in the ring cover the round trip.
-    const int dealt = p.tiles_n - int(gridDim.x);
+    const int dealt = max(0, items - int(gridDim.x));
     unsigned int* work = p.counters + kWholeWorkCounter;
     for (;;) {
       unsigned int raw = 0;
@@ -290,7 +352,10 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
       const int tile = next_tile(seq);
       if (tile < 0) break;
       const int as = seq & 1;
-      const int n = tile * p.tile_rows + pcol;  // first of this thread's eight columns
+      // the item's weight tile and the first row of its block in C
+      const int nt = Maps::kExperts ? tile % p.tiles_n : tile;
+      const int m_base = Maps::kExperts ? (tile / p.tiles_n) * kExpertBlockRows : 0;
+      const int n = nt * p.tile_rows + pcol;    // first of this thread's eight columns
       const bool keep = pcol < p.tile_rows;     // tile_rows is a multiple of 8: a piece is all inside or all outside
       mbar_wait(acc_full_bar(as), uint32_t(seq >> 1) & 1u, ctx, WB_DEV_TIMEOUT_EPILOGUE);
       tc_fence_after_sync();
@@ -298,6 +363,48 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
       if (t == 0) WB_TRACE_SEG(seq, 2, trace_now());
 #endif
       const uint32_t t_acc = tmem_base + (uint32_t(quad * 32) << 16) + (as ? Base::ACC_COL1 : 0);
+      if constexpr (Maps::kSilu) {
+        // Chunks of 16 rows pass through shared memory as f32: thread t takes row t / 8 and hidden columns 8 (t % 8) .. + 7
+        // (gate in columns 0 .. 63 of the staged row, up in 64 .. 127); four neighbouring lanes share a scale block.
+        static_assert(SBUFS == 2 && EB == 4, "two f32 staging buffers");
+        const int kblocks = maps.inter >> 5, i8 = t & 7;
+#pragma unroll 1
+        for (int ch = 0; ch < nchunks; ++ch) {
+          uint32_t r[16];
+          tmem_ld_32x16(t_acc + ch * 16, r);
+          tmem_ld_wait();
+          if (ch == nchunks - 1) {  // accumulator fully read: hand it back to the MMA warp
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty_bar(as));
+          }
+          const uint32_t buf = staging_base + (chunk_ctr & 1u) * uint32_t(Cfg::STAGING_BUF_BYTES);
+          ++chunk_ctr;
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(buf + uint32_t(j * 128 + nl) * 4u), "r"(r[j]) : "memory");
+          asm volatile("bar.sync 1, 128;" ::: "memory");  // (the next chunk's barrier orders these reads before the buffer's reuse)
+          const int m = ch * 16 + (t >> 3);
+          const uint32_t src = buf + uint32_t((t >> 3) * 128 + i8 * 8) * 4u;
+          float y[8];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            float4 g, u;
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(g.x), "=f"(g.y), "=f"(g.z), "=f"(g.w) : "r"(src + 16u * h) : "memory");
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w) : "r"(src + 256u + 16u * h) : "memory");
+            // (rounded to bf16 first, as in silu_quantize_block)
+            silu_mul_bf16x2(pack_bf16x2(g.x, g.y), pack_bf16x2(u.x, u.y), y[4 * h + 0], y[4 * h + 1]);
+            silu_mul_bf16x2(pack_bf16x2(g.z, g.w), pack_bf16x2(u.z, u.w), y[4 * h + 2], y[4 * h + 3]);
+          }
+          const int row = m_base + m;
+          const bool real = m < p.M && WB_CHECK(m < kExpertBlockRows && nt < p.tiles_n, kCheckOutputIndex, (long long)row << 32 | unsigned(nt));
+          mxfp4_encode_group<8>(y, real, row, nt * 2 + (i8 >> 2), i8 & 3, maps.inter, kblocks, maps.k_atoms, maps.q, nullptr, maps.scale_packed);
+          if (nt == p.tiles_n - 1 && i8 == 0 && real)  // the K blocks that pad the atoms to whole pipeline stages
+            for (int kb = kblocks; kb < maps.k_atoms * 4; ++kb)
+              reinterpret_cast<uint8_t*>(packed_scale_word(maps.scale_packed, maps.k_atoms, row, kb >> 2))[kb & 3] = WB_SF_PAD;
+        }
+        continue;
+      }
       if (p.tma_store) {
         // Every 16-row chunk is transposed into a dense [16][tile_rows] block of the output type in one of two
         // staging buffers and leaves through one TMA store (clipped at M and N by the copy engine). The stores are
@@ -333,7 +440,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
           if (t == 0) bulk_wait_group_read<0>();  // the previous chunk's store has read the other buffer
           asm volatile("bar.sync 1, 128;" ::: "memory");
           if (t == 0) {
-            tma_store_2d(&tmC, buf, tile * p.tile_rows, ch * 16);
+            tma_store_2d(&maps.c, buf, nt * p.tile_rows, m_base + ch * 16);
             bulk_commit_group();
           }
         }
@@ -371,7 +478,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
           float4 lo, hi;
           asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w) : "r"(src) : "memory");
           asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w) : "r"(src + 16u) : "memory");
-          OutT* dst = C + size_t(m) * p.ldc + n;
+          OutT* dst = C + size_t(m_base + m) * p.ldc + n;
           if (!WB_CHECK(m >= 0 && m < p.M && n >= 0 && n < p.N, kCheckOutputIndex, (long long)m << 32 | unsigned(n))) continue;
           if (p.c_vec && n + 8 <= p.N) {
             if constexpr (sizeof(OutT) == 4) {
