@@ -1568,7 +1568,8 @@ struct ExpertMlpPlan {
 static ExpertMlpPlan plan_expert_mlp(int T, int E, int K, int inter, int N, int top_k, bool decode_packing) {
   ExpertMlpPlan p;
   const long long n = (long long)T * top_k;
-  // At most 128 tokens: no expert can get more than one 128-row block, and the decode kernel streams the weights once.
+  // At most 128 tokens: no expert can get more than one 128-row block, and the decode kernel streams the weights once
+  // (16 tokens, 8 experts, top-2, K = 4096, inter = 7168: 75 us against 186 us in 256-row tiles and single steps).
   p.decode = decode_packing && T <= wb::kExpertBlockRows;
   p.block = p.decode ? wb::kExpertBlockRows : 256;
   const long long blocks = p.decode ? (n < E ? n : E) : (n + (long long)E * 255 + 255) / 256;

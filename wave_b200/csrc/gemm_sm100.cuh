@@ -156,7 +156,9 @@ struct AlignedMaps {
 // a scale block of its row: the block maximum needs no shuffle, the codes of a block are one 16-byte store and the four
 // blocks of a tile are one word of a packed scale atom. inter % 128 == 0 (a scale atom and both row blocks then belong
 // to one tile).
-// Instead of [rows, 2 inter] bf16 written here and read back by a second kernel, [rows, inter / 2] bytes leave.
+// Instead of [rows, 2 inter] bf16 written here and read back by a second kernel, [rows, inter / 2] bytes leave: with the
+// launches and passes that go with it (library softmax and top-k, two scale repacks, silu_and_mul) the whole MLP of 4096
+// tokens, 8 experts, top-2, K = 4096, inter = 7168 went from 515 to 379 us per call.
 template <int G>
 struct SiluMaps : AlignedMaps<G> {
   static constexpr bool kSilu = true;
