@@ -1073,17 +1073,15 @@ int wb200_quantize_mxfp4(const void* x, int x_dtype, long long ldx, int rows, in
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int k_atoms = wb::sf_k_atoms(K);
-  const int total_rows = scale_packed ? wb::sf_row_blocks(rows) * 128 : rows;
   const int q_vec = (reinterpret_cast<uintptr_t>(q) & 15) == 0;
-  const long long warps = (long long)total_rows * ((k_atoms + 7) / 8);
-  const unsigned blocks = unsigned((warps + 7) / 8);
+  const unsigned blocks = unsigned(wb::sf_row_blocks(rows)) * 16u * unsigned((k_atoms + 7) / 8);
   if (x_dtype == WB200_F32)
-    wb::quantize_mxfp4_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), ldx, rows, total_rows, K,
+    wb::quantize_mxfp4_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), ldx, rows, K,
                                                             static_cast<uint8_t*>(q), q_vec, static_cast<uint8_t*>(scale_rowmajor),
                                                             static_cast<uint8_t*>(scale_packed), k_atoms);
   else
     wb::quantize_mxfp4_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(x), ldx, rows, total_rows, K, static_cast<uint8_t*>(q), q_vec,
+        static_cast<const __nv_bfloat16*>(x), ldx, rows, K, static_cast<uint8_t*>(q), q_vec,
         static_cast<uint8_t*>(scale_rowmajor), static_cast<uint8_t*>(scale_packed), k_atoms);
   WB_CUDA(cudaGetLastError());
   return WB200_OK;

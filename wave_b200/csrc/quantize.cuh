@@ -20,8 +20,9 @@
 //   * the four scale bytes of a group leave as one 32-bit word, row-major and in the packed layout alike (a word of an
 //     atom is the four K blocks of one row), and padding bytes are written by the same pass;
 //   * the codes of a block are gathered in one lane (4 x 4 transpose in the group): one 16-byte store per lane.
-// 28672 x 8192 bf16, codes and both scale layouts (602 MB): 160 us (3.8 TB/s) -> 117 us (5.2 TB/s); 3000 x 8192 with packed scales only: 23 us (with the padding
-// kernel that the pass absorbs) -> 14.8 us.
+// 28672 x 8192 bf16, codes and both scale layouts (602 MB): 160 us (3.8 TB/s) -> 123 us, and 119 us (5.1 TB/s) with the
+// words of a packed-scale sector written together; 3000 x 8192 with packed scales only: 23 us (with the padding kernel that
+// the pass absorbs) -> 14.8 us.
 #pragma once
 #include "ptx.cuh"
 #include "scales.cuh"
@@ -221,20 +222,23 @@ __device__ __forceinline__ uint32_t* packed_scale_word(uint8_t* base, int k_atom
   return reinterpret_cast<uint32_t*>(base + (size_t(r >> 7) * k_atoms + atom) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4);
 }
 
-// One warp per (row, 32 K blocks); rows are walked up to total_rows, past `rows` (the padding rows of the packed scales)
-// only the padding byte is written. x rows are 16-byte aligned; q rows 16-byte aligned when q_vec.
+// One warp per (row, 32 K blocks). The 8 warps of a CTA take the same 32 K blocks of 8 rows of a 128-row block: two
+// neighbouring rows of each of its four 32-row groups. Their scale words of one atom are 32 consecutive bytes of the packed
+// layout, so the words are exchanged through shared memory and every 32-byte sector is written once (a warp that writes its
+// own 8 words touches 8 sectors with 4 bytes each). Rows past `rows` (the padding rows of the packed scales) get the padding byte
+// only. x rows are 16-byte aligned; q rows 16-byte aligned when q_vec. Grid: 16 x row blocks x chunks of 32 K blocks.
 template <typename InT>
 __global__ void __launch_bounds__(256)
-quantize_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int total_rows, int K, uint8_t* __restrict__ q, int q_vec,
+quantize_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int K, uint8_t* __restrict__ q, int q_vec,
                       uint8_t* __restrict__ scale_rm, uint8_t* __restrict__ scale_packed, int k_atoms) {
+  __shared__ uint32_t words[8][8];  // [atom of the chunk][word of the sector]
   pdl_launch_dependents();
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kblocks = K >> 5;
   const unsigned chunks = unsigned(k_atoms + 7) >> 3;
-  const unsigned wid = blockIdx.x * 8u + (threadIdx.x >> 5);
-  const int r = int(wid / chunks);
-  if (r >= total_rows) return;
-  const int kb0 = int(wid - unsigned(r) * chunks) * 32;
+  const unsigned group = blockIdx.x / chunks;  // 8 rows
+  const int kb0 = int(blockIdx.x - group * chunks) * 32;
+  const int r = int(group >> 4) * 128 + (warp & 3) * 32 + int(group & 15) * 2 + (warp >> 2);
   const bool real = r < rows;
   uint4 codes;
   uint32_t scales;
@@ -249,7 +253,6 @@ quantize_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int to
       d[0] = codes.x; d[1] = codes.y; d[2] = codes.z; d[3] = codes.w;
     }
   }
-  if (sub == 0 && scale_packed && (kb0 >> 2) + g < k_atoms) *packed_scale_word(scale_packed, k_atoms, r, (kb0 >> 2) + g) = scales;
   if (sub == 1 && scale_rm && real) {
     uint8_t* d = scale_rm + (long long)r * kblocks + kb0 + g * 4;
     if ((kblocks & 3) == 0 && (reinterpret_cast<uintptr_t>(scale_rm) & 3) == 0) {
@@ -259,6 +262,14 @@ quantize_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int to
       for (int u = 0; u < 4; ++u)
         if (kb0 + g * 4 + u < kblocks) d[u] = uint8_t(scales >> (8 * u));
     }
+  }
+  if (scale_packed) {
+    if (sub == 0) words[g][warp] = scales;  // word (row of the pair, 32-row group) of the sector
+    __syncthreads();
+    const int atom = (kb0 >> 2) + (threadIdx.x >> 3);
+    if (threadIdx.x < 64 && atom < k_atoms)
+      reinterpret_cast<uint32_t*>(scale_packed + (size_t(group >> 4) * k_atoms + atom) * 512 + (group & 15) * 32)[threadIdx.x & 7] =
+          words[threadIdx.x >> 3][threadIdx.x & 7];
   }
 }
 
