@@ -164,6 +164,14 @@ int wb200_repack_scales_grouped(const void* src, long long src_row_stride, int n
 int wb200_quantize_mxfp4(const void* x, int x_dtype, long long ldx, int rows, int K, void* q, void* scale_rowmajor,
                          void* scale_packed, void* stream);
 
+/* wb200_quantize_mxfp4 and wb200_mxfp4_gemm in one call, the GEMM launched as the programmatic dependent of the
+ * quantiser: x [M, K] (f32 or bf16) is quantised to q_scratch [M, K/2] (16-byte aligned) and scale_scratch
+ * (wb200_packed_scale_bytes(M, K)), and the GEMM's set-up, and on the M <= 128 path its first ring of weight loads, run
+ * while the quantiser does. Other arguments as wb200_mxfp4_gemm; WB200_OVERLAP_PREVIOUS is refused. */
+int wb200_mxfp4_gemm_quantize_a(int M, int N, int K, const void* x, int x_dtype, long long ldx, void* q_scratch, void* scale_scratch,
+                                const void* b, const void* b_scale_packed, void* c, int c_dtype, long long ldc, void* workspace,
+                                size_t workspace_bytes, unsigned flags, void* stream);
+
 /* Grouped GEMM driven by DEVICE routing arrays, for rows laid out by wb200_moe_align_block_size with
  * block_size = 256: a [max_rows, K/2] holds the routed rows of all experts, every expert padded to whole
  * 256-row blocks; expert_ids[i] (device) is the expert of block i; *num_rows (device) the padded total, row

@@ -84,6 +84,7 @@ EXPORTED_SYMBOLS = (
     "wb200_mxfp4_moe_gemm",
     "wb200_mxfp4_expert_mlp_workspace_bytes",
     "wb200_mxfp4_expert_mlp",
+    "wb200_mxfp4_gemm_quantize_a",
     "wb200_moe_align_block_size",
     "wb200_moe_gather_rows",
     "wb200_silu_and_mul",
@@ -203,6 +204,9 @@ def load() -> ctypes.CDLL:
     lib.wb200_silu_and_mul.restype = c_int
     lib.wb200_silu_and_mul.argtypes = [c_void_p, c_void_p, c_ll, c_ll, c_int, c_int, c_int, c_void_p, c_ll, c_void_p,
                                        c_void_p, c_void_p, c_void_p, c_void_p]
+    lib.wb200_mxfp4_gemm_quantize_a.restype = c_int
+    lib.wb200_mxfp4_gemm_quantize_a.argtypes = [c_int, c_int, c_int, c_void_p, c_int, c_ll, c_void_p, c_void_p, c_void_p, c_void_p,
+                                                c_void_p, c_int, c_ll, c_void_p, c_size_t, c_uint, c_void_p]
     lib.wb200_mxfp4_expert_mlp_workspace_bytes.restype = c_size_t
     lib.wb200_mxfp4_expert_mlp_workspace_bytes.argtypes = [c_int] * 6
     lib.wb200_mxfp4_expert_mlp.restype = c_int

@@ -1437,6 +1437,20 @@ int wb200_mxfp4_gemm_repack_a(int M, int N, int K, const void* a, const void* a_
   return rc;
 }
 
+int wb200_mxfp4_gemm_quantize_a(int M, int N, int K, const void* x, int x_dtype, long long ldx, void* q_scratch, void* scale_scratch,
+                                const void* b, const void* b_scale_packed, void* c, int c_dtype, long long ldc, void* workspace,
+                                size_t workspace_bytes, unsigned flags, void* stream) {
+  if (!scale_scratch) return fail(WB200_ERR_INVALID_ARG, "gemm_quantize_a: null scratch for the packed activation scales");
+  if (flags & WB200_OVERLAP_PREVIOUS)  // the quantiser reads x at once
+    return fail(WB200_ERR_INVALID_ARG, "gemm_quantize_a: WB200_OVERLAP_PREVIOUS is not available here");
+  int rc = wb200_quantize_mxfp4(x, x_dtype, ldx, M, K, q_scratch, nullptr, scale_scratch, stream);
+  if (rc) return rc;
+  tl_dependent_launch = true;  // the GEMM is the quantiser's programmatic dependent
+  rc = wb200_mxfp4_gemm(M, N, K, q_scratch, scale_scratch, b, b_scale_packed, c, c_dtype, ldc, workspace, workspace_bytes, flags, stream);
+  tl_dependent_launch = false;
+  return rc;
+}
+
 extern "C++" {
 template <int CG, int BN>
 static int launch_mxfp8(int c_dtype, const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,

@@ -38,7 +38,6 @@ class MXFP4Linear(torch.nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lead = x.shape[:-1]
         x2 = x.reshape(-1, self.in_features)
-        q, _, sf = ops.quantize_mxfp4(x2, want_rowmajor=False, want_packed=True)
         out = torch.empty(x2.shape[0], self.out_features, dtype=self.output_dtype, device=x.device)
         packed = self._packed
         if x2.shape[0] <= 128:
@@ -46,5 +45,5 @@ class MXFP4Linear(torch.nn.Module):
                 h = ops.decode_tile_rows(self.out_features, x.device)
                 self._packed_decode = self._packed if h == 128 else ops.repack_scales(self.weight_scales, tile_rows=h)
             packed = self._packed_decode
-        ops.scaled_gemm_packed(q, sf, self.weight_codes, packed, out)
+        ops.quantized_gemm(x2, self.weight_codes, packed, out)
         return out.reshape(*lead, self.out_features)

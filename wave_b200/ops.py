@@ -227,6 +227,38 @@ def scaled_gemm_packed(a: torch.Tensor, a_sf: PackedScales, b: torch.Tensor, b_s
         _lib.check(rc)
 
 
+def quantized_gemm(x: torch.Tensor, b: torch.Tensor, b_sf: PackedScales, c: torch.Tensor) -> None:
+    """c[M, N] = dequant(quantise(x)) @ dequant(b).T for f32 or bf16 x [M, K]: `quantize_mxfp4` and `scaled_gemm_packed` in
+    one native call, the GEMM set up (and, for M <= 128, its first weight loads issued) while the quantiser runs."""
+    lib = _lib.load()
+    if not x.is_cuda:
+        raise ValueError("x must be a CUDA tensor; wave_b200 has no CPU path")
+    if x.dtype not in _DTYPE_CODE or x.dim() != 2:
+        raise ValueError(f"x must be a 2-D float32 or bfloat16 tensor, got {x.dtype} {tuple(x.shape)}")
+    if x.stride(1) != 1:
+        x = x.contiguous()
+    (M, K), N = x.shape, b.shape[0]
+    if b.shape[1] * 2 != K or (b_sf.rows, b_sf.K) != (N, K) or c.dtype not in _DTYPE_CODE or tuple(c.shape) != (M, N) or c.stride(1) != 1:
+        raise ValueError("operand and scale shapes do not agree")
+    flags = _lib.PATH_AUTO
+    if b_sf.tile_rows != 128:
+        if (M > 128) != (b_sf.tile_rows == 224):
+            raise ValueError(f"b's scales are packed per {b_sf.tile_rows}-row tile, which M = {M} does not read")
+        flags |= _lib.B_TILE_ROWS(b_sf.tile_rows)
+    q_bytes = (M * K // 2 + 255) // 256 * 256
+    scratch = torch.empty(q_bytes + packed_scale_bytes(M, K), dtype=torch.uint8, device=x.device)
+    with torch.cuda.device(x.device):
+        ws_ptr = ws_bytes = 0
+        if M <= 128 or split_k_pays():
+            ws_bytes = int(lib.wb200_mxfp4_gemm_workspace_bytes(M, N, K))
+            if ws_bytes:
+                ws_ptr = _workspace(x.device, ws_bytes, "skinny" if M <= 128 else "splitk").data_ptr()
+        _lib.check(lib.wb200_mxfp4_gemm_quantize_a(M, N, K, x.data_ptr(), _DTYPE_CODE[x.dtype], x.stride(0) if M > 1 else K,
+                                                   scratch.data_ptr(), scratch.data_ptr() + q_bytes, b.data_ptr(),
+                                                   b_sf.data.data_ptr(), c.data_ptr(), _DTYPE_CODE[c.dtype],
+                                                   c.stride(0) if M > 1 else N, ws_ptr, ws_bytes, flags, _stream()))
+
+
 _FP8_FORMATS = {torch.float8_e5m2: _lib.E5M2, torch.float8_e4m3fn: _lib.E4M3}
 
 
