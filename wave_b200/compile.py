@@ -192,7 +192,14 @@ class ScaledGemmKernel:
                 raise ValueError(f"b must be packed E2M1 [N, K/2] = [{N}, {K // 2}], got {tuple(b.shape)}")
         if self._static is not None and self._static != (M, N, K):
             raise ValueError(f"kernel was built for (M, N, K) = {self._static}, called with {(M, N, K)}")
-        a_sf = a_scale if isinstance(a_scale, ops.PackedScales) else self._pack_activation_scales(a_scale, M, K)
+        rowmajor = None
+        if isinstance(a_scale, ops.PackedScales):
+            a_sf = a_scale
+        else:  # packed by the call below, ahead of the GEMM
+            rowmajor = self._check_scale(a_scale, M, K, "a_scale")
+            if rowmajor.stride(1) != 1:
+                rowmajor = rowmajor.contiguous()
+            a_sf = ops.PackedScales(self._a_scale_buffer(rowmajor.device, M, K), M, K)
         if isinstance(b_scale, ops.PackedScales):
             b_sf = b_scale
         else:
@@ -200,7 +207,7 @@ class ScaledGemmKernel:
             b_sf = self._weight_scales.get(self._check_scale(b_scale, N, K, "b_scale"), self._weight_tile_rows(M, N, idx))
         fmt = _lib.E5M2 if t.element_format == "f8e5m2" else _lib.E4M3
         flags = self.options.kernel_path | self._raster_flags() | (_lib.ACCUMULATE if t.accumulate else 0)
-        ops.scaled_gemm_mxfp8_packed(a, a_sf, b, b_sf, c, fmt, flags, b_fp4=b_fp4)
+        ops.scaled_gemm_mxfp8_packed(a, a_sf, b, b_sf, c, fmt, flags, b_fp4=b_fp4, a_scale=rowmajor)
 
     def _invoke_checked(self, a, a_scale, b, b_scale, c) -> None:
         t = self.template

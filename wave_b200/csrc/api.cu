@@ -1521,6 +1521,20 @@ int wb200_mxfp8_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
               : launch_mxfp8<1, 256>(c_dtype, *dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, accumulate, s, elem_format);
 }
 
+int wb200_mxfp8_gemm_repack_a(int M, int N, int K, const void* a, const void* a_scale, long long a_scale_stride, void* a_scale_scratch,
+                              const void* b, const void* b_scale_packed, void* c, int c_dtype, long long ldc, int elem_format,
+                              void* workspace, size_t workspace_bytes, unsigned flags, void* stream) {
+  if (!a_scale_scratch) return fail(WB200_ERR_INVALID_ARG, "mxfp8_gemm_repack_a: null scratch for the packed activation scales");
+  tl_dependent_launch = (flags & WB200_OVERLAP_PREVIOUS) != 0;
+  int rc = wb200_repack_scales(a_scale, a_scale_stride, M, K, a_scale_scratch, stream);
+  tl_dependent_launch = false;
+  if (rc) return rc;
+  tl_dependent_launch = true;  // the GEMM is the repack kernel's programmatic dependent
+  rc = wb200_mxfp8_gemm(M, N, K, a, a_scale_scratch, b, b_scale_packed, c, c_dtype, ldc, elem_format, workspace, workspace_bytes, flags, stream);
+  tl_dependent_launch = false;
+  return rc;
+}
+
 int wb200_mxfp4_gemm_skinny_noalloc(int M, int N, int K, const void* a, const void* a_scale_packed, const void* b,
                                     const void* b_scale_packed, void* c, int c_dtype, long long ldc, unsigned flags,
                                     void* stream) {

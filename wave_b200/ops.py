@@ -285,10 +285,13 @@ def quantize_mxfp8(x: torch.Tensor, dtype: torch.dtype = torch.float8_e5m2, want
 
 
 def scaled_gemm_mxfp8_packed(a: torch.Tensor, a_sf: PackedScales, b: torch.Tensor, b_sf: PackedScales, c: torch.Tensor,
-                             elem_format: int | None = None, flags: int = 0, b_fp4: bool = False) -> None:
+                             elem_format: int | None = None, flags: int = 0, b_fp4: bool = False,
+                             a_scale: torch.Tensor | None = None) -> None:
     """c [M, N] = dequant(a) @ dequant(b)^T for 8-bit operands a [M, K], b [N, K] (torch float8 tensors, or
     int8 / uint8 bytes with `elem_format` given) and packed E8M0 scales, on the current stream.
-    b_fp4: the mixed pair — b is packed E2M1, [N, K/2] uint8 as for the MXFP4 GEMM, a stays 8-bit (K % 128 == 0)."""
+    b_fp4: the mixed pair — b is packed E2M1, [N, K/2] uint8 as for the MXFP4 GEMM, a stays 8-bit (K % 128 == 0).
+    a_scale: row-major scales of a ([M, K/32], unit column stride), packed into a_sf's memory first in the same native call,
+    the GEMM set up while that kernel runs."""
     lib = _lib.load()
     if elem_format is None:
         if a.dtype not in _FP8_FORMATS:
@@ -316,6 +319,12 @@ def scaled_gemm_mxfp8_packed(a: torch.Tensor, a_sf: PackedScales, b: torch.Tenso
         ws_bytes = int(lib.wb200_mxfp4_gemm_workspace_bytes(M, N, K))
         ws_ptr = _workspace(a.device, ws_bytes, "skinny").data_ptr()
     with torch.cuda.device(a.device):
+        if a_scale is not None:
+            _lib.check(lib.wb200_mxfp8_gemm_repack_a(M, N, K, a.data_ptr(), a_scale.data_ptr(), a_scale.stride(0) if M > 1 else K // 32,
+                                                     a_sf.data.data_ptr(), b.data_ptr(), b_sf.data.data_ptr(), c.data_ptr(),
+                                                     _DTYPE_CODE[c.dtype], c.stride(0) if M > 1 else N, elem_format, ws_ptr, ws_bytes,
+                                                     flags, _stream()))
+            return
         _lib.check(lib.wb200_mxfp8_gemm(M, N, K, a.data_ptr(), a_sf.data.data_ptr(), b.data_ptr(), b_sf.data.data_ptr(),
                                         c.data_ptr(), _DTYPE_CODE[c.dtype], c.stride(0) if M > 1 else N, elem_format, ws_ptr,
                                         ws_bytes, flags, _stream()))
