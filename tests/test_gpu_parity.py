@@ -1071,3 +1071,33 @@ def test_run_bench_option_reports_kernel_time(tmp_path):
     check(c, a, a_s, b, b_s)
     rep = json.loads((tmp_path / "bench.json").read_text())["benchmarks"][0]
     assert rep["time_unit"] == "us" and rep["iterations"] == 3 and 0 < rep["min_time"] <= rep["real_time"] < 1e5
+
+
+@pytest.mark.parametrize("shape", [(129, 128, 10240), (512, 2048, 16000), (300, 1000, 10016), (700, 900, 16384), (512, 512, 12000),
+                                   (1024, 1030, 10272)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_split_k_inside_a_cluster(shape, out_dtype):
+    """Few output tiles and K >= 40 K blocks without a workspace: the slices of a tile run on the CTA pairs of one cluster. One
+    tile and the most that 2, 3 and 4 slices take; ragged M, N and K, C with an unaligned row pitch, accumulation, and the
+    same bits on every run."""
+    M, N, K = shape
+    a, a_s, b, b_s = random_problem(M, N, K, seed=M + N + K, lo=125, hi=129)
+    ad, bd = a.to(DEV), b.to(DEV)
+    asp, bsp = ops.repack_scales(a_s.to(DEV)), ops.repack_scales(b_s.to(DEV))
+    ref = orc.scaled_gemm(a, a_s, b, b_s)
+    wide = torch.full((M, N + 3), float("nan"), dtype=out_dtype, device=DEV)
+    c = wide[:, 1:N + 1]
+    ops.scaled_gemm_packed(ad, asp, bd, bsp, c)
+    check(c.contiguous(), a, a_s, b, b_s, ref=ref)
+    assert bool(wide[:, 0].isnan().all()) and bool(wide[:, N + 1:].isnan().all())
+    again = torch.empty(M, N, dtype=out_dtype, device=DEV)
+    for _ in range(3):
+        ops.scaled_gemm_packed(ad, asp, bd, bsp, again)
+        assert torch.equal(again, c)
+    if out_dtype == torch.float32:
+        base = torch.randn(M, N, generator=torch.Generator().manual_seed(M))
+        acc = base.to(DEV)
+        ops.scaled_gemm_packed(ad, asp, bd, bsp, acc, _lib.ACCUMULATE)
+        tol = orc.f32_tolerance(orc.dequant_mxfp4(a, a_s), orc.dequant_mxfp4(b, b_s), ref, K)
+        assert bool(((acc.cpu() - (ref + base)).abs() <= tol + 1e-6 * base.abs()).all())
+    ops.check_device_status()

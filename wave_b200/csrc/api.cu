@@ -2,6 +2,7 @@
 // launches. Plays the role of the reference's native launch shim
 // (wave_lang/kernel/wave/runtime/runtime.cpp:123-263) for the MXFP4 scaled-GEMM kernels.
 #include "../../include/wave_b200.h"
+#include "gemm_cluster_splitk_sm100.cuh"
 #include "gemm_sm100.cuh"
 #include "moe.cuh"
 #include "multi_gpu.cuh"
@@ -641,6 +642,96 @@ int launch_splitk(const DeviceInfo& dev, int slices, int M, int N, int K, const 
                                                                                   static_cast<OutT*>(c), ldc, accumulate);
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
+}
+
+// ------------------------------------------------------------------------------------------
+// split-K inside a cluster: few output tiles, no workspace (gemm_cluster_splitk_sm100.cuh)
+// ------------------------------------------------------------------------------------------
+template <int BN, typename OutT>
+int cluster_splitk_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int slices, long long tiles, cudaStream_t stream) {
+  using Split = wb::ClusterSplitCfg<BN, OutT>;
+  static bool smem_set[kMaxDevices] = {};
+  int rc = set_smem(wb::mxfp4_gemm_cluster_splitk_kernel<BN, OutT>, Split::SMEM_BYTES, smem_set);
+  if (rc) return rc;
+  cfg.gridDim = dim3(unsigned(tiles) * 2 * slices, 1, 1);
+  cfg.blockDim = dim3(192, 1, 1);
+  cfg.dynamicSmemBytes = Split::SMEM_BYTES;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2 * slices;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = tl_dependent_launch ? 2 : 1;
+  return WB200_OK;
+}
+
+// Clusters of `slices` CTA pairs that run at one time on the current device (a cluster does not cross a GPC, so this is less
+// than SMs / CTAs); 0 where they cannot.
+int clusters_in_flight(int slices) {
+  static int known[kMaxDevices][wb::kMaxClusterSlices + 1];
+  static std::mutex mu;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  std::lock_guard<std::mutex> lk(mu);
+  int& n = known[dev][slices];
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    int count = 0;
+    const bool saved = tl_dependent_launch;
+    tl_dependent_launch = false;
+    if (cluster_splitk_config<128, float>(cfg, attr, slices, 1, nullptr) != WB200_OK ||
+        cudaOccupancyMaxActiveClusters(&count, wb::mxfp4_gemm_cluster_splitk_kernel<128, float>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      count = 0;
+    }
+    tl_dependent_launch = saved;
+    n = count > 0 ? count : -1;
+  }
+  return n > 0 ? n : 0;
+}
+
+template <int BN, typename OutT>
+int launch_cluster_splitk(const DeviceInfo& dev, int slices, int M, int N, int K, const void* a, const void* as, const void* b,
+                          const void* bs, void* c, long long ldc, int accumulate, cudaStream_t stream) {
+  using Cfg = wb::GemmCfg<2, BN, int(sizeof(OutT))>;
+  wb::PlainMaps maps;
+  int rc;
+  if ((rc = make_operand_map(&maps.m[0], a, M, K / 2, Cfg::BM))) return rc;
+  if ((rc = make_operand_map(&maps.m[1], b, N, K / 2, Cfg::B_ROWS))) return rc;
+  if ((rc = make_scale_map(&maps.m[2], as, wb::sf_row_blocks(M), wb::sf_k_atoms(K), 1))) return rc;
+  if ((rc = make_scale_map(&maps.m[3], bs, wb::sf_row_blocks(N), wb::sf_k_atoms(K), Cfg::SFB_BLOCKS))) return rc;
+  maps.m[4] = maps.m[0];  // not used: C leaves through plain stores
+  wb::GemmParams p = {};
+  p.c = c;
+  p.M = M; p.N = N; p.K = K;
+  p.ldc = int(ldc);
+  p.tiles_m = (M + 255) / 256;
+  p.tiles_n = (N + BN - 1) / BN;
+  p.group_n = std::max(1, std::min(tl_group_n, p.tiles_n));
+  p.vec_ok = ((reinterpret_cast<uintptr_t>(c) & 15) == 0 && (ldc * (long long)sizeof(OutT)) % 16 == 0) ? 1 : 0;
+  p.accumulate = accumulate;
+  p.status = dev.status_ptr;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  if ((rc = cluster_splitk_config<BN, OutT>(cfg, attr, slices, (long long)p.tiles_m * p.tiles_n, stream))) return rc;
+  WB_CUDA(cudaLaunchKernelEx(&cfg, wb::mxfp4_gemm_cluster_splitk_kernel<BN, OutT>, maps, p, slices));
+  return WB200_OK;
+}
+
+// Slices for a shape that AUTO would give to the CTA-pair tile kernel: as many as let all its 256 x 128 tiles run in one
+// wave of clusters (a second wave costs a whole launch again: 512 x 4096 x 4096, 64 tiles, 10.2 us plain, 19.2 us with 2
+// slices), and only from K = 40 x 256 up: at 32 K blocks the exchange takes what the slices save (1024 x 1024 x 8192: 12.4
+// plain, 11.9 with 2), at 16 more (256 x 4096 x 4096: 9.5 against 10.5).
+int cluster_splitk_slices(int M, int N, int K) {
+  if ((K + 255) / 256 < 40) return 0;
+  const long long tiles = (long long)((M + 255) / 256) * ((N + 127) / 128);
+  for (int s = wb::kMaxClusterSlices; s >= 2; --s)
+    if (tiles <= clusters_in_flight(s)) return s;
+  return 0;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1397,6 +1488,14 @@ int wb200_mxfp4_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
     if (c_dtype == WB200_F32)
       return dispatch_skinny<float>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, workspace, accumulate, s);
     return dispatch_skinny<__nv_bfloat16>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, workspace, accumulate, s);
+  }
+  if ((flags & WB200_PATH_MASK) == WB200_PATH_AUTO && path == WB200_PATH_TILE_2CTA && !(flags & (WB200_TILE_N128 | WB200_TILE_N192))) {
+    const int cluster_slices = cluster_splitk_slices(M, N, K);
+    if (cluster_slices) {
+      if (c_dtype == WB200_F32)
+        return launch_cluster_splitk<128, float>(*dev, cluster_slices, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, accumulate, s);
+      return launch_cluster_splitk<128, __nv_bfloat16>(*dev, cluster_slices, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, accumulate, s);
+    }
   }
   // Narrow problems fill more SMs with 128-wide tiles.
   int bn = (flags & WB200_TILE_N128) ? 128 : (flags & WB200_TILE_N192) ? 192 : 256;
