@@ -246,17 +246,26 @@ def quantized_gemm(x: torch.Tensor, b: torch.Tensor, b_sf: PackedScales, c: torc
             raise ValueError(f"b's scales are packed per {b_sf.tile_rows}-row tile, which M = {M} does not read")
         flags |= _lib.B_TILE_ROWS(b_sf.tile_rows)
     q_bytes = (M * K // 2 + 255) // 256 * 256
-    scratch = torch.empty(q_bytes + packed_scale_bytes(M, K), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
+    scratch = torch.empty(q_bytes + (M + 127) // 128 * ((K + 255) // 256) * 1024, dtype=torch.uint8, device=x.device)
+
+    def run():
         ws_ptr = ws_bytes = 0
         if M <= 128 or split_k_pays():
             ws_bytes = int(lib.wb200_mxfp4_gemm_workspace_bytes(M, N, K))
             if ws_bytes:
                 ws_ptr = _workspace(x.device, ws_bytes, "skinny" if M <= 128 else "splitk").data_ptr()
-        _lib.check(lib.wb200_mxfp4_gemm_quantize_a(M, N, K, x.data_ptr(), _DTYPE_CODE[x.dtype], x.stride(0) if M > 1 else K,
-                                                   scratch.data_ptr(), scratch.data_ptr() + q_bytes, b.data_ptr(),
-                                                   b_sf.data.data_ptr(), c.data_ptr(), _DTYPE_CODE[c.dtype],
-                                                   c.stride(0) if M > 1 else N, ws_ptr, ws_bytes, flags, _stream()))
+        q = scratch.data_ptr()
+        return lib.wb200_mxfp4_gemm_quantize_a(M, N, K, x.data_ptr(), _DTYPE_CODE[x.dtype], x.stride(0) if M > 1 else K, q, q + q_bytes,
+                                               b.data_ptr(), b_sf.data.data_ptr(), c.data_ptr(), _DTYPE_CODE[c.dtype],
+                                               c.stride(0) if M > 1 else N, ws_ptr, ws_bytes, flags, _stream())
+
+    if x.device.index is None or x.device.index == torch.cuda.current_device():
+        rc = run()
+    else:
+        with torch.cuda.device(x.device):
+            rc = run()
+    if rc:
+        _lib.check(rc)
 
 
 _FP8_FORMATS = {torch.float8_e5m2: _lib.E5M2, torch.float8_e4m3fn: _lib.E4M3}
