@@ -129,6 +129,10 @@ size_t wb200_packed_scale_bytes(int rows, int K);
  * range keeps both packings. The reference prepares its weight scales per kernel variant in the same way
  * (e8m0_shuffle for the preshuffle templates, wave_lang/kernel/wave/utils/mxfp_utils.py:113-128). */
 int wb200_decode_tile_rows(int N);
+/* The same for the mixed pair (8-bit activations, 4-bit weights, WB200_B_FP4): where it returns a height above 128 (up to
+ * 208; two atom rows per tile) the decode kernel puts the weights on the MMA's N side. Only wb200_mxfp8_gemm with
+ * WB200_B_FP4 and M <= 128 reads such a packing. */
+int wb200_mixed_decode_tile_rows(int N);
 size_t wb200_packed_scale_bytes_tiled(int rows, int K, int tile_rows);
 int wb200_repack_scales_tiled(const void* scales, long long row_stride, int rows, int K, int tile_rows, void* packed,
                               void* stream);

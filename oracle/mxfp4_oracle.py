@@ -131,10 +131,11 @@ def pack_scales(scale: torch.Tensor) -> torch.Tensor:
 
 def pack_scales_tiled(scale: torch.Tensor, tile_rows: int) -> torch.Tensor:
     """Weight-scale packing per tile of `tile_rows` rows. Up to 128 (a multiple of 8; the decode kernel's tiles): every
-    tile gets an atom row of its own, its rows in atom rows 0 .. tile_rows - 1 and the padding byte above. 224 (the
-    tile kernel's 224-column tiles): two atom rows per tile, rows 0..127 and 128..223 of the tile. Inside an atom the
+    tile gets an atom row of its own, its rows in atom rows 0 .. tile_rows - 1 and the padding byte above. Above 128 (up to
+    208: the mixed decode kernel's tiles; 224: the tile kernel's 224-column tiles): two atom rows per tile, rows 0..127 and
+    128.. of the tile. Inside an atom the
     layout is `pack_scales`'s; tile_rows = 128 is `pack_scales` itself."""
-    assert tile_rows == 224 or (tile_rows % 8 == 0 and 8 <= tile_rows <= 128)
+    assert tile_rows == 224 or (tile_rows % 8 == 0 and 8 <= tile_rows <= 208)
     rows, kb = scale.shape
     tiles = (rows + tile_rows - 1) // tile_rows
     span = (tile_rows + 127) // 128 * 128  # rows of packed storage per tile

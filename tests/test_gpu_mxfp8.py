@@ -329,3 +329,36 @@ def test_mixed_pair_golden_small(out_dtype):
     if out_dtype == torch.float32:
         torch.testing.assert_close(c.cpu(), ref, atol=2e-3, rtol=1e-3)  # the reference's tolerance for its 8-bit test
     check_mixed(c, x, xs, w, ws)
+
+
+@pytest.mark.parametrize("M", [1, 16, 33, 64, 128])
+@pytest.mark.parametrize("N,K", [(28672, 256), (28672 - 72, 384), (60000, 128), (20001, 128)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_mixed_decode_with_weights_on_the_n_side(M, N, K, out_dtype):
+    """The mixed pair's decode kernel on scales packed per tile of more than 128 rows: one and two tiles per SM, ragged last
+    tile, odd N (scalar stores), few K blocks (fewer than stages), accumulation into a column block of a wider C, packing
+    bit-exact, E4M3 and E5M2."""
+    h = ops.decode_tile_rows(N, mixed=True)
+    if h <= 128:
+        pytest.skip("this part's SM count gives tiles of at most 128 rows")
+    fmt = torch.float8_e4m3fn if K != 384 else torch.float8_e5m2
+    a, a_s, b, b_s = mixed_problem(M, N, K, 900 + M + K, fmt)
+    ad, bd, a_sf = a.to(DEV), b.to(DEV), ops.repack_scales(a_s.to(DEV))
+    b_sf = ops.repack_scales(b_s.to(DEV), tile_rows=h)
+    assert torch.equal(b_sf.data.cpu(), orc.pack_scales_tiled(b_s, h))
+    c = torch.full((M, N), float("nan"), dtype=out_dtype, device=DEV)
+    ops.scaled_gemm_mxfp8_packed(ad, a_sf, bd, b_sf, c, b_fp4=True)
+    check_mixed(c, a, a_s, b, b_s)
+    usual = torch.empty_like(c)
+    ops.scaled_gemm_mxfp8_packed(ad, a_sf, bd, ops.repack_scales(b_s.to(DEV)), usual, b_fp4=True, flags=_lib.PATH_TILE_1CTA)
+    bits = torch.int32 if out_dtype == torch.float32 else torch.int16
+    assert torch.equal(c.view(bits), usual.view(bits))  # every output's sum over K is made in the same order
+    wide = torch.ones(M, N + 8, dtype=out_dtype, device=DEV)
+    ops.scaled_gemm_mxfp8_packed(ad, a_sf, bd, b_sf, wide[:, :N], b_fp4=True, flags=_lib.ACCUMULATE)
+    ref = (usual.float() + 1.0) if out_dtype == torch.float32 else None
+    if ref is not None:
+        assert torch.equal(wide[:, :N], ref)
+    assert bool((wide[:, N:] == 1).all())
+    with pytest.raises(RuntimeError):  # no MXFP4 kernel reads this packing
+        ops.scaled_gemm_packed(bd[:M], ops.repack_scales(b_s[:M].to(DEV)), bd, b_sf, torch.empty(M, N, dtype=out_dtype, device=DEV))
+    ops.check_device_status()

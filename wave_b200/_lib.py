@@ -66,6 +66,7 @@ EXPORTED_SYMBOLS = (
     "wb200_debug_checks_selftest",
     "wb200_packed_scale_bytes",
     "wb200_decode_tile_rows",
+    "wb200_mixed_decode_tile_rows",
     "wb200_packed_scale_bytes_tiled",
     "wb200_repack_scales_tiled",
     "wb200_repack_scales",
@@ -157,6 +158,8 @@ def load() -> ctypes.CDLL:
     lib.wb200_packed_scale_bytes.argtypes = [c_int, c_int]
     lib.wb200_decode_tile_rows.restype = c_int
     lib.wb200_decode_tile_rows.argtypes = [c_int]
+    lib.wb200_mixed_decode_tile_rows.restype = c_int
+    lib.wb200_mixed_decode_tile_rows.argtypes = [c_int]
     lib.wb200_packed_scale_bytes_tiled.restype = c_size_t
     lib.wb200_packed_scale_bytes_tiled.argtypes = [c_int, c_int, c_int]
     lib.wb200_repack_scales_tiled.restype = c_int

@@ -204,7 +204,7 @@ class ScaledGemmKernel:
             b_sf = b_scale
         else:
             idx = a.device.index if a.device.index is not None else torch.cuda.current_device()
-            b_sf = self._weight_scales.get(self._check_scale(b_scale, N, K, "b_scale"), self._weight_tile_rows(M, N, idx))
+            b_sf = self._weight_scales.get(self._check_scale(b_scale, N, K, "b_scale"), self._weight_tile_rows(M, N, idx, b_fp4))
         fmt = _lib.E5M2 if t.element_format == "f8e5m2" else _lib.E4M3
         flags = self.options.kernel_path | self._raster_flags() | (_lib.ACCUMULATE if t.accumulate else 0)
         ops.scaled_gemm_mxfp8_packed(a, a_sf, b, b_sf, c, fmt, flags, b_fp4=b_fp4, a_scale=rowmajor)
@@ -283,16 +283,16 @@ class ScaledGemmKernel:
             raise ValueError(f"{name} must be [{rows}, {K // ops.SCALE_GROUP_SIZE}], got {tuple(s.shape)}")
         return s
 
-    def _weight_tile_rows(self, M: int, N: int, dev_index: int) -> int:
+    def _weight_tile_rows(self, M: int, N: int, dev_index: int, mixed: bool = False) -> int:
         """Rows per tile the weight scales are packed for: the decode kernel's balanced tile height for M <= 128 (every
         SM gets the same number of weight tiles, `ops.decode_tile_rows`), 128 otherwise. Weights are packed once per
         (weight, height) and cached, so a weight used at both ends of the M range keeps two packings."""
         if M > 128 or not self.options.decode_tiled_weight_scales:
             return 128
-        key = (N, dev_index)
+        key = (N, dev_index, mixed)
         h = self._tile_rows.get(key)
         if h is None:
-            h = self._tile_rows[key] = ops.decode_tile_rows(N, dev_index)
+            h = self._tile_rows[key] = ops.decode_tile_rows(N, dev_index, mixed)
         return h
 
     def drop_cached_weights(self, b_scale: torch.Tensor | None = None) -> None:

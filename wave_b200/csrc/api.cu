@@ -4,6 +4,7 @@
 #include "../../include/wave_b200.h"
 #include "gemm_cluster_splitk_sm100.cuh"
 #include "gemm_sm100.cuh"
+#include "mixed_decode_sm100.cuh"
 #include "moe.cuh"
 #include "multi_gpu.cuh"
 #include "quantize.cuh"
@@ -947,6 +948,67 @@ int dispatch_skinny_experts(const DeviceInfo& dev, const RoutedGemm& g, int T, v
   return launch_skinny_experts<128, 6, Maps>(dev, g, T, c, ldc, hidden, counters, stream);
 }
 
+// Tile height of the mixed (8-bit activations, 4-bit weights) decode kernel with the weights on the MMA's N side: the fewest
+// rounds of at most 208-row tiles that cover N with the same number of tiles on every SM. 0 where that kernel is not
+// used: less than one 128-row tile per SM (the K-split kernel spreads those better), or a height of at most 128, where it
+// multiplies no more weight rows per MMA than the whole-tile kernel.
+int mixed_decode_tile_rows(int sm_count, int N) {
+  if ((N + 127) / 128 < sm_count) return 0;
+  const long long per_round = (long long)sm_count * wb::kMixedTileRowsMax;
+  const long long slots = (N + per_round - 1) / per_round * sm_count;
+  const int h = int(((N + slots - 1) / slots + 7) / 8 * 8);
+  return h > 128 && h <= wb::kMixedTileRowsMax ? h : 0;
+}
+
+template <int NP, typename OutT>
+int launch_mixed_decode(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b, const void* bs,
+                        void* c, long long ldc, int accumulate, cudaStream_t stream, int elem_format) {
+  using Cfg = wb::MixedDecodeCfg<NP>;
+  wb::MixedDecodeMaps maps;
+  const int tile_rows = tl_b_tile_rows, blocks = (tile_rows + 127) / 128, tiles_n = (N + tile_rows - 1) / tile_rows;
+  int rc;
+  if ((rc = make_operand_map_u4(&maps.w, b, N, K, tile_rows))) return rc;
+  if ((rc = make_operand_map(&maps.x, a, M, K, NP))) return rc;
+  if ((rc = make_scale_map(&maps.sfw, bs, tiles_n * blocks, wb::sf_k_atoms(K), blocks, 1))) return rc;
+  if ((rc = make_scale_map(&maps.sfx, as, 1, wb::sf_k_atoms(K), 1, 1))) return rc;
+  wb::MixedDecodeParams p;
+  p.c = c;
+  p.M = M; p.N = N;
+  p.ldc = int(ldc);
+  p.tiles_n = tiles_n;
+  p.tile_rows = tile_rows;
+  p.num_kb = K / 128;
+  p.accumulate = accumulate;
+  p.dependent = tl_dependent_launch ? 1 : 0;
+  p.elem_format = elem_format;
+  p.vec_ok = ((reinterpret_cast<uintptr_t>(c) & 15) == 0 && (ldc * (long long)sizeof(OutT)) % 16 == 0) ? 1 : 0;
+  p.status = dev.status_ptr;
+  auto kernel = wb::mixed_decode_kernel<NP, OutT>;
+  static bool smem_set[kMaxDevices] = {};
+  if ((rc = set_smem(kernel, Cfg::SMEM_BYTES, smem_set))) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(tiles_n < dev.sm_count ? tiles_n : dev.sm_count), 1, 1);
+  cfg.blockDim = dim3(192, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = tl_dependent_launch ? 1 : 0;
+  WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
+  return WB200_OK;
+}
+
+template <typename OutT>
+int dispatch_mixed_decode(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b, const void* bs,
+                          void* c, long long ldc, int accumulate, cudaStream_t s, int elem_format) {
+  if (M <= 16) return launch_mixed_decode<16, OutT>(dev, M, N, K, a, as, b, bs, c, ldc, accumulate, s, elem_format);
+  if (M <= 32) return launch_mixed_decode<32, OutT>(dev, M, N, K, a, as, b, bs, c, ldc, accumulate, s, elem_format);
+  if (M <= 64) return launch_mixed_decode<64, OutT>(dev, M, N, K, a, as, b, bs, c, ldc, accumulate, s, elem_format);
+  return launch_mixed_decode<128, OutT>(dev, M, N, K, a, as, b, bs, c, ldc, accumulate, s, elem_format);
+}
+
 template <typename OutT, int EB = 4>
 int dispatch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
                     const void* bs, void* c, long long ldc, void* ws, int accumulate, cudaStream_t stream,
@@ -1067,7 +1129,16 @@ int wb200_decode_tile_rows(int N) {
   return decode_tile_rows(dev->sm_count, N);
 }
 
-static bool tile_rows_ok(int tile_rows) { return (tile_rows >= 8 && tile_rows <= 128 && tile_rows % 8 == 0) || tile_rows == 224; }
+int wb200_mixed_decode_tile_rows(int N) {
+  DeviceInfo* dev;
+  if (N <= 0 || get_device(&dev)) return 128;
+  const int h = mixed_decode_tile_rows(dev->sm_count, N);
+  return h ? h : decode_tile_rows(dev->sm_count, N);
+}
+
+static bool tile_rows_ok(int tile_rows) {
+  return (tile_rows >= 8 && tile_rows <= wb::kMixedTileRowsMax && tile_rows % 8 == 0) || tile_rows == 224;
+}
 static int tiled_row_blocks(int rows, int tile_rows) { return (rows + tile_rows - 1) / tile_rows * ((tile_rows + 127) / 128); }
 
 size_t wb200_packed_scale_bytes_tiled(int rows, int K, int tile_rows) {
@@ -1104,7 +1175,7 @@ static int repack_scales_impl(const void* src, long long src_row_stride, int row
 
 int wb200_repack_scales_tiled(const void* src, long long src_row_stride, int rows, int K, int tile_rows, void* dst, void* stream) {
   if (!tile_rows_ok(tile_rows))
-    return fail(WB200_ERR_INVALID_ARG, "repack_scales_tiled: %d rows per tile (8 .. 128 in steps of 8, or 224)", tile_rows);
+    return fail(WB200_ERR_INVALID_ARG, "repack_scales_tiled: %d rows per tile (8 .. 208 in steps of 8, or 224)", tile_rows);
   return repack_scales_impl(src, src_row_stride, rows, K, dst, stream, false, tile_rows);
 }
 
@@ -1579,8 +1650,10 @@ int wb200_mxfp8_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
     explicit TileRowsScope(int h) : saved(tl_b_tile_rows) { tl_b_tile_rows = h; }
     ~TileRowsScope() { tl_b_tile_rows = saved; }
   } tile_rows_scope(b_tile_rows_from_flags(flags));
-  if (tl_b_tile_rows > 128)
-    return fail(WB200_ERR_UNSUPPORTED, "mxfp8_gemm: weight scales packed per %d-row tile (the 8-bit GEMM reads heights of 8 .. 128 on its M <= 128 path)", tl_b_tile_rows);
+  const bool wide_mixed = tl_b_tile_rows > 128 && tl_b_tile_rows <= wb::kMixedTileRowsMax && (elem_format & WB200_B_FP4);
+  if (tl_b_tile_rows > 128 && !wide_mixed)
+    return fail(WB200_ERR_UNSUPPORTED, "mxfp8_gemm: weight scales packed per %d-row tile (the 8-bit GEMM reads heights of 8 .. 128, with "
+                "4-bit weights up to %d, on its M <= 128 path)", tl_b_tile_rows, wb::kMixedTileRowsMax);
   struct DependentScope {  // restores the previous value on every return path
     bool saved;
     explicit DependentScope(bool on) : saved(tl_dependent_launch) { if (on) tl_dependent_launch = true; }
@@ -1606,6 +1679,11 @@ int wb200_mxfp8_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
     if (!ws_ok)
       return fail(WB200_ERR_WORKSPACE, "the skinny path needs a 16-byte aligned workspace of %zu bytes (got %zu)",
                   skinny_workspace_bytes(dev->sm_count, M), workspace ? workspace_bytes : size_t(0));
+    if (wide_mixed) {
+      if (c_dtype == WB200_F32)
+        return dispatch_mixed_decode<float>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, accumulate, s, elem_format);
+      return dispatch_mixed_decode<__nv_bfloat16>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, accumulate, s, elem_format);
+    }
     if (c_dtype == WB200_F32)
       return dispatch_skinny<float, 8>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, workspace, accumulate, s, elem_format);
     return dispatch_skinny<__nv_bfloat16, 8>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, workspace, accumulate, s, elem_format);

@@ -50,14 +50,15 @@ def packed_scale_bytes(rows: int, K: int) -> int:
     return int(_lib.load().wb200_packed_scale_bytes(rows, K))
 
 
-def decode_tile_rows(N: int, device=None) -> int:
+def decode_tile_rows(N: int, device=None, mixed: bool = False) -> int:
     """Tile height of the M <= 128 kernel for which every SM of `device` gets the same number of weight tiles (a multiple
-    of 8, at most 128; 128 when the usual packing is as good). Pack a weight's scales with it to use it."""
-    lib = _lib.load()
+    of 8, at most 128; 128 when the usual packing is as good). Pack a weight's scales with it to use it. mixed: for 8-bit
+    activations with 4-bit weights, where heights up to 208 are read too."""
+    fn = _lib.load().wb200_mixed_decode_tile_rows if mixed else _lib.load().wb200_decode_tile_rows
     if device is None:
-        return int(lib.wb200_decode_tile_rows(int(N)))
+        return int(fn(int(N)))
     with torch.cuda.device(device):
-        return int(lib.wb200_decode_tile_rows(int(N)))
+        return int(fn(int(N)))
 
 
 def repack_scales(scale: torch.Tensor, out: torch.Tensor | None = None, tile_rows: int = 128) -> PackedScales:
@@ -311,8 +312,9 @@ def scaled_gemm_mxfp8_packed(a: torch.Tensor, a_sf: PackedScales, b: torch.Tenso
             raise ValueError(f"{name} must be a contiguous 2-D CUDA tensor of 8-bit elements")
     M, K = a.shape
     N = b.shape[0]
-    if a_sf.tile_rows != 128 or b_sf.tile_rows > 128 or (b_sf.tile_rows != 128 and M > 128):
-        raise ValueError("the 8-bit GEMM reads per-tile weight scales (tile_rows < 128) on its M <= 128 path only")
+    if a_sf.tile_rows != 128 or b_sf.tile_rows > (208 if b_fp4 else 128) or (b_sf.tile_rows != 128 and M > 128):
+        raise ValueError("the 8-bit GEMM reads per-tile weight scales (tile_rows < 128, with 4-bit weights up to 208) on its "
+                         "M <= 128 path only")
     if b_sf.tile_rows != 128:
         flags |= _lib.B_TILE_ROWS(b_sf.tile_rows)
     if b_fp4:
