@@ -359,6 +359,6 @@ def test_mixed_decode_with_weights_on_the_n_side(M, N, K, out_dtype):
     if ref is not None:
         assert torch.equal(wide[:, :N], ref)
     assert bool((wide[:, N:] == 1).all())
-    with pytest.raises(RuntimeError):  # no MXFP4 kernel reads this packing
+    with pytest.raises(ValueError):  # no MXFP4 kernel reads this packing
         ops.scaled_gemm_packed(bd[:M], ops.repack_scales(b_s[:M].to(DEV)), bd, b_sf, torch.empty(M, N, dtype=out_dtype, device=DEV))
     ops.check_device_status()

@@ -76,7 +76,7 @@ def repack_scales(scale: torch.Tensor, out: torch.Tensor | None = None, tile_row
     tiled = tile_rows != 128
     nbytes = int(lib.wb200_packed_scale_bytes_tiled(rows, K, tile_rows)) if tiled else packed_scale_bytes(rows, K)
     if tiled and nbytes == 0:
-        raise ValueError(f"repack_scales: {tile_rows} rows per tile (8 .. 128 in steps of 8)")
+        raise ValueError(f"repack_scales: {tile_rows} rows per tile (8 .. 208 in steps of 8, or 224)")
     if out is None:
         out = torch.empty(nbytes, dtype=torch.uint8, device=scale.device)
     elif out.numel() < nbytes or out.dtype != torch.uint8 or not out.is_contiguous():
