@@ -7,6 +7,8 @@
 // row from memory but takes the MMAs of 128 (the 8-bit containers), and with the loads left out the kernel ran no faster:
 // 34.8 of 34.2 us at M = 16, N = 28672, K = 8192. Here the activations take the lanes (M of 128 are real) and up to 208 weight
 // rows the columns: half the MMAs per weight row. The activation tile is also fetched half as often.
+// N = 28672, K = 8192 (117 MB of weights), per launch: M = 1 / 16 / 64 / 128: 34.2 / 34.2 / 36.9 / 40.2 -> 25.2 / 25.6 / 27.7 /
+// 30.9 us; what remains is the rate at which the copy engine expands (26.7 us with the MMAs left out before).
 //   * one CTA per SM walks tiles blockIdx.x, + gridDim.x, ..: the tile height is chosen on the host so that every SM gets the
 //     same number of tiles (wb200_mixed_decode_tile_rows);
 //   * a tile of more than 128 rows has two rows of scale atoms (rows 0 .. 127 and 128 .. of the tile);
