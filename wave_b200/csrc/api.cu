@@ -144,6 +144,24 @@ static int b_tile_rows_from_flags(unsigned flags) {
   const unsigned h8 = (flags & WB200_B_TILE_ROWS_MASK) >> WB200_B_TILE_ROWS_SHIFT;
   return h8 == 0 ? 128 : int(h8) * 8;
 }
+// Row-major activation scales of the call in progress (wb200_mxfp4_gemm_repack_a): kernels that have a scale warp take them
+// as they are, for the others the launcher packs them into the caller's scratch first (pack_row_scales).
+struct PendingRowScales {
+  const void* src = nullptr;
+  long long stride = 0;
+  void* scratch = nullptr;
+};
+static thread_local PendingRowScales tl_row_scales;
+static int pack_row_scales(int M, int K, cudaStream_t stream);
+static wb::RowScales row_scales_param(int M, int K) {
+  wb::RowScales s;
+  s.base = static_cast<const uint8_t*>(tl_row_scales.src);
+  s.stride = tl_row_scales.stride;
+  s.rows = M;
+  s.kblocks = K / 32;
+  s.vec = ((reinterpret_cast<uintptr_t>(s.base) & 7) == 0 && s.stride % 8 == 0) ? 1 : 0;
+  return s;
+}
 struct GroupNScope {  // restores the previous value on every return path
   int saved;
   explicit GroupNScope(unsigned flags) : saved(tl_group_n) { tl_group_n = group_n_from_flags(flags); }
@@ -255,12 +273,12 @@ int make_output_map_dense(CUtensorMap* map, void* c, int M, int N, long long ldc
 }
 
 // EB: bits per operand element (4: MXFP4, 8: MXFP8 with elem_format 0 = E4M3 / 1 = E5M2).
-template <int CG, int BN, typename OutT, int EB = 4>
-int launch_tile(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
+template <int CG, int BN, typename OutT, int EB, typename Maps>
+int launch_tile_maps(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
                 const void* bs, void* c, long long ldc, int sfa_row_blocks, int sfb_row_blocks, int accumulate,
-                cudaStream_t stream, int elem_format = 0) {
+                cudaStream_t stream, int elem_format) {
   using Cfg = wb::GemmCfg<CG, BN, int(sizeof(OutT)), EB>;
-  wb::PlainMaps maps;
+  Maps maps;
   CUtensorMap& tmA = maps.m[0];
   CUtensorMap& tmC = maps.m[4];
   const long long row_bytes = (long long)K * EB / 8;
@@ -269,8 +287,13 @@ int launch_tile(const DeviceInfo& dev, int M, int N, int K, const void* a, const
   rc = weights_are_fp4(EB, elem_format) ? make_operand_map_u4(&maps.m[1], b, N, K, Cfg::B_ROWS)
                                         : make_operand_map(&maps.m[1], b, N, row_bytes, Cfg::B_ROWS);
   if (rc) return rc;
-  rc = make_scale_map(&maps.m[2], as, sfa_row_blocks, wb::sf_k_atoms(K), 1, Cfg::SF_ATOMS);
-  if (rc) return rc;
+  if constexpr (Maps::kRowScales) {
+    maps.a_scales = row_scales_param(M, K);
+    maps.m[2] = maps.m[0];  // not used
+  } else {
+    rc = make_scale_map(&maps.m[2], as, sfa_row_blocks, wb::sf_k_atoms(K), 1, Cfg::SF_ATOMS);
+    if (rc) return rc;
+  }
   rc = make_scale_map(&maps.m[3], bs, sfb_row_blocks, wb::sf_k_atoms(K), Cfg::SFB_BLOCKS, Cfg::SF_ATOMS);
   if (rc) return rc;
   wb::GemmParams p;
@@ -292,7 +315,7 @@ int launch_tile(const DeviceInfo& dev, int M, int N, int K, const void* a, const
     tmC = tmA;  // never dereferenced by the kernel on the direct-store path
   }
   p.status = dev.status_ptr;
-  auto kernel = wb::mxfp4_gemm_kernel<CG, BN, OutT, wb::PlainMaps, EB>;
+  auto kernel = wb::mxfp4_gemm_kernel<CG, BN, OutT, Maps, EB>;
   static bool smem_set[kMaxDevices] = {};
   rc = set_smem(kernel, Cfg::SMEM_BYTES, smem_set);
   if (rc) return rc;
@@ -301,7 +324,7 @@ int launch_tile(const DeviceInfo& dev, int M, int N, int K, const void* a, const
   const int grid = int(tiles < units ? tiles : units) * CG;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
+  cfg.blockDim = dim3(Cfg::THREADS + (Maps::kRowScales ? 32 : 0), 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -315,6 +338,20 @@ int launch_tile(const DeviceInfo& dev, int M, int N, int K, const void* a, const
   cfg.numAttrs = tl_dependent_launch ? 2 : 1;
   WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   return WB200_OK;
+}
+
+template <int CG, int BN, typename OutT, int EB = 4>
+int launch_tile(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
+                const void* bs, void* c, long long ldc, int sfa_row_blocks, int sfb_row_blocks, int accumulate,
+                cudaStream_t stream, int elem_format = 0) {
+  if constexpr (EB == 4 && CG == 2 && BN != 224) {
+    if (tl_row_scales.src)
+      return launch_tile_maps<CG, BN, OutT, EB, wb::RowScaleMaps>(dev, M, N, K, a, as, b, bs, c, ldc, sfa_row_blocks, sfb_row_blocks, accumulate,
+                                                                  stream, elem_format);
+  }
+  if (int rc = pack_row_scales(M, K, stream)) return rc;
+  return launch_tile_maps<CG, BN, OutT, EB, wb::PlainMaps>(dev, M, N, K, a, as, b, bs, c, ldc, sfa_row_blocks, sfb_row_blocks, accumulate, stream,
+                                                           elem_format);
 }
 
 template <int CG, int BN>
@@ -557,6 +594,7 @@ int launch_splitk(const DeviceInfo& dev, int slices, int M, int N, int K, const 
                   const void* bs, void* c, long long ldc, void* workspace, int accumulate, cudaStream_t stream) {
   constexpr int CG = 2, BN = 256;
   using Cfg = wb::GemmCfg<CG, BN, 4>;
+  if (int rc = pack_row_scales(M, K, stream)) return rc;
   static wb::GroupedMaps maps;
   static std::mutex mu;
   std::lock_guard<std::mutex> lk(mu);
@@ -701,6 +739,7 @@ int launch_cluster_splitk(const DeviceInfo& dev, int slices, int M, int N, int K
   using Cfg = wb::GemmCfg<2, BN, int(sizeof(OutT))>;
   wb::PlainMaps maps;
   int rc;
+  if ((rc = pack_row_scales(M, K, stream))) return rc;
   if ((rc = make_operand_map(&maps.m[0], a, M, K / 2, Cfg::BM))) return rc;
   if ((rc = make_operand_map(&maps.m[1], b, N, K / 2, Cfg::B_ROWS))) return rc;
   if ((rc = make_scale_map(&maps.m[2], as, wb::sf_row_blocks(M), wb::sf_k_atoms(K), 1))) return rc;
@@ -742,10 +781,10 @@ size_t skinny_workspace_bytes(int sm_count, int M) {
   return kCounterBytes + size_t(2) * sm_count * M * 128 * sizeof(float);
 }
 
-template <int NP, int STAGES, typename OutT, int EB = 4>
-int launch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
+template <int NP, int STAGES, typename OutT, int EB, bool RS>
+int launch_skinny_scales(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
                   const void* bs, void* c, long long ldc, void* ws, int accumulate, cudaStream_t stream,
-                  int elem_format = 0) {
+                  int elem_format) {
   using Cfg = wb::SkinnyCfg<NP, STAGES, EB>;
   CUtensorMap tmW, tmX, tmSFW, tmSFX;
   const long long row_bytes = (long long)K * EB / 8;
@@ -755,9 +794,15 @@ int launch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, con
   if (rc) return rc;
   rc = make_scale_map(&tmSFW, bs, wb::sf_row_blocks(N), wb::sf_k_atoms(K), 1, Cfg::SF_ATOMS);
   if (rc) return rc;
-  rc = make_scale_map(&tmSFX, as, 1, wb::sf_k_atoms(K), 1, Cfg::SF_ATOMS);
-  if (rc) return rc;
   wb::SkinnyParams p;
+  if constexpr (RS) {
+    p.x_scales = row_scales_param(M, K);
+    tmSFX = tmX;  // not used
+  } else {
+    rc = make_scale_map(&tmSFX, as, 1, wb::sf_k_atoms(K), 1, Cfg::SF_ATOMS);
+    if (rc) return rc;
+    p.x_scales = {};
+  }
   p.c = c;
   p.counters = static_cast<unsigned int*>(ws);
   p.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + kCounterBytes);
@@ -769,7 +814,7 @@ int launch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, con
   p.dependent = tl_dependent_launch ? 1 : 0;
   p.elem_format = elem_format;
   p.status = dev.status_ptr;
-  auto kernel = wb::mxfp4_skinny_kernel<NP, STAGES, OutT, EB>;
+  auto kernel = wb::mxfp4_skinny_kernel<NP, STAGES, OutT, EB, RS>;
   static bool smem_set[kMaxDevices] = {};
   rc = set_smem(kernel, Cfg::SMEM_BYTES, smem_set);
   if (rc) return rc;
@@ -777,7 +822,7 @@ int launch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, con
   const int grid = int(units < dev.sm_count ? units : dev.sm_count);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(192, 1, 1);
+  cfg.blockDim = dim3(RS ? 224 : 192, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -788,6 +833,16 @@ int launch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, con
   WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, tmW, tmX, tmSFW, tmSFX, p));
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
+}
+
+template <int NP, int STAGES, typename OutT, int EB = 4>
+int launch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
+                  const void* bs, void* c, long long ldc, void* ws, int accumulate, cudaStream_t stream, int elem_format = 0) {
+  if constexpr (EB == 4) {
+    if (tl_row_scales.src)
+      return launch_skinny_scales<NP, STAGES, OutT, EB, true>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
+  }
+  return launch_skinny_scales<NP, STAGES, OutT, EB, false>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
 }
 
 // Whole N tiles taken from an atomic counter instead of a K split (skinny_whole_sm100.cuh), when there is at least one
@@ -820,13 +875,13 @@ int decode_tile_rows(int sm_count, int N) {
   return (h >= 88 && h < 128) ? h : 128;
 }
 
-template <int NP, int STAGES, typename OutT, int EB = 4, int WR = 128, int SBUFS = 2>
-int launch_skinny_whole(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
+template <int NP, int STAGES, typename OutT, int EB, int WR, int SBUFS, typename Maps>
+int launch_skinny_whole_maps(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
                         const void* bs, void* c, long long ldc, void* ws, int accumulate, cudaStream_t stream,
-                        int elem_format = 0) {
+                        int elem_format) {
   using Base = wb::SkinnyCfg<NP, STAGES, EB, WR>;
   using Cfg = wb::SkinnyWholeCfg<NP, STAGES, EB, WR, SBUFS>;
-  wb::SkinnyMaps maps = {};
+  Maps maps = {};
   const long long row_bytes = (long long)K * EB / 8;
   const int tile_rows = tl_b_tile_rows;  // 128 with the usual packing of the weight scales
   const int tiles_n = (N + tile_rows - 1) / tile_rows;
@@ -836,8 +891,13 @@ int launch_skinny_whole(const DeviceInfo& dev, int M, int N, int K, const void* 
   if (rc) return rc;
   rc = make_scale_map(&maps.sfw, bs, tiles_n, wb::sf_k_atoms(K), 1, Base::SF_ATOMS);
   if (rc) return rc;
-  rc = make_scale_map(&maps.sfx, as, 1, wb::sf_k_atoms(K), 1, Base::SF_ATOMS);
-  if (rc) return rc;
+  if constexpr (Maps::kRowScales) {
+    maps.x_scales = row_scales_param(M, K);
+    maps.sfx = maps.x;  // not used
+  } else {
+    rc = make_scale_map(&maps.sfx, as, 1, wb::sf_k_atoms(K), 1, Base::SF_ATOMS);
+    if (rc) return rc;
+  }
   wb::SkinnyWholeParams p;
   p.c = c;
   p.counters = static_cast<unsigned int*>(ws);
@@ -858,13 +918,13 @@ int launch_skinny_whole(const DeviceInfo& dev, int M, int N, int K, const void* 
     if (rc) return rc;
   }
   p.status = dev.status_ptr;
-  auto kernel = wb::mxfp4_skinny_whole_kernel<NP, STAGES, OutT, EB, WR, SBUFS>;
+  auto kernel = wb::mxfp4_skinny_whole_kernel<NP, STAGES, OutT, EB, WR, SBUFS, Maps>;
   static bool smem_set[kMaxDevices] = {};
   rc = set_smem(kernel, Cfg::SMEM_BYTES, smem_set);
   if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(dev.sm_count, 1, 1);  // one CTA per SM; every CTA's first tile is its own index (tiles >= SMs)
-  cfg.blockDim = dim3(192, 1, 1);
+  cfg.blockDim = dim3(Maps::kRowScales ? 224 : 192, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -875,6 +935,18 @@ int launch_skinny_whole(const DeviceInfo& dev, int M, int N, int K, const void* 
   WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
+}
+
+template <int NP, int STAGES, typename OutT, int EB = 4, int WR = 128, int SBUFS = 2>
+int launch_skinny_whole(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
+                        const void* bs, void* c, long long ldc, void* ws, int accumulate, cudaStream_t stream, int elem_format = 0) {
+  if constexpr (EB == 4) {
+    if (tl_row_scales.src)
+      return launch_skinny_whole_maps<NP, STAGES, OutT, EB, WR, SBUFS, wb::SkinnyRowScaleMaps>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate,
+                                                                                               stream, elem_format);
+  }
+  return launch_skinny_whole_maps<NP, STAGES, OutT, EB, WR, SBUFS, wb::SkinnyMaps>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream,
+                                                                                   elem_format);
 }
 
 // The tiles of all experts of a decode step in one launch (SkinnyExpertMaps). T: tokens = rows of a block that can be real.
@@ -1146,16 +1218,22 @@ size_t wb200_packed_scale_bytes_tiled(int rows, int K, int tile_rows) {
   return size_t(tiled_row_blocks(rows, tile_rows)) * wb::sf_k_atoms(K) * 512;
 }
 
-static int repack_scales_impl(const void* src, long long src_row_stride, int rows, int K, void* dst, void* stream,
-                              bool broadcast, int block_rows = 128) {
+static int check_repack(const void* src, long long src_row_stride, int rows, int K, const void* dst, bool broadcast) {
   if (rows <= 0 || K <= 0 || K % 32 != 0)
     return fail(WB200_ERR_INVALID_ARG, "repack_scales: rows = %d, K = %d (K must be a positive multiple of 32)", rows, K);
   if (!src || !dst) return fail(WB200_ERR_INVALID_ARG, "repack_scales: null pointer");
   if (src_row_stride < (broadcast ? 1 : K / 32))
     return fail(WB200_ERR_INVALID_ARG, "repack_scales: row stride %lld < %d", src_row_stride, broadcast ? 1 : K / 32);
   if (reinterpret_cast<uintptr_t>(dst) & 15) return fail(WB200_ERR_ALIGNMENT, "repack_scales: dst must be 16-byte aligned");
+  return WB200_OK;
+}
+
+static int repack_scales_impl(const void* src, long long src_row_stride, int rows, int K, void* dst, void* stream,
+                              bool broadcast, int block_rows = 128) {
+  int rc = check_repack(src, src_row_stride, rows, K, dst, broadcast);
+  if (rc) return rc;
   DeviceInfo* dev;
-  int rc = get_device(&dev);
+  rc = get_device(&dev);
   if (rc) return rc;
   const int k_atoms = wb::sf_k_atoms(K);
   dim3 grid((k_atoms + 7) / 8, tiled_row_blocks(rows, block_rows));
@@ -1171,6 +1249,21 @@ static int repack_scales_impl(const void* src, long long src_row_stride, int row
   WB_CUDA(cudaLaunchKernelEx(&cfg, wb::repack_scales_kernel, static_cast<const uint8_t*>(src), src_row_stride, rows, K / 32,
                              k_atoms, static_cast<uint8_t*>(dst), broadcast, tl_dependent_launch, block_rows));
   return WB200_OK;
+}
+
+extern "C++" {
+namespace {
+// Packs the row-major scales of the call in progress, if there are any, into its scratch; the kernel launched next is the
+// repack kernel's programmatic dependent.
+int pack_row_scales(int M, int K, cudaStream_t stream) {
+  if (!tl_row_scales.src) return WB200_OK;
+  const PendingRowScales s = tl_row_scales;
+  tl_row_scales = {};
+  int rc = repack_scales_impl(s.src, s.stride, M, K, s.scratch, stream, false);
+  if (rc == WB200_OK) tl_dependent_launch = true;
+  return rc;
+}
+}  // namespace
 }
 
 int wb200_repack_scales_tiled(const void* src, long long src_row_stride, int rows, int K, int tile_rows, void* dst, void* stream) {
@@ -1597,14 +1690,13 @@ int wb200_mxfp4_gemm_repack_a(int M, int N, int K, const void* a, const void* a_
                               void* a_scale_scratch, const void* b, const void* b_scale_packed, void* c, int c_dtype,
                               long long ldc, void* workspace, size_t workspace_bytes, unsigned flags, void* stream) {
   if (!a_scale_scratch) return fail(WB200_ERR_INVALID_ARG, "gemm_repack_a: null scratch for the packed activation scales");
-  tl_dependent_launch = (flags & WB200_OVERLAP_PREVIOUS) != 0;  // the repack kernel itself overlaps the previous kernel's tail
-  int rc = wb200_repack_scales(a_scale, a_scale_stride, M, K, a_scale_scratch, stream);
-  tl_dependent_launch = false;
+  int rc = check_repack(a_scale, a_scale_stride, M, K, a_scale_scratch, false);
   if (rc) return rc;
-  tl_dependent_launch = true;  // the GEMM is the repack kernel's programmatic dependent
-  rc = wb200_mxfp4_gemm(M, N, K, a, a_scale_scratch, b, b_scale_packed, c, c_dtype, ldc, workspace, workspace_bytes, flags, stream);
-  tl_dependent_launch = false;
-  return rc;
+  struct PendingScope {  // restores the previous state on every return path
+    PendingScope(const void* src, long long stride, void* scratch) { tl_row_scales = {src, stride, scratch}; }
+    ~PendingScope() { tl_row_scales = {}; tl_dependent_launch = false; }
+  } pending(a_scale, a_scale_stride, a_scale_scratch);
+  return wb200_mxfp4_gemm(M, N, K, a, a_scale_scratch, b, b_scale_packed, c, c_dtype, ldc, workspace, workspace_bytes, flags, stream);
 }
 
 int wb200_mxfp4_gemm_quantize_a(int M, int N, int K, const void* x, int x_dtype, long long ldx, void* q_scratch, void* scale_scratch,

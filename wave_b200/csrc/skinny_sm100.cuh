@@ -19,6 +19,7 @@
 //     published skips the write of its own. Nobody spins on another CTA.
 #pragma once
 #include "ptx.cuh"
+#include "row_scales.cuh"
 #include <cuda_bf16.h>
 
 namespace wb {
@@ -86,6 +87,7 @@ struct SkinnyParams {
   int accumulate;  // add to the values already in C instead of overwriting them
   int dependent;   // launched as the programmatic dependent of the kernel that writes the activations' packed scales
   int elem_format; // 8-bit operands only: 0 = E4M3, 1 = E5M2
+  RowScales x_scales;
   int* status;
 };
 
@@ -105,8 +107,9 @@ __device__ __forceinline__ int skinny_owner(long long total, int g, int u) {
   return c;
 }
 
-template <int NP, int STAGES, typename OutT, int EB = 4>
-__global__ void __launch_bounds__(192, 1)
+// RS: the activations' scales are p.x_scales, row-major, brought into the stages by a seventh warp (row_scales.cuh).
+template <int NP, int STAGES, typename OutT, int EB = 4, bool RS = false>
+__global__ void __launch_bounds__(RS ? 224 : 192, 1)
 mxfp4_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                     const __grid_constant__ CUtensorMap tmSFW, const __grid_constant__ CUtensorMap tmSFX,
                     const SkinnyParams p) {
@@ -134,7 +137,7 @@ mxfp4_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full_bar(s), 1);
+      mbar_init(full_bar(s), RS ? 2 : 1);
       mbar_init(empty_bar(s), 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -183,14 +186,14 @@ mxfp4_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       const uint32_t fb = full_bar(p_stage);
       if (elect_one()) {
         // 4-bit weights expanded by the copy engine (EB == 8 only) count with their packed size
-        if (part != 1) mbar_expect_tx(fb, Cfg::STAGE_BYTES - ((EB == 8 && (p.elem_format & 0x10)) ? Cfg::W_BYTES / 2 : 0));
+        if (part != 1) mbar_expect_tx(fb, Cfg::STAGE_BYTES - (RS ? Cfg::SF_BYTES : 0) - ((EB == 8 && (p.elem_format & 0x10)) ? Cfg::W_BYTES / 2 : 0));
         if (part != 2) {
           tma_load_2d_hint(sW, &tmW, p_kb * 128, p_tile * 128, fb, stream_policy);
           tma_load_2d(sSFW, &tmSFW, p_kb * (Cfg::SF_ATOMS * 128), p_tile, fb);
         }
         if (part != 1) {
           tma_load_2d_hint(sX, &tmX, p_kb * 128, 0, fb, keep_policy);
-          tma_load_2d(sSFX, &tmSFX, p_kb * (Cfg::SF_ATOMS * 128), 0, fb);
+          if constexpr (!RS) tma_load_2d(sSFX, &tmSFX, p_kb * (Cfg::SF_ATOMS * 128), 0, fb);
         }
       }
       __syncwarp();
@@ -289,6 +292,22 @@ mxfp4_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+    }
+  } else if (RS && warp == 6) {
+    // ------------------------------------------------------------------ the activations' scales, row-major, into the stages
+    if constexpr (RS) {
+      static_assert(EB == 4, "a stage of 256 K");
+      if (p.dependent) pdl_wait();
+      uint32_t stage = 0, phase = 0;
+      for (int seg = 0; seg < nseg; ++seg) {
+        int tile, kbs, kbe;
+        segment(seg, tile, kbs, kbe);
+        feed_row_scales<(NP + 31) / 32, STAGES>(
+            p.x_scales, 0, lane, kbs, kbe, stage, phase,
+            [&](uint32_t st) { return smem_base + st * Cfg::STAGE_BYTES + Cfg::W_BYTES + Cfg::X_BYTES + Cfg::SF_BYTES; },
+            [&](uint32_t st, uint32_t ph) { mbar_wait(empty_bar(st), ph ^ 1u, ctx, WB_DEV_TIMEOUT_PRODUCER); },
+            [&](uint32_t st) { mbar_arrive(full_bar(st)); });
       }
     }
   } else {

@@ -64,10 +64,15 @@ struct SkinnyWholeParams {
 
 // The tensor maps of a launch over one weight.
 struct SkinnyMaps {
-  static constexpr bool kExperts = false, kSilu = false;
+  static constexpr bool kExperts = false, kSilu = false, kRowScales = false;
   CUtensorMap w, sfw;  // weights and their packed scales
   CUtensorMap x, sfx;  // activations and their packed scales
   CUtensorMap c;
+};
+// The same with the activations' scales row-major (sfx is not used): a seventh warp brings them into the stages.
+struct SkinnyRowScaleMaps : SkinnyMaps {
+  static constexpr bool kRowScales = true;
+  RowScales x_scales;
 };
 // A decode step of a mixture-of-experts layer (at most 128 tokens, so at most 128 rows per expert): the tiles of every
 // expert that received tokens, in one launch. x holds one block of 128 rows per such expert (moe_align_block_size with
@@ -80,7 +85,7 @@ struct SkinnyMaps {
 // quantised: codes q [rows, inter / 2] and packed scales. inter % 64 == 0.
 template <int G, bool SILU>
 struct SkinnyExpertMaps {
-  static constexpr bool kExperts = true, kSilu = SILU;
+  static constexpr bool kExperts = true, kSilu = SILU, kRowScales = false;
   CUtensorMap w[G], sfw[G];
   CUtensorMap x, sfx;
   CUtensorMap c;
@@ -96,7 +101,7 @@ struct SkinnyExpertMaps {
 constexpr int kExpertBlockRows = 128;
 
 template <int NP, int STAGES, typename OutT, int EB = 4, int WR = 128, int SBUFS = 2, typename Maps = SkinnyMaps>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(Maps::kRowScales ? 224 : 192, 1)
 mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholeParams p) {
   using Base = SkinnyCfg<NP, STAGES, EB, WR>;
   using Cfg = SkinnyWholeCfg<NP, STAGES, EB, WR, SBUFS>;
@@ -110,7 +115,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
 #ifdef WB200_TRACE
   if (threadIdx.x == 0) WB_TRACE_SET(0, trace_now());  // timeline marks as in skinny_sm100.cuh; a "segment" is a tile here
 #endif
-  if (warp == 0 && lane < 4) {  // the copy engine fetches a descriptor on first use: start that now
+  if (warp == 0 && lane < (Maps::kRowScales ? 3 : 4)) {  // the copy engine fetches a descriptor on first use: start that now
     if constexpr (Maps::kExperts) prefetch_tensormap((lane & 1) ? &maps.sfx : &maps.x);
     else prefetch_tensormap(lane == 0 ? &maps.w : lane == 1 ? &maps.sfw : lane == 2 ? &maps.x : &maps.sfx);
   }
@@ -136,7 +141,8 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
       uint32_t count = 1;                                  // full / empty stage, accumulator full, tile number written
       const int q = b - 2 * STAGES;
       if (q >= 2 && q < 4) count = 4;                       // accumulator drained: one arrival per epilogue warp
-      else if (q >= 4 + IQ && q < 4 + 2 * IQ) count = 5;    // tile number read by the MMA warp and the four epilogue warps
+      else if (q >= 4 + IQ && q < 4 + 2 * IQ) count = 5 + (Maps::kRowScales ? 1 : 0);  // tile number read by the MMA, epilogue and scale warps
+      else if (Maps::kRowScales && b < STAGES) count = 2;   // a stage's loads, and its activation scales
       mbar_init(bar_base + 8u * b, count);
     }
     if (lane == 0) *abort_flag = 0u;
@@ -189,7 +195,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
       // and the epilogue keeps the tile's own columns
       // (4-bit weights expanded by the copy engine, EB == 8 only, count with their packed size: 64 bytes per row)
       if (part != 1)
-        mbar_expect_tx(fb, Cfg::STAGE_BYTES - Base::W_BYTES + uint32_t(p.tile_rows) * ((EB == 8 && (p.elem_format & 0x10)) ? 64u : 128u));
+        mbar_expect_tx(fb, Cfg::STAGE_BYTES - Base::W_BYTES - (Maps::kRowScales ? Base::SF_BYTES : 0) + uint32_t(p.tile_rows) * ((EB == 8 && (p.elem_format & 0x10)) ? 64u : 128u));
       if (part != 2) {
         if constexpr (Maps::kSilu) {
           tma_load_2d_hint(sW, tm_w, kb * 128, w_tile * 64, fb, stream_policy);
@@ -201,7 +207,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
       }
       if (part != 1) {
         tma_load_2d_hint(sX, &maps.x, kb * 128, block * kExpertBlockRows, fb, keep_policy);
-        tma_load_2d(sSFX, &maps.sfx, kb * (Base::SF_ATOMS * 128), block, fb);
+        if constexpr (!Maps::kRowScales) tma_load_2d(sSFX, &maps.sfx, kb * (Base::SF_ATOMS * 128), block, fb);
       }
     }
     __syncwarp();
@@ -336,6 +342,21 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+    }
+  } else if (Maps::kRowScales && warp == 6) {
+    // ------------------------------------------------------------------ the activations' scales, row-major, into the stages
+    if constexpr (Maps::kRowScales) {
+      static_assert(EB == 4, "a stage of 256 K");
+      if (p.dependent) pdl_wait();
+      uint32_t stage = 0, phase = 0;
+      for (int seq = 0;; ++seq) {
+        if (next_tile(seq) < 0) break;
+        feed_row_scales<(NP + 31) / 32, STAGES>(
+            maps.x_scales, 0, lane, 0, p.num_kb, stage, phase,
+            [&](uint32_t st) { return smem_base + st * Cfg::STAGE_BYTES + Base::W_BYTES + Base::X_BYTES + Base::SF_BYTES; },
+            [&](uint32_t st, uint32_t ph) { mbar_wait(empty_bar(st), ph ^ 1u, ctx, WB_DEV_TIMEOUT_PRODUCER); },
+            [&](uint32_t st) { mbar_arrive(full_bar(st)); });
       }
     }
   } else {
