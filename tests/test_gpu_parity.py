@@ -1101,3 +1101,27 @@ def test_split_k_inside_a_cluster(shape, out_dtype):
         tol = orc.f32_tolerance(orc.dequant_mxfp4(a, a_s), orc.dequant_mxfp4(b, b_s), ref, K)
         assert bool(((acc.cpu() - (ref + base)).abs() <= tol + 1e-6 * base.abs()).all())
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 640, 992), (16, 28672, 256), (33, 1000, 1184), (64, 19072, 288), (100, 28672 - 40, 512), (128, 4096, 2080),
+                                   (129, 512, 32), (300, 700, 1184), (1000, 384, 4128), (2048, 4096, 512), (2050, 8192, 288)])
+@pytest.mark.parametrize("offset,extra", [(0, 0), (8, 8), (3, 5)])
+def test_row_major_activation_scales_give_the_bits_of_packed_ones(M, N, K, offset, extra):
+    """The call that takes a_scale row-major (a warp of the GEMM brings it into the stages) against the same GEMM on scales packed
+    beforehand, for every kernel that has that warp: K blocks that end inside a stage, rows that end inside a tile, several
+    tiles per CTA, row pitches and bases that allow 8-byte loads and that do not."""
+    a, a_s, b, b_s = random_problem(M, N, K, seed=M + N + K + offset)
+    wide = torch.full((M, offset + K // 32 + extra), 255, dtype=torch.uint8, device=DEV)
+    view = wide[:, offset:offset + K // 32]
+    view.copy_(a_s.to(DEV))
+    kernel, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    gemm = wb.wave_compile(options, kernel)
+    ad, bd, bsd = a.to(DEV), b.to(DEV), b_s.to(DEV)
+    c = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    gemm(ad, view, bd, bsd, c)
+    ref = torch.full_like(c, float("nan"))
+    h = ops.decode_tile_rows(N) if M <= 128 else 128
+    ops.scaled_gemm_packed(ad, ops.repack_scales(a_s.to(DEV)), bd, ops.repack_scales(bsd, tile_rows=h), ref)
+    assert torch.equal(c.view(torch.int16), ref.view(torch.int16))
+    check(c, a, a_s, b, b_s)
+    ops.check_device_status()

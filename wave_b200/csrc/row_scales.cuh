@@ -20,13 +20,18 @@ struct RowScales {
   int vec;              // base and stride are multiples of 8: whole 8-byte loads
 };
 
-// The scales of K blocks 8 kb .. 8 kb + 7 of one row; the padding byte outside the matrix.
+// The scales of K blocks 8 kb .. 8 kb + 7 of one row; the padding byte outside the matrix. The 8-byte load is predicated and
+// nothing selects on its result, so that it stays in flight until the stage it belongs to is written.
 __device__ __forceinline__ uint2 row_scales_of(const RowScales& s, int row, int kb) {
   uint2 v = make_uint2(0x01010101u * WB_SF_PAD, 0x01010101u * WB_SF_PAD);
   const int left = s.kblocks - kb * 8;
-  if (row >= s.rows || left <= 0) return v;
   const uint8_t* p = s.base + (long long)row * s.stride + kb * 8;
-  if (s.vec && left >= 8) return *reinterpret_cast<const uint2*>(p);
+  if (s.vec && left >= 8) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t@p ld.global.v2.b32 {%0, %1}, [%2];\n\t}"
+                 : "+r"(v.x), "+r"(v.y) : "l"(p), "r"(int(row < s.rows)) : "memory");
+    return v;
+  }
+  if (row >= s.rows || left <= 0) return v;
   uint32_t w[2] = {v.x, v.y};
 #pragma unroll
   for (int j = 0; j < 8; ++j)
