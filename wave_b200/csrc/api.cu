@@ -340,12 +340,19 @@ int launch_tile_maps(const DeviceInfo& dev, int M, int N, int K, const void* a, 
   return WB200_OK;
 }
 
+#ifndef WB_RS_STAGES
+#define WB_RS_STAGES 32
+#endif
+// Most pipeline stages per CTA pair for which the tile kernel takes a's scales row-major.
+constexpr int kRowScaleStages = WB_RS_STAGES;
+
 template <int CG, int BN, typename OutT, int EB = 4>
 int launch_tile(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
                 const void* bs, void* c, long long ldc, int sfa_row_blocks, int sfb_row_blocks, int accumulate,
                 cudaStream_t stream, int elem_format = 0) {
   if constexpr (EB == 4 && CG == 2 && BN != 224) {
-    if (tl_row_scales.src)
+    const long long tiles = (long long)((M + 255) / 256) * ((N + BN - 1) / BN), units = dev.sm_count / 2;
+    if (tl_row_scales.src && (tiles + units - 1) / units * ((K + 255) / 256) <= kRowScaleStages)
       return launch_tile_maps<CG, BN, OutT, EB, wb::RowScaleMaps>(dev, M, N, K, a, as, b, bs, c, ldc, sfa_row_blocks, sfb_row_blocks, accumulate,
                                                                   stream, elem_format);
   }

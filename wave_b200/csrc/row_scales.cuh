@@ -4,9 +4,8 @@
 // (scales.cuh) by a kernel of its own costs a launch on the host and, on the device, its own start and end in front
 // of every GEMM: 2 to 3 us, a tenth of a decode step. Here one extra warp of the GEMM brings the scales of every pipeline
 // stage straight into the stage's atoms: a lane reads the eight scale bytes (one stage = 256 K) of rows lane, lane + 32, ..
-// and writes two 16-byte lines, exactly what the packed array holds there. It runs as far ahead as the ring of stages allows,
-// with the loads of the next four stages in registers, so the latency of a load is not in the way; a row's bytes of
-// four consecutive stages share a 32-byte sector.
+// and writes two 16-byte lines, exactly what the packed array holds there. It runs as far ahead as the ring of stages allows;
+// a row's bytes of four consecutive stages share a 32-byte sector.
 #pragma once
 #include "ptx.cuh"
 #include "scales.cuh"
@@ -44,14 +43,16 @@ __device__ __forceinline__ uint2 row_scales_of(const RowScales& s, int row, int 
 template <int R, int STAGES, typename Atoms, typename Wait, typename Signal>
 __device__ __forceinline__ void feed_row_scales(const RowScales& s, int row0, int lane, int kb0, int kb1, uint32_t& stage, uint32_t& phase,
                                                 Atoms atoms, Wait wait, Signal signal) {
-  constexpr int D = 4;  // stages whose scales are in registers
+  // The loads of D stages go out together, between two fences: a fence waits for the loads before it, so one that is
+  // in flight across the fence of a stage costs that stage its whole latency (1.1 us a stage instead of ~0.25).
+  constexpr int D = 8;
   constexpr uint32_t kPad = 0x01010101u * WB_SF_PAD;
-  uint2 v[D][R];
-#pragma unroll
-  for (int d = 0; d < D; ++d)
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[d][r] = (kb0 + d < kb1) ? row_scales_of(s, row0 + r * 32 + lane, kb0 + d) : make_uint2(kPad, kPad);
   for (int kb = kb0; kb < kb1; kb += D) {
+    uint2 v[D][R];
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[d][r] = (kb + d < kb1) ? row_scales_of(s, row0 + r * 32 + lane, kb + d) : make_uint2(kPad, kPad);
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       if (kb + d >= kb1) break;
@@ -64,10 +65,6 @@ __device__ __forceinline__ void feed_row_scales(const RowScales& s, int row0, in
       fence_proxy_async_smem();  // the tensor core's copy reads them through the async proxy
       __syncwarp();
       if (lane == 0) signal(stage);
-      if (kb + d + D < kb1) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[d][r] = row_scales_of(s, row0 + r * 32 + lane, kb + d + D);
-      }
       if (++stage == STAGES) { stage = 0; phase ^= 1u; }
     }
   }
