@@ -273,12 +273,13 @@ int make_output_map_dense(CUtensorMap* map, void* c, int M, int N, long long ldc
 }
 
 // EB: bits per operand element (4: MXFP4, 8: MXFP8 with elem_format 0 = E4M3 / 1 = E5M2).
-template <int CG, int BN, typename OutT, int EB, typename Maps>
-int launch_tile_maps(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
+template <int CG, int BN, typename OutT, int EB = 4>
+int launch_tile(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
                 const void* bs, void* c, long long ldc, int sfa_row_blocks, int sfb_row_blocks, int accumulate,
-                cudaStream_t stream, int elem_format) {
+                cudaStream_t stream, int elem_format = 0) {
   using Cfg = wb::GemmCfg<CG, BN, int(sizeof(OutT)), EB>;
-  Maps maps;
+  wb::PlainMaps maps;
+  if (int rc = pack_row_scales(M, K, stream)) return rc;
   CUtensorMap& tmA = maps.m[0];
   CUtensorMap& tmC = maps.m[4];
   const long long row_bytes = (long long)K * EB / 8;
@@ -287,13 +288,8 @@ int launch_tile_maps(const DeviceInfo& dev, int M, int N, int K, const void* a, 
   rc = weights_are_fp4(EB, elem_format) ? make_operand_map_u4(&maps.m[1], b, N, K, Cfg::B_ROWS)
                                         : make_operand_map(&maps.m[1], b, N, row_bytes, Cfg::B_ROWS);
   if (rc) return rc;
-  if constexpr (Maps::kRowScales) {
-    maps.a_scales = row_scales_param(M, K);
-    maps.m[2] = maps.m[0];  // not used
-  } else {
-    rc = make_scale_map(&maps.m[2], as, sfa_row_blocks, wb::sf_k_atoms(K), 1, Cfg::SF_ATOMS);
-    if (rc) return rc;
-  }
+  rc = make_scale_map(&maps.m[2], as, sfa_row_blocks, wb::sf_k_atoms(K), 1, Cfg::SF_ATOMS);
+  if (rc) return rc;
   rc = make_scale_map(&maps.m[3], bs, sfb_row_blocks, wb::sf_k_atoms(K), Cfg::SFB_BLOCKS, Cfg::SF_ATOMS);
   if (rc) return rc;
   wb::GemmParams p;
@@ -315,7 +311,7 @@ int launch_tile_maps(const DeviceInfo& dev, int M, int N, int K, const void* a, 
     tmC = tmA;  // never dereferenced by the kernel on the direct-store path
   }
   p.status = dev.status_ptr;
-  auto kernel = wb::mxfp4_gemm_kernel<CG, BN, OutT, Maps, EB>;
+  auto kernel = wb::mxfp4_gemm_kernel<CG, BN, OutT, wb::PlainMaps, EB>;
   static bool smem_set[kMaxDevices] = {};
   rc = set_smem(kernel, Cfg::SMEM_BYTES, smem_set);
   if (rc) return rc;
@@ -324,7 +320,7 @@ int launch_tile_maps(const DeviceInfo& dev, int M, int N, int K, const void* a, 
   const int grid = int(tiles < units ? tiles : units) * CG;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(Cfg::THREADS + (Maps::kRowScales ? 32 : 0), 1, 1);
+  cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -338,27 +334,6 @@ int launch_tile_maps(const DeviceInfo& dev, int M, int N, int K, const void* a, 
   cfg.numAttrs = tl_dependent_launch ? 2 : 1;
   WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   return WB200_OK;
-}
-
-#ifndef WB_RS_STAGES
-#define WB_RS_STAGES 32
-#endif
-// Most pipeline stages per CTA pair for which the tile kernel takes a's scales row-major.
-constexpr int kRowScaleStages = WB_RS_STAGES;
-
-template <int CG, int BN, typename OutT, int EB = 4>
-int launch_tile(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
-                const void* bs, void* c, long long ldc, int sfa_row_blocks, int sfb_row_blocks, int accumulate,
-                cudaStream_t stream, int elem_format = 0) {
-  if constexpr (EB == 4 && CG == 2 && BN != 224) {
-    const long long tiles = (long long)((M + 255) / 256) * ((N + BN - 1) / BN), units = dev.sm_count / 2;
-    if (tl_row_scales.src && (tiles + units - 1) / units * ((K + 255) / 256) <= kRowScaleStages)
-      return launch_tile_maps<CG, BN, OutT, EB, wb::RowScaleMaps>(dev, M, N, K, a, as, b, bs, c, ldc, sfa_row_blocks, sfb_row_blocks, accumulate,
-                                                                  stream, elem_format);
-  }
-  if (int rc = pack_row_scales(M, K, stream)) return rc;
-  return launch_tile_maps<CG, BN, OutT, EB, wb::PlainMaps>(dev, M, N, K, a, as, b, bs, c, ldc, sfa_row_blocks, sfb_row_blocks, accumulate, stream,
-                                                           elem_format);
 }
 
 template <int CG, int BN>
@@ -845,10 +820,11 @@ int launch_skinny_scales(const DeviceInfo& dev, int M, int N, int K, const void*
 template <int NP, int STAGES, typename OutT, int EB = 4>
 int launch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
                   const void* bs, void* c, long long ldc, void* ws, int accumulate, cudaStream_t stream, int elem_format = 0) {
-  if constexpr (EB == 4) {
+  if constexpr (EB == 4 && NP <= wb::kRowScaleRows) {
     if (tl_row_scales.src)
       return launch_skinny_scales<NP, STAGES, OutT, EB, true>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
   }
+  if (int rc = pack_row_scales(M, K, stream)) return rc;
   return launch_skinny_scales<NP, STAGES, OutT, EB, false>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
 }
 
@@ -947,11 +923,12 @@ int launch_skinny_whole_maps(const DeviceInfo& dev, int M, int N, int K, const v
 template <int NP, int STAGES, typename OutT, int EB = 4, int WR = 128, int SBUFS = 2>
 int launch_skinny_whole(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
                         const void* bs, void* c, long long ldc, void* ws, int accumulate, cudaStream_t stream, int elem_format = 0) {
-  if constexpr (EB == 4) {
+  if constexpr (EB == 4 && NP <= wb::kRowScaleRows) {
     if (tl_row_scales.src)
       return launch_skinny_whole_maps<NP, STAGES, OutT, EB, WR, SBUFS, wb::SkinnyRowScaleMaps>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate,
                                                                                                stream, elem_format);
   }
+  if (int rc = pack_row_scales(M, K, stream)) return rc;
   return launch_skinny_whole_maps<NP, STAGES, OutT, EB, WR, SBUFS, wb::SkinnyMaps>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream,
                                                                                    elem_format);
 }

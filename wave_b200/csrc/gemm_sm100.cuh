@@ -25,7 +25,6 @@
 #pragma once
 #include "ptx.cuh"
 #include "quantize.cuh"
-#include "row_scales.cuh"
 #include <cuda_bf16.h>
 
 namespace wb {
@@ -107,15 +106,8 @@ struct GemmParams {
 // The tensor maps of one launch, passed by value as a kernel parameter. Index: 0 = a, 1 = b,
 // 2 = packed a scales, 3 = packed b scales, 4 = c. map(g, i): map i of group g.
 struct PlainMaps {
-  static constexpr bool kGrouped = false, kAligned = false, kSilu = false, kRowScales = false;
+  static constexpr bool kGrouped = false, kAligned = false, kSilu = false;
   CUtensorMap m[5];
-  __device__ __forceinline__ const CUtensorMap* map(int, int i) const { return &m[i]; }
-};
-// The same with a's scales row-major (map 2 is not used): a seventh warp brings them into the stages.
-struct RowScaleMaps {
-  static constexpr bool kGrouped = false, kAligned = false, kSilu = false, kRowScales = true;
-  CUtensorMap m[5];
-  RowScales a_scales;
   __device__ __forceinline__ const CUtensorMap* map(int, int i) const { return &m[i]; }
 };
 // Grouped (per-expert) launch: five maps per group, each describing only that group's rows, so that
@@ -123,7 +115,7 @@ struct RowScaleMaps {
 // tiles over the groups, rows the row count of each group.
 constexpr int kMaxGroups = 32;
 struct GroupedMaps {
-  static constexpr bool kGrouped = true, kAligned = false, kSilu = false, kRowScales = false;
+  static constexpr bool kGrouped = true, kAligned = false, kSilu = false;
   CUtensorMap m[kMaxGroups * 5];
   void* c_base[kMaxGroups];  // first output row of each group, for the stores that do not go through its tensor map
   int tile_start[kMaxGroups + 1];
@@ -144,7 +136,7 @@ struct GroupedMaps {
 // parameter block, which the host copies on every launch, is 2.5 KB for up to 8 experts and 8.7 KB for up to 32.
 template <int G>
 struct AlignedMaps {
-  static constexpr bool kGrouped = true, kAligned = true, kSilu = false, kRowScales = false;
+  static constexpr bool kGrouped = true, kAligned = true, kSilu = false;
   CUtensorMap rows_map[3];   // a, packed a scales, c
   CUtensorMap w_map[2 * G];  // b, packed b scales of every expert
   void* c_base;
@@ -358,7 +350,7 @@ __device__ __forceinline__ void stage_chunk32(uint32_t buf, int lane, int half, 
 }
 
 template <int CG, int BN, typename OutT, typename Maps, int EB = 4>
-__global__ void __launch_bounds__(Maps::kRowScales ? 224 : 192, 1)
+__global__ void __launch_bounds__(192, 1)
 mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
   using Cfg = GemmCfg<CG, BN, int(sizeof(OutT)), EB>;
   constexpr int STAGES = Cfg::STAGES;
@@ -387,7 +379,7 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full_bar(s), 1 + (Maps::kRowScales ? CG : 0));  // the loads, and the scale warp of every CTA
+      mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -460,11 +452,11 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
 #endif
         if (elect_one()) {
           // 4-bit weights expanded by the copy engine (EB == 8 kernels only): the transaction count is the packed size
-          if (leader) mbar_expect_tx(full_bar(stage), (Cfg::LOAD_BYTES - (Maps::kRowScales ? Cfg::SFA_BYTES : 0) - ((EB == 8 && (p.elem_format & 0x10)) ? Cfg::B_BYTES / 2 : 0)) * CG);
+          if (leader) mbar_expect_tx(full_bar(stage), (Cfg::LOAD_BYTES - ((EB == 8 && (p.elem_format & 0x10)) ? Cfg::B_BYTES / 2 : 0)) * CG);
           tma_load_2d<CG>(sA, tm_a, kb * 128, a_row, fb);
           tma_load_2d<CG>(sB, tm_b, kb * 128, b_row, fb);
           // scale factors: SF_ATOMS atoms of 512 bytes (128 32-bit words) per 128-row block and stage
-          if constexpr (!Maps::kRowScales) tma_load_2d<CG>(sSFA, tm_sfa, kb * (Cfg::SF_ATOMS * 128), sfa_rb, fb);
+          tma_load_2d<CG>(sSFA, tm_sfa, kb * (Cfg::SF_ATOMS * 128), sfa_rb, fb);
           if constexpr (Maps::kSilu) {  // the gate rows' block, then the up rows'
             tma_load_2d<CG>(sSFB, tm_sfb, kb * (Cfg::SF_ATOMS * 128), nt, fb);
             tma_load_2d<CG>(sSFB + Cfg::SF_ATOMS * 512, tm_sfb, kb * (Cfg::SF_ATOMS * 128), maps.inter / 128 + nt, fb);
@@ -512,7 +504,7 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
           const uint32_t t_sfa = tmem_base + Cfg::SF_COL + sf_set * Cfg::SF_SET_COLS;
           const uint32_t t_sfb = t_sfa + 8;
           if (++sf_set == Cfg::SF_SETS) sf_set = 0;
-          mbar_wait<Maps::kRowScales && CG == 2>(full_bar(stage), phase, ctx, WB_DEV_TIMEOUT_MMA_FULL);
+          mbar_wait(full_bar(stage), phase, ctx, WB_DEV_TIMEOUT_MMA_FULL);
           tc_fence_after_sync();
           const uint32_t sA = smem_base + stage * Cfg::STAGE_BYTES;
           const uint32_t sB = sA + Cfg::A_BYTES;
@@ -561,25 +553,6 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
         ++it;
-      }
-    }
-  } else if (Maps::kRowScales && warp == 6) {
-    // ------------------------------------------------------------------ a's scales, row-major, into the stages
-    if constexpr (Maps::kRowScales) {
-      static_assert(EB == 4, "a stage of 256 K");
-      uint32_t stage = 0, phase = 0;
-      pdl_wait();
-      for (int t = first_tile; t < num_tiles; t += tile_step) {
-        int mt, nt, rows;
-        decode_tile(maps, p, t, tiles_m, mt, nt, rows);
-        feed_row_scales<4, STAGES>(
-            maps.a_scales, (mt * CG + int(rank)) * Cfg::BM, lane, 0, num_kb, stage, phase,
-            [&](uint32_t st) { return smem_base + st * Cfg::STAGE_BYTES + Cfg::A_BYTES + Cfg::B_BYTES; },
-            [&](uint32_t st, uint32_t ph) { mbar_wait(empty_bar(st), ph ^ 1u, ctx, WB_DEV_TIMEOUT_PRODUCER); },
-            [&](uint32_t st) {
-              if constexpr (CG == 2) mbar_arrive_cluster(mapa_shared(full_bar(st), 0));
-              else mbar_arrive(full_bar(st));
-            });
       }
     }
   } else {

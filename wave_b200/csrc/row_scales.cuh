@@ -1,11 +1,14 @@
-// Activation scales taken row-major by the GEMM kernels themselves.
+// Activation scales of a decode GEMM (M <= 32) taken row-major by the GEMM kernel itself.
 //
 // The reference-facing call hands over a_scale as [M, K/32]. Packing it into the layout tcgen05.cp reads
-// (scales.cuh) by a kernel of its own costs a launch on the host and, on the device, its own start and end in front
-// of every GEMM: 2 to 3 us, a tenth of a decode step. Here one extra warp of the GEMM brings the scales of every pipeline
-// stage straight into the stage's atoms: a lane reads the eight scale bytes (one stage = 256 K) of rows lane, lane + 32, ..
-// and writes two 16-byte lines, exactly what the packed array holds there. It runs as far ahead as the ring of stages allows;
-// a row's bytes of four consecutive stages share a 32-byte sector.
+// (scales.cuh) by a kernel of its own costs a launch on the host and, on the device, about a microsecond in front of every
+// GEMM. Here one extra warp of the decode kernels brings the scales of every pipeline stage straight into the stage's
+// atoms: a lane reads the eight scale bytes (one stage = 256 K) of its row and writes two 16-byte lines, exactly what the
+// packed array holds there. It runs as far ahead as the ring of stages allows.
+// M = 16, N = 28672, K = 8192, replayed from a graph: 23.6 -> 22.6 us, launched eagerly 26.2 -> 24.2; 16 x 4096 x 4096 eagerly
+// 24.8 -> 19.5. Up to 32 rows only: the fence that hands a stage to the tensor core and the loads cost up to a microsecond a
+// stage when four rows per lane are read (128 x 8192 x 8192: 31.4 -> 42.0 us), and the 128-row stages of the tile kernel
+// cannot wait for that either (8192^3: 178 -> 500 us).
 #pragma once
 #include "ptx.cuh"
 #include "scales.cuh"
@@ -38,30 +41,27 @@ __device__ __forceinline__ uint2 row_scales_of(const RowScales& s, int row, int 
   return make_uint2(w[0], w[1]);
 }
 
-// Feeds stages with the scales of K blocks [kb0, kb1) (in stages of 256 K) of rows row0 .. row0 + 32 R - 1. atoms(stage): shared
-// address of the stage's two atoms; wait(stage, phase): the stage is free; signal(stage): by one lane, the scales are there.
-template <int R, int STAGES, typename Atoms, typename Wait, typename Signal>
-__device__ __forceinline__ void feed_row_scales(const RowScales& s, int row0, int lane, int kb0, int kb1, uint32_t& stage, uint32_t& phase,
-                                                Atoms atoms, Wait wait, Signal signal) {
-  // The loads of D stages go out together, between two fences: a fence waits for the loads before it, so one that is
-  // in flight across the fence of a stage costs that stage its whole latency (1.1 us a stage instead of ~0.25).
+constexpr int kRowScaleRows = 32;  // one row per lane
+
+// Feeds stages with the scales of K blocks [kb0, kb1) (in stages of 256 K). atoms(stage): shared address of the stage's two
+// atoms; wait(stage, phase): the stage is free; signal(stage): by one lane, the scales are there.
+template <int STAGES, typename Atoms, typename Wait, typename Signal>
+__device__ __forceinline__ void feed_row_scales(const RowScales& s, int lane, int kb0, int kb1, uint32_t& stage, uint32_t& phase, Atoms atoms,
+                                                Wait wait, Signal signal) {
+  // The loads of D stages go out together, between two fences: a fence waits for the loads before it.
   constexpr int D = 8;
   constexpr uint32_t kPad = 0x01010101u * WB_SF_PAD;
   for (int kb = kb0; kb < kb1; kb += D) {
-    uint2 v[D][R];
+    uint2 v[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d)
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[d][r] = (kb + d < kb1) ? row_scales_of(s, row0 + r * 32 + lane, kb + d) : make_uint2(kPad, kPad);
+    for (int d = 0; d < D; ++d) v[d] = (kb + d < kb1) ? row_scales_of(s, lane, kb + d) : make_uint2(kPad, kPad);
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       if (kb + d >= kb1) break;
       wait(stage, phase);
-      const uint32_t line = atoms(stage) + uint32_t(lane) * 16u;
-      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(line), "r"(v[d][0].x), "r"(R > 1 ? v[d][1 % R].x : kPad),
-                   "r"(R > 2 ? v[d][2 % R].x : kPad), "r"(R > 3 ? v[d][3 % R].x : kPad) : "memory");
-      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(line + 512u), "r"(v[d][0].y), "r"(R > 1 ? v[d][1 % R].y : kPad),
-                   "r"(R > 2 ? v[d][2 % R].y : kPad), "r"(R > 3 ? v[d][3 % R].y : kPad) : "memory");
+      const uint32_t line = atoms(stage) + uint32_t(lane) * 16u;  // rows lane, lane + 32, .. of the atom
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %2, %2};" ::"r"(line), "r"(v[d].x), "r"(kPad) : "memory");
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %2, %2};" ::"r"(line + 512u), "r"(v[d].y), "r"(kPad) : "memory");
       fence_proxy_async_smem();  // the tensor core's copy reads them through the async proxy
       __syncwarp();
       if (lane == 0) signal(stage);

@@ -347,13 +347,13 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
   } else if (Maps::kRowScales && warp == 6) {
     // ------------------------------------------------------------------ the activations' scales, row-major, into the stages
     if constexpr (Maps::kRowScales) {
-      static_assert(EB == 4, "a stage of 256 K");
+      static_assert(EB == 4 && NP <= kRowScaleRows, "a stage of 256 K, one row per lane");
       if (p.dependent) pdl_wait();
       uint32_t stage = 0, phase = 0;
       for (int seq = 0;; ++seq) {
         if (next_tile(seq) < 0) break;
-        feed_row_scales<(NP + 31) / 32, STAGES>(
-            maps.x_scales, 0, lane, 0, p.num_kb, stage, phase,
+        feed_row_scales<STAGES>(
+            maps.x_scales, lane, 0, p.num_kb, stage, phase,
             [&](uint32_t st) { return smem_base + st * Cfg::STAGE_BYTES + Base::W_BYTES + Base::X_BYTES + Base::SF_BYTES; },
             [&](uint32_t st, uint32_t ph) { mbar_wait(empty_bar(st), ph ^ 1u, ctx, WB_DEV_TIMEOUT_PRODUCER); },
             [&](uint32_t st) { mbar_arrive(full_bar(st)); });
