@@ -1125,3 +1125,25 @@ def test_row_major_activation_scales_give_the_bits_of_packed_ones(M, N, K, offse
     assert torch.equal(c.view(torch.int16), ref.view(torch.int16))
     check(c, a, a_s, b, b_s)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("N,K", [(128, 256), (500, 1024), (1024, 8192), (1030, 12288), (4096, 4064), (9472, 4096), (9601, 4096), (18816, 512),
+                                 (14336, 4096)])
+@pytest.mark.parametrize("M", [1, 16, 17, 64, 128])
+def test_decode_calls_with_few_weight_tiles(M, N, K):
+    """M <= 128 with fewer 128-row weight tiles than SMs: the K-split kernel, the two tile kernels or a cluster per tile, by M and the
+    size of the weight; either side of every line of that rule. Same call as a user's (AUTO, with a workspace)."""
+    a, a_s, b, b_s = random_problem(M, N, K, seed=M + N + K)
+    ad, bd = a.to(DEV), b.to(DEV)
+    a_sf, b_sf = ops.repack_scales(a_s.to(DEV)), ops.repack_scales(b_s.to(DEV))
+    ref = orc.scaled_gemm(a, a_s, b, b_s)
+    for out_dtype in (torch.bfloat16, torch.float32):
+        c = torch.full((M, N), float("nan"), dtype=out_dtype, device=DEV)
+        ops.scaled_gemm_packed(ad, a_sf, bd, b_sf, c)
+        check(c, a, a_s, b, b_s, ref=ref)
+    base = torch.randn(M, N, generator=torch.Generator().manual_seed(N))
+    acc = base.to(DEV)
+    ops.scaled_gemm_packed(ad, a_sf, bd, b_sf, acc, _lib.ACCUMULATE)
+    tol = orc.f32_tolerance(orc.dequant_mxfp4(a, a_s), orc.dequant_mxfp4(b, b_s), ref, K)
+    assert bool(((acc.cpu() - (ref + base)).abs() <= tol + 1e-6 * base.abs()).all())
+    ops.check_device_status()

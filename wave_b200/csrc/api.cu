@@ -1094,6 +1094,27 @@ int dispatch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, c
   return launch_skinny<128, 6, OutT, EB>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
 }
 
+// What AUTO runs for M <= 128 on the usual packing of the weight scales when there are fewer 128-row weight tiles than SMs
+// (with more, the whole-tile decode kernel is the fastest at every M).
+enum class DecodeRoute { kSkinny, kTile1, kTile2, kCluster };
+// The K-split kernel keeps all SMs streaming, but every CTA ends with partial tiles of M x 128 sums that meet in memory: with
+// M = 64 that costs more than the stream (64 x 2048 x 4096: 51 us), and with few K blocks per SM at M = 16 too. It is
+// the fastest only up to 16 rows and from eight 256-deep K blocks per SM up. us, K split against the tile kernel:
+//   M = 16: N x K = 1024 x 1024 8.7 / 4.8, 2048 x 4096 19.0 / 7.8, 4096 x 4096 12.5 / 8.8, 8192 x 1024 11.0 / 5.3;
+//           14336 x 4096 12.1 / 13.4, 4096 x 14336 14.3 / 18.3, 8192 x 8192 13.5 / 16.2, 16384 x 16384 28.6 / 30.5
+//   M = 32: 4096 x 4096 16.9 / 9.0, 8192 x 8192 16.4 / 13.2, 14336 x 4096 14.1 / 13.1, 16384 x 16384 30.5 / 30.9
+//   M = 128: 1024 x 8192 101 / 11.3, 4096 x 4096 48.0 / 9.0, 8192 x 8192 30.8 / 13.5, 16384 x 16384 43.5 / 31.5
+// Of the tile kernels, CTA pairs (256 x 128 tiles) fetch the weights of a tile through two SMs: ahead from 16 K blocks up
+// while a pair per tile fits (1024 x 8192 11.0 / 12.7, 8192 x 8192 13.2 / 14.3), behind otherwise (8192 x 1024 6.0 / 5.3,
+// 14336 x 4096 13.4 / 11.2). Where K is long enough and the tiles are few, a cluster per tile.
+DecodeRoute decode_route(int sm_count, int M, int N, int K) {
+  const int tiles = (N + 127) / 128, kb = (K + 255) / 256;
+  if (tiles >= sm_count) return DecodeRoute::kSkinny;
+  if (cluster_splitk_slices(M, N, K)) return DecodeRoute::kCluster;
+  if (M <= 16 && (long long)tiles * kb >= 8ll * sm_count) return DecodeRoute::kSkinny;
+  return tiles * 2 <= sm_count && kb >= 16 ? DecodeRoute::kTile2 : DecodeRoute::kTile1;
+}
+
 // ------------------------------------------------------------------------------------------
 // allocation-free skinny entry point: its scratch lives in the library image
 // ------------------------------------------------------------------------------------------
@@ -1606,9 +1627,19 @@ int wb200_mxfp4_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
   const int slices = splitk_slices(dev->sm_count, M, N, K);
   const bool splitk_ok = slices >= 2 && workspace && workspace_bytes >= splitk_workspace_bytes(slices, M, N) &&
                          (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && N % 4 == 0;
+  int route_bn = 0;  // tile width that the decode rule has chosen with the path
   if (path == WB200_PATH_AUTO) {
     const bool ws_ok = workspace && workspace_bytes >= skinny_workspace_bytes(dev->sm_count, M);
-    if (M <= 128 && ws_ok) path = WB200_PATH_SKINNY;
+    if (M <= 128 && ws_ok) {
+      path = WB200_PATH_SKINNY;
+      if (tl_b_tile_rows == 128 && !(flags & (WB200_TILE_N128 | WB200_TILE_N192))) {
+        const DecodeRoute route = decode_route(dev->sm_count, M, N, K);
+        if (route != DecodeRoute::kSkinny) {
+          path = route == DecodeRoute::kTile1 ? WB200_PATH_TILE_1CTA : WB200_PATH_TILE_2CTA;
+          if (route != DecodeRoute::kCluster) route_bn = 128;
+        }
+      }
+    }
     // split-K pays from three slices up; with two, 128-wide tiles do better (1024 x 2048 x 16000: 21.7 us
     // with two slices, 18.6 us with 128-wide tiles, 24.3 us with neither)
     else if (splitk_ok && slices >= 3 && !(flags & (WB200_TILE_N128 | WB200_TILE_N192))) path = WB200_PATH_TILE_SPLITK;
@@ -1637,7 +1668,7 @@ int wb200_mxfp4_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
       return dispatch_skinny<float>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, workspace, accumulate, s);
     return dispatch_skinny<__nv_bfloat16>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, workspace, accumulate, s);
   }
-  if ((flags & WB200_PATH_MASK) == WB200_PATH_AUTO && path == WB200_PATH_TILE_2CTA && !(flags & (WB200_TILE_N128 | WB200_TILE_N192))) {
+  if ((flags & WB200_PATH_MASK) == WB200_PATH_AUTO && path == WB200_PATH_TILE_2CTA && !route_bn && !(flags & (WB200_TILE_N128 | WB200_TILE_N192))) {
     const int cluster_slices = cluster_splitk_slices(M, N, K);
     if (cluster_slices) {
       if (c_dtype == WB200_F32)
@@ -1666,6 +1697,7 @@ int wb200_mxfp4_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
     }
   }
   if (wide224) bn = 224;
+  if (route_bn) bn = route_bn;
   return dispatch_tile(path, bn, c_dtype, *dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc,
                        wb::sf_row_blocks(M), wb::sf_row_blocks(N), accumulate, s);
 }
