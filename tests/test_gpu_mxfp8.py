@@ -362,3 +362,18 @@ def test_mixed_decode_with_weights_on_the_n_side(M, N, K, out_dtype):
     with pytest.raises(ValueError):  # no MXFP4 kernel reads this packing
         ops.scaled_gemm_packed(bd[:M], ops.repack_scales(b_s[:M].to(DEV)), bd, b_sf, torch.empty(M, N, dtype=out_dtype, device=DEV))
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("N,K", [(128, 128), (1024, 8192), (1100, 1024), (4096, 4096), (4096, 12288), (9600, 2048), (14336, 1024)])
+@pytest.mark.parametrize("M", [1, 16, 32, 33, 128])
+@pytest.mark.parametrize("b_fp4", [False, True])
+def test_8bit_decode_calls_with_few_weight_tiles(M, N, K, b_fp4):
+    """M <= 128 with fewer 128-row weight tiles than SMs: either side of every line of the rule that picks the K-split kernel or one
+    of the two tile kernels."""
+    problem_of, check_of = (mixed_problem, check_mixed) if b_fp4 else (problem, check)
+    a, a_s, b, b_s = problem_of(M, N, K, M + N + K, torch.float8_e4m3fn)
+    c = torch.full((M, N), float("nan"), dtype=torch.float32, device=DEV)
+    a_sf, b_sf = ops.repack_scales(a_s.to(DEV)), ops.repack_scales(b_s.to(DEV))
+    ops.scaled_gemm_mxfp8_packed(a.to(DEV), a_sf, b.to(DEV), b_sf, c, b_fp4=b_fp4)
+    check_of(c, a, a_s, b, b_s)
+    ops.check_device_status()

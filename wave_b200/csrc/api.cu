@@ -1115,6 +1115,20 @@ DecodeRoute decode_route(int sm_count, int M, int N, int K) {
   return tiles * 2 <= sm_count && kb >= 16 ? DecodeRoute::kTile2 : DecodeRoute::kTile1;
 }
 
+// The same for 8-bit operands and the mixed pair (K blocks of 128). us, K split against the better tile kernel:
+//   M = 16: 1024 x 1024 11.3 / 5.8, 1024 x 8192 18.7 / 16.9 (mixed 24.3 / 16.6), 4096 x 1024 13.2 / 6.0; 4096 x 4096 11.6 / 12.5
+//           (11.0 / 11.9), 8192 x 8192 19.2 / 20.0 (16.2 / 18.3), 14336 x 4096 17.3 / 21.6 (15.0 / 20.1)
+//   M = 32: 4096 x 4096 15.4 / 11.6, 8192 x 8192 21.4 / 20.8, 14336 x 4096 19.4 / 16.4; 4096 x 14336 23.2 / 27.2, 16384 x 16384
+//           50.8 / 51.9 (37.0 / 41.2)
+//   M = 128: 1024 x 8192 102 / 17.3, 4096 x 4096 34.9 / 12.0, 8192 x 8192 36.8 / 21.3, 16384 x 16384 68.3 / 53.3
+DecodeRoute decode_route_8bit(int sm_count, int M, int N, int K) {
+  const int tiles = (N + 127) / 128, kb = (K + 127) / 128;
+  if (tiles >= sm_count) return DecodeRoute::kSkinny;
+  if (M <= 16 && (long long)tiles * kb >= 6ll * sm_count) return DecodeRoute::kSkinny;
+  if (M <= 32 && kb >= 96 && (long long)tiles * kb >= 20ll * sm_count) return DecodeRoute::kSkinny;
+  return tiles * 2 <= sm_count && kb >= 16 ? DecodeRoute::kTile2 : DecodeRoute::kTile1;
+}
+
 // ------------------------------------------------------------------------------------------
 // allocation-free skinny entry point: its scratch lives in the library image
 // ------------------------------------------------------------------------------------------
@@ -1777,7 +1791,17 @@ int wb200_mxfp8_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
   const int accumulate = (flags & WB200_ACCUMULATE) ? 1 : 0;
   const bool ws_ok = workspace && workspace_bytes >= skinny_workspace_bytes(dev->sm_count, M) &&
                      (reinterpret_cast<uintptr_t>(workspace) & 15) == 0;
-  if (path == WB200_PATH_AUTO) path = (M <= 128 && ws_ok) ? WB200_PATH_SKINNY : (M > 128) ? WB200_PATH_TILE_2CTA : WB200_PATH_TILE_1CTA;
+  bool n128 = (flags & WB200_TILE_N128) != 0;
+  if (path == WB200_PATH_AUTO) {
+    path = (M <= 128 && ws_ok) ? WB200_PATH_SKINNY : (M > 128) ? WB200_PATH_TILE_2CTA : WB200_PATH_TILE_1CTA;
+    if (path == WB200_PATH_SKINNY && tl_b_tile_rows == 128 && !n128) {
+      const DecodeRoute route = decode_route_8bit(dev->sm_count, M, N, K);
+      if (route != DecodeRoute::kSkinny) {
+        path = route == DecodeRoute::kTile1 ? WB200_PATH_TILE_1CTA : WB200_PATH_TILE_2CTA;
+        n128 = true;
+      }
+    }
+  }
   if (tl_b_tile_rows != 128 && path != WB200_PATH_SKINNY)
     return fail(WB200_ERR_UNSUPPORTED, "mxfp8_gemm: weight scales packed per %d-row tile are read by the M <= 128 kernel only, which needs "
                 "a workspace (M = %d, path %u)", tl_b_tile_rows, M, path);
@@ -1796,7 +1820,6 @@ int wb200_mxfp8_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
       return dispatch_skinny<float, 8>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, workspace, accumulate, s, elem_format);
     return dispatch_skinny<__nv_bfloat16, 8>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, workspace, accumulate, s, elem_format);
   }
-  bool n128 = (flags & WB200_TILE_N128) != 0;
   if (!n128 && (flags & WB200_PATH_MASK) == WB200_PATH_AUTO)
     n128 = (long long)((M + 127) / 128) * ((N + 255) / 256) < dev->sm_count;
   if (path == WB200_PATH_TILE_2CTA)
