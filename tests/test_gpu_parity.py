@@ -1147,3 +1147,20 @@ def test_decode_calls_with_few_weight_tiles(M, N, K):
     tol = orc.f32_tolerance(orc.dequant_mxfp4(a, a_s), orc.dequant_mxfp4(b, b_s), ref, K)
     assert bool(((acc.cpu() - (ref + base)).abs() <= tol + 1e-6 * base.abs()).all())
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("rows,N,K", [(1, 640, 416), (32, 28672, 256), (128, 1000, 992), (129, 512, 288), (1000, 4096, 512)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_linear_in_one_call_gives_the_bits_of_quantiser_and_gemm(rows, N, K, dtype):
+    """MXFP4Linear's single native call against wb200_quantize_mxfp4 followed by the GEMM, also for a column block of a wider x and
+    for a transposed x, which is copied."""
+    g = torch.Generator().manual_seed(rows + N)
+    layer = wb.MXFP4Linear.from_float((torch.randn(N, K, generator=g) * 0.02).to(DEV), output_dtype=dtype)
+    wide = torch.randn(rows, K + 32, generator=g).to(dtype).to(DEV)
+    for x in (wide[:, :K].contiguous(), wide[:, 16:K + 16], wide[:, :K].t().contiguous().t()):
+        y = layer(x)
+        q, _, sf = wb.quantize_mxfp4(x, want_rowmajor=False)
+        ref = torch.empty(rows, N, dtype=dtype, device=DEV)
+        ops.scaled_gemm_packed(q, sf, layer.weight_codes, layer._packed_decode if rows <= 128 else layer._packed, ref)
+        assert torch.equal(y, ref)
+    ops.check_device_status()
