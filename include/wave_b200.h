@@ -296,7 +296,7 @@ int wb200_mxfp8_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
                      size_t workspace_bytes, unsigned flags, void* stream);
 /* The same with row-major activation scales ([M, K/32], row stride in bytes), packed into a_scale_scratch
  * (wb200_packed_scale_bytes(M, K) bytes) first; the GEMM is launched as the repack kernel's programmatic dependent, as in
- * wb200_mxfp4_gemm_repack_a. */
+ * wb200_mxfp4_gemm_repack_a. WB200_PATH_AUTO with M <= 128 takes a tile path here where few weight tiles make it faster. */
 int wb200_mxfp8_gemm_repack_a(int M, int N, int K, const void* a, const void* a_scale, long long a_scale_stride, void* a_scale_scratch,
                               const void* b, const void* b_scale_packed, void* c, int c_dtype, long long ldc, int elem_format,
                               void* workspace, size_t workspace_bytes, unsigned flags, void* stream);

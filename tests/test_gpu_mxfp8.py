@@ -369,11 +369,13 @@ def test_mixed_decode_with_weights_on_the_n_side(M, N, K, out_dtype):
 @pytest.mark.parametrize("b_fp4", [False, True])
 def test_8bit_decode_calls_with_few_weight_tiles(M, N, K, b_fp4):
     """M <= 128 with fewer 128-row weight tiles than SMs: either side of every line of the rule that picks the K-split kernel or one
-    of the two tile kernels."""
+    of the two tile kernels in the template call."""
     problem_of, check_of = (mixed_problem, check_mixed) if b_fp4 else (problem, check)
     a, a_s, b, b_s = problem_of(M, N, K, M + N + K, torch.float8_e4m3fn)
     c = torch.full((M, N), float("nan"), dtype=torch.float32, device=DEV)
-    a_sf, b_sf = ops.repack_scales(a_s.to(DEV)), ops.repack_scales(b_s.to(DEV))
-    ops.scaled_gemm_mxfp8_packed(a.to(DEV), a_sf, b.to(DEV), b_sf, c, b_fp4=b_fp4)
+    template, subs = wb.get_scaled_gemm_mxfp8_kernel((M, N, K), wb.ScaledMMAType.F32_16x16x128_F8F6F4, "f8e4m3fn", wb.f32,
+                                                     weight_format="f4e2m1fn" if b_fp4 else None)
+    gemm = wb.wave_compile(wb.set_default_run_config(wb.WaveCompileOptions(subs=subs)), template)
+    gemm(a.to(DEV), a_s.to(DEV), b.to(DEV), b_s.to(DEV), c)
     check_of(c, a, a_s, b, b_s)
     ops.check_device_status()

@@ -1755,6 +1755,10 @@ static int launch_mxfp8(int c_dtype, const DeviceInfo& dev, int M, int N, int K,
 }
 }  // extern "C++"
 
+// Set while wb200_mxfp8_gemm_repack_a, the form behind the template call, runs: AUTO then follows decode_route_8bit. On its own
+// wb200_mxfp8_gemm keeps its documented choice (the skinny path whenever M <= 128 and a workspace is passed).
+static thread_local bool tl_route_8bit = false;
+
 int wb200_mxfp8_gemm(int M, int N, int K, const void* a, const void* a_scale_packed, const void* b,
                      const void* b_scale_packed, void* c, int c_dtype, long long ldc, int elem_format, void* workspace,
                      size_t workspace_bytes, unsigned flags, void* stream) {
@@ -1794,7 +1798,7 @@ int wb200_mxfp8_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
   bool n128 = (flags & WB200_TILE_N128) != 0;
   if (path == WB200_PATH_AUTO) {
     path = (M <= 128 && ws_ok) ? WB200_PATH_SKINNY : (M > 128) ? WB200_PATH_TILE_2CTA : WB200_PATH_TILE_1CTA;
-    if (path == WB200_PATH_SKINNY && tl_b_tile_rows == 128 && !n128) {
+    if (tl_route_8bit && path == WB200_PATH_SKINNY && tl_b_tile_rows == 128 && !n128) {
       const DecodeRoute route = decode_route_8bit(dev->sm_count, M, N, K);
       if (route != DecodeRoute::kSkinny) {
         path = route == DecodeRoute::kTile1 ? WB200_PATH_TILE_1CTA : WB200_PATH_TILE_2CTA;
@@ -1838,8 +1842,9 @@ int wb200_mxfp8_gemm_repack_a(int M, int N, int K, const void* a, const void* a_
   tl_dependent_launch = false;
   if (rc) return rc;
   tl_dependent_launch = true;  // the GEMM is the repack kernel's programmatic dependent
+  tl_route_8bit = true;
   rc = wb200_mxfp8_gemm(M, N, K, a, a_scale_scratch, b, b_scale_packed, c, c_dtype, ldc, elem_format, workspace, workspace_bytes, flags, stream);
-  tl_dependent_launch = false;
+  tl_dependent_launch = tl_route_8bit = false;
   return rc;
 }
 
