@@ -1159,7 +1159,7 @@ def test_linear_in_one_call_gives_the_bits_of_quantiser_and_gemm(rows, N, K, dty
     wide = torch.randn(rows, K + 32, generator=g).to(dtype).to(DEV)
     for x in (wide[:, :K].contiguous(), wide[:, 16:K + 16], wide[:, :K].t().contiguous().t()):
         y = layer(x)
-        q, _, sf = wb.quantize_mxfp4(x, want_rowmajor=False)
+        q, _, sf = ops.quantize_mxfp4(x, want_rowmajor=False)
         ref = torch.empty(rows, N, dtype=dtype, device=DEV)
         ops.scaled_gemm_packed(q, sf, layer.weight_codes, layer._packed_decode if rows <= 128 else layer._packed, ref)
         assert torch.equal(y, ref)
