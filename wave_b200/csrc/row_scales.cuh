@@ -43,21 +43,26 @@ __device__ __forceinline__ uint2 row_scales_of(const RowScales& s, int row, int 
 
 constexpr int kRowScaleRows = 32;  // one row per lane
 
-// Feeds stages with the scales of K blocks [kb0, kb1) (in stages of 256 K). atoms(stage): shared address of the stage's two
+// Feeds `count` stages; stage i takes K block (kb0 + i) mod num_kb (in stages of 256 K), so that a run over several tiles is
+// one sequence: the loads for the next tile's stages are not held up at its start. atoms(stage): shared address of its two
 // atoms; wait(stage, phase): the stage is free; signal(stage): by one lane, the scales are there.
 template <int STAGES, typename Atoms, typename Wait, typename Signal>
-__device__ __forceinline__ void feed_row_scales(const RowScales& s, int lane, int kb0, int kb1, uint32_t& stage, uint32_t& phase, Atoms atoms,
-                                                Wait wait, Signal signal) {
+__device__ __forceinline__ void feed_row_scales(const RowScales& s, int lane, int kb0, int num_kb, int count, uint32_t& stage, uint32_t& phase,
+                                                Atoms atoms, Wait wait, Signal signal) {
   // The loads of D stages go out together, between two fences: a fence waits for the loads before it.
   constexpr int D = 8;
   constexpr uint32_t kPad = 0x01010101u * WB_SF_PAD;
-  for (int kb = kb0; kb < kb1; kb += D) {
+  int kb = kb0;
+  for (int i = 0; i < count; i += D) {
     uint2 v[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) v[d] = (kb + d < kb1) ? row_scales_of(s, lane, kb + d) : make_uint2(kPad, kPad);
+    for (int d = 0; d < D; ++d) {
+      v[d] = (i + d < count) ? row_scales_of(s, lane, kb) : make_uint2(kPad, kPad);
+      if (++kb == num_kb) kb = 0;
+    }
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      if (kb + d >= kb1) break;
+      if (i + d >= count) break;
       wait(stage, phase);
       const uint32_t line = atoms(stage) + uint32_t(lane) * 16u;  // rows lane, lane + 32, .. of the atom
       asm volatile("st.shared.v4.b32 [%0], {%1, %2, %2, %2};" ::"r"(line), "r"(v[d].x), "r"(kPad) : "memory");

@@ -300,15 +300,11 @@ mxfp4_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       static_assert(EB == 4 && NP <= kRowScaleRows, "a stage of 256 K, one row per lane");
       if (p.dependent) pdl_wait();
       uint32_t stage = 0, phase = 0;
-      for (int seg = 0; seg < nseg; ++seg) {
-        int tile, kbs, kbe;
-        segment(seg, tile, kbs, kbe);
-        feed_row_scales<STAGES>(
-            p.x_scales, lane, kbs, kbe, stage, phase,
-            [&](uint32_t st) { return smem_base + st * Cfg::STAGE_BYTES + Cfg::W_BYTES + Cfg::X_BYTES + Cfg::SF_BYTES; },
-            [&](uint32_t st, uint32_t ph) { mbar_wait(empty_bar(st), ph ^ 1u, ctx, WB_DEV_TIMEOUT_PRODUCER); },
-            [&](uint32_t st) { mbar_arrive(full_bar(st)); });
-      }
+      feed_row_scales<STAGES>(
+          p.x_scales, lane, head_kbs, nkb, u1 - u0, stage, phase,
+          [&](uint32_t st) { return smem_base + st * Cfg::STAGE_BYTES + Cfg::W_BYTES + Cfg::X_BYTES + Cfg::SF_BYTES; },
+          [&](uint32_t st, uint32_t ph) { mbar_wait(empty_bar(st), ph ^ 1u, ctx, WB_DEV_TIMEOUT_PRODUCER); },
+          [&](uint32_t st) { mbar_arrive(full_bar(st)); });
     }
   } else {
     // ------------------------------------------------------------------ epilogue warps 2..5

@@ -353,7 +353,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
       for (int seq = 0;; ++seq) {
         if (next_tile(seq) < 0) break;
         feed_row_scales<STAGES>(
-            maps.x_scales, lane, 0, p.num_kb, stage, phase,
+            maps.x_scales, lane, 0, p.num_kb, p.num_kb, stage, phase,
             [&](uint32_t st) { return smem_base + st * Cfg::STAGE_BYTES + Base::W_BYTES + Base::X_BYTES + Base::SF_BYTES; },
             [&](uint32_t st, uint32_t ph) { mbar_wait(empty_bar(st), ph ^ 1u, ctx, WB_DEV_TIMEOUT_PRODUCER); },
             [&](uint32_t st) { mbar_arrive(full_bar(st)); });
