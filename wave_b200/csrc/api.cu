@@ -153,6 +153,11 @@ struct PendingRowScales {
 };
 static thread_local PendingRowScales tl_row_scales;
 static int pack_row_scales(int M, int K, cudaStream_t stream);
+// The decode kernels take them as they are where they can be read eight bytes at a time; byte by byte the scale warp is slower than
+// the repack kernel it replaces (15 x 5803 x 5344, pitch 167 bytes, from a graph: 14.3 against 12.6 us).
+static bool takes_row_scales() {
+  return tl_row_scales.src && (reinterpret_cast<uintptr_t>(tl_row_scales.src) & 7) == 0 && tl_row_scales.stride % 8 == 0;
+}
 static wb::RowScales row_scales_param(int M, int K) {
   wb::RowScales s;
   s.base = static_cast<const uint8_t*>(tl_row_scales.src);
@@ -821,7 +826,7 @@ template <int NP, int STAGES, typename OutT, int EB = 4>
 int launch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
                   const void* bs, void* c, long long ldc, void* ws, int accumulate, cudaStream_t stream, int elem_format = 0) {
   if constexpr (EB == 4 && NP <= wb::kRowScaleRows) {
-    if (tl_row_scales.src)
+    if (takes_row_scales())
       return launch_skinny_scales<NP, STAGES, OutT, EB, true>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
   }
   if (int rc = pack_row_scales(M, K, stream)) return rc;
@@ -924,7 +929,7 @@ template <int NP, int STAGES, typename OutT, int EB = 4, int WR = 128, int SBUFS
 int launch_skinny_whole(const DeviceInfo& dev, int M, int N, int K, const void* a, const void* as, const void* b,
                         const void* bs, void* c, long long ldc, void* ws, int accumulate, cudaStream_t stream, int elem_format = 0) {
   if constexpr (EB == 4 && NP <= wb::kRowScaleRows) {
-    if (tl_row_scales.src)
+    if (takes_row_scales())
       return launch_skinny_whole_maps<NP, STAGES, OutT, EB, WR, SBUFS, wb::SkinnyRowScaleMaps>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate,
                                                                                                stream, elem_format);
   }
@@ -1099,9 +1104,9 @@ int dispatch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, c
 enum class DecodeRoute { kSkinny, kTile1, kTile2, kCluster };
 // The K-split kernel keeps all SMs streaming, but every CTA ends with partial tiles of M x 128 sums that meet in memory: with
 // M = 64 that costs more than the stream (64 x 2048 x 4096: 51 us), and with few K blocks per SM at M = 16 too. It is
-// the fastest only up to 16 rows and from eight 256-deep K blocks per SM up. us, K split against the tile kernel:
+// the fastest only up to 16 rows and from six 256-deep K blocks per SM up. us, K split against the tile kernel:
 //   M = 16: N x K = 1024 x 1024 8.7 / 4.8, 2048 x 4096 19.0 / 7.8, 4096 x 4096 12.5 / 8.8, 8192 x 1024 11.0 / 5.3;
-//           14336 x 4096 12.1 / 13.4, 4096 x 14336 14.3 / 18.3, 8192 x 8192 13.5 / 16.2, 16384 x 16384 28.6 / 30.5
+//           5803 x 5344 (M = 15) 12.6 / 14.8, 14336 x 4096 12.1 / 13.4, 4096 x 14336 14.3 / 18.3, 8192 x 8192 13.5 / 16.2, 16384 x 16384 28.6 / 30.5
 //   M = 32: 4096 x 4096 16.9 / 9.0, 8192 x 8192 16.4 / 13.2, 14336 x 4096 14.1 / 13.1, 16384 x 16384 30.5 / 30.9
 //   M = 128: 1024 x 8192 101 / 11.3, 4096 x 4096 48.0 / 9.0, 8192 x 8192 30.8 / 13.5, 16384 x 16384 43.5 / 31.5
 // Of the tile kernels, CTA pairs (256 x 128 tiles) fetch the weights of a tile through two SMs: ahead from 16 K blocks up
@@ -1111,7 +1116,7 @@ DecodeRoute decode_route(int sm_count, int M, int N, int K) {
   const int tiles = (N + 127) / 128, kb = (K + 255) / 256;
   if (tiles >= sm_count) return DecodeRoute::kSkinny;
   if (cluster_splitk_slices(M, N, K)) return DecodeRoute::kCluster;
-  if (M <= 16 && (long long)tiles * kb >= 8ll * sm_count) return DecodeRoute::kSkinny;
+  if (M <= 16 && (long long)tiles * kb >= 6ll * sm_count) return DecodeRoute::kSkinny;
   return tiles * 2 <= sm_count && kb >= 16 ? DecodeRoute::kTile2 : DecodeRoute::kTile1;
 }
 
