@@ -488,6 +488,23 @@ def test_224_wide_tiles_on_weight_scales_packed_for_them(shape, out_dtype):
     ops.check_device_status()
 
 
+@pytest.mark.parametrize("shape", [(256, 448, 10240), (300, 1000, 16000), (129, 224, 12288), (700, 900, 10272)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_224_wide_tiles_with_few_tiles_and_a_long_k(shape, out_dtype):
+    """The sizes at which the usual packing of the weight scales goes to the cluster split-K kernel, whose 128-wide tiles cannot
+    read a packing per 224 rows: the call stays on the 224-wide tile kernel. One N tile, several, and a ragged last one."""
+    M, N, K = shape
+    a, a_s, b, b_s = random_problem(M, N, K, seed=M + N)
+    ad, bd, a_sf = a.to(DEV), b.to(DEV), ops.repack_scales(a_s.to(DEV))
+    c224 = torch.full((M, N), float("nan"), dtype=out_dtype, device=DEV)
+    ops.scaled_gemm_packed(ad, a_sf, bd, ops.repack_scales(b_s.to(DEV), tile_rows=224), c224)
+    check(c224, a, a_s, b, b_s)
+    c256 = torch.full((M, N), float("nan"), dtype=out_dtype, device=DEV)
+    ops.scaled_gemm_packed(ad, a_sf, bd, ops.repack_scales(b_s.to(DEV)), c256, _lib.PATH_TILE_2CTA)
+    bits = torch.int16 if out_dtype == torch.bfloat16 else torch.int32
+    assert torch.equal(c224.view(bits), c256.view(bits))
+
+
 def test_tiled_weight_scales_are_refused_where_no_kernel_reads_them():
     N, K = 28672, 256
     h = ops.decode_tile_rows(N)

@@ -1687,7 +1687,9 @@ int wb200_mxfp4_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
       return dispatch_skinny<float>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, workspace, accumulate, s);
     return dispatch_skinny<__nv_bfloat16>(*dev, M, N, K, a, a_scale_packed, b, b_scale_packed, c, ldc, workspace, accumulate, s);
   }
-  if ((flags & WB200_PATH_MASK) == WB200_PATH_AUTO && path == WB200_PATH_TILE_2CTA && !route_bn && !(flags & (WB200_TILE_N128 | WB200_TILE_N192))) {
+  // (the cluster kernel's 128-wide tiles read the usual packing of the weight scales only)
+  if ((flags & WB200_PATH_MASK) == WB200_PATH_AUTO && path == WB200_PATH_TILE_2CTA && !wide224 && !route_bn &&
+      !(flags & (WB200_TILE_N128 | WB200_TILE_N192))) {
     const int cluster_slices = cluster_splitk_slices(M, N, K);
     if (cluster_slices) {
       if (c_dtype == WB200_F32)
