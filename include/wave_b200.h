@@ -223,8 +223,9 @@ int wb200_silu_and_mul(const void* x1, const void* x2, long long ld1, long long 
  * rows; w2[e]: [N, inter/2]; w1_scale / w2_scale: their scales from wb200_repack_scales (HOST arrays of device
  * pointers). The gate|up GEMM rounds its sums to bf16 and writes silu(gate) * up already quantised, the codes of
  * wb200_mxfp4_moe_gemm + wb200_silu_and_mul.
- * w1_scale_decode (may be NULL; used for T <= 128): w1's scales packed in the row order of 128-row tiles of 64 gate rows
- * and the 64 up rows of the same hidden columns. Limits: E <= 32, inter % 128 == 0, K % 32 == 0, N % 32 == 0.
+ * Every call reads the weights and scales as they are in memory then. w1_scale_decode is not read (pass NULL): the form for
+ * T <= 128 took a second packing of w1's scales from it, which could fall behind w1_scale.
+ * Limits: E <= 32, inter % 128 == 0, K % 32 == 0, N % 32 == 0.
  * workspace: 16-byte aligned, of the size the first function returns (0 for arguments outside the limits). */
 size_t wb200_mxfp4_expert_mlp_workspace_bytes(int T, int E, int K, int inter, int N, int top_k);
 int wb200_mxfp4_expert_mlp(int T, int E, int K, int inter, int N, int top_k, const void* x, int x_dtype, long long ldx,

@@ -12,6 +12,7 @@ from conftest import GOLDEN
 from oracle import moe_oracle
 from oracle import mxfp4_oracle as orc
 from wave_b200 import moe, ops
+from wave_b200.grouped import ExpertWeights
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -348,4 +349,46 @@ def test_expert_mlp_single_call_form_special_logits(T):
     first = torch.full((T, E), -30.0, device=DEV)
     first[:, :k] = 0.0
     torch.testing.assert_close(mlp(x, tied).float() * 3.0, mlp(x, first).float(), rtol=2 ** -7, atol=1e-6)
+    ops.check_device_status()
+
+
+def _small_expert_mlp(seed, E=4, K=256, inter=128, N=96, k=2):
+    g = torch.Generator().manual_seed(seed)
+    w1 = [orc.quantize_mxfp4(torch.randn(2 * inter, K, generator=g) * 0.05) for _ in range(E)]
+    w2 = [orc.quantize_mxfp4(torch.randn(N, inter, generator=g) * 0.05) for _ in range(E)]
+    mlp = wb.MXFP4ExpertMLP([q.to(DEV) for q, _ in w1], [s.to(DEV) for _, s in w1], [q.to(DEV) for q, _ in w2], [s.to(DEV) for _, s in w2],
+                            top_k=k)
+    return w1, w2, mlp
+
+
+@pytest.mark.parametrize("T", [1, 16, 128, 200])
+@pytest.mark.parametrize("how", ["object", "in place", "in place under a graph"])
+def test_expert_mlp_reads_the_weights_as_they_are_at_the_call(T, how):
+    """Weights replaced between two calls, as another object, in place, and in place between the capture and the replay of a
+    graph: the second result is that of the new weights (other codes and other scales), at decode and prefill sizes.
+    Tolerance as in test_expert_mlp_single_call_form."""
+    k = 2
+    _, w2, mlp = _small_expert_mlp(1, k=k)
+    new = [(q, s + 2) for q, s in _small_expert_mlp(2, k=k)[0]]
+    g = torch.Generator().manual_seed(3)
+    x, logits = torch.randn(T, mlp.K, generator=g).to(torch.bfloat16), torch.randn(T, mlp.E, generator=g)
+    xd, ld = x.to(DEV), logits.to(DEV)
+    mlp(xd, ld)
+    if how.endswith("graph"):
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = mlp(xd, ld)
+    if how == "object":
+        mlp.w1 = ExpertWeights([q.to(DEV) for q, _ in new], [s.to(DEV) for _, s in new])
+    else:
+        for e, (q, s) in enumerate(new):
+            mlp.w1.b[e].copy_(q)
+            ops.repack_scales(s.to(DEV), out=mlp.w1.b_sf[e].data)
+    if how.endswith("graph"):
+        graph.replay()
+    else:
+        out = mlp(xd, ld)
+    ref = moe_oracle.expert_mlp(x, [q for q, _ in new], [s for _, s in new], [q for q, _ in w2], [s for _, s in w2], logits, k)
+    assert float((out.cpu().float() - ref).norm() / ref.norm()) < 1.5e-2
     ops.check_device_status()

@@ -953,7 +953,8 @@ int launch_skinny_experts(const DeviceInfo& dev, const RoutedGemm& g, int T, voi
                            Maps::kSilu ? g.N : ldc)))
       return rc;
     if ((rc = make_operand_map(&maps.w[e], g.b_ptrs[e], g.N, g.K / 2, Maps::kSilu ? 64 : 128))) return rc;
-    if ((rc = make_scale_map(&maps.sfw[e], g.b_sf_ptrs[e], tiles_n, k_atoms, 1, Base::SF_ATOMS))) return rc;
+    if constexpr (Maps::kSilu) maps.w_scale[e] = static_cast<const uint8_t*>(g.b_sf_ptrs[e]);
+    else if ((rc = make_scale_map(&maps.sfw[e], g.b_sf_ptrs[e], tiles_n, k_atoms, 1, Base::SF_ATOMS))) return rc;
   }
   if ((rc = make_operand_map(&maps.x, g.a, g.max_rows, g.K / 2, NP))) return rc;
   if ((rc = make_scale_map(&maps.sfx, g.a_sf, wb::sf_row_blocks(g.max_rows), k_atoms, 1, Base::SF_ATOMS))) return rc;
@@ -963,6 +964,8 @@ int launch_skinny_experts(const DeviceInfo& dev, const RoutedGemm& g, int T, voi
   maps.num_rows = g.num_rows;
   wb::SkinnyWholeParams p = {};
   if constexpr (Maps::kSilu) {
+    maps.sfw[0] = maps.sfx;  // not used
+    maps.w_k_atoms = k_atoms;
     maps.inter = hidden->inter;
     maps.k_atoms = wb::sf_k_atoms(hidden->inter);
     maps.q = static_cast<uint8_t*>(hidden->q);
@@ -988,7 +991,7 @@ int launch_skinny_experts(const DeviceInfo& dev, const RoutedGemm& g, int T, voi
   const long long items = (long long)maps.max_blocks * tiles_n;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(items < dev.sm_count ? items : dev.sm_count), 1, 1);
-  cfg.blockDim = dim3(192, 1, 1);
+  cfg.blockDim = dim3(Maps::kScaleWarp ? 224 : 192, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -1911,12 +1914,12 @@ struct ExpertMlpPlan {
   int block, cap;  // rows per routing block, rows of the routed matrices (the worst case of the routing)
   size_t counters, weight, ids, inverse, expert_ids, num_rows, a, a_sf, q, q_sf, y, total;
 };
-static ExpertMlpPlan plan_expert_mlp(int T, int E, int K, int inter, int N, int top_k, bool decode_packing) {
+static ExpertMlpPlan plan_expert_mlp(int T, int E, int K, int inter, int N, int top_k) {
   ExpertMlpPlan p;
   const long long n = (long long)T * top_k;
   // At most 128 tokens: no expert can get more than one 128-row block, and the decode kernel streams the weights once
   // (16 tokens, 8 experts, top-2, K = 4096, inter = 7168: 75 us against 186 us in 256-row tiles and single steps).
-  p.decode = decode_packing && T <= wb::kExpertBlockRows;
+  p.decode = T <= wb::kExpertBlockRows;
   p.block = p.decode ? wb::kExpertBlockRows : 256;
   const long long blocks = p.decode ? (n < E ? n : E) : (n + (long long)E * 255 + 255) / 256;
   p.cap = int(blocks * p.block);
@@ -1948,7 +1951,7 @@ static int check_expert_mlp(int T, int E, int K, int inter, int N, int top_k) {
 
 size_t wb200_mxfp4_expert_mlp_workspace_bytes(int T, int E, int K, int inter, int N, int top_k) {
   if (check_expert_mlp(T, E, K, inter, N, top_k)) return 0;
-  return std::max(plan_expert_mlp(T, E, K, inter, N, top_k, true).total, plan_expert_mlp(T, E, K, inter, N, top_k, false).total);
+  return plan_expert_mlp(T, E, K, inter, N, top_k).total;
 }
 
 int wb200_mxfp4_expert_mlp(int T, int E, int K, int inter, int N, int top_k, const void* x, int x_dtype, long long ldx,
@@ -1965,7 +1968,7 @@ int wb200_mxfp4_expert_mlp(int T, int E, int K, int inter, int N, int top_k, con
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (ldx * (x_dtype == WB200_F32 ? 4 : 2)) % 16 != 0)
     return fail(WB200_ERR_ALIGNMENT, "expert_mlp: x rows must be 16-byte aligned");
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return fail(WB200_ERR_ALIGNMENT, "expert_mlp: the workspace must be 16-byte aligned");
-  const ExpertMlpPlan plan = plan_expert_mlp(T, E, K, inter, N, top_k, w1_scale_decode != nullptr);
+  const ExpertMlpPlan plan = plan_expert_mlp(T, E, K, inter, N, top_k);
   if (workspace_bytes < plan.total) return fail(WB200_ERR_WORKSPACE, "expert_mlp: workspace of %zu bytes needed (got %zu)", plan.total, workspace_bytes);
   DeviceInfo* dev;
   if ((rc = get_device(&dev))) return rc;
@@ -2002,7 +2005,7 @@ int wb200_mxfp4_expert_mlp(int T, int E, int K, int inter, int N, int top_k, con
     DependentScope() { tl_dependent_launch = true; }
     ~DependentScope() { tl_dependent_launch = saved; }
   } dependent_scope;
-  const RoutedGemm up{E, plan.cap, expert_ids, num_rows, 2 * inter, K, ws + plan.a, ws + plan.a_sf, w1, plan.decode ? w1_scale_decode : w1_scale};
+  const RoutedGemm up{E, plan.cap, expert_ids, num_rows, 2 * inter, K, ws + plan.a, ws + plan.a_sf, w1, w1_scale};
   const RoutedGemm down{E, plan.cap, expert_ids, num_rows, N, inter, ws + plan.q, ws + plan.q_sf, w2, w2_scale};
   const HiddenOut hidden{inter, ws + plan.q, ws + plan.q_sf};
   void* y = ws + plan.y;

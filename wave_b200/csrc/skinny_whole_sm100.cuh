@@ -64,14 +64,14 @@ struct SkinnyWholeParams {
 
 // The tensor maps of a launch over one weight.
 struct SkinnyMaps {
-  static constexpr bool kExperts = false, kSilu = false, kRowScales = false;
+  static constexpr bool kExperts = false, kSilu = false, kRowScales = false, kScaleWarp = false;
   CUtensorMap w, sfw;  // weights and their packed scales
   CUtensorMap x, sfx;  // activations and their packed scales
   CUtensorMap c;
 };
 // The same with the activations' scales row-major (sfx is not used): a seventh warp brings them into the stages.
 struct SkinnyRowScaleMaps : SkinnyMaps {
-  static constexpr bool kRowScales = true;
+  static constexpr bool kRowScales = true, kScaleWarp = true;
   RowScales x_scales;
 };
 // A decode step of a mixture-of-experts layer (at most 128 tokens, so at most 128 rows per expert): the tiles of every
@@ -81,12 +81,15 @@ struct SkinnyRowScaleMaps : SkinnyMaps {
 // real, in whole waves of 74 CTA pairs; here the weights are streamed once at the decode kernel's rate: the whole MLP of 16
 // tokens, 8 experts, top-2, K = 4096, inter = 7168 (371 MB of weights) went from 186 to 75 us per call.
 // Silu form: w holds `inter` gate rows and then `inter` up rows; a tile is 64 gate rows (lanes 0 .. 63) and the 64 up rows
-// of the same hidden columns (lanes 64 .. 127), its scales packed in that row order, and what leaves is silu(gate) * up
-// quantised: codes q [rows, inter / 2] and packed scales. inter % 64 == 0.
+// of the same hidden columns (lanes 64 .. 127), whose scales a seventh warp joins from the usual packing
+// (feed_gate_up_scales), and what leaves is silu(gate) * up quantised: codes q [rows, inter / 2] and packed scales.
+// inter % 128 == 0.
 template <int G, bool SILU>
 struct SkinnyExpertMaps {
-  static constexpr bool kExperts = true, kSilu = SILU, kRowScales = false;
-  CUtensorMap w[G], sfw[G];
+  static constexpr bool kExperts = true, kSilu = SILU, kRowScales = false, kScaleWarp = SILU;
+  CUtensorMap w[G], sfw[SILU ? 1 : G];
+  const uint8_t* w_scale[SILU ? G : 1];  // packed scales of [2 inter, K]
+  int w_k_atoms;
   CUtensorMap x, sfx;
   CUtensorMap c;
   int num_groups;
@@ -101,7 +104,7 @@ struct SkinnyExpertMaps {
 constexpr int kExpertBlockRows = 128;
 
 template <int NP, int STAGES, typename OutT, int EB = 4, int WR = 128, int SBUFS = 2, typename Maps = SkinnyMaps>
-__global__ void __launch_bounds__(Maps::kRowScales ? 224 : 192, 1)
+__global__ void __launch_bounds__(Maps::kScaleWarp ? 224 : 192, 1)
 mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholeParams p) {
   using Base = SkinnyCfg<NP, STAGES, EB, WR>;
   using Cfg = SkinnyWholeCfg<NP, STAGES, EB, WR, SBUFS>;
@@ -141,8 +144,8 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
       uint32_t count = 1;                                  // full / empty stage, accumulator full, tile number written
       const int q = b - 2 * STAGES;
       if (q >= 2 && q < 4) count = 4;                       // accumulator drained: one arrival per epilogue warp
-      else if (q >= 4 + IQ && q < 4 + 2 * IQ) count = 5 + (Maps::kRowScales ? 1 : 0);  // tile number read by the MMA, epilogue and scale warps
-      else if (Maps::kRowScales && b < STAGES) count = 2;   // a stage's loads, and its activation scales
+      else if (q >= 4 + IQ && q < 4 + 2 * IQ) count = 5 + (Maps::kScaleWarp ? 1 : 0);  // tile number read by the MMA, epilogue and scale warps
+      else if (Maps::kScaleWarp && b < STAGES) count = 2;   // a stage's loads, and what the scale warp brings
       mbar_init(bar_base + 8u * b, count);
     }
     if (lane == 0) *abort_flag = 0u;
@@ -173,7 +176,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
       const int e = __ldcg(maps.expert_ids + block);
       if (e < 0 || e >= maps.num_groups) return false;  // never written by a correct router; do not index out of the table
       tm_w = &maps.w[e];
-      tm_sfw = &maps.sfw[e];
+      if constexpr (!Maps::kSilu) tm_sfw = &maps.sfw[e];
     } else {
       w_tile = item;
       tm_w = &maps.w;
@@ -195,7 +198,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
       // and the epilogue keeps the tile's own columns
       // (4-bit weights expanded by the copy engine, EB == 8 only, count with their packed size: 64 bytes per row)
       if (part != 1)
-        mbar_expect_tx(fb, Cfg::STAGE_BYTES - Base::W_BYTES - (Maps::kRowScales ? Base::SF_BYTES : 0) + uint32_t(p.tile_rows) * ((EB == 8 && (p.elem_format & 0x10)) ? 64u : 128u));
+        mbar_expect_tx(fb, Cfg::STAGE_BYTES - Base::W_BYTES - (Maps::kScaleWarp ? Base::SF_BYTES : 0) + uint32_t(p.tile_rows) * ((EB == 8 && (p.elem_format & 0x10)) ? 64u : 128u));
       if (part != 2) {
         if constexpr (Maps::kSilu) {
           tma_load_2d_hint(sW, tm_w, kb * 128, w_tile * 64, fb, stream_policy);
@@ -203,7 +206,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
         } else {
           tma_load_2d_hint(sW, tm_w, kb * 128, w_tile * p.tile_rows, fb, stream_policy);
         }
-        tma_load_2d(sSFW, tm_sfw, kb * (Base::SF_ATOMS * 128), w_tile, fb);
+        if constexpr (!Maps::kSilu) tma_load_2d(sSFW, tm_sfw, kb * (Base::SF_ATOMS * 128), w_tile, fb);
       }
       if (part != 1) {
         tma_load_2d_hint(sX, &maps.x, kb * 128, block * kExpertBlockRows, fb, keep_policy);
@@ -344,8 +347,25 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
-  } else if (Maps::kRowScales && warp == 6) {
-    // ------------------------------------------------------------------ the activations' scales, row-major, into the stages
+  } else if (Maps::kScaleWarp && warp == 6) {
+    // ------------------------------------------------------------------ scales that the copy engine cannot bring as the MMA reads them
+    if constexpr (Maps::kSilu) {
+      if (p.dependent) pdl_wait();  // the routing arrays are the kernels' before this one
+      uint32_t stage = 0, phase = 0;
+      for (int seq = 0;; ++seq) {
+        const int item = next_tile(seq);
+        if (item < 0) break;
+        const int blk = item / p.tiles_n, nt = item - blk * p.tiles_n;
+        const int e = __ldcg(maps.expert_ids + blk);  // (an item the producer has located: a valid expert)
+        const uint8_t* gate = maps.w_scale[e] + size_t(nt >> 1) * maps.w_k_atoms * 512 + lane * 16 + (nt & 1) * 8;
+        feed_gate_up_scales<STAGES>(
+            gate, gate + size_t(maps.inter >> 7) * maps.w_k_atoms * 512, lane, p.num_kb, stage, phase,
+            [&](uint32_t st) { return smem_base + st * Cfg::STAGE_BYTES + Base::W_BYTES + Base::X_BYTES; },
+            [&](uint32_t st, uint32_t ph) { mbar_wait(empty_bar(st), ph ^ 1u, ctx, WB_DEV_TIMEOUT_PRODUCER); },
+            [&](uint32_t st) { mbar_arrive(full_bar(st)); });
+      }
+    }
+    // the activations' scales, row-major, into the stages
     if constexpr (Maps::kRowScales) {
       static_assert(EB == 4 && NP <= kRowScaleRows, "a stage of 256 K, one row per lane");
       if (p.dependent) pdl_wait();

@@ -15,7 +15,6 @@ the alignment kernel wrote, so a forward pass has no host synchronisation.
 
 from __future__ import annotations
 
-import ctypes
 from dataclasses import dataclass
 
 import torch
@@ -172,20 +171,6 @@ class MXFP4ExpertMLP:
             raise ValueError("w1 must be [E][2 I, K/2] and w2 [E][K_out, I/2] for the same E and I")
         self.top_k = top_k
         self.E, self.K, self.I = len(self.w1), self.w1.K, self.w1.N // 2
-        # The single-call path (one native entry, fused kernels) covers what its kernels are built for; anything else runs
-        # the same steps one by one.
-        self._fused = self.E <= 32 and self.I % 128 == 0 and self.w2.N % 32 == 0
-        if self._fused:
-            # decode packing of w1's scales: the row order of tiles of 64 gate rows and the 64 up rows of the same columns
-            self._w1_decode = [self._decode_scales(p) for p in self.w1.b_sf]
-            self._w1_decode_ptrs = (ctypes.c_void_p * self.E)(*[t.data_ptr() for t in self._w1_decode])
-
-    def _decode_scales(self, packed: ops.PackedScales) -> torch.Tensor:
-        """Packed scales of [2 I, K] in blocks of 128 rows -> blocks of 64 gate rows and the matching 64 up rows. A block
-        holds, per atom, 32 lines of four 4-byte words, one word per group of 32 rows."""
-        blocks = self.I // 128
-        words = packed.data.view(torch.int32).view(2, blocks, -1, 32, 2, 2)  # half, block, atom, line, 64-row half, group
-        return words.permute(1, 4, 2, 3, 0, 5).contiguous().view(-1)  # block, 64-row half, atom, line, gate|up, group
 
     def route(self, router_logits: torch.Tensor):
         score = torch.softmax(router_logits, dim=-1, dtype=torch.float32)
@@ -193,11 +178,15 @@ class MXFP4ExpertMLP:
         return weight.contiguous(), ids.contiguous()
 
     def _takes_fused(self, x: torch.Tensor, logits: torch.Tensor) -> bool:
-        """What the native single call accepts; other inputs take the step-by-step form and its checks."""
-        return (self._fused and type(self).route is MXFP4ExpertMLP.route and 0 < self.top_k <= self.E and x.is_cuda and
+        """What the native single call (one entry, fused kernels) is built for; anything else takes the same steps one by one,
+        with their checks. w1 and w2 are looked at as they are now: a caller may have replaced them."""
+        w1, w2 = self.w1, self.w2
+        return (self.E <= 32 and self.I % 128 == 0 and w2.N % 32 == 0 and len(w1) == len(w2) == self.E and
+                (w1.N, w1.K, w2.K) == (2 * self.I, self.K, self.I) and
+                type(self).route is MXFP4ExpertMLP.route and 0 < self.top_k <= self.E and x.is_cuda and
                 x.dim() == 2 and x.shape[0] > 0 and x.shape[1] == self.K and x.dtype in ops._DTYPE_CODE and
                 tuple(logits.shape) == (x.shape[0], self.E) and logits.device == x.device and
-                self.w1.b[0].device == x.device and logits.dtype in (torch.float32, torch.bfloat16, torch.float16))
+                w1.b[0].device == x.device and logits.dtype in (torch.float32, torch.bfloat16, torch.float16))
 
     def _forward_fused(self, x: torch.Tensor, logits: torch.Tensor) -> torch.Tensor:
         lib = _lib.load()
@@ -216,7 +205,7 @@ class MXFP4ExpertMLP:
             _lib.check(lib.wb200_mxfp4_expert_mlp(
                 *shape, x.data_ptr(), ops._DTYPE_CODE[x.dtype], x.stride(0) if T > 1 else self.K, logits.data_ptr(),
                 ops._DTYPE_CODE[logits.dtype], logits.stride(0) if T > 1 else self.E, self.w1._b_ptrs, self.w1._sf_ptrs,
-                self._w1_decode_ptrs, self.w2._b_ptrs, self.w2._sf_ptrs, out.data_ptr(), N, ws.data_ptr(), nbytes, _stream()))
+                None, self.w2._b_ptrs, self.w2._sf_ptrs, out.data_ptr(), N, ws.data_ptr(), nbytes, _stream()))
         return out
 
     def forward(self, x: torch.Tensor, router_logits: torch.Tensor) -> torch.Tensor:
