@@ -392,3 +392,24 @@ def test_expert_mlp_reads_the_weights_as_they_are_at_the_call(T, how):
     ref = moe_oracle.expert_mlp(x, [q for q, _ in new], [s for _, s in new], [q for q, _ in w2], [s for _, s in w2], logits, k)
     assert float((out.cpu().float() - ref).norm() / ref.norm()) < 1.5e-2
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("T", [16, 200])
+@pytest.mark.parametrize("where", ["instance", "subclass", "class"])
+def test_expert_mlp_calls_the_router_it_was_given(T, where, monkeypatch):
+    """A `route` of the caller's own, wherever it was set, decides the experts: negated logits through the library's router
+    give the result of the same logits through a router that negates them. Both sides run the same GEMMs on the same codes;
+    the weights may differ in the last bits of the softmax, an output by one rounding to bf16."""
+    mlp = _small_expert_mlp(1)[2]
+    g = torch.Generator().manual_seed(T)
+    x, logits = torch.randn(T, mlp.K, generator=g).to(torch.bfloat16).to(DEV), torch.randn(T, mlp.E, generator=g).to(DEV)
+    expected = mlp(x, -logits).float()
+    library = wb.MXFP4ExpertMLP.route
+    if where == "instance":
+        mlp.route = lambda r: library(mlp, -r)
+    elif where == "subclass":
+        mlp.__class__ = type("Routed", (wb.MXFP4ExpertMLP,), {"route": lambda self, r: library(self, -r)})
+    else:
+        monkeypatch.setattr(wb.MXFP4ExpertMLP, "route", lambda self, r: library(self, -r))
+    out = mlp(x, logits).float()
+    assert bool(((out - expected).abs() <= 2 ** -7 * expected.abs() + 1e-6 * expected.abs().max()).all())
