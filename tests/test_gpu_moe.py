@@ -413,3 +413,15 @@ def test_expert_mlp_calls_the_router_it_was_given(T, where, monkeypatch):
         monkeypatch.setattr(wb.MXFP4ExpertMLP, "route", lambda self, r: library(self, -r))
     out = mlp(x, logits).float()
     assert bool(((out - expected).abs() <= 2 ** -7 * expected.abs() + 1e-6 * expected.abs().max()).all())
+
+
+@pytest.mark.parametrize("T", [1, 16, 200])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_expert_mlp_takes_logits_with_overlapping_rows(T, dtype):
+    """Logits whose rows share memory: one row for all tokens (stride 0), and rows that start one expert apart."""
+    mlp = _small_expert_mlp(1)[2]
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, mlp.K, generator=g).to(torch.bfloat16).to(DEV)
+    flat = torch.randperm(T + mlp.E, generator=g).to(dtype).to(DEV)
+    for logits in (flat[:mlp.E].expand(T, mlp.E), flat.as_strided((T, mlp.E), (1, 1)), flat[:mlp.E].flip(0).expand(T, mlp.E)):
+        assert torch.equal(mlp(x, logits), mlp(x, logits.contiguous()))

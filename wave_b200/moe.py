@@ -194,7 +194,7 @@ class MXFP4ExpertMLP:
             x = x.contiguous()
         if logits.dtype == torch.float16:
             logits = logits.float()
-        if logits.stride(1) != 1:
+        if logits.stride(1) != 1 or (logits.shape[0] > 1 and logits.stride(0) < self.E):  # overlapping rows, as of an expanded bias
             logits = logits.contiguous()
         T, N = x.shape[0], self.w2.N
         shape = (T, self.E, self.K, self.I, N, self.top_k)
