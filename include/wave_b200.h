@@ -161,7 +161,8 @@ int wb200_repack_scales_grouped(const void* src, long long src_row_stride, int n
 /* Activation quantiser: x [rows, K] (f32 when x_dtype == WB200_F32, bf16 when WB200_BF16, row pitch ldx
  * elements, 16-byte aligned rows) -> packed E2M1 codes q [rows, K/2] and E8M0 scales, written row-major
  * (scale_rowmajor [rows, K/32], may be NULL) and/or in the packed layout the GEMM reads (scale_packed,
- * wb200_packed_scale_bytes(rows, K) bytes, may be NULL; padding bytes are filled too). Per 32-element
+ * wb200_packed_scale_bytes(rows, K) bytes, may be NULL; padding bytes are filled too). q is 4-byte aligned, the scale arrays
+ * may start at any byte (a GEMM that reads scale_packed wants it 16-byte aligned). Per 32-element
  * block: scale exponent floor(log2(amax)) - 2, values rounded to the nearest E2M1 value, ties to the even
  * code. The reference names this step as its direction ("fused dynamic quantization",
  * wave_lang/kernel/wave/templates/test_kernels.py:74) but ships no quantiser; its tests feed random
@@ -170,8 +171,8 @@ int wb200_quantize_mxfp4(const void* x, int x_dtype, long long ldx, int rows, in
                          void* scale_packed, void* stream);
 
 /* wb200_quantize_mxfp4 and wb200_mxfp4_gemm in one call, the GEMM launched as the programmatic dependent of the
- * quantiser: x [M, K] (f32 or bf16) is quantised to q_scratch [M, K/2] (16-byte aligned) and scale_scratch
- * (wb200_packed_scale_bytes(M, K)), and the GEMM's set-up, and on the M <= 128 path its first ring of weight loads, run
+ * quantiser: x [M, K] (f32 or bf16) is quantised to q_scratch [M, K/2] and scale_scratch
+ * (wb200_packed_scale_bytes(M, K)), both 16-byte aligned, and the GEMM's set-up, and on the M <= 128 path its first ring of weight loads, run
  * while the quantiser does. Other arguments as wb200_mxfp4_gemm; WB200_OVERLAP_PREVIOUS is refused. */
 int wb200_mxfp4_gemm_quantize_a(int M, int N, int K, const void* x, int x_dtype, long long ldx, void* q_scratch, void* scale_scratch,
                                 const void* b, const void* b_scale_packed, void* c, int c_dtype, long long ldc, void* workspace,

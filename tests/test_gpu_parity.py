@@ -691,6 +691,24 @@ def test_quantizer_bit_exact_against_oracle(rows, K, dtype):
     assert torch.equal(packed.data.cpu(), orc.pack_scales(es))
 
 
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 4, 12])
+@pytest.mark.parametrize("rows,K", [(1, 32), (130, 416)])
+def test_quantizer_writes_scale_arrays_that_start_at_any_byte(rows, K, offset):
+    """The C entry with both scale arrays `offset` bytes into a buffer: the oracle's bytes, padding included, and nothing beside them."""
+    x = torch.randn(rows, K, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16)
+    q_ref, s_ref = orc.quantize_mxfp4(x.float())
+    packed_ref = orc.pack_scales(s_ref)
+    xd, q = x.to(DEV), torch.empty(rows, K // 2, dtype=torch.uint8, device=DEV)
+    rm = torch.full((s_ref.numel() + 32,), 0xEE, dtype=torch.uint8, device=DEV)
+    pk = torch.full((packed_ref.numel() + 32,), 0xEE, dtype=torch.uint8, device=DEV)
+    _lib.check(_lib.load().wb200_quantize_mxfp4(xd.data_ptr(), _lib.WB200_BF16, K, rows, K, q.data_ptr(), rm.data_ptr() + offset,
+                                                pk.data_ptr() + offset, torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(q.cpu(), q_ref)
+    for buf, ref in ((rm.cpu(), s_ref.reshape(-1)), (pk.cpu(), packed_ref.reshape(-1))):
+        assert torch.equal(buf[offset:offset + ref.numel()], ref)
+        assert bool((buf[:offset] == 0xEE).all()) and bool((buf[offset + ref.numel():] == 0xEE).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_quantizer_marks_blocks_with_nan_or_inf(dtype):
     """A NaN or an infinity in a block gives scale byte 255 (E8M0's NaN) and codes 0, bit-exact against the oracle;

@@ -66,6 +66,10 @@ def test_argument_validation_returns_codes_and_messages(lib):
     assert lib.wb200_repack_scales(p16, 1, 16, 40, p16, None) == _lib.WB200_ERR_INVALID_ARG
     assert lib.wb200_repack_scales(None, 2, 16, 64, p16, None) == _lib.WB200_ERR_INVALID_ARG
     assert lib.wb200_repack_scales(p16, 1, 16, 64, p16, None) == _lib.WB200_ERR_INVALID_ARG
+    # quantise + GEMM: scratch that the GEMM cannot read is refused before the quantiser runs (there is no GPU here to run it on)
+    for q, sf in ((p16 + 4, p16), (p16, p16 + 1), (p16, p16 + 8)):
+        assert lib.wb200_mxfp4_gemm_quantize_a(16, 16, 64, p16, 0, 64, q, sf, p16, p16, p16, 0, 16, 0, 0, 0, None) == _lib.WB200_ERR_ALIGNMENT
+        assert b"16-byte aligned" in lib.wb200_last_error()
     with pytest.raises(ValueError):
         _lib.check(_lib.WB200_ERR_INVALID_ARG)
 

@@ -1745,7 +1745,10 @@ int wb200_mxfp4_gemm_quantize_a(int M, int N, int K, const void* x, int x_dtype,
   if (!scale_scratch) return fail(WB200_ERR_INVALID_ARG, "gemm_quantize_a: null scratch for the packed activation scales");
   if (flags & WB200_OVERLAP_PREVIOUS)  // the quantiser reads x at once
     return fail(WB200_ERR_INVALID_ARG, "gemm_quantize_a: WB200_OVERLAP_PREVIOUS is not available here");
-  int rc = wb200_quantize_mxfp4(x, x_dtype, ldx, M, K, q_scratch, nullptr, scale_scratch, stream);
+  // what the GEMM will refuse is refused before the quantiser writes anything
+  int rc = check_common(M, N, K, q_scratch, scale_scratch, b, b_scale_packed, c, c_dtype, ldc);
+  if (rc) return rc;
+  rc = wb200_quantize_mxfp4(x, x_dtype, ldx, M, K, q_scratch, nullptr, scale_scratch, stream);
   if (rc) return rc;
   tl_dependent_launch = true;  // the GEMM is the quantiser's programmatic dependent
   rc = wb200_mxfp4_gemm(M, N, K, q_scratch, scale_scratch, b, b_scale_packed, c, c_dtype, ldc, workspace, workspace_bytes, flags, stream);

@@ -267,9 +267,16 @@ quantize_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int K,
     if (sub == 0) words[g][warp] = scales;  // word (row of the pair, 32-row group) of the sector
     __syncthreads();
     const int atom = (kb0 >> 2) + (threadIdx.x >> 3);
-    if (threadIdx.x < 64 && atom < k_atoms)
-      reinterpret_cast<uint32_t*>(scale_packed + (size_t(group >> 4) * k_atoms + atom) * 512 + (group & 15) * 32)[threadIdx.x & 7] =
-          words[threadIdx.x >> 3][threadIdx.x & 7];
+    if (threadIdx.x < 64 && atom < k_atoms) {
+      uint8_t* d = scale_packed + (size_t(group >> 4) * k_atoms + atom) * 512 + (group & 15) * 32 + (threadIdx.x & 7) * 4;
+      const uint32_t word = words[threadIdx.x >> 3][threadIdx.x & 7];
+      if ((reinterpret_cast<uintptr_t>(scale_packed) & 3) == 0) {
+        *reinterpret_cast<uint32_t*>(d) = word;
+      } else {  // an array that a caller placed at any byte
+#pragma unroll
+        for (int u = 0; u < 4; ++u) d[u] = uint8_t(word >> (8 * u));
+      }
+    }
   }
 }
 
