@@ -425,3 +425,24 @@ def test_expert_mlp_takes_logits_with_overlapping_rows(T, dtype):
     flat = torch.randperm(T + mlp.E, generator=g).to(dtype).to(DEV)
     for logits in (flat[:mlp.E].expand(T, mlp.E), flat.as_strided((T, mlp.E), (1, 1)), flat[:mlp.E].flip(0).expand(T, mlp.E)):
         assert torch.equal(mlp(x, logits), mlp(x, logits.contiguous()))
+
+
+@pytest.mark.parametrize("num_rows", [1, 200, 256, 300, 511, 600])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_routed_gemm_with_a_row_count_inside_a_block(num_rows, out_dtype):
+    """num_rows that is not whole 256-row blocks (or lies past the buffers): the rows below it are computed, the blocks at or past it are
+    left alone."""
+    from test_gpu_parity import check, random_problem
+    R, N, K = 512, 320, 256
+    a, a_s, _, _ = random_problem(R, 1, K, seed=9)
+    weights = [random_problem(1, N, K, seed=10 + e)[2:] for e in range(2)]
+    experts = ExpertWeights([b.to(DEV) for b, _ in weights], [s.to(DEV) for _, s in weights])
+    c = torch.full((R, N), -1.0, dtype=out_dtype, device=DEV)
+    moe.moe_scaled_gemm(a.to(DEV), a_s.to(DEV), experts, torch.tensor([1, 0], dtype=torch.int32, device=DEV),
+                        torch.tensor([num_rows], dtype=torch.int32, device=DEV), c)
+    for block, (b, b_s) in ((0, weights[1]), (1, weights[0])):
+        lo, hi = 256 * block, min(256 * (block + 1), num_rows)
+        if lo < hi:
+            check(c[lo:hi], a[lo:hi], a_s[lo:hi], b, b_s)
+        else:
+            assert bool((c[lo:] == -1.0).all())

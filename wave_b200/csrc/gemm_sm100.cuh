@@ -206,13 +206,19 @@ __device__ __forceinline__ void raster_tile(int t, int tiles_m, int tiles_n, int
   nt = n0 + (r - mt * gw);
 }
 
-// Number of tile ids of this launch. Aligned form: from what the routing kernels wrote.
+// The rows of this launch: as a count of M tiles and, in the aligned form, as what the routing kernels wrote (a caller of the
+// grouped GEMM may end inside a tile).
+struct RowSpan {
+  int tiles_m, rows;
+};
+// Number of tile ids of this launch.
 template <typename Maps>
-__device__ __forceinline__ int count_tiles(const Maps& maps, const GemmParams& p, int& tiles_m) {
-  tiles_m = p.tiles_m;
+__device__ __forceinline__ int count_tiles(const Maps& maps, const GemmParams& p, RowSpan& span) {
+  span = {p.tiles_m, p.M};
   if constexpr (Maps::kAligned) {
-    tiles_m = min(maps.tiles_m_cap, __ldcg(maps.num_rows) / maps.tile_rows);
-    return tiles_m * p.tiles_n;
+    span.rows = min(maps.tiles_m_cap * maps.tile_rows, __ldcg(maps.num_rows));
+    span.tiles_m = (span.rows + maps.tile_rows - 1) / maps.tile_rows;
+    return span.tiles_m * p.tiles_n;
   } else if constexpr (Maps::kGrouped) {
     return maps.interleave ? maps.num_groups * maps.tiles_max : maps.tile_start[maps.num_groups];
   } else {
@@ -221,9 +227,9 @@ __device__ __forceinline__ int count_tiles(const Maps& maps, const GemmParams& p
 }
 
 // Tile id -> M tile, N tile, rows of its group; returns the group, or -1 for an id that names no tile (interleaved walk
-// over groups of unequal size). tiles_m: from count_tiles.
+// over groups of unequal size). span: from count_tiles.
 template <typename Maps>
-__device__ __forceinline__ int decode_tile(const Maps& maps, const GemmParams& p, int t, int tiles_m, int& mt, int& nt,
+__device__ __forceinline__ int decode_tile(const Maps& maps, const GemmParams& p, int t, const RowSpan& span, int& mt, int& nt,
                                            int& rows, void** c_base = nullptr) {
   if constexpr (!Maps::kGrouped) {
     raster_tile(t, p.tiles_m, p.tiles_n, p.group_n, mt, nt);
@@ -231,10 +237,10 @@ __device__ __forceinline__ int decode_tile(const Maps& maps, const GemmParams& p
     if (c_base) *c_base = p.c;
     return 0;
   } else if constexpr (Maps::kAligned) {
-    raster_tile(t, tiles_m, p.tiles_n, p.group_n, mt, nt);
+    raster_tile(t, span.tiles_m, p.tiles_n, p.group_n, mt, nt);
     const int e = __ldcg(maps.expert_ids + mt);
     if (e < 0 || e >= maps.num_groups) return -1;  // never written by a correct router; do not index out of the table
-    rows = tiles_m * maps.tile_rows;
+    rows = span.rows;
     if (c_base) *c_base = maps.c_base;
     return e;
   } else {
@@ -408,8 +414,8 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
 
   // The routing arrays of an aligned launch are written by the kernels before this one: every role waits for them.
   if constexpr (Maps::kAligned) pdl_wait();
-  int tiles_m;
-  const int num_tiles = count_tiles(maps, p, tiles_m);
+  RowSpan span;
+  const int num_tiles = count_tiles(maps, p, span);
   const int first_tile = (CG == 2) ? (blockIdx.x >> 1) : blockIdx.x;
   const int tile_step = (CG == 2) ? (gridDim.x >> 1) : gridDim.x;
   const int num_kb = (p.K + Cfg::BK - 1) / Cfg::BK;
@@ -424,7 +430,7 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
     pdl_wait();  // the packed activation scales may be written by the kernel launched just before this one
     for (int t = first_tile; t < num_tiles; t += tile_step) {
       int mt, nt, rows;
-      const int group = decode_tile(maps, p, t, tiles_m, mt, nt, rows);
+      const int group = decode_tile(maps, p, t, span, mt, nt, rows);
       if (Maps::kGrouped && group < 0) continue;
       const CUtensorMap *tm_a = maps.map(group, 0), *tm_b = maps.map(group, 1), *tm_sfa = maps.map(group, 2), *tm_sfb = maps.map(group, 3);
       const int a_row = (mt * CG + int(rank)) * Cfg::BM;
@@ -482,7 +488,7 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
         uint32_t sfb_group = 0;
         if constexpr ((BN % 128 != 0 && !Cfg::TILED_SFB) || Maps::kGrouped) {
           int mt, nt, rows;
-          if (decode_tile(maps, p, t, tiles_m, mt, nt, rows) < 0) continue;
+          if (decode_tile(maps, p, t, span, mt, nt, rows) < 0) continue;
           sfb_group = uint32_t((nt * BN) % 128) / 32u;
         }
         const int as = it & 1;
@@ -569,7 +575,7 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
     for (int t = first_tile; t < num_tiles; t += tile_step) {
       int mt, nt, rows;
       void* c_group = nullptr;
-      const int group = decode_tile(maps, p, t, tiles_m, mt, nt, rows, &c_group);
+      const int group = decode_tile(maps, p, t, span, mt, nt, rows, &c_group);
       if (Maps::kGrouped && group < 0) continue;
       const int as = it & 1;
       mbar_wait(acc_full_bar(as), uint32_t(it >> 1) & 1u, ctx, WB_DEV_TIMEOUT_EPILOGUE);
