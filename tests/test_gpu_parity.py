@@ -1092,6 +1092,39 @@ def test_overlap_previous_chain_gives_the_same_bits(shape):
     ops.check_device_status()
 
 
+def test_a_weight_quantised_two_launches_ahead_of_an_overlapping_gemm():
+    """quantise w -> GEMM on another weight -> GEMM on w, both GEMMs flagged WB200_OVERLAP_PREVIOUS: the kernel before the second
+    GEMM does not write w, so that GEMM may load w at once, and the quantiser has to be done by then. w's memory holds the
+    other of two weights before every round, so a value read too early is a wrong one."""
+    N, K, M = 16384, 8192, 16
+    lib, g = _lib.load(), torch.Generator(device=DEV).manual_seed(5)
+    ws = [torch.randn(N, K, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2)]
+    q, pk = torch.empty(N, K // 2, dtype=torch.uint8, device=DEV), torch.empty(ops.packed_scale_bytes(N, K), dtype=torch.uint8, device=DEV)
+    a, _, a_sf = ops.quantize_mxfp4(torch.randn(M, K, generator=g, device=DEV))
+    q1, _, sf1 = ops.quantize_mxfp4(torch.randn(1024, K, generator=g, device=DEV))
+    c1, w_sf = torch.empty(M, 1024, dtype=torch.bfloat16, device=DEV), ops.PackedScales(pk, N, K)
+
+    def quantise(w):
+        _lib.check(lib.wb200_quantize_mxfp4(w.data_ptr(), _lib.WB200_BF16, K, N, K, q.data_ptr(), None, pk.data_ptr(),
+                                            torch.cuda.current_stream().cuda_stream))
+
+    refs = []
+    for w in ws:
+        quantise(w)
+        torch.cuda.synchronize()
+        refs.append(torch.empty(M, N, dtype=torch.bfloat16, device=DEV))
+        ops.scaled_gemm_packed(a, a_sf, q, w_sf, refs[-1])
+    outs = [torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(6)]
+    for i, c in enumerate(outs):  # no synchronisation in between
+        quantise(ws[i & 1])
+        ops.scaled_gemm_packed(a, a_sf, q1, sf1, c1, _lib.OVERLAP_PREVIOUS)
+        ops.scaled_gemm_packed(a, a_sf, q, w_sf, c, _lib.OVERLAP_PREVIOUS)
+    torch.cuda.synchronize()
+    for i, c in enumerate(outs):
+        assert torch.equal(c.view(torch.int16), refs[i & 1].view(torch.int16))
+    ops.check_device_status()
+
+
 def test_run_bench_option_reports_kernel_time(tmp_path):
     """options.run_bench: after the call the kernel is timed on the device and the report goes to
     benchmark_results_file (the reference hands its module to a benchmark tool, compile.py:317-329)."""

@@ -1340,8 +1340,8 @@ int wb200_repack_scales_grouped(const void* src, long long src_row_stride, int n
   return WB200_OK;
 }
 
-int wb200_quantize_mxfp4(const void* x, int x_dtype, long long ldx, int rows, int K, void* q, void* scale_rowmajor,
-                         void* scale_packed, void* stream) {
+static int quantize_mxfp4_impl(const void* x, int x_dtype, long long ldx, int rows, int K, void* q, void* scale_rowmajor,
+                               void* scale_packed, bool release, void* stream) {
   if (rows <= 0 || K <= 0 || K % 32 != 0)
     return fail(WB200_ERR_INVALID_ARG, "quantize: rows = %d, K = %d (K must be a positive multiple of 32)", rows, K);
   if (!x || !q || (!scale_rowmajor && !scale_packed)) return fail(WB200_ERR_INVALID_ARG, "quantize: null pointer");
@@ -1360,13 +1360,18 @@ int wb200_quantize_mxfp4(const void* x, int x_dtype, long long ldx, int rows, in
   if (x_dtype == WB200_F32)
     wb::quantize_mxfp4_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), ldx, rows, K,
                                                             static_cast<uint8_t*>(q), q_vec, static_cast<uint8_t*>(scale_rowmajor),
-                                                            static_cast<uint8_t*>(scale_packed), k_atoms);
+                                                            static_cast<uint8_t*>(scale_packed), k_atoms, release);
   else
     wb::quantize_mxfp4_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(
         static_cast<const __nv_bfloat16*>(x), ldx, rows, K, static_cast<uint8_t*>(q), q_vec,
-        static_cast<uint8_t*>(scale_rowmajor), static_cast<uint8_t*>(scale_packed), k_atoms);
+        static_cast<uint8_t*>(scale_rowmajor), static_cast<uint8_t*>(scale_packed), k_atoms, release);
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
+}
+
+int wb200_quantize_mxfp4(const void* x, int x_dtype, long long ldx, int rows, int K, void* q, void* scale_rowmajor,
+                         void* scale_packed, void* stream) {
+  return quantize_mxfp4_impl(x, x_dtype, ldx, rows, K, q, scale_rowmajor, scale_packed, false, stream);
 }
 
 int wb200_moe_align_block_size(const void* topk_ids, int ids_are_int64, int num_ids, int num_experts, int block_size,
@@ -1748,7 +1753,7 @@ int wb200_mxfp4_gemm_quantize_a(int M, int N, int K, const void* x, int x_dtype,
   // what the GEMM will refuse is refused before the quantiser writes anything
   int rc = check_common(M, N, K, q_scratch, scale_scratch, b, b_scale_packed, c, c_dtype, ldc);
   if (rc) return rc;
-  rc = wb200_quantize_mxfp4(x, x_dtype, ldx, M, K, q_scratch, nullptr, scale_scratch, stream);
+  rc = quantize_mxfp4_impl(x, x_dtype, ldx, M, K, q_scratch, nullptr, scale_scratch, true, stream);
   if (rc) return rc;
   tl_dependent_launch = true;  // the GEMM is the quantiser's programmatic dependent
   rc = wb200_mxfp4_gemm(M, N, K, q_scratch, scale_scratch, b, b_scale_packed, c, c_dtype, ldc, workspace, workspace_bytes, flags, stream);

@@ -54,7 +54,7 @@ moe_align_block_size_kernel(const IdT* __restrict__ ids, int n, int E, int block
   __shared__ int totals[kMoeMaxExperts];
   __shared__ int starts[kMoeMaxExperts];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  pdl_launch_dependents();
+  if (dependent) pdl_launch_dependents();  // (in a chain of the library's own; see quantize_mxfp4_kernel)
   if (sorted_ids)
     for (int i = tid; i < sorted_cap; i += blockDim.x) sorted_ids[i] = n;
   for (int e = lane; e < E; e += 32) next[warp][e] = 0;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(256)
 moe_combine_kernel(const T* __restrict__ y, long long ldy, const int* __restrict__ row_of,
                    const float* __restrict__ weight, int tokens, int top_k, int cols, T* __restrict__ out,
                    long long ldo, int dependent) {
-  pdl_launch_dependents();
+  if (dependent) pdl_launch_dependents();  // (in a chain of the library's own; see quantize_mxfp4_kernel)
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int cvec = (cols + 7) >> 3;
   if (dependent) pdl_wait();

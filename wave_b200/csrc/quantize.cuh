@@ -227,12 +227,15 @@ __device__ __forceinline__ uint32_t* packed_scale_word(uint8_t* base, int k_atom
 // layout, so the words are exchanged through shared memory and every 32-byte sector is written once (a warp that writes its
 // own 8 words touches 8 sectors with 4 bytes each). Rows past `rows` (the padding rows of the packed scales) get the padding byte
 // only. x rows are 16-byte aligned; q rows 16-byte aligned when q_vec. Grid: 16 x row blocks x chunks of 32 K blocks.
+// release: the library launches this kernel's programmatic dependent right behind it, which waits before it reads a scale
+// or a code. Otherwise it does not let dependents start early: what it writes may be the WEIGHTS of a GEMM two launches
+// on, which WB200_OVERLAP_PREVIOUS allows to be read before that GEMM's wait.
 template <typename InT>
 __global__ void __launch_bounds__(256)
 quantize_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int K, uint8_t* __restrict__ q, int q_vec,
-                      uint8_t* __restrict__ scale_rm, uint8_t* __restrict__ scale_packed, int k_atoms) {
+                      uint8_t* __restrict__ scale_rm, uint8_t* __restrict__ scale_packed, int k_atoms, int release) {
   __shared__ uint32_t words[8][8];  // [atom of the chunk][word of the sector]
-  pdl_launch_dependents();
+  if (release) pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kblocks = K >> 5;
   const unsigned chunks = unsigned(k_atoms + 7) >> 3;
@@ -334,7 +337,7 @@ __global__ void __launch_bounds__(256)
 quantize_scatter_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int K, int copies,
                               const int* __restrict__ dst_rows, uint8_t* __restrict__ q, int q_vec, uint8_t* __restrict__ scale_rm,
                               uint8_t* __restrict__ scale_packed, int k_atoms, int dependent) {
-  pdl_launch_dependents();
+  if (dependent) pdl_launch_dependents();  // (in a chain of the library's own; see quantize_mxfp4_kernel)
   const int lane = threadIdx.x & 31;
   const int kblocks = K >> 5;
   const unsigned chunks = unsigned(k_atoms + 7) >> 3;
