@@ -566,6 +566,74 @@ def test_two_streams_run_skinny_gemms_at_the_same_time():
     ops.check_device_status()
 
 
+@pytest.mark.parametrize("kind,M,N,K", [("fp4", 64, 28672, 1024), ("fp4", 256, 4096, 4096), ("fp4", 16, 1024, 12320), ("fp8", 16, 14336, 2048),
+                                        ("mixed", 64, 28672, 2048), ("fp8", 300, 4096, 2048)])
+def test_two_streams_pack_activation_scales_at_the_same_time(kind, M, N, K):
+    """ONE kernel object called from two unordered streams at sizes whose activation scales are packed ahead of the GEMM (decode
+    above 32 rows, tile and cluster kernels, rows of scales that are not whole 8-byte words, 8-bit operands): every stream
+    packs into memory of its own. The scales of the two problems are powers of two apart, so that a block read from the
+    other one shows. Reference: the same call alone, bit for bit."""
+    g = torch.Generator().manual_seed(M + N)
+    if kind == "fp4":
+        kernel, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    else:
+        kernel, subs = wb.get_scaled_gemm_mxfp8_kernel((M, N, K), wb.ScaledMMAType.F32_16x16x128_F8F6F4, "f8e4m3fn", wb.bf16,
+                                                       weight_format="f4e2m1fn" if kind == "mixed" else None)
+        options = wb.WaveCompileOptions(subs=subs)
+    gemm = wb.wave_compile(wb.set_default_run_config(options), kernel)
+
+    def operand(rows, bits):
+        t = torch.randint(0, 256, (rows, K * bits // 8), dtype=torch.uint8, generator=g)
+        return (t if bits == 4 else (t & 0xBF).view(torch.float8_e4m3fn)).to(DEV)
+
+    b = operand(N, 8 if kind == "fp8" else 4)
+    b_s = torch.randint(124, 131, (N, K // 32), dtype=torch.uint8, generator=g).to(DEV)
+    xs = [(operand(M, 4 if kind == "fp4" else 8), torch.randint(110 + 20 * i, 115 + 20 * i, (M, K // 32), dtype=torch.uint8, generator=g).to(DEV))
+          for i in range(2)]
+    outs = [torch.empty(M, N, dtype=torch.bfloat16, device=DEV) for _ in xs]
+    refs = [torch.empty(M, N, dtype=torch.bfloat16, device=DEV) for _ in xs]
+    for (a, a_s), c in zip(xs, refs):
+        gemm(a, a_s, b, b_s, c)
+        torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(DEV) for _ in xs]
+    for rep in range(20):
+        for st, (a, a_s), c in zip(streams, xs, outs):
+            with torch.cuda.stream(st):
+                gemm(a, a_s, b, b_s, c)
+    torch.cuda.synchronize()
+    for c, ref in zip(outs, refs):
+        assert torch.equal(c.view(torch.int16), ref.view(torch.int16))
+    ops.check_device_status()
+
+
+def test_scratch_of_a_captured_call_outlives_a_larger_call():
+    """A graph holds the address of the scratch it packs into: a larger call on the same stream takes new memory and leaves the old
+    one to the graph, whatever is allocated afterwards."""
+    N, K = 4096, 2048
+    kernel, options = wb.get_tagged_mxfp4_gemm((64, N, K), output_dtype=wb.bf16)
+    options.dynamic_symbols = ["M"]
+    gemm = wb.wave_compile(wb.set_default_run_config(options), kernel)
+    a, a_s, b, b_s = (t.to(DEV) for t in random_problem(512, N, K, seed=77))
+    c = torch.empty(64, N, dtype=torch.bfloat16, device=DEV)
+    stream, graph = torch.cuda.Stream(DEV), torch.cuda.CUDAGraph()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        gemm(a[:64], a_s[:64], b, b_s, c)
+    torch.cuda.synchronize()
+    ref = c.clone()
+    with torch.cuda.graph(graph, stream=stream):
+        gemm(a[:64], a_s[:64], b, b_s, c)
+    small = list(gemm._a_scale_buf.values())[0][-1]
+    with torch.cuda.stream(stream):
+        gemm(a, a_s, b, b_s, torch.empty(512, N, dtype=torch.bfloat16, device=DEV))
+    torch.cuda.synchronize()
+    assert list(gemm._a_scale_buf.values())[0][0] is small and list(gemm._a_scale_buf.values())[0][-1] is not small
+    c.fill_(float("nan"))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(c.view(torch.int16), ref.view(torch.int16))
+
+
 # ---------------------------------------------------------------------------------------------
 # grouped (MoE) GEMM
 # ---------------------------------------------------------------------------------------------

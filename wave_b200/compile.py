@@ -119,7 +119,7 @@ class ScaledGemmKernel:
         self.options = options
         self.asm = ""  # the reference exposes generated code here; nothing is generated at run time
         self._weight_scales = ops.WeightScaleCache()
-        self._a_scale_buf: dict[int, torch.Tensor] = {}
+        self._a_scale_buf: dict[tuple[int, int], list[torch.Tensor]] = {}  # (device, stream) -> scratches, the one in use last
         self._workspaces = ops.WorkspacePool()  # this object's own: calls through another object may overlap with these
         self._plans: dict = {}
         self._tile_rows: dict = {}
@@ -320,14 +320,15 @@ class ScaledGemmKernel:
         return _lib.GROUP_N(max(1, min(254, (int(g) * block_n) // 256)))
 
     def _a_scale_buffer(self, device, M, K):
-        idx = device.index or 0
+        """Scratch for the packed activation scales of a call on the current stream: calls on other streams may overlap with it
+        and have their own. One that a larger call has outgrown stays (a captured graph may hold its address); as every
+        new one has at least twice the size, what stays is smaller than what is in use."""
+        idx = device.index if device.index is not None else torch.cuda.current_device()
         need = ops.packed_scale_bytes(M, K)
-        buf = self._a_scale_buf.get(idx)
-        if buf is None or buf.numel() < need:
-            buf = torch.empty(need, dtype=torch.uint8, device=device)
-            self._a_scale_buf[idx] = buf
-            self._plans.clear()  # plans hold the old buffer
-        return buf
+        bufs = self._a_scale_buf.setdefault((idx, torch.cuda.current_stream(idx).cuda_stream), [])
+        if not bufs or bufs[-1].numel() < need:
+            bufs.append(torch.empty(max(need, 2 * bufs[-1].numel()) if bufs else need, dtype=torch.uint8, device=device))
+        return bufs[-1]
 
     def _pack_activation_scales(self, a_scale, M, K):
         if isinstance(a_scale, ops.PackedScales):
