@@ -1160,6 +1160,42 @@ def test_overlap_previous_chain_gives_the_same_bits(shape):
     ops.check_device_status()
 
 
+@pytest.mark.parametrize("strided", [False, True])
+def test_overlap_previous_waits_for_the_weight_scales_the_call_packs_itself(strided):
+    """A call that has to pack its weight's scales puts a kernel that writes them in front of its GEMM: that call is not launched as
+    the kernel's early dependent, the next one is. Both through the remembered plan and through the general form (strided a)."""
+    M, N, K = 16, 28672, 512
+    a, a_s, b, b_s = random_problem(M, N, K, seed=3)
+    kernel, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    options.overlap_previous = True
+    gemm = wb.wave_compile(wb.set_default_run_config(options), kernel)
+    lib, seen = _lib.load(), []
+
+    class Recorder:
+        def __getattr__(self, name):
+            fn = getattr(lib, name)
+            if not name.startswith("wb200_mxfp4_gemm") or name.endswith("bytes"):
+                return fn
+            return lambda *args: (seen.append(args[-2]), fn(*args))[1]
+
+    gemm._lib = Recorder()
+    ad = a.to(DEV)
+    if strided:
+        wide = torch.zeros(M, K // 2 + 16, dtype=torch.uint8, device=DEV)
+        wide[:, :K // 2] = ad
+        ad = wide[:, :K // 2]
+    bd, a_sd, b_sd = b.to(DEV), a_s.to(DEV), b_s.to(DEV)
+    with pytest.MonkeyPatch.context() as mp:
+        mp.setattr(_lib, "load", lambda: gemm._lib)
+        for call in range(3):
+            if call == 2:
+                b_sd.copy_(b_s)  # a new version: packed again
+            c = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+            gemm(ad, a_sd, bd, b_sd, c)
+            check(c, a, a_s, b, b_s)
+    assert [bool(f & _lib.OVERLAP_PREVIOUS) for f in seen] == [False, True, False]
+
+
 def test_a_weight_quantised_two_launches_ahead_of_an_overlapping_gemm():
     """quantise w -> GEMM on another weight -> GEMM on w, both GEMMs flagged WB200_OVERLAP_PREVIOUS: the kernel before the second
     GEMM does not write w, so that GEMM may load w at once, and the quantiser has to be done by then. w's memory holds the

@@ -158,7 +158,10 @@ class ScaledGemmKernel:
         if M > 128 and ws_bytes and not ops.split_k_pays() and (flags & _lib.PATH_MASK) != _lib.PATH_TILE_SPLITK:
             ws_ptr = ws_bytes = 0  # eager call: stay on the plain tile path (see ops.split_k_pays)
         tile_rows = self._weight_tile_rows(M, N, dev_index)
+        packings = self._weight_scales.packings
         b_sf = self._weight_scales.get(b_scale, tile_rows)
+        if self._weight_scales.packings != packings:
+            flags &= ~_lib.OVERLAP_PREVIOUS  # the kernel that precedes the GEMM has become the one that writes its weight scales
         if tile_rows != 128:
             flags |= _lib.B_TILE_ROWS(tile_rows)
         lib = self._lib
@@ -273,7 +276,10 @@ class ScaledGemmKernel:
             b_sf = b_scale
         else:
             idx = a.device.index if a.device.index is not None else torch.cuda.current_device()
+            packings = self._weight_scales.packings
             b_sf = self._weight_scales.get(self._check_scale(b_scale, N, K, "b_scale"), self._weight_tile_rows(M, N, idx))
+            if self._weight_scales.packings != packings:
+                flags &= ~_lib.OVERLAP_PREVIOUS  # as in _launch
         ops.scaled_gemm_packed(a, a_sf, b, b_sf, c, flags)  # adds the tile-height bits a tiled packing needs
 
     @staticmethod

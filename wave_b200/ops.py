@@ -353,6 +353,7 @@ class WeightScaleCache:
 
     def __init__(self, capacity: int = 64):
         self.capacity = capacity
+        self.packings = 0  # launched so far: a call that moves it has put a repack kernel in front of its GEMM
         self._entries: OrderedDict = OrderedDict()
 
     def get(self, scale: torch.Tensor, tile_rows: int = 128) -> PackedScales:
@@ -365,6 +366,7 @@ class WeightScaleCache:
                 return packed
             del self._entries[key]  # same address, another (or a dead) tensor: the packing is not this tensor's
         packed = repack_scales(scale, tile_rows=tile_rows)
+        self.packings += 1
         self._entries[key] = (weakref.ref(scale), packed)
         while len(self._entries) > self.capacity:
             self._entries.popitem(last=False)
