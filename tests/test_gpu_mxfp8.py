@@ -379,3 +379,20 @@ def test_8bit_decode_calls_with_few_weight_tiles(M, N, K, b_fp4):
     gemm(a.to(DEV), a_s.to(DEV), b.to(DEV), b_s.to(DEV), c)
     check_of(c, a, a_s, b, b_s)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("path", [_lib.PATH_TILE_1CTA, _lib.PATH_TILE_2CTA, _lib.PATH_SKINNY])
+@pytest.mark.parametrize("N", [18952, 20480])
+def test_mixed_template_with_a_forced_path(path, N):
+    """M <= 128 at an N whose decode height for the mixed pair is above 128 and for other pairs is 128: the tile kernels take the usual
+    packing, the decode kernels theirs."""
+    M, K = 16, 256
+    if not ops.decode_tile_rows(N, mixed=True) > 128 == ops.decode_tile_rows(N):
+        pytest.skip("this part's SM count gives other heights")
+    a, a_s, b, b_s = mixed_problem(M, N, K, N, torch.float8_e4m3fn)
+    template, subs = wb.get_scaled_gemm_mxfp8_kernel((M, N, K), wb.ScaledMMAType.F32_16x16x128_F8F6F4, "f8e4m3fn", wb.f32, weight_format="f4e2m1fn")
+    gemm = wb.wave_compile(wb.set_default_run_config(wb.WaveCompileOptions(subs=subs, kernel_path=path)), template)
+    c = torch.full((M, N), float("nan"), dtype=torch.float32, device=DEV)
+    gemm(a.to(DEV), a_s.to(DEV), b.to(DEV), b_s.to(DEV), c)
+    check_mixed(c, a, a_s, b, b_s)
+    ops.check_device_status()

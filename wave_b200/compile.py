@@ -295,6 +295,8 @@ class ScaledGemmKernel:
         (weight, height) and cached, so a weight used at both ends of the M range keeps two packings."""
         if M > 128 or not self.options.decode_tiled_weight_scales:
             return 128
+        if self.options.kernel_path in (_lib.PATH_TILE_1CTA, _lib.PATH_TILE_2CTA):
+            mixed = False  # no tile kernel reads the mixed pair's heights
         key = (N, dev_index, mixed)
         h = self._tile_rows.get(key)
         if h is None:
