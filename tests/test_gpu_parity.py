@@ -1300,11 +1300,11 @@ def test_row_major_activation_scales_give_the_bits_of_packed_ones(M, N, K, offse
 
 
 @pytest.mark.parametrize("N,K", [(128, 256), (500, 1024), (1024, 8192), (1030, 12288), (4096, 4064), (9472, 4096), (9601, 4096), (18816, 512),
-                                 (14336, 4096)])
-@pytest.mark.parametrize("M", [1, 16, 17, 64, 128])
+                                 (14336, 4096), (2048, 16000), (4096, 10240), (5803, 5376), (8192, 8192), (11001, 4096)])
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 64, 128])
 def test_decode_calls_with_few_weight_tiles(M, N, K):
-    """M <= 128 with fewer 128-row weight tiles than SMs: the K-split kernel, the two tile kernels or a cluster per tile, by M and the
-    size of the weight; either side of every line of that rule. Same call as a user's (AUTO, with a workspace)."""
+    """M <= 128 with fewer 128-row weight tiles than SMs: the K-split kernel, the two tile kernels or a cluster per tile, by M, the
+    size of the weight, that of the activations and the alignment of C's rows; either side of every line of that rule. Same call as a user's (AUTO, with a workspace)."""
     a, a_s, b, b_s = random_problem(M, N, K, seed=M + N + K)
     ad, bd = a.to(DEV), b.to(DEV)
     a_sf, b_sf = ops.repack_scales(a_s.to(DEV)), ops.repack_scales(b_s.to(DEV))

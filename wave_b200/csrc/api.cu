@@ -250,6 +250,11 @@ int check_common(int M, int N, int K, const void* a, const void* as, const void*
   return WB200_OK;
 }
 
+// Every row of C starts on 16 bytes: wide stores and TMA stores are possible.
+bool rows_aligned(const void* c, long long ldc, int c_dtype) {
+  return (reinterpret_cast<uintptr_t>(c) & 15) == 0 && ldc * (c_dtype == WB200_F32 ? 4 : 2) % 16 == 0;
+}
+
 // ------------------------------------------------------------------------------------------
 // tile paths
 // ------------------------------------------------------------------------------------------
@@ -1105,22 +1110,38 @@ int dispatch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, c
 // What AUTO runs for M <= 128 on the usual packing of the weight scales when there are fewer 128-row weight tiles than SMs
 // (with more, the whole-tile decode kernel is the fastest at every M).
 enum class DecodeRoute { kSkinny, kTile1, kTile2, kCluster };
-// The K-split kernel keeps all SMs streaming, but every CTA ends with partial tiles of M x 128 sums that meet in memory: with
-// M = 64 that costs more than the stream (64 x 2048 x 4096: 51 us), and with few K blocks per SM at M = 16 too. It is
-// the fastest only up to 16 rows and from six 256-deep K blocks per SM up. us, K split against the tile kernel:
-//   M = 16: N x K = 1024 x 1024 8.7 / 4.8, 2048 x 4096 19.0 / 7.8, 4096 x 4096 12.5 / 8.8, 8192 x 1024 11.0 / 5.3;
-//           5803 x 5344 (M = 15) 12.6 / 14.8, 14336 x 4096 12.1 / 13.4, 4096 x 14336 14.3 / 18.3, 8192 x 8192 13.5 / 16.2, 16384 x 16384 28.6 / 30.5
-//   M = 32: 4096 x 4096 16.9 / 9.0, 8192 x 8192 16.4 / 13.2, 14336 x 4096 14.1 / 13.1, 16384 x 16384 30.5 / 30.9
-//   M = 128: 1024 x 8192 101 / 11.3, 4096 x 4096 48.0 / 9.0, 8192 x 8192 30.8 / 13.5, 16384 x 16384 43.5 / 31.5
+// The K-split kernel keeps all SMs streaming, but every CTA ends with partial tiles of M x 128 sums that meet in memory: that
+// costs more with every 16 rows and with every CTA that shares a tile. A tile kernel walks K in one CTA, or CTA pair, per
+// tile: ~0.2 us per 256-deep K block whatever M is. Its CTAs also read the same activations: where these are
+// fewer than 128 KB together it is slower, by up to a half. us with the weights in memory (not in L2), K split / the
+// tile kernel or cluster that would be next:
+//   M = 1:   4096 x 4096 12.6 / 10.5, 3072 x 8192 11.4 / 13.8, 2048 x 12288 13.0 / 14.5, 2048 x 16000 14.1 / 19.0, 4096 x 14336 13.7 / 19.7
+//   M = 16:  1024 x 12288 18.7 / 10.1, 2048 x 8192 12.9 / 11.4, 2048 x 12288 13.8 / 12.0, 2048 x 16384 14.8 / 12.7, 4096 x 10240 12.8 / 14.3
+//   M = 17:  8192 x 8192 15.7 / 17.4, 8192 x 6144 14.7 / 12.7, 14336 x 6144 16.9 / 17.9, 14336 x 4096 14.1 / 13.1, 4096 x 4096 18.0 / 10.8
+//   M = 32:  8192 x 8192 16.0 / 13.2, 16384 x 8192 21.2 / 17.2, 14336 x 4096 14.3 / 12.5
+//   M = 128: 1024 x 16384 106 / 11.1, 4096 x 4096 48.0 / 9.0, 14336 x 4096 25.1 / 11.0
+// Rows of C that are not 16-byte aligned are stored element by element, which the tile kernels, one row per lane, pay for more:
+//   N x K = 5803 x 5376, M = 17: 14.0 / 12.2, M = 32: 14.3 / 14.4; 11001 x 4096, M = 32: 14.1 / 16.2, M = 128: 26.2 / 29.3.
 // Of the tile kernels, CTA pairs (256 x 128 tiles) fetch the weights of a tile through two SMs: ahead from 16 K blocks up
-// while a pair per tile fits (1024 x 8192 11.0 / 12.7, 8192 x 8192 13.2 / 14.3), behind otherwise (8192 x 1024 6.0 / 5.3,
-// 14336 x 4096 13.4 / 11.2). Where K is long enough and the tiles are few, a cluster per tile.
-DecodeRoute decode_route(int sm_count, int M, int N, int K) {
+// while a pair per tile fits (1024 x 6144 9.5 / 10.5 for one CTA per tile, 2048 x 8192 11.5 / 13.1), behind otherwise
+// (14336 x 4096 15.1 / 13.2; unaligned 5803 x 5376, M = 32: 17.5 / 14.4). Where K is long enough and the tiles are few, a cluster
+// per tile: always ahead above 16 rows (M = 17: 4096 x 14336 16.3 / 18.2 for the K split, 2048 x 10240 14.5 / 19.7).
+constexpr long long kRouteActivationBytes = 128 << 10;
+DecodeRoute decode_route(int sm_count, int M, int N, int K, bool c_aligned) {
   const int tiles = (N + 127) / 128, kb = (K + 255) / 256;
   if (tiles >= sm_count) return DecodeRoute::kSkinny;
-  if (cluster_splitk_slices(M, N, K)) return DecodeRoute::kCluster;
-  if (M <= 16 && (long long)tiles * kb >= 6ll * sm_count) return DecodeRoute::kSkinny;
-  return tiles * 2 <= sm_count && kb >= 16 ? DecodeRoute::kTile2 : DecodeRoute::kTile1;
+  const long long units = (long long)tiles * kb, sms = sm_count;
+  const bool few_activations = (long long)M * K / 2 < kRouteActivationBytes;
+  const int slices = cluster_splitk_slices(M, N, K);
+  const bool pairs = tiles * 2 <= sm_count;  // a CTA pair per tile fits
+  if (M <= 16) {
+    if (units >= 10 * sms || (few_activations && (units >= 6 * sms || (kb >= 24 && units >= 5 * sms && (!slices || M < 4)))))
+      return DecodeRoute::kSkinny;
+  } else if (!slices) {
+    if ((M <= 32 && few_activations && kb >= (pairs ? 32 : 24) && units >= 10 * sms) || (!c_aligned && units >= 9 * sms)) return DecodeRoute::kSkinny;
+  }
+  if (slices) return DecodeRoute::kCluster;
+  return (c_aligned || M <= 16 || !few_activations) && pairs && kb >= 16 ? DecodeRoute::kTile2 : DecodeRoute::kTile1;
 }
 
 // The same for 8-bit operands and the mixed pair (K blocks of 128). us, K split against the better tile kernel:
@@ -1660,7 +1681,7 @@ int wb200_mxfp4_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
     if (M <= 128 && ws_ok) {
       path = WB200_PATH_SKINNY;
       if (tl_b_tile_rows == 128 && !(flags & (WB200_TILE_N128 | WB200_TILE_N192))) {
-        const DecodeRoute route = decode_route(dev->sm_count, M, N, K);
+        const DecodeRoute route = decode_route(dev->sm_count, M, N, K, rows_aligned(c, ldc, c_dtype));
         if (route != DecodeRoute::kSkinny) {
           path = route == DecodeRoute::kTile1 ? WB200_PATH_TILE_1CTA : WB200_PATH_TILE_2CTA;
           if (route != DecodeRoute::kCluster) route_bn = 128;
