@@ -364,8 +364,9 @@ def test_mixed_decode_with_weights_on_the_n_side(M, N, K, out_dtype):
     ops.check_device_status()
 
 
-@pytest.mark.parametrize("N,K", [(128, 128), (1024, 8192), (1100, 1024), (4096, 4096), (4096, 12288), (9600, 2048), (14336, 1024)])
-@pytest.mark.parametrize("M", [1, 16, 32, 33, 128])
+@pytest.mark.parametrize("N,K", [(128, 128), (1024, 8192), (1100, 1024), (4096, 4096), (4096, 12288), (9600, 2048), (14336, 1024),
+                                 (2048, 12288), (5803, 5376), (8192, 4096), (4096, 14336)])
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 128])
 @pytest.mark.parametrize("b_fp4", [False, True])
 def test_8bit_decode_calls_with_few_weight_tiles(M, N, K, b_fp4):
     """M <= 128 with fewer 128-row weight tiles than SMs: either side of every line of the rule that picks the K-split kernel or one

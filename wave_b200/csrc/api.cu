@@ -1144,18 +1144,26 @@ DecodeRoute decode_route(int sm_count, int M, int N, int K, bool c_aligned) {
   return (c_aligned || M <= 16 || !few_activations) && pairs && kb >= 16 ? DecodeRoute::kTile2 : DecodeRoute::kTile1;
 }
 
-// The same for 8-bit operands and the mixed pair (K blocks of 128). us, K split against the better tile kernel:
-//   M = 16: 1024 x 1024 11.3 / 5.8, 1024 x 8192 18.7 / 16.9 (mixed 24.3 / 16.6), 4096 x 1024 13.2 / 6.0; 4096 x 4096 11.6 / 12.5
-//           (11.0 / 11.9), 8192 x 8192 19.2 / 20.0 (16.2 / 18.3), 14336 x 4096 17.3 / 21.6 (15.0 / 20.1)
-//   M = 32: 4096 x 4096 15.4 / 11.6, 8192 x 8192 21.4 / 20.8, 14336 x 4096 19.4 / 16.4; 4096 x 14336 23.2 / 27.2, 16384 x 16384
-//           50.8 / 51.9 (37.0 / 41.2)
-//   M = 128: 1024 x 8192 102 / 17.3, 4096 x 4096 34.9 / 12.0, 8192 x 8192 36.8 / 21.3, 16384 x 16384 68.3 / 53.3
-DecodeRoute decode_route_8bit(int sm_count, int M, int N, int K) {
+// The same for 8-bit operands and the mixed pair (K blocks of 128). us with the weights in memory, K split / the better tile kernel,
+// 8-bit (mixed) weights:
+//   M = 16:  1024 x 4096 17.9 / 11.0, 4096 x 4096 11.8 / 12.2, 2048 x 6144 13.6 / 16.4 (12.9 / 14.1), 1024 x 8192 18.1 / 17.1 (19.3 / 16.9), 14336 x 4096 17.2 / 20.7 (14.4 / 18.3)
+//   M = 17:  4096 x 4096 15.6 / 11.8, 14336 x 4096 18.8 / 22.1 (16.3 / 18.8), 2048 x 16384 22.4 / 29.6 (21.4 / 29.1)
+//   M = 32:  8192 x 4096 16.0 / 12.7, 14336 x 4096 19.3 / 15.8, 8192 x 8192 21.2 / 20.7, 10240 x 8192 (20.0 / 22.1), 4096 x 10240 20.5 / 21.1 (19.0 / 20.6), 2048 x 16384 23.7 / 29.4 (22.3 / 29.2)
+//   M = 48:  4096 x 4096 19.8 / 11.7, 4096 x 16384 27.6 / 31.0 (24.4 / 29.8);  M = 64: 4096 x 16384 31.2 / 30.7 (27.9 / 30.0)
+//   M = 128: 1024 x 8192 102 / 17.3, 4096 x 4096 34.5 / 11.9
+// Unaligned rows of C: 5803 x 5376, M = 17: 16.3 / 18.2, M = 128: 33.7 / 31.7; 11001 x 4096, M = 32: 17.9 / 18.6, M = 128: 30.9 / 34.0.
+DecodeRoute decode_route_8bit(int sm_count, int M, int N, int K, bool mixed, bool c_aligned) {
   const int tiles = (N + 127) / 128, kb = (K + 127) / 128;
   if (tiles >= sm_count) return DecodeRoute::kSkinny;
-  if (M <= 16 && (long long)tiles * kb >= 6ll * sm_count) return DecodeRoute::kSkinny;
-  if (M <= 32 && kb >= 96 && (long long)tiles * kb >= 20ll * sm_count) return DecodeRoute::kSkinny;
-  return tiles * 2 <= sm_count && kb >= 16 ? DecodeRoute::kTile2 : DecodeRoute::kTile1;
+  const long long units = (long long)tiles * kb, sms = sm_count;
+  const bool few_activations = (long long)M * K < kRouteActivationBytes;
+  bool k_split;
+  if (M <= 16) k_split = units >= 6 * sms || (kb >= 32 && units >= 5 * sms) || (kb >= 128 && units >= 3 * sms);
+  else if (M <= 32) k_split = units >= 8 * sms && (kb > (mixed ? 48 : 64) || (kb > 24 && few_activations) || !c_aligned);
+  else if (M <= 64) k_split = units >= 13 * sms && ((M <= 48 && kb >= 96) || !c_aligned);
+  else k_split = !c_aligned && units >= 16 * sms;
+  if (k_split) return DecodeRoute::kSkinny;
+  return tiles * 2 <= sm_count && (kb >= 32 || (kb >= 16 && !few_activations)) ? DecodeRoute::kTile2 : DecodeRoute::kTile1;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1838,7 +1846,7 @@ int wb200_mxfp8_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
   if (path == WB200_PATH_AUTO) {
     path = (M <= 128 && ws_ok) ? WB200_PATH_SKINNY : (M > 128) ? WB200_PATH_TILE_2CTA : WB200_PATH_TILE_1CTA;
     if (tl_route_8bit && path == WB200_PATH_SKINNY && tl_b_tile_rows == 128 && !n128) {
-      const DecodeRoute route = decode_route_8bit(dev->sm_count, M, N, K);
+      const DecodeRoute route = decode_route_8bit(dev->sm_count, M, N, K, (elem_format & WB200_B_FP4) != 0, rows_aligned(c, ldc, c_dtype));
       if (route != DecodeRoute::kSkinny) {
         path = route == DecodeRoute::kTile1 ? WB200_PATH_TILE_1CTA : WB200_PATH_TILE_2CTA;
         n128 = true;
