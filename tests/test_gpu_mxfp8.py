@@ -397,3 +397,28 @@ def test_mixed_template_with_a_forced_path(path, N):
     gemm(a.to(DEV), a_s.to(DEV), b.to(DEV), b_s.to(DEV), c)
     check_mixed(c, a, a_s, b, b_s)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("M,K,N,cols,out_dtype", [
+    (1, 384, 20480, 20480, torch.bfloat16), (16, 512, 20480, 20480, torch.float32), (17, 512, 20480, 20480, torch.bfloat16),
+    (32, 1024, 20480, 20480, torch.float32), (33, 1024, 20480, 20480, torch.bfloat16),
+    (33, 1152, 20480, 20480, torch.bfloat16), (128, 3968, 18952, 18952, torch.bfloat16), (128, 4096, 18952, 18952, torch.float32),  # 32 K per row
+    (16, 6144, 18952, 18952, torch.bfloat16), (16, 6272, 18952, 18952, torch.bfloat16),  # low tiles over a long K
+    (8, 1920, 28671, 28671, torch.bfloat16), (8, 2048, 28671, 28671, torch.bfloat16), (9, 2304, 28671, 28671, torch.float32),  # odd N
+    (8, 2048, 20481, 20481, torch.bfloat16), (9, 2304, 20481, 20481, torch.bfloat16), (17, 4352, 20480, 20483, torch.bfloat16),
+])
+def test_mixed_template_either_side_of_the_height_rule(M, K, N, cols, out_dtype):
+    """The template call with 4-bit weights at sizes either side of every line that decides between the mixed pair's tile height and the
+    other pairs': few K per row, C's rows aligned to 16 bytes or not (odd N, a column block of a wider C), 16 rows over a long K.
+    The result is the oracle's whichever is taken."""
+    a, a_s, b, b_s = mixed_problem(M, N, K, M + N + K, torch.float8_e4m3fn)
+    template, subs = wb.get_scaled_gemm_mxfp8_kernel((M, N, K), wb.ScaledMMAType.F32_16x16x128_F8F6F4, "f8e4m3fn",
+                                                     wb.f32 if out_dtype == torch.float32 else wb.bf16, weight_format="f4e2m1fn")
+    gemm = wb.wave_compile(wb.set_default_run_config(wb.WaveCompileOptions(subs=subs)), template)
+    wide = torch.full((M, cols), float("nan"), dtype=out_dtype, device=DEV)
+    c = wide[:, :N]
+    gemm(a.to(DEV), a_s.to(DEV), b.to(DEV), b_s.to(DEV), c)
+    rows = sorted({0, M // 2, M - 1})  # sampled: the oracle multiplies on the CPU
+    check_mixed(c[rows].contiguous(), a[rows], a_s[rows], b, b_s)
+    assert bool(wide[:, N:].isnan().all())
+    ops.check_device_status()

@@ -207,7 +207,8 @@ class ScaledGemmKernel:
             b_sf = b_scale
         else:
             idx = a.device.index if a.device.index is not None else torch.cuda.current_device()
-            b_sf = self._weight_scales.get(self._check_scale(b_scale, N, K, "b_scale"), self._weight_tile_rows(M, N, idx, b_fp4))
+            tile_rows = self._mixed_tile_rows(M, N, K, c, idx) if b_fp4 else self._weight_tile_rows(M, N, idx)
+            b_sf = self._weight_scales.get(self._check_scale(b_scale, N, K, "b_scale"), tile_rows)
         fmt = _lib.E5M2 if t.element_format == "f8e5m2" else _lib.E4M3
         flags = self.options.kernel_path | self._raster_flags() | (_lib.ACCUMULATE if t.accumulate else 0)
         ops.scaled_gemm_mxfp8_packed(a, a_sf, b, b_sf, c, fmt, flags, b_fp4=b_fp4, a_scale=rowmajor)
@@ -295,13 +296,31 @@ class ScaledGemmKernel:
         (weight, height) and cached, so a weight used at both ends of the M range keeps two packings."""
         if M > 128 or not self.options.decode_tiled_weight_scales:
             return 128
-        if self.options.kernel_path in (_lib.PATH_TILE_1CTA, _lib.PATH_TILE_2CTA):
-            mixed = False  # no tile kernel reads the mixed pair's heights
         key = (N, dev_index, mixed)
         h = self._tile_rows.get(key)
         if h is None:
             h = self._tile_rows[key] = ops.decode_tile_rows(N, dev_index, mixed)
         return h
+
+    def _mixed_tile_rows(self, M: int, N: int, K: int, c: torch.Tensor, dev_index: int) -> int:
+        """The same for the mixed pair, whose decode kernel reads heights above 128. Each of its tiles ends with M rows of C that
+        one lane writes per row, while the kernels for the other heights write whole rows: it needs the K for that, 32
+        for every row of C that is written 16 bytes at a time, 256 where C's rows are not 16-byte aligned. us against the other
+        height, bf16: N = 28672, K = 512: M = 16 6.0 / 6.1, M = 48 6.6 / 6.6; N = 22208, K = 1024: M = 32 8.0 / 8.1, M = 64 9.5 / 8.9, M = 128 12.7 / 9.8; K = 4096: M = 128 20.8 / 23.5;
+        unaligned N = 28671, K = 2048: M = 8 11.8 / 11.9, M = 64 28.1 / 15.9, K = 8192: M = 32 35.8 / 35.8, M = 128 64.8 / 51.0. Up to
+        16 rows the usual packing takes the K-split kernel, which is ahead of low tiles over a long K (N = 19200, M = 16: K = 6144
+        18.8 / 19.0, K = 16384 42.2 / 38.1; N = 22208, K = 16384 45.8 / 45.3) and in unaligned stores (N = 22201, K = 4096, M = 8 15.7 /
+        16.2, M = 16 18.9 / 16.6)."""
+        usual = self._weight_tile_rows(M, N, dev_index)
+        if M > 128 or self.options.kernel_path in (_lib.PATH_TILE_1CTA, _lib.PATH_TILE_2CTA):
+            return usual  # no tile kernel reads a height above 128
+        wide = self._weight_tile_rows(M, N, dev_index, mixed=True)
+        k_split = M <= 16 and usual == 128
+        if k_split and K > 6144 and wide < 152:
+            return usual
+        if c.data_ptr() % 16 == 0 and (c.stride(0) if M > 1 else N) * c.element_size() % 16 == 0:
+            return wide if K >= 32 * max(M, 16) else usual
+        return wide if K >= 256 * max(M, 8) and not (k_split and M > 8) else usual
 
     def drop_cached_weights(self, b_scale: torch.Tensor | None = None) -> None:
         """Forget the packed copy of `b_scale` (of every weight when None). The kernel repacks a weight's scales on
