@@ -173,7 +173,7 @@ int wb200_quantize_mxfp4(const void* x, int x_dtype, long long ldx, int rows, in
 /* wb200_quantize_mxfp4 and wb200_mxfp4_gemm in one call, the GEMM launched as the programmatic dependent of the
  * quantiser: x [M, K] (f32 or bf16) is quantised to q_scratch [M, K/2] and scale_scratch
  * (wb200_packed_scale_bytes(M, K)), both 16-byte aligned, and the GEMM's set-up, and on the M <= 128 path its first ring of weight loads, run
- * while the quantiser does. Other arguments as wb200_mxfp4_gemm; WB200_OVERLAP_PREVIOUS is refused. */
+ * while the quantiser does (an ordinary launch for M > 128 where rows of c are not 16-byte aligned). Other arguments as wb200_mxfp4_gemm; WB200_OVERLAP_PREVIOUS is refused. */
 int wb200_mxfp4_gemm_quantize_a(int M, int N, int K, const void* x, int x_dtype, long long ldx, void* q_scratch, void* scale_scratch,
                                 const void* b, const void* b_scale_packed, void* c, int c_dtype, long long ldc, void* workspace,
                                 size_t workspace_bytes, unsigned flags, void* stream);

@@ -1782,9 +1782,14 @@ int wb200_mxfp4_gemm_quantize_a(int M, int N, int K, const void* x, int x_dtype,
   // what the GEMM will refuse is refused before the quantiser writes anything
   int rc = check_common(M, N, K, q_scratch, scale_scratch, b, b_scale_packed, c, c_dtype, ldc);
   if (rc) return rc;
-  rc = quantize_mxfp4_impl(x, x_dtype, ldx, M, K, q_scratch, nullptr, scale_scratch, true, stream);
+  // The GEMM is the quantiser's programmatic dependent, but for the tile kernels where rows of C are not 16-byte aligned: those are
+  // bound by their element-wise stores and were slower for it (us dependent / ordinary: 512 x 5803 x 5344 48.0 / 44.8,
+  // 512 x 4001 x 4096 33.5 / 31.9, 2000 x 5803 x 5344 163 / 156, 300 x 11001 x 4096 65.9 / 67.5; aligned: 512 x 5808 x 5344 16.4 / 16.6,
+  // 300 x 11000 x 4096 16.0 / 17.2, 3000 x 8192 x 8192 83.7 / 84.5).
+  const bool dependent = M <= 128 || rows_aligned(c, ldc, c_dtype);
+  rc = quantize_mxfp4_impl(x, x_dtype, ldx, M, K, q_scratch, nullptr, scale_scratch, dependent, stream);
   if (rc) return rc;
-  tl_dependent_launch = true;  // the GEMM is the quantiser's programmatic dependent
+  tl_dependent_launch = dependent;
   rc = wb200_mxfp4_gemm(M, N, K, q_scratch, scale_scratch, b, b_scale_packed, c, c_dtype, ldc, workspace, workspace_bytes, flags, stream);
   tl_dependent_launch = false;
   return rc;
