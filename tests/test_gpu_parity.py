@@ -566,6 +566,36 @@ def test_two_streams_run_skinny_gemms_at_the_same_time():
     ops.check_device_status()
 
 
+def test_workspace_of_a_captured_call_outlives_a_larger_call(monkeypatch):
+    """The graph of a decode GEMM writes its counters and partial tiles where the workspace was at the capture. Blocks of that size
+    that are allocated after a larger call has made a new workspace are not written by a replay."""
+    monkeypatch.setattr(ops, "_pool", ops.WorkspacePool())
+    N, K = 4096, 16384  # at 16 rows the K-split kernel, which uses the workspace
+    a, a_s, b, b_s = random_problem(128, N, K, seed=78)
+    a_sf, b_sf = [ops.repack_scales(a_s[:m].to(DEV)) for m in (16, 128)], ops.repack_scales(b_s.to(DEV))
+    ad, bd = a.to(DEV), b.to(DEV)
+    c = torch.empty(16, N, dtype=torch.bfloat16, device=DEV)
+    stream, graph = torch.cuda.Stream(DEV), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        ops.scaled_gemm_packed(ad[:16], a_sf[0], bd, b_sf, c, _lib.PATH_SKINNY)
+    torch.cuda.synchronize()
+    ref = c.clone()
+    with torch.cuda.graph(graph, stream=stream):
+        ops.scaled_gemm_packed(ad[:16], a_sf[0], bd, b_sf, c, _lib.PATH_SKINNY)
+    key = (0, stream.cuda_stream, "skinny")
+    small = ops._pool._by_key[key].data_ptr(), ops._pool._by_key[key].numel()
+    with torch.cuda.stream(stream):
+        ops.scaled_gemm_packed(ad, a_sf[1], bd, b_sf, torch.empty(128, N, dtype=torch.bfloat16, device=DEV), _lib.PATH_SKINNY)
+        assert ops._pool._by_key[key].numel() >= 2 * small[1]
+        blocks = [torch.full((small[1],), 7, dtype=torch.uint8, device=DEV) for _ in range(4)]
+    torch.cuda.synchronize()
+    assert all(not (t.data_ptr() < small[0] + small[1] and small[0] < t.data_ptr() + t.numel()) for t in blocks)
+    c.fill_(float("nan"))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(c.view(torch.int16), ref.view(torch.int16)) and all(bool((t == 7).all()) for t in blocks)
+
+
 @pytest.mark.parametrize("kind,M,N,K", [("fp4", 64, 28672, 1024), ("fp4", 256, 4096, 4096), ("fp4", 16, 1024, 12320), ("fp8", 16, 14336, 2048),
                                         ("mixed", 64, 28672, 2048), ("fp8", 300, 4096, 2048)])
 def test_two_streams_pack_activation_scales_at_the_same_time(kind, M, N, K):

@@ -142,11 +142,14 @@ class WorkspacePool:
     functional entry points share a module-level one.
 
     Workspaces are created and initialised eagerly. While a stream is being captured into a CUDA graph nothing
-    is allocated: the call uses the workspace an earlier eager call (the warm-up) made for that device and kind.
+    is allocated: the call uses the workspace an earlier eager call (the warm-up) made for that device and kind. The graph
+    keeps its address, so one that a larger call outgrows stays; as every new one has at least twice the size, what stays
+    is smaller than what is in use. `clear` gives everything back: not while a graph is still to be replayed.
     """
 
     def __init__(self):
         self._by_key: dict = {}
+        self._outgrown: list = []
 
     def get(self, device: torch.device, nbytes: int, kind: str) -> torch.Tensor:
         idx = device.index if device.index is not None else torch.cuda.current_device()
@@ -161,6 +164,9 @@ class WorkspacePool:
                     return w
             raise RuntimeError("this GEMM needs a workspace, which cannot be created while a CUDA graph is being captured: "
                                "call it once eagerly (with the same shapes) before the capture")
+        if ws is not None:
+            self._outgrown.append(ws)
+            nbytes = max(nbytes, 2 * ws.numel())
         ws = torch.empty(nbytes, dtype=torch.uint8, device=torch.device("cuda", idx))
         with torch.cuda.device(idx):
             _lib.check(_lib.load().wb200_workspace_init(ws.data_ptr(), nbytes, _stream()))
@@ -169,6 +175,7 @@ class WorkspacePool:
 
     def clear(self) -> None:
         self._by_key.clear()
+        self._outgrown.clear()
 
 
 _pool = WorkspacePool()
