@@ -1309,9 +1309,9 @@ def test_split_k_inside_a_cluster(shape, out_dtype):
                                    (129, 512, 32), (300, 700, 1184), (1000, 384, 4128), (2048, 4096, 512), (2050, 8192, 288)])
 @pytest.mark.parametrize("offset,extra", [(0, 0), (8, 8), (3, 5)])
 def test_row_major_activation_scales_give_the_bits_of_packed_ones(M, N, K, offset, extra):
-    """The call that takes a_scale row-major (a warp of the GEMM brings it into the stages) against the same GEMM on scales packed
-    beforehand, for every kernel that has that warp: K blocks that end inside a stage, rows that end inside a tile, several
-    tiles per CTA, row pitches and bases that allow 8-byte loads and that do not."""
+    """The call that takes a_scale row-major against the same GEMM on scales packed beforehand, for every path of the call: the sizes at
+    which it packs them itself ahead of the GEMM (nearly all of these; the next test is for the kernels that take them as they
+    are), K blocks that end inside a stage, rows that end inside a tile, row pitches and bases of any alignment."""
     a, a_s, b, b_s = random_problem(M, N, K, seed=M + N + K + offset)
     wide = torch.full((M, offset + K // 32 + extra), 255, dtype=torch.uint8, device=DEV)
     view = wide[:, offset:offset + K // 32]
@@ -1327,6 +1327,44 @@ def test_row_major_activation_scales_give_the_bits_of_packed_ones(M, N, K, offse
     assert torch.equal(c.view(torch.int16), ref.view(torch.int16))
     check(c, a, a_s, b, b_s)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K,pad,path", [
+    (16, 28672, 288, 7, 0), (32, 28672, 2336, 7, 0), (1, 28672, 4096, 0, 0), (5, 57344, 2816, 8, 0),  # whole tiles: one and more rounds
+    (17, 19000, 3104, 7, 0), (32, 18816 + 128, 512, 0, 0),
+    (16, 9472, 4128, 7, 0), (3, 14336, 4096, 0, 0), (16, 4096, 10272, 7, 0),  # K split
+    (17, 1000, 2336, 7, _lib.PATH_SKINNY), (32, 640, 8192, 0, _lib.PATH_SKINNY), (1, 128, 32, 7, _lib.PATH_SKINNY), (30, 300, 12576, 15, _lib.PATH_SKINNY),
+])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_decode_kernels_take_row_major_scales_as_they_are(M, N, K, pad, path, out_dtype):
+    """The warp that brings row-major scales into the stages, in both decode kernels: fewer and more K blocks than ring stages, runs over
+    several tiles, the last K blocks of a row (K / 32 not a multiple of 8 with a padded pitch), fewer rows than lanes. Bits of
+    the same GEMM on packed scales, the oracle's values, and a scratch that stays as it was: no repack kernel ran."""
+    a, a_s, b, b_s = random_problem(M, N, K, seed=M + N + K)
+    pitch = (K // 32 + pad) // 8 * 8 if pad else K // 32
+    assert pitch >= K // 32 and pitch % 8 == 0
+    wide = torch.full((M + 1, pitch), 255, dtype=torch.uint8, device=DEV)
+    view = wide[1:, :K // 32]
+    view.copy_(a_s.to(DEV))
+    lib, h = _lib.load(), ops.decode_tile_rows(N)
+    if path:
+        h = 128
+    flags = path | _lib.B_TILE_ROWS(h)
+    b_sf, ad, bd = ops.repack_scales(b_s.to(DEV), tile_rows=h), a.to(DEV), b.to(DEV)
+    scratch = torch.full((ops.packed_scale_bytes(M, K),), 0xEE, dtype=torch.uint8, device=DEV)
+    ws_bytes = int(lib.wb200_mxfp4_gemm_workspace_bytes(M, N, K))
+    c = torch.full((M, N), float("nan"), dtype=out_dtype, device=DEV)
+    for _ in range(2):
+        _lib.check(lib.wb200_mxfp4_gemm_repack_a(M, N, K, ad.data_ptr(), view.data_ptr(), pitch, scratch.data_ptr(), bd.data_ptr(),
+                                                 b_sf.data.data_ptr(), c.data_ptr(), ops._DTYPE_CODE[out_dtype], N,
+                                                 ops._workspace(ad.device, ws_bytes).data_ptr(), ws_bytes, flags,
+                                                 torch.cuda.current_stream().cuda_stream))
+    assert bool((scratch == 0xEE).all())
+    ref = torch.full_like(c, float("nan"))
+    ops.scaled_gemm_packed(ad, ops.repack_scales(a_s.to(DEV)), bd, b_sf, ref, path)
+    bits = torch.int16 if out_dtype == torch.bfloat16 else torch.int32
+    assert torch.equal(c.view(bits), ref.view(bits))
+    check(c, a, a_s, b, b_s)
 
 
 @pytest.mark.parametrize("N,K", [(128, 256), (500, 1024), (1024, 8192), (1030, 12288), (4096, 4064), (9472, 4096), (9601, 4096), (18816, 512),

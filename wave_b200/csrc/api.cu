@@ -164,7 +164,6 @@ static wb::RowScales row_scales_param(int M, int K) {
   s.stride = tl_row_scales.stride;
   s.rows = M;
   s.kblocks = K / 32;
-  s.vec = ((reinterpret_cast<uintptr_t>(s.base) & 7) == 0 && s.stride % 8 == 0) ? 1 : 0;
   return s;
 }
 struct GroupNScope {  // restores the previous value on every return path

@@ -16,10 +16,9 @@
 namespace wb {
 
 struct RowScales {
-  const uint8_t* base;  // [rows, kblocks] bytes
-  long long stride;     // bytes between rows
+  const uint8_t* base;  // [rows, kblocks] bytes; a multiple of 8
+  long long stride;     // bytes between rows; a multiple of 8
   int rows, kblocks;
-  int vec;              // base and stride are multiples of 8: whole 8-byte loads
 };
 
 // The scales of K blocks 8 kb .. 8 kb + 7 of one row; the padding byte outside the matrix. The 8-byte load is predicated and
@@ -28,7 +27,7 @@ __device__ __forceinline__ uint2 row_scales_of(const RowScales& s, int row, int 
   uint2 v = make_uint2(0x01010101u * WB_SF_PAD, 0x01010101u * WB_SF_PAD);
   const int left = s.kblocks - kb * 8;
   const uint8_t* p = s.base + (long long)row * s.stride + kb * 8;
-  if (s.vec && left >= 8) {
+  if (left >= 8) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t@p ld.global.v2.b32 {%0, %1}, [%2];\n\t}"
                  : "+r"(v.x), "+r"(v.y) : "l"(p), "r"(int(row < s.rows)) : "memory");
     return v;
