@@ -705,8 +705,10 @@ def main():
         "metric": metric, "value": value, "unit": unit, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "mxfp4",
         "data": "synthetic", "config": config, "clocks": clocks,
+        # of the workloads above only M = 16 runs on a kernel that takes the activation scales row-major (at most 32 rows, a weight
+        # tile or more per SM, scale rows of whole 8-byte words)
         "gpu_launches": (1 if M <= 32 else 2) * args.steps,
-        "gpu_launches_note": "activation-scale repack + GEMM per timed step (up to 32 rows the GEMM alone); the kernel-only, sustained, decode and sharded loops launch more",
+        "gpu_launches_note": "activation-scale repack + GEMM per timed step (M = 16: the GEMM alone); the kernel-only, sustained, decode and sharded loops launch more",
         "roofline": roofline,
     }
     if e2e:

@@ -43,8 +43,8 @@ __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { retu
 // for the kernels that follow (the decode GEMM's tile counter).
 // Latency-bound. Every warp owns a contiguous run of ids: it counts them per expert in its own row of a table, one scan over
 // the rows gives every warp its first position per expert, and a second walk over the run places the ids; positions are
-// in flat order because the runs are. Three CTA barriers in all, where a walk in chunks of 1024 ids with a scan per
-// chunk took 18 us for 8192 ids.
+// in flat order because the runs are. Three CTA barriers in all, where there was a walk in chunks of 1024 ids with a scan per
+// chunk: 8192 ids of 8 experts 14.5 -> 9.2 us (calls back to back from a graph), 32768 of 256 experts 123 -> 92, 32 ids 3.4 -> 3.3.
 template <typename IdT>
 __global__ void __launch_bounds__(1024)
 moe_align_block_size_kernel(const IdT* __restrict__ ids, int n, int E, int block_size, int sorted_cap,

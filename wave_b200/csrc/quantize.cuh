@@ -164,7 +164,8 @@ template <> struct Raw8<float> { using type = Raw8f; };
 template <> struct Raw8<__nv_bfloat16> { using type = uint4; };
 
 // Scale byte of a block whose largest magnitude has the f32 pattern `amax_bits` (the rule at the head of this file) and
-// the factor that brings its values to codes: 2^(127 - byte), 0 for a block with a NaN or an infinity (codes 0).
+// the factor that brings its values to codes: 2^(127 - byte). (Byte 255, a block with a NaN or an infinity, has none: the callers
+// write codes 0 there whatever the product is.)
 __device__ __forceinline__ int mxfp4_scale_byte(uint32_t amax_bits) {
   const int e = int(amax_bits >> 23);
   if (e == 255) return 255;

@@ -5,8 +5,8 @@
 // GEMM. Here one extra warp of the decode kernels brings the scales of every pipeline stage straight into the stage's
 // atoms: a lane reads the eight scale bytes (one stage = 256 K) of its row and writes two 16-byte lines, exactly what the
 // packed array holds there. It runs as far ahead as the ring of stages allows.
-// M = 16, N = 28672, K = 8192, replayed from a graph: 23.6 -> 22.6 us, launched eagerly 26.2 -> 24.2; 16 x 4096 x 4096 eagerly
-// 24.8 -> 19.5. Up to 32 rows only: the fence that hands a stage to the tensor core and the loads cost up to a microsecond a
+// M = 16, N = 28672, K = 8192, 24 calls on as many weights in one graph: 23.8 -> 22.8 us a call, launched eagerly 32.4 -> 28.9;
+// 16 x 14336 x 4096 14.1 -> 13.4, eagerly 20.8 -> 17.4. (A graph of one call each gains 0.2 to 0.3 us.) Up to 32 rows only: the fence that hands a stage to the tensor core and the loads cost up to a microsecond a
 // stage when four rows per lane are read (128 x 8192 x 8192: 31.4 -> 42.0 us), and the 128-row stages of the tile kernel
 // cannot wait for that either (8192^3: 178 -> 500 us).
 #pragma once

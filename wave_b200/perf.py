@@ -80,9 +80,9 @@ def time_shape(M, N, K, out_dtype=torch.bfloat16, iters: int = 20, validate: boo
 
 
 def time_moe(tokens=4096, experts=8, top_k=2, K=4096, inter=7168, iters=10, device="cuda:0"):
-    """Device time of every step of the MXFP4 expert MLP at the grouped-GEMM benchmark's sizes
-    (8 experts x [14336, 4096] gate|up weights, 4096 tokens, top-2): microseconds per step and, for the
-    memory-bound steps, the bytes they must move / that time."""
+    """Time of the MXFP4 expert MLP at the grouped-GEMM benchmark's sizes (8 experts x [14336, 4096] gate|up weights, 4096 tokens,
+    top-2): every step of the step-by-step form (microseconds and, for the memory-bound steps, the bytes they must move /
+    that time), that form as a whole, and the single native call that `MXFP4ExpertMLP` makes."""
     from . import moe, ops
     from .grouped import moe_scaled_gemm
     dev = torch.device(device)
@@ -120,7 +120,8 @@ def time_moe(tokens=4096, experts=8, top_k=2, K=4096, inter=7168, iters=10, devi
          int(post.item()) * (2 * inter * 2 + inter // 2 + inter // 32)),
         ("grouped GEMM down", lambda: moe_scaled_gemm(hq, hs, mlp.w2, expert_ids, post, y), None),
         ("combine", lambda: moe.combine(y, inverse, weight.reshape(-1), top_k, out), R * K * 2 + tokens * K * 2),
-        ("whole forward", lambda: mlp(x, logits), None),
+        ("the steps, one by one", lambda: mlp._forward_steps(x, logits), None),
+        ("single native call", lambda: mlp(x, logits), None),
     ]
     rows = []
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -517,7 +518,7 @@ def main(argv=None):
     ap.add_argument("--mxfp8-fp4-weights", action="store_true", help="time the mixed pair: E4M3 activations, packed E2M1 weights")
     ap.add_argument("--compare-cublaslt", action="store_true", help="context: time cuBLASLt's block-scaled FP4 GEMM on the same operands")
     ap.add_argument("--k-sharded", action="store_true", help="under torchrun: time the K-sharded GEMM against GEMM + NCCL reduce-scatter")
-    ap.add_argument("--moe", action="store_true", help="time the steps of the MXFP4 expert MLP instead of the shape sweep")
+    ap.add_argument("--moe", action="store_true", help="time the MXFP4 expert MLP and its steps instead of the shape sweep")
     ap.add_argument("--timeline", nargs=3, type=int, metavar=("M", "N", "K"),
                     help="per-CTA timeline of the skinny kernel (needs the --trace build of the library, see skinny_timeline)")
     ap.add_argument("--save", default=None, help="with --timeline: write the raw marks to this .npy file")
