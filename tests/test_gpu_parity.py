@@ -1006,6 +1006,35 @@ def test_cuda_graph_replay_of_a_decode_call():
     ops.check_device_status()
 
 
+def test_graphed_gemm_keeps_the_kernel_object_alive():
+    """The graph holds addresses of memory that belongs to the kernel object (workspace, scratch, packed weight scales): a graph whose
+    maker dropped that object still has it, and gives the same result after its memory could have been handed out again."""
+    import gc
+    import weakref
+    from wave_b200.graphs import GraphedScaledGemm
+    M, N, K = 16, 4096, 1024
+    a, a_s, b, b_s = random_problem(M, N, K, seed=12)
+    dev = [t.to(DEV) for t in (a, a_s, b, b_s)]
+    c = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+
+    def make():
+        kernel, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+        gemm = wb.wave_compile(wb.set_default_run_config(options), kernel)
+        return GraphedScaledGemm(gemm, *dev, c), weakref.ref(gemm)
+
+    graphed, gemm = make()
+    gc.collect()
+    assert gemm() is not None
+    blocks = [torch.full((n,), 255, dtype=torch.uint8, device=DEV) for n in (1 << 14, 1 << 18, 1 << 20, 1 << 22) for _ in range(4)]
+    c.fill_(float("nan"))
+    graphed.replay()
+    check(c, a, a_s, b, b_s)
+    assert all(bool((t == 255).all()) for t in blocks)
+    del graphed
+    gc.collect()
+    assert gemm() is None
+
+
 def test_bounded_wait_reports_timeout_and_context_stays_usable():
     """A wait that nothing satisfies gives up after its limit, the kernel ends normally, the status word
     carries the code, and the next GEMM on the same context is correct."""

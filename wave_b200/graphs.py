@@ -24,6 +24,7 @@ class GraphedScaledGemm:
 
     def __init__(self, gemm, a, a_scale, b, b_scale, c, warmup: int = 2):
         self.tensors = (a, a_scale, b, b_scale, c)
+        self.gemm = gemm  # owns the workspace, the scratch and the packed weight scales that the graph holds the addresses of
         side = torch.cuda.Stream(a.device)
         side.wait_stream(torch.cuda.current_stream(a.device))
         with torch.cuda.stream(side):
