@@ -1006,6 +1006,38 @@ def test_cuda_graph_replay_of_a_decode_call():
     ops.check_device_status()
 
 
+def test_packed_weight_scales_of_a_captured_call_outlive_their_eviction():
+    """One kernel object over more weights than its cache holds, captured into one graph: every captured call keeps the packing it was
+    given, also after later calls have evicted it and `drop_cached_weights` has emptied the cache."""
+    M, N, K, n = 16, 2048, 1024, 4
+    kernel, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    gemm = wb.wave_compile(wb.set_default_run_config(options), kernel)
+    gemm._weight_scales.capacity = 2
+    probs = [random_problem(M, N, K, seed=40 + i) for i in range(n)]
+    dev = [[t.to(DEV) for t in p] for p in probs]
+    outs = [torch.empty(M, N, dtype=torch.bfloat16, device=DEV) for _ in probs]
+    side, graph = torch.cuda.Stream(DEV), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        for p, c in zip(dev, outs):
+            gemm(*p, c)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        for p, c in zip(dev, outs):
+            gemm(*p, c)
+    assert len(gemm._weight_scales._entries) <= 2 and len(gemm._weight_scales._captured) == n
+    for p, ref, c in zip(dev, probs, outs):  # before any replay: a packing made in the capture holds nothing yet
+        gemm(*p, c)
+        check(c, *ref)
+    gemm.drop_cached_weights()
+    blocks = [torch.full((ops.packed_scale_bytes(N, K),), 255, dtype=torch.uint8, device=DEV) for _ in range(16)]
+    for c in outs:
+        c.fill_(float("nan"))
+    graph.replay()
+    for p, c in zip(probs, outs):
+        check(c, *p)
+    assert all(bool((t == 255).all()) for t in blocks)
+
+
 def test_graphed_gemm_keeps_the_kernel_object_alive():
     """The graph holds addresses of memory that belongs to the kernel object (workspace, scratch, packed weight scales): a graph whose
     maker dropped that object still has it, and gives the same result after its memory could have been handed out again."""

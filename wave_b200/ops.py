@@ -364,12 +364,15 @@ class WeightScaleCache:
     that the allocator places at a freed tensor's address therefore never meets the old packing, and an in-place
     write (which bumps the version of every view) makes the next call repack. What the cache cannot see is a write
     through a raw pointer (a C extension, a CUDA graph replay that rewrites the scales): call `clear()` — or
-    `ScaledGemmKernel.drop_cached_weights()` — after such a write."""
+    `ScaledGemmKernel.drop_cached_weights()` — after such a write. A packing that a captured call was given stays in memory
+    as long as the cache, whatever is evicted or dropped: the graph holds its address. One that is made while a graph is
+    captured is filled by the replays only and not given to any other call."""
 
     def __init__(self, capacity: int = 64):
         self.capacity = capacity
         self.packings = 0  # launched so far: a call that moves it has put a repack kernel in front of its GEMM
         self._entries: OrderedDict = OrderedDict()
+        self._captured: dict = {}
 
     def get(self, scale: torch.Tensor, tile_rows: int = 128) -> PackedScales:
         key = (scale.data_ptr(), tuple(scale.shape), scale.stride(), scale.device.index, scale._version, tile_rows)
@@ -378,14 +381,23 @@ class WeightScaleCache:
             owner, packed = hit
             if owner() is scale:
                 self._entries.move_to_end(key)
+                self._keep_if_captured(packed)
                 return packed
             del self._entries[key]  # same address, another (or a dead) tensor: the packing is not this tensor's
         packed = repack_scales(scale, tile_rows=tile_rows)
         self.packings += 1
+        if self._keep_if_captured(packed):
+            return packed
         self._entries[key] = (weakref.ref(scale), packed)
         while len(self._entries) > self.capacity:
             self._entries.popitem(last=False)
         return packed
+
+    def _keep_if_captured(self, packed: PackedScales) -> bool:
+        if not torch.cuda.is_current_stream_capturing():
+            return False
+        self._captured[id(packed)] = packed
+        return True
 
     def drop(self, scale: torch.Tensor) -> None:
         """Forget every packing made from this tensor's memory (any version)."""
