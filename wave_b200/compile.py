@@ -306,11 +306,13 @@ class ScaledGemmKernel:
         """The same for the mixed pair, whose decode kernel reads heights above 128. Each of its tiles ends with M rows of C that
         one lane writes per row, while the kernels for the other heights write whole rows: it needs the K for that, 32
         for every row of C that is written 16 bytes at a time, 256 where C's rows are not 16-byte aligned. us against the other
-        height, bf16: N = 28672, K = 512: M = 16 6.0 / 6.1, M = 48 6.6 / 6.6; N = 22208, K = 1024: M = 32 8.0 / 8.1, M = 64 9.5 / 8.9, M = 128 12.7 / 9.8; K = 4096: M = 128 20.8 / 23.5;
-        unaligned N = 28671, K = 2048: M = 8 11.8 / 11.9, M = 64 28.1 / 15.9, K = 8192: M = 32 35.8 / 35.8, M = 128 64.8 / 51.0. Up to
-        16 rows the usual packing takes the K-split kernel, which is ahead of low tiles over a long K (N = 19200, M = 16: K = 6144
-        18.8 / 19.0, K = 16384 42.2 / 38.1; N = 22208, K = 16384 45.8 / 45.3) and in unaligned stores (N = 22201, K = 4096, M = 8 15.7 /
-        16.2, M = 16 18.9 / 16.6)."""
+        height, bf16:
+          aligned: N = 28672, K = 512: M = 16 6.0 / 6.1, M = 48 6.6 / 6.6; N = 22208, K = 1024: M = 32 8.0 / 8.1,
+            M = 64 9.5 / 8.9, M = 128 12.7 / 9.8, K = 4096: M = 128 20.8 / 23.5;
+          unaligned: N = 28671, K = 2048: M = 8 11.8 / 11.9, M = 64 28.1 / 15.9, K = 8192: M = 32 35.8 / 35.8, M = 128 64.8 / 51.0.
+        Up to 16 rows the usual packing takes the K-split kernel, which is ahead of low tiles over a long K (N = 19200, M = 16:
+        K = 6144 18.8 / 19.0, K = 16384 42.2 / 38.1; N = 22208, K = 16384 45.8 / 45.3) and in unaligned stores (N = 22201,
+        K = 4096: M = 8 15.7 / 16.2, M = 16 18.9 / 16.6)."""
         usual = self._weight_tile_rows(M, N, dev_index)
         if M > 128 or self.options.kernel_path in (_lib.PATH_TILE_1CTA, _lib.PATH_TILE_2CTA):
             return usual  # no tile kernel reads a height above 128
