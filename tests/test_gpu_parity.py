@@ -636,6 +636,37 @@ def test_two_streams_pack_activation_scales_at_the_same_time(kind, M, N, K):
     ops.check_device_status()
 
 
+def test_graphed_calls_of_one_object_have_scratch_of_their_own_and_allocate_none():
+    """Two graphs over one kernel object, each warmed up on a stream of its own, and an eager call: three scratches, none of them made
+    during a capture. Replays of both graphs and eager calls on three streams at once give the results of the calls alone."""
+    from wave_b200.graphs import GraphedScaledGemm
+    M, N, K = 64, 28672, 1024
+    kernel, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    gemm = wb.wave_compile(wb.set_default_run_config(options), kernel)
+    a, _, b, b_s = (t.to(DEV) for t in random_problem(M, N, K, seed=3))
+    scales = [torch.randint(110 + 8 * i, 115 + 8 * i, (M, K // 32), dtype=torch.uint8, device=DEV) for i in range(3)]
+    outs = [torch.empty(M, N, dtype=torch.bfloat16, device=DEV) for _ in range(3)]
+    refs = []
+    for a_s in scales:
+        gemm(a, a_s, b, b_s, outs[0])
+        torch.cuda.synchronize()
+        refs.append(outs[0].clone())
+    graphs = [GraphedScaledGemm(gemm, a, scales[i], b, b_s, outs[i]) for i in range(2)]
+    made = {key: [t.data_ptr() for t in bufs] for key, bufs in gemm._a_scale_buf.items()}
+    plans = {p[3].data_ptr() for p in gemm._plans.values()}
+    assert len(made) == 3 and plans == {v[0] for v in made.values()}  # (main stream and two warm-ups; the captures use those)
+    streams = [torch.cuda.Stream(DEV) for _ in range(3)]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for st, run in zip(streams, (graphs[0].replay, graphs[1].replay, lambda: gemm(a, scales[2], b, b_s, outs[2]))):
+            with torch.cuda.stream(st):
+                run()
+    torch.cuda.synchronize()
+    for c, ref in zip(outs, refs):
+        assert torch.equal(c.view(torch.int16), ref.view(torch.int16))
+    ops.check_device_status()
+
+
 def test_scratch_of_a_captured_call_outlives_a_larger_call():
     """A graph holds the address of the scratch it packs into: a larger call on the same stream takes new memory and leaves the old
     one to the graph, whatever is allocated afterwards."""

@@ -120,6 +120,7 @@ class ScaledGemmKernel:
         self.asm = ""  # the reference exposes generated code here; nothing is generated at run time
         self._weight_scales = ops.WeightScaleCache()
         self._a_scale_buf: dict[tuple[int, int], list[torch.Tensor]] = {}  # (device, stream) -> scratches, the one in use last
+        self._a_scale_last: dict[int, tuple[int, int]] = {}  # device -> key of the scratch that was asked for last
         self._workspaces = ops.WorkspacePool()  # this object's own: calls through another object may overlap with these
         self._plans: dict = {}
         self._tile_rows: dict = {}
@@ -270,7 +271,8 @@ class ScaledGemmKernel:
             plan = (M, N, K, a_buf, ws_ptr, ws_bytes, flags, ops._DTYPE_CODE[c.dtype], idx, ws)
             sig = (a.shape, a.stride(), a.dtype, a_scale.shape, a_scale.stride(), b.shape, b.stride(), b_scale.shape,
                    c.shape, c.stride(), c.dtype, a.device, torch.cuda.current_stream(a.device).cuda_stream)
-            self._plans[sig] = plan
+            if not torch.cuda.is_current_stream_capturing():  # (every capture takes the memory of its own warm-up)
+                self._plans[sig] = plan
             return self._launch(plan, a, a_scale, b, b_scale, c)
         a_sf = self._pack_activation_scales(a_scale, M, K)
         if isinstance(b_scale, ops.PackedScales):
@@ -351,12 +353,20 @@ class ScaledGemmKernel:
     def _a_scale_buffer(self, device, M, K):
         """Scratch for the packed activation scales of a call on the current stream: calls on other streams may overlap with it
         and have their own. One that a larger call has outgrown stays (a captured graph may hold its address); as every
-        new one has at least twice the size, what stays is smaller than what is in use."""
+        new one has at least twice the size, what stays is smaller than what is in use. A captured call takes the scratch of
+        the stream that asked for one last, which is its warm-up's: allocating in a capture takes milliseconds."""
         idx = device.index if device.index is not None else torch.cuda.current_device()
         need = ops.packed_scale_bytes(M, K)
-        bufs = self._a_scale_buf.setdefault((idx, torch.cuda.current_stream(idx).cuda_stream), [])
-        if not bufs or bufs[-1].numel() < need:
-            bufs.append(torch.empty(max(need, 2 * bufs[-1].numel()) if bufs else need, dtype=torch.uint8, device=device))
+        key = (idx, torch.cuda.current_stream(idx).cuda_stream)
+        bufs = self._a_scale_buf.get(key)
+        if bufs is None or bufs[-1].numel() < need:
+            last = self._a_scale_buf.get(self._a_scale_last.get(idx))
+            if last is not None and last[-1].numel() >= need and torch.cuda.is_current_stream_capturing():
+                return last[-1]
+            size = max(need, 2 * bufs[-1].numel()) if bufs else need
+            bufs = self._a_scale_buf.setdefault(key, [])
+            bufs.append(torch.empty(size, dtype=torch.uint8, device=device))
+        self._a_scale_last[idx] = key
         return bufs[-1]
 
     def _pack_activation_scales(self, a_scale, M, K):

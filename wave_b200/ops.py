@@ -142,13 +142,14 @@ class WorkspacePool:
     functional entry points share a module-level one.
 
     Workspaces are created and initialised eagerly. While a stream is being captured into a CUDA graph nothing
-    is allocated: the call uses the workspace an earlier eager call (the warm-up) made for that device and kind. The graph
+    is allocated: the call uses the workspace that the eager call before it (the warm-up) got for that device and kind. The graph
     keeps its address, so one that a larger call outgrows stays; as every new one has at least twice the size, what stays
     is smaller than what is in use. `clear` gives everything back: not while a graph is still to be replayed.
     """
 
     def __init__(self):
         self._by_key: dict = {}
+        self._last: dict = {}  # (device, kind) -> key of the workspace that was asked for last
         self._outgrown: list = []
 
     def get(self, device: torch.device, nbytes: int, kind: str) -> torch.Tensor:
@@ -157,10 +158,12 @@ class WorkspacePool:
         key = (idx, torch.cuda.current_stream(idx).cuda_stream, kind)
         ws = self._by_key.get(key)
         if ws is not None and ws.numel() >= nbytes:
+            self._last[idx, kind] = key
             return ws
         if capturing:
-            for (d, _, k), w in self._by_key.items():
-                if d == idx and k == kind and w.numel() >= nbytes:
+            last = self._by_key.get(self._last.get((idx, kind)))
+            for w in ([] if last is None else [last]) + [w for (d, _, k), w in self._by_key.items() if d == idx and k == kind]:
+                if w.numel() >= nbytes:
                     return w
             raise RuntimeError("this GEMM needs a workspace, which cannot be created while a CUDA graph is being captured: "
                                "call it once eagerly (with the same shapes) before the capture")
@@ -171,10 +174,12 @@ class WorkspacePool:
         with torch.cuda.device(idx):
             _lib.check(_lib.load().wb200_workspace_init(ws.data_ptr(), nbytes, _stream()))
         self._by_key[key] = ws
+        self._last[idx, kind] = key
         return ws
 
     def clear(self) -> None:
         self._by_key.clear()
+        self._last.clear()
         self._outgrown.clear()
 
 
