@@ -34,6 +34,7 @@ def seed_torch():
 def built_library():
     """Build the CUDA library if needed (nvcc cross-compiles without a GPU) and return its path."""
     from wave_b200 import build
+    build.build_fast()
     return build.build()
 
 

@@ -1496,3 +1496,97 @@ def test_linear_in_one_call_gives_the_bits_of_quantiser_and_gemm(rows, N, K, dty
         ops.scaled_gemm_packed(q, sf, layer.weight_codes, layer._packed_decode if rows <= 128 else layer._packed, ref)
         assert torch.equal(y, ref)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K,kind", [(8, 640, 416, "fp4"), (300, 512, 1024, "fp4"), (16, 1024, 512, "fp8"), (16, 1024, 512, "mixed")])
+def test_a_repeated_call_follows_its_tensors(M, N, K, kind):
+    """The second call with tensors of the same form is recognised in native code. It reads the tensors it is given (other activations, other
+    weights, scales rewritten in place, another stream, a transposed operand, a wider output), and refuses what the first call would. Each
+    result has the bits of a fresh kernel object's first call."""
+    def operands(seed):
+        g = torch.Generator().manual_seed(seed)
+        if kind == "fp4":
+            return [t.to(DEV) for t in random_problem(M, N, K, seed=seed)]
+        x, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+        b = ops.quantize_mxfp8(w, torch.float8_e4m3fn) if kind == "fp8" else ops.quantize_mxfp4(w)
+        return [*ops.quantize_mxfp8(x, torch.float8_e4m3fn)[:2], *b[:2]]
+
+    def compiled():
+        if kind == "fp4":
+            t, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+        else:
+            t, subs = wb.get_scaled_gemm_mxfp8_kernel((M, N, K), wb.ScaledMMAType.F32_16x16x128_F8F6F4, "f8e4m3fn", wb.bf16,
+                                                      weight_format="f4e2m1fn" if kind == "mixed" else None)
+            options = wb.WaveCompileOptions(subs=subs)
+        return wb.wave_compile(wb.set_default_run_config(options), t)
+
+    gemm = compiled()
+    wide = torch.full((M, N + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+
+    def expect(args, c=None):
+        c = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV) if c is None else c
+        ref = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+        gemm(*args, c)
+        compiled()(*args, ref)
+        assert torch.equal(c, ref)
+
+    one, two = operands(1), operands(2)
+    for args in (one, one, two, two, one[:2] + two[2:], one):
+        expect(args)
+    one[3].copy_(two[3])  # in place: the version counter moves
+    expect(one)
+    expect(one)
+    for _ in range(2):
+        expect(one, wide[:, :N])
+        expect(one, wide[:, 1:N + 1])  # rows that are not 16-byte aligned
+    assert bool((wide[:, N + 1:] == 7.0).all())
+    bits = one[0].view(torch.uint8)
+    expect([bits.t().contiguous().t().view(one[0].dtype), *one[1:]])
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream(DEV)
+    with torch.cuda.stream(side):
+        expect(one)
+        expect(two)
+    side.synchronize()
+    with torch.inference_mode():
+        expect([one[0].clone(), *one[1:]])
+    good = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    for bad in ([one[0][:-1], *one[1:], good], [one[0], one[1][:, :-1], *one[2:], good], [*one, good[:, :-1]], [*one, good.float()],
+                [*one[:3], one[3][:-1], good], [one[0].cpu(), *one[1:], good], [*one[:2], one[2][:-1], one[3], good]):
+        with pytest.raises(ValueError):
+            gemm(*bad)
+    gemm.drop_cached_weights()
+    expect(one)
+    ops.check_device_status()
+
+
+def test_a_repeated_linear_call_follows_its_tensors():
+    """MXFP4Linear: second and later calls, at several batch sizes, with strided, transposed, 1-D and 3-D inputs, on another stream, in a
+    captured graph; each has the bits of the call that a new layer makes first."""
+    N, K = 640, 416
+    g = torch.Generator().manual_seed(1)
+    layer = wb.MXFP4Linear.from_float((torch.randn(N, K, generator=g) * 0.02).to(DEV))
+    wide = torch.randn(200, K + 32, generator=g).to(torch.bfloat16).to(DEV)
+
+    def expect(x):
+        y, ref = layer(x), wb.MXFP4Linear(layer.weight_codes, layer.weight_scales)(x)
+        assert y.shape == (*x.shape[:-1], N) and torch.equal(y, ref)
+
+    for _ in range(2):
+        for x in (wide[:3, :K], wide[:200, 16:K + 16], wide[:8, :K].float(), wide[0, :K], wide[:6, :K].reshape(2, 3, K), wide[:, :K].t().contiguous().t()):
+            expect(x)
+        with torch.cuda.stream(torch.cuda.Stream(DEV)):
+            expect(wide[:3, :K])
+            torch.cuda.current_stream().synchronize()
+    with pytest.raises(RuntimeError):
+        layer(wide[:3, :K - 32])
+    with pytest.raises(ValueError):
+        layer(wide[:3, 1:K + 1])  # rows that are not 16-byte aligned
+    x = wide[:4, :K].contiguous()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = layer(x)
+    x.copy_(wide[10:14, :K])
+    graph.replay()
+    assert torch.equal(y, layer(wide[10:14, :K]))
+    ops.check_device_status()

@@ -278,6 +278,24 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_fast = None
+
+
+def fast():
+    """The host module for repeated calls (csrc/fast_call.cpp), bound to the loaded library."""
+    global _fast
+    if _fast is None:
+        lib = load()
+        try:
+            from . import _fast as module
+        except ImportError as e:
+            raise RuntimeError(f"wave_b200._fast cannot be loaded ({e}): build it with `python -m wave_b200.build`") from e
+        module.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.wb200_mxfp4_gemm_repack_a, lib.wb200_mxfp8_gemm_repack_a,
+                                                                      lib.wb200_mxfp4_gemm_quantize_a, lib.wb200_mxfp4_gemm_workspace_bytes)))
+        _fast = module
+    return _fast
+
+
 def check(rc: int) -> None:
     """Turn a status code of the C ABI into the exception class the reference would raise."""
     if rc == WB200_OK:

@@ -1,4 +1,4 @@
-"""Build libwave_b200.so in-tree with nvcc for sm_100a (`python -m wave_b200.build`)."""
+"""Build libwave_b200.so (nvcc, sm_100a) and the host module _fast.so (g++) in-tree: `python -m wave_b200.build`."""
 
 from __future__ import annotations
 
@@ -65,6 +65,31 @@ def build(force: bool = False, verbose: bool = False, trace: bool = False, check
     return out
 
 
+FAST_OUT = PKG / "_fast.so"
+FAST_SOURCE = CSRC / "fast_call.cpp"
+
+
+def build_fast(force: bool = False) -> Path:
+    """Compile `wave_b200._fast` (csrc/fast_call.cpp, against the installed torch) if it is missing or older than its source."""
+    if not force and FAST_OUT.exists() and FAST_SOURCE.stat().st_mtime <= FAST_OUT.stat().st_mtime:
+        return FAST_OUT
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    nvcc = Path(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc").resolve()
+    includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", nvcc.parent.parent / "include",
+                Path(sysconfig.get_paths()["include"])]
+    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-I{i}" for i in includes), str(FAST_SOURCE), "-o", str(FAST_OUT), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           "-ltorch_cuda", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed ({res.returncode}):\n{res.stdout}\n{res.stderr}")
+    return FAST_OUT
+
+
 if __name__ == "__main__":
+    print(build_fast(force="--force" in sys.argv))
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv, trace="--trace" in sys.argv, checks="--checks" in sys.argv,
                 mma_ceiling="--mma-ceiling" in sys.argv))

@@ -1,0 +1,394 @@
+// Repeated calls of the Python front ends, in native code: `wave_b200._fast`.
+//
+// A scaled GEMM of a small problem runs for 5 to 30 microseconds on the GPU, and so long did the Python code take that leads
+// to it (the counterpart of the reference's invoke path, wave_lang/kernel/wave/utils/run_utils.py:62-134, which it
+// measures with profile_python_wrapper): building the key of a call from shapes and strides, the look-up of the weight's packed
+// scales and of the workspace, sixteen arguments through ctypes. Here a call that was made before is recognised from the
+// tensors themselves and goes straight to the C ABI of include/wave_b200.h; whatever is not recognised returns None, and the
+// Python code does what it always did (all checks, all error messages) and then registers what it found.
+//
+// What is kept: per kernel object, the signatures (sizes, strides, types, device, stream, alignment of the output) of at most
+// kMaxPlans calls with their scratch, and at most kMaxWeights packings of weight scales, each found by the tensor it was made from
+// (a weak reference), its version counter and its address, as WeightScaleCache does. Nothing about activations or outputs
+// is kept but their shapes. Calls under stream capture, on another device than the current one, with tensor subclasses, under
+// functional transforms, or with inference tensors are left to the Python code.
+// us per call, calls back to back: 1024^3 f32 16.9 -> 8.2 (the GPU's time now), MXFP4Linear 8 x 14336 x 4096 26.8 -> 15.6.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <algorithm>
+#include <vector>
+
+namespace {
+
+constexpr size_t kMaxPlans = 64, kMaxWeights = 64;
+constexpr int kF32 = 0, kBF16 = 1;  // WB200_F32, WB200_BF16
+
+struct Abi {
+  int (*gemm_repack_a)(int, int, int, const void*, const void*, long long, void*, const void*, const void*, void*, int, long long, void*, size_t,
+                       unsigned, void*);
+  int (*mxfp8_gemm_repack_a)(int, int, int, const void*, const void*, long long, void*, const void*, const void*, void*, int, long long, int, void*,
+                             size_t, unsigned, void*);
+  int (*gemm_quantize_a)(int, int, int, const void*, int, long long, void*, void*, const void*, const void*, void*, int, long long, void*, size_t,
+                         unsigned, void*);
+  size_t (*gemm_workspace_bytes)(int, int, int);
+} abi;
+
+// An ordinary CUDA tensor: no subclass, no wrapper of a functional transform, no inference tensor.
+bool plain(PyObject* o) {
+  if (Py_TYPE(o) != reinterpret_cast<PyTypeObject*>(THPVariableClass)) return false;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  static const c10::DispatchKeySet keys = c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::ADInplaceOrView}) |
+                                          c10::getAutogradRelatedKeySetFromBackend(c10::BackendComponent::CUDABit) |
+                                          c10::getAutocastRelatedKeySetFromBackend(c10::BackendComponent::CUDABit);
+  return t.key_set() == keys && t.layout() == at::kStrided;
+}
+
+struct Signature {
+  int64_t size[2], stride[2];
+  at::ScalarType type;
+  bool operator==(const Signature& o) const {
+    return size[0] == o.size[0] && size[1] == o.size[1] && stride[0] == o.stride[0] && stride[1] == o.stride[1] && type == o.type;
+  }
+};
+bool signature_of(const at::Tensor& t, int device, Signature* s) {
+  if (t.dim() != 2 || t.device().index() != device) return false;
+  s->size[0] = t.size(0);
+  s->size[1] = t.size(1);
+  s->stride[0] = t.stride(0);
+  s->stride[1] = t.stride(1);
+  s->type = t.scalar_type();
+  return true;
+}
+
+// Every row of a matrix with unit column stride starts on 16 bytes.
+bool rows_aligned(const at::Tensor& c) {
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0 && (c.size(0) == 1 || c.stride(0) * int64_t(c.element_size()) % 16 == 0);
+}
+
+struct CallKey {  // order: a, a_scale, b, b_scale, c
+  Signature sig[5];
+  int device;
+  cudaStream_t stream;
+  bool aligned, tiled;
+  long path;
+  bool operator==(const CallKey& o) const {
+    return stream == o.stream && device == o.device && aligned == o.aligned && tiled == o.tiled && path == o.path && std::equal(sig, sig + 5, o.sig);
+  }
+};
+struct Plan {
+  CallKey key;
+  int M, N, K;
+  int elem_format;  // -1: MXFP4
+  unsigned flags;
+  at::Tensor scratch, workspace;  // packed activation scales; workspace (undefined: none)
+  size_t workspace_bytes;
+  int tile_rows;
+};
+struct Weight {
+  c10::weak_intrusive_ptr<c10::TensorImpl> owner;
+  const c10::TensorImpl* impl;
+  const void* ptr;
+  uint32_t version;
+  int tile_rows;
+  at::Tensor packed;
+};
+
+struct Calls {
+  std::vector<Plan> plans;
+  std::vector<Weight> weights;
+  size_t next_plan = 0, next_weight = 0, last_plan = 0;
+
+  const Plan* find(const CallKey& key) {
+    if (last_plan < plans.size() && plans[last_plan].key == key) return &plans[last_plan];
+    for (size_t i = 0; i < plans.size(); ++i)
+      if (plans[i].key == key) {
+        last_plan = i;
+        return &plans[i];
+      }
+    return nullptr;
+  }
+  const Weight* find(const at::Tensor& scale, int tile_rows) {
+    const c10::TensorImpl* impl = scale.unsafeGetTensorImpl();
+    for (const Weight& w : weights)
+      // (an address that another tensor has taken over belongs to a new object, and the reference to the old one has expired)
+      if (w.impl == impl && w.tile_rows == tile_rows && !w.owner.expired() && w.ptr == scale.data_ptr() && w.version == scale._version()) return &w;
+    return nullptr;
+  }
+};
+
+struct PyCalls {
+  PyObject_HEAD
+  Calls* calls;
+};
+
+bool key_of(PyObject* const* args, CallKey* key) {
+  for (int i = 0; i < 5; ++i)
+    if (!plain(args[i])) return false;
+  const at::Tensor& a = THPVariable_Unpack(args[0]);
+  key->device = a.device().index();
+  if (key->device != c10::cuda::current_device()) return false;
+  for (int i = 0; i < 5; ++i)
+    if (!signature_of(THPVariable_Unpack(args[i]), key->device, &key->sig[i])) return false;
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return false;
+  key->stream = c10::cuda::getCurrentCUDAStream(key->device).stream();
+  key->aligned = rows_aligned(THPVariable_Unpack(args[4]));
+  key->tiled = PyObject_IsTrue(args[5]) == 1;
+  key->path = PyLong_AsLong(args[6]);
+  return true;
+}
+
+PyObject* fail(const std::exception& e) {
+  PyErr_SetString(PyExc_RuntimeError, e.what());
+  return nullptr;
+}
+
+// call(a, a_scale, b, b_scale, c, tiled, path) -> status of the launch, or None: not a call that is known here
+PyObject* calls_call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  if (n != 7) {
+    PyErr_SetString(PyExc_TypeError, "call takes 7 arguments");
+    return nullptr;
+  }
+  try {
+    Calls& calls = *reinterpret_cast<PyCalls*>(self)->calls;
+    CallKey key;
+    if (calls.plans.empty() || !key_of(args, &key)) {
+      if (PyErr_Occurred()) return nullptr;
+      Py_RETURN_NONE;
+    }
+    const Plan* found = calls.find(key);
+    const Weight* weight = found ? calls.find(THPVariable_Unpack(args[3]), found->tile_rows) : nullptr;
+    if (!weight) Py_RETURN_NONE;
+    // another thread may change the tables while the lock is released: what the launch reads is held here
+    const at::Tensor scratch = found->scratch, workspace = found->workspace, packed = weight->packed;
+    const int M = found->M, N = found->N, K = found->K, elem_format = found->elem_format;
+    const size_t ws_bytes = found->workspace_bytes;
+    const unsigned flags = found->flags;
+    const void* ptr[4];
+    for (int i = 0; i < 3; ++i) ptr[i] = THPVariable_Unpack(args[i]).data_ptr();
+    void* c = THPVariable_Unpack(args[4]).data_ptr();
+    const int c_type = key.sig[4].type == at::kFloat ? kF32 : kBF16;
+    const long long a_scale_stride = M > 1 ? key.sig[1].stride[0] : K / 32, ldc = M > 1 ? key.sig[4].stride[0] : N;
+    void* ws = workspace.defined() ? workspace.data_ptr() : nullptr;
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    if (elem_format < 0)
+      rc = abi.gemm_repack_a(M, N, K, ptr[0], ptr[1], a_scale_stride, scratch.data_ptr(), ptr[2], packed.data_ptr(), c, c_type, ldc, ws, ws_bytes, flags,
+                             key.stream);
+    else
+      rc = abi.mxfp8_gemm_repack_a(M, N, K, ptr[0], ptr[1], a_scale_stride, scratch.data_ptr(), ptr[2], packed.data_ptr(), c, c_type, ldc, elem_format,
+                                   ws, ws_bytes, flags, key.stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(rc);
+  } catch (const std::exception& e) {
+    return fail(e);
+  }
+}
+
+// add(a, a_scale, b, b_scale, c, tiled, path, (M, N, K, elem_format, flags, tile_rows, workspace_bytes), packed, scratch, workspace or None):
+// the Python code has just made this call with these arguments.
+PyObject* calls_add(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  if (n != 11) {
+    PyErr_SetString(PyExc_TypeError, "add takes 11 arguments");
+    return nullptr;
+  }
+  try {
+    Calls& calls = *reinterpret_cast<PyCalls*>(self)->calls;
+    Plan p;
+    Py_ssize_t ws_bytes = 0;
+    if (!PyArg_ParseTuple(args[7], "iiiiIin", &p.M, &p.N, &p.K, &p.elem_format, &p.flags, &p.tile_rows, &ws_bytes)) return nullptr;
+    if (!key_of(args, &p.key) || !THPVariable_Check(args[8]) || !THPVariable_Check(args[9])) {
+      if (PyErr_Occurred()) return nullptr;
+      Py_RETURN_NONE;
+    }
+    const at::ScalarType c_type = p.key.sig[4].type;
+    if (p.key.sig[4].stride[1] != 1 || (c_type != at::kFloat && c_type != at::kBFloat16)) Py_RETURN_NONE;
+    p.scratch = THPVariable_Unpack(args[9]);
+    if (args[10] != Py_None) p.workspace = THPVariable_Unpack(args[10]);
+    p.workspace_bytes = size_t(ws_bytes);
+    if (const Plan* old = calls.find(p.key)) {
+      const_cast<Plan&>(*old) = p;
+    } else if (calls.plans.size() < kMaxPlans) {
+      calls.plans.push_back(p);
+    } else {
+      calls.plans[calls.next_plan++ % kMaxPlans] = p;
+    }
+    const at::Tensor& scale = THPVariable_Unpack(args[3]);
+    if (!calls.find(scale, p.tile_rows)) {
+      const auto gone = std::remove_if(calls.weights.begin(), calls.weights.end(), [&](const Weight& w) {
+        return w.owner.expired() || (w.impl == scale.unsafeGetTensorImpl() && w.tile_rows == p.tile_rows);
+      });
+      calls.weights.erase(gone, calls.weights.end());
+      Weight w{c10::weak_intrusive_ptr<c10::TensorImpl>(scale.getIntrusivePtr()), scale.unsafeGetTensorImpl(), scale.data_ptr(),
+               uint32_t(scale._version()), p.tile_rows, THPVariable_Unpack(args[8])};
+      if (calls.weights.size() < kMaxWeights) calls.weights.push_back(std::move(w));
+      else calls.weights[calls.next_weight++ % kMaxWeights] = std::move(w);
+    }
+    Py_RETURN_NONE;
+  } catch (const std::exception& e) {
+    return fail(e);
+  }
+}
+
+PyObject* calls_clear(PyObject* self, PyObject*) {
+  Calls& calls = *reinterpret_cast<PyCalls*>(self)->calls;
+  calls.plans.clear();
+  calls.weights.clear();
+  Py_RETURN_NONE;
+}
+
+// ---------------------------------------------------------------------------------------------
+// workspaces of the functional entry points, as WorkspacePool holds them
+// ---------------------------------------------------------------------------------------------
+struct Workspaces {
+  struct Entry {
+    int device;
+    cudaStream_t stream;
+    at::Tensor ws;
+  };
+  std::vector<Entry> entries;
+};
+struct PyWorkspaces {
+  PyObject_HEAD
+  Workspaces* table;
+};
+// put(device, stream, workspace)
+PyObject* workspaces_put(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  if (n != 3 || !THPVariable_Check(args[2])) {
+    PyErr_SetString(PyExc_TypeError, "put takes a device index, a stream and a tensor");
+    return nullptr;
+  }
+  const int device = int(PyLong_AsLong(args[0]));
+  auto stream = reinterpret_cast<cudaStream_t>(PyLong_AsUnsignedLongLong(args[1]));
+  if (PyErr_Occurred()) return nullptr;
+  auto& entries = reinterpret_cast<PyWorkspaces*>(self)->table->entries;
+  for (auto& e : entries)
+    if (e.device == device && e.stream == stream) {
+      e.ws = THPVariable_Unpack(args[2]);
+      Py_RETURN_NONE;
+    }
+  entries.push_back({device, stream, THPVariable_Unpack(args[2])});
+  Py_RETURN_NONE;
+}
+PyObject* workspaces_clear(PyObject* self, PyObject*) {
+  reinterpret_cast<PyWorkspaces*>(self)->table->entries.clear();
+  Py_RETURN_NONE;
+}
+
+template <typename Object, typename Data, Data* Object::*Field>
+PyObject* object_new(PyTypeObject* type, PyObject*, PyObject*) {
+  PyObject* self = type->tp_alloc(type, 0);
+  if (self) reinterpret_cast<Object*>(self)->*Field = new Data;
+  return self;
+}
+template <typename Object, typename Data, Data* Object::*Field>
+void object_free(PyObject* self) {
+  delete (reinterpret_cast<Object*>(self)->*Field);
+  Py_TYPE(self)->tp_free(self);
+}
+
+// linear(x, weight_codes, packed_scales, tile_rows, output dtype, workspaces) -> dequant(quantise(x)) @ dequant(W)^T, or None: left to
+// the Python code. packed_scales: of weight_codes, per tile_rows rows; the caller has chosen them for this number of rows.
+PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 6) {
+    PyErr_SetString(PyExc_TypeError, "linear takes 6 arguments");
+    return nullptr;
+  }
+  try {
+    if (!plain(args[0]) || !plain(args[1]) || !plain(args[2]) || !THPDtype_Check(args[4])) Py_RETURN_NONE;
+    const at::Tensor &x = THPVariable_Unpack(args[0]), &w = THPVariable_Unpack(args[1]), &packed = THPVariable_Unpack(args[2]);
+    const int device = x.device().index();
+    const at::ScalarType x_type = x.scalar_type(), out_type = reinterpret_cast<THPDtype*>(args[4])->scalar_type;
+    const int64_t dims = x.dim();
+    if (device != c10::cuda::current_device() || w.device().index() != device || packed.device().index() != device || dims < 1 || w.dim() != 2 ||
+        !w.is_contiguous() || (x_type != at::kFloat && x_type != at::kBFloat16) || (out_type != at::kFloat && out_type != at::kBFloat16))
+      Py_RETURN_NONE;
+    const int64_t K = w.size(1) * 2, N = w.size(0);
+    if (x.size(dims - 1) != K || K == 0 || x.numel() == 0) Py_RETURN_NONE;
+    const int64_t M = x.numel() / K;
+    const bool strided = dims == 2 && x.stride(1) == 1 && x.stride(0) >= K;
+    if (!(strided || x.is_contiguous()) || M > 0x7fffffff || N > 0x7fffffff) Py_RETURN_NONE;
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) Py_RETURN_NONE;
+    const auto stream = c10::cuda::getCurrentCUDAStream(device);
+    at::Tensor ws;
+    size_t ws_bytes = 0;
+    if (M <= 128) {
+      ws_bytes = abi.gemm_workspace_bytes(int(M), int(N), int(K));
+      for (const auto& e : reinterpret_cast<PyWorkspaces*>(args[5])->table->entries)
+        if (e.device == device && e.stream == stream.stream()) ws = e.ws;
+      if (!ws.defined() || size_t(ws.numel()) < ws_bytes) Py_RETURN_NONE;
+    }
+    const long tile_rows = PyLong_AsLong(args[3]);
+    if (PyErr_Occurred()) return nullptr;
+    std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = N;
+    const at::Tensor out = at::detail::empty_cuda(shape, out_type, x.device(), c10::nullopt);
+    const int64_t q_bytes = (M * K / 2 + 255) / 256 * 256;
+    const at::Tensor scratch = at::detail::empty_cuda({q_bytes + (M + 127) / 128 * ((K + 255) / 256) * 1024}, at::kByte, x.device(), c10::nullopt);
+    uint8_t* q = static_cast<uint8_t*>(scratch.data_ptr());
+    const unsigned flags = tile_rows == 128 ? 0u : unsigned(tile_rows / 8) << 16;  // WB200_B_TILE_ROWS
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = abi.gemm_quantize_a(int(M), int(N), int(K), x.data_ptr(), x_type == at::kFloat ? kF32 : kBF16, strided && M > 1 ? x.stride(0) : K, q, q + q_bytes,
+                             w.data_ptr(), packed.data_ptr(), out.data_ptr(), out_type == at::kFloat ? kF32 : kBF16, N,
+                             ws.defined() ? ws.data_ptr() : nullptr, ws_bytes, flags, stream.stream());
+    Py_END_ALLOW_THREADS
+    if (rc) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(out);
+  } catch (const std::exception& e) {
+    return fail(e);
+  }
+}
+
+// bind(gemm_repack_a, mxfp8_gemm_repack_a, gemm_quantize_a, gemm_workspace_bytes): addresses in the loaded library
+PyObject* bind(PyObject*, PyObject* args) {
+  unsigned long long p[4];
+  if (!PyArg_ParseTuple(args, "KKKK", &p[0], &p[1], &p[2], &p[3])) return nullptr;
+  abi.gemm_repack_a = reinterpret_cast<decltype(abi.gemm_repack_a)>(p[0]);
+  abi.mxfp8_gemm_repack_a = reinterpret_cast<decltype(abi.mxfp8_gemm_repack_a)>(p[1]);
+  abi.gemm_quantize_a = reinterpret_cast<decltype(abi.gemm_quantize_a)>(p[2]);
+  abi.gemm_workspace_bytes = reinterpret_cast<decltype(abi.gemm_workspace_bytes)>(p[3]);
+  Py_RETURN_NONE;
+}
+
+#define FASTCALL(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL
+PyMethodDef calls_methods[] = {{"call", FASTCALL(calls_call), nullptr}, {"add", FASTCALL(calls_add), nullptr},
+                               {"clear", calls_clear, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyMethodDef workspaces_methods[] = {{"put", FASTCALL(workspaces_put), nullptr}, {"clear", workspaces_clear, METH_NOARGS, nullptr},
+                                    {nullptr, nullptr, 0, nullptr}};
+PyMethodDef module_methods[] = {{"bind", bind, METH_VARARGS, nullptr}, {"linear", FASTCALL(linear), nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_fast", nullptr, -1, module_methods, nullptr, nullptr, nullptr, nullptr};
+
+template <typename Object, typename Data, Data* Object::*Field>
+bool add_type(PyObject* module, const char* name, const char* qualified, PyMethodDef* methods) {
+  static PyTypeObject type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+  type.tp_name = qualified;
+  type.tp_basicsize = sizeof(Object);
+  type.tp_flags = Py_TPFLAGS_DEFAULT;
+  type.tp_methods = methods;
+  type.tp_new = object_new<Object, Data, Field>;
+  type.tp_dealloc = object_free<Object, Data, Field>;
+  if (PyType_Ready(&type) < 0) return false;
+  return PyModule_AddObjectRef(module, name, reinterpret_cast<PyObject*>(&type)) == 0;
+}
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__fast() {
+  PyObject* m = PyModule_Create(&module_def);
+  if (!m) return nullptr;
+  if (!add_type<PyCalls, Calls, &PyCalls::calls>(m, "Calls", "wave_b200._fast.Calls", calls_methods) ||
+      !add_type<PyWorkspaces, Workspaces, &PyWorkspaces::table>(m, "Workspaces", "wave_b200._fast.Workspaces", workspaces_methods)) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import torch
 
-from . import ops
+from . import _lib, ops
 from .lang import as_output_dtype
 
 
@@ -36,6 +36,18 @@ class MXFP4Linear(torch.nn.Module):
         return cls(q, s, output_dtype)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        rows = x.numel() // self.in_features
+        packed = self._packed if rows > 128 else self._packed_decode
+        if packed is not None:
+            # a call whose tensors need no preparation; anything else comes back unhandled
+            y = _lib.fast().linear(x, self._buffers.get("weight_codes"), packed.data, packed.tile_rows, self.output_dtype, ops._pool.fast)
+            if type(y) is int:
+                _lib.check(y)
+            elif y is not None:
+                return y
+        return self._forward_checked(x)
+
+    def _forward_checked(self, x: torch.Tensor) -> torch.Tensor:
         lead = x.shape[:-1]
         x2 = x.reshape(-1, self.in_features)
         out = torch.empty(x2.shape[0], self.out_features, dtype=self.output_dtype, device=x.device)

@@ -151,6 +151,13 @@ class WorkspacePool:
         self._by_key: dict = {}
         self._last: dict = {}  # (device, kind) -> key of the workspace that was asked for last
         self._outgrown: list = []
+        self._fast = None  # the "skinny" ones of eager calls, for the native linear call
+
+    @property
+    def fast(self):
+        if self._fast is None:
+            self._fast = _lib.fast().Workspaces()
+        return self._fast
 
     def get(self, device: torch.device, nbytes: int, kind: str) -> torch.Tensor:
         idx = device.index if device.index is not None else torch.cuda.current_device()
@@ -159,6 +166,8 @@ class WorkspacePool:
         ws = self._by_key.get(key)
         if ws is not None and ws.numel() >= nbytes:
             self._last[idx, kind] = key
+            if kind == "skinny" and not capturing:
+                self.fast.put(idx, key[1], ws)
             return ws
         if capturing:
             last = self._by_key.get(self._last.get((idx, kind)))
@@ -175,12 +184,16 @@ class WorkspacePool:
             _lib.check(_lib.load().wb200_workspace_init(ws.data_ptr(), nbytes, _stream()))
         self._by_key[key] = ws
         self._last[idx, kind] = key
+        if kind == "skinny":
+            self.fast.put(idx, key[1], ws)
         return ws
 
     def clear(self) -> None:
         self._by_key.clear()
         self._last.clear()
         self._outgrown.clear()
+        if self._fast is not None:
+            self._fast.clear()
 
 
 _pool = WorkspacePool()
