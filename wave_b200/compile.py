@@ -126,6 +126,7 @@ class ScaledGemmKernel:
         self._tile_rows: dict = {}
         self._lib = _lib.load()
         self._fast = _lib.fast().Calls()  # calls made before, recognised in native code
+        self._bound_lib = self._lib  # the library that module calls: not used once `_lib` is another object
         self._static = None
         if template.shape is not None and not options.dynamic_symbols:
             self._static = tuple(template.shape)
@@ -143,10 +144,11 @@ class ScaledGemmKernel:
             finally:
                 self._in_bench = False
             return None
-        options = self.options
-        rc = self._fast.call(a, a_scale, b, b_scale, c, options.decode_tiled_weight_scales, options.kernel_path)
-        if rc is not None:
-            return _lib.check(rc) if rc else None
+        if self._lib is self._bound_lib:
+            options = self.options
+            rc = self._fast.call(a, a_scale, b, b_scale, c, options.decode_tiled_weight_scales, options.kernel_path)
+            if rc is not None:
+                return _lib.check(rc) if rc else None
         # Next: plain tensors whose (shape, dtype, stride, device) signature was validated before.
         # The signature check is what stands between the caller and the C ABI on every call, so it is
         # done once per distinct signature and remembered.
