@@ -130,7 +130,12 @@ size_t wb200_packed_scale_bytes(int rows, int K);
  * range keeps both packings. The reference prepares its weight scales per kernel variant in the same way
  * (e8m0_shuffle for the preshuffle templates, wave_lang/kernel/wave/utils/mxfp_utils.py:113-128). */
 int wb200_decode_tile_rows(int N);
-/* The same for the mixed pair (8-bit activations, 4-bit weights, WB200_B_FP4): where it returns a height above 128 (up to
+/* The height for calls of one M and K (weight_bits / activation_bits: 4 or 8; c_rows_aligned: every row of c starts on 16 bytes),
+ * 128 where the usual packing is the faster one: also with fewer 128-row tiles than SMs, where one low tile per SM is ahead of cutting K
+ * as long as K is short for the height, and with a thin last round over a short K. A height for which N has fewer tiles than SMs is
+ * read only if it is the lowest one with at most one tile per SM. */
+int wb200_decode_tile_rows_for(int M, int N, int K, int weight_bits, int activation_bits, int c_rows_aligned);
+/* wb200_decode_tile_rows for the mixed pair (8-bit activations, 4-bit weights, WB200_B_FP4): where it returns a height above 128 (up to
  * 208; two atom rows per tile) the decode kernel puts the weights on the MMA's N side. Only wb200_mxfp8_gemm with
  * WB200_B_FP4 and M <= 128 reads such a packing. */
 int wb200_mixed_decode_tile_rows(int N);

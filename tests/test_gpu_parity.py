@@ -1590,3 +1590,47 @@ def test_a_repeated_linear_call_follows_its_tensors():
     graph.replay()
     assert torch.equal(y, layer(wide[10:14, :K]))
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("N,K", [(8, 32), (1000, 2048), (4096, 4096), (5803, 5376), (11001, 8192), (14336, 4096), (14335, 2080), (17800, 8192), (18900, 4096),
+                                 (17408, 10240), (20480, 4096), (20483, 1024)])
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 64, 128])
+def test_low_decode_tiles_match_the_usual_packing(M, N, K):
+    """One low weight tile per SM, and several of them over a short K, in the template call: heights from 8 to 128, tiles that end past N, K
+    that ends inside a stage, rows of C that are 16-byte aligned or not. Against the oracle (the bars of every decode kernel: one
+    bf16 ulp, or the f32 bound) and the same call on the usual packing."""
+    a, a_s, b, b_s = random_problem(M, N, K, seed=M + N + K)
+    ad, asd, bd, bsd = a.to(DEV), a_s.to(DEV), b.to(DEV), b_s.to(DEV)
+    ref = orc.scaled_gemm(a, a_s, b, b_s)
+    for out_dtype in (torch.bfloat16, torch.float32):
+        outs = []
+        for tiled in (True, False):
+            kernel, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.TORCH_DTYPE_TO_WAVE[out_dtype])
+            options.decode_tiled_weight_scales = tiled
+            c = torch.full((M, N), float("nan"), dtype=out_dtype, device=DEV)
+            wb.wave_compile(options, kernel)(ad, asd, bd, bsd, c)
+            outs.append(c)
+        for c in outs:
+            check(c, a, a_s, b, b_s, ref=ref)
+        h = ops.decode_tile_rows_for(M, N, K, c_aligned=ops.rows_aligned(c))
+        assert h % 8 == 0 and 8 <= h <= 128
+    if h != 128 and N % 8 == 0:  # added into a C that holds values
+        acc = torch.ones(M, N, device=DEV)
+        ops.scaled_gemm_packed(ad, ops.repack_scales(asd), bd, ops.repack_scales(bsd, tile_rows=h), acc, _lib.ACCUMULATE)
+        check(acc, a, a_s, b, b_s, ref=ref + 1.0)
+    ops.check_device_status()
+
+
+def test_linear_layer_first_used_at_another_decode_batch():
+    """One layer at batch sizes that read different packings of its weight scales, in any order."""
+    N, K = 14336, 512
+    g = torch.Generator().manual_seed(3)
+    w = torch.randn(N, K, generator=g) * 0.02
+    wq, ws = orc.quantize_mxfp4(w)
+    layer = wb.MXFP4Linear.from_float(w.to(DEV), output_dtype=torch.bfloat16)
+    for rows in (128, 4, 128, 33, 200, 1):
+        x = torch.randn(rows, K, generator=g)
+        xq, xs = orc.quantize_mxfp4(x)
+        check_bf16(layer(x.to(DEV)), orc.scaled_gemm(xq, xs, wq, ws))
+    assert layer._packed.tile_rows == 128
+    ops.check_device_status()

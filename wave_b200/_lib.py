@@ -66,6 +66,7 @@ EXPORTED_SYMBOLS = (
     "wb200_debug_checks_selftest",
     "wb200_packed_scale_bytes",
     "wb200_decode_tile_rows",
+    "wb200_decode_tile_rows_for",
     "wb200_mixed_decode_tile_rows",
     "wb200_packed_scale_bytes_tiled",
     "wb200_repack_scales_tiled",
@@ -158,6 +159,8 @@ def load() -> ctypes.CDLL:
     lib.wb200_packed_scale_bytes.argtypes = [c_int, c_int]
     lib.wb200_decode_tile_rows.restype = c_int
     lib.wb200_decode_tile_rows.argtypes = [c_int]
+    lib.wb200_decode_tile_rows_for.restype = c_int
+    lib.wb200_decode_tile_rows_for.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int]
     lib.wb200_mixed_decode_tile_rows.restype = c_int
     lib.wb200_mixed_decode_tile_rows.argtypes = [c_int]
     lib.wb200_packed_scale_bytes_tiled.restype = c_size_t
@@ -291,7 +294,8 @@ def fast():
         except ImportError as e:
             raise RuntimeError(f"wave_b200._fast cannot be loaded ({e}): build it with `python -m wave_b200.build`") from e
         module.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.wb200_mxfp4_gemm_repack_a, lib.wb200_mxfp8_gemm_repack_a,
-                                                                      lib.wb200_mxfp4_gemm_quantize_a, lib.wb200_mxfp4_gemm_workspace_bytes)))
+                                                                      lib.wb200_mxfp4_gemm_quantize_a, lib.wb200_mxfp4_gemm_workspace_bytes,
+                                                                      lib.wb200_decode_tile_rows_for)))
         _fast = module
     return _fast
 

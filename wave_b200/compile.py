@@ -165,7 +165,7 @@ class ScaledGemmKernel:
         M, N, K, a_buf, ws_ptr, ws_bytes, flags, dtype_code, dev_index, _ws_keepalive = plan
         if M > 128 and ws_bytes and not ops.split_k_pays() and (flags & _lib.PATH_MASK) != _lib.PATH_TILE_SPLITK:
             ws_ptr = ws_bytes = 0  # eager call: stay on the plain tile path (see ops.split_k_pays)
-        tile_rows = self._weight_tile_rows(M, N, dev_index)
+        tile_rows = self._weight_tile_rows(M, N, K, c, dev_index)
         packings = self._weight_scales.packings
         b_sf = self._weight_scales.get(b_scale, tile_rows)
         if self._weight_scales.packings != packings:
@@ -225,7 +225,7 @@ class ScaledGemmKernel:
             b_sf = b_scale
         else:
             idx = a.device.index if a.device.index is not None else torch.cuda.current_device()
-            tile_rows = self._mixed_tile_rows(M, N, K, c, idx) if b_fp4 else self._weight_tile_rows(M, N, idx)
+            tile_rows = self._mixed_tile_rows(M, N, K, c, idx) if b_fp4 else self._weight_tile_rows(M, N, K, c, idx)
             b_sf = self._weight_scales.get(self._check_scale(b_scale, N, K, "b_scale"), tile_rows)
         fmt = _lib.E5M2 if t.element_format == "f8e5m2" else _lib.E4M3
         flags = self.options.kernel_path | self._raster_flags() | (_lib.ACCUMULATE if t.accumulate else 0)
@@ -305,7 +305,7 @@ class ScaledGemmKernel:
         else:
             idx = a.device.index if a.device.index is not None else torch.cuda.current_device()
             packings = self._weight_scales.packings
-            b_sf = self._weight_scales.get(self._check_scale(b_scale, N, K, "b_scale"), self._weight_tile_rows(M, N, idx))
+            b_sf = self._weight_scales.get(self._check_scale(b_scale, N, K, "b_scale"), self._weight_tile_rows(M, N, K, c, idx))
             if self._weight_scales.packings != packings:
                 flags &= ~_lib.OVERLAP_PREVIOUS  # as in _launch
         ops.scaled_gemm_packed(a, a_sf, b, b_sf, c, flags)  # adds the tile-height bits a tiled packing needs
@@ -317,16 +317,24 @@ class ScaledGemmKernel:
             raise ValueError(f"{name} must be [{rows}, {K // ops.SCALE_GROUP_SIZE}], got {tuple(s.shape)}")
         return s
 
-    def _weight_tile_rows(self, M: int, N: int, dev_index: int, mixed: bool = False) -> int:
-        """Rows per tile the weight scales are packed for: the decode kernel's balanced tile height for M <= 128 (every
-        SM gets the same number of weight tiles, `ops.decode_tile_rows`), 128 otherwise. Weights are packed once per
-        (weight, height) and cached, so a weight used at both ends of the M range keeps two packings."""
+    def _weight_tile_rows(self, M: int, N: int, K: int, c: torch.Tensor, dev_index: int, mixed: bool = False) -> int:
+        """Rows per tile the weight scales are packed for: 128, or for M <= 128 the height that is the decode kernel's fastest for
+        the call (`ops.decode_tile_rows_for`; with a forced path `ops.decode_tile_rows`, which that path reads). Weights are
+        packed once per (weight, height) and cached, so a weight used at both ends of the M range keeps two packings.
+        mixed: the height of the mixed pair's own kernel."""
         if M > 128 or not self.options.decode_tiled_weight_scales:
             return 128
-        key = (N, dev_index, mixed)
+        forced = self.options.kernel_path != _lib.PATH_AUTO
+        aligned = mixed or forced or ops.rows_aligned(c)
+        key = (M, N, K, aligned, dev_index, mixed, forced)
         h = self._tile_rows.get(key)
         if h is None:
-            h = self._tile_rows[key] = ops.decode_tile_rows(N, dev_index, mixed)
+            if mixed or forced:
+                h = ops.decode_tile_rows(N, dev_index, mixed)
+            else:
+                t = self.template
+                h = ops.decode_tile_rows_for(M, N, K, dev_index, t.weight_bits, t.element_bits, aligned)
+            self._tile_rows[key] = h
         return h
 
     def _mixed_tile_rows(self, M: int, N: int, K: int, c: torch.Tensor, dev_index: int) -> int:
@@ -340,10 +348,12 @@ class ScaledGemmKernel:
         Up to 16 rows the usual packing takes the K-split kernel, which is ahead of low tiles over a long K (N = 19200, M = 16:
         K = 6144 18.8 / 19.0, K = 16384 42.2 / 38.1; N = 22208, K = 16384 45.8 / 45.3) and in unaligned stores (N = 22201,
         K = 4096: M = 8 15.7 / 16.2, M = 16 18.9 / 16.6)."""
-        usual = self._weight_tile_rows(M, N, dev_index)
+        usual = self._weight_tile_rows(M, N, K, c, dev_index)
         if M > 128 or self.options.kernel_path in (_lib.PATH_TILE_1CTA, _lib.PATH_TILE_2CTA):
             return usual  # no tile kernel reads a height above 128
-        wide = self._weight_tile_rows(M, N, dev_index, mixed=True)
+        wide = self._weight_tile_rows(M, N, K, c, dev_index, mixed=True)
+        if wide <= 128:
+            return usual
         k_split = M <= 16 and usual == 128
         if k_split and K > 6144 and wide < 152:
             return usual

@@ -837,15 +837,51 @@ int launch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, con
   return launch_skinny_scales<NP, STAGES, OutT, EB, false>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
 }
 
+// The tile height (a multiple of 8, at most 128) for which `rounds` tiles on every SM cover N, with the fewest rounds.
+int balanced_tile_rows(int sm_count, int N) {
+  const long long slots = ((N + 127) / 128 + sm_count - 1) / sm_count * (long long)sm_count;
+  return std::min(128, int(((N + slots - 1) / slots + 7) / 8 * 8));
+}
+
+enum class DecodePair { kFp4, kFp8, kMixed };  // operand types: MXFP4, 8-bit, 8-bit activations with 4-bit weights
+// Fewer 128-row weight tiles than SMs: whether the whole-tile kernel on tiles of h rows, one per SM, is ahead of what the usual packing
+// would take (K split, tile kernel or cluster per tile). No tile is cut along K, so nothing meets in memory and the kernel ends
+// a microsecond after its stream; what it costs is one SM's chain of MMAs, ~0.26 us per stage however few rows a
+// tile has, so a long K needs high tiles. us, usual packing / h rows, bf16, weights in memory:
+//   MXFP4, M = 1:    4096 x 1024 5.8 / 4.8, 4096 x 4096 11.2 / 8.9, 14336 x 4096 13.2 / 9.8, 2048 x 8192 13.6 / 13.0, 4096 x 8192 12.3 / 13.0,
+//                    8192 x 8192 14.2 / 13.1, 14336 x 8192 17.2 / 14.4, 8192 x 14336 17.9 / 19.3, 11008 x 14336 20.7 / 19.6
+//   M = 32:          4096 x 4096 9.8 / 9.0, 14336 x 4096 13.9 / 10.3, 5808 x 8192 13.4 / 13.3, 14336 x 8192 16.9 / 14.8, 5808 x 10240 14.9 / 15.3
+//   M = 64:          2048 x 1024 5.9 / 6.0, 8192 x 1024 6.6 / 6.2, 8192 x 4096 10.4 / 10.7, 14336 x 4096 11.9 / 11.7, 11008 x 10240 18.1 / 18.1,
+//                    14336 x 14336 25.9 / 23.2
+//   M = 128:         14336 x 4096 11.9 / 12.7, 17408 x 10240 22.4 / 21.4, 8192 x 14336 19.4 / 24.5
+//   rows of C not 16-byte aligned (the tile kernels store them element by element, one row per lane): M = 128: 4001 x 1024 22.7 / 8.2,
+//                    14335 x 4096 26.5 / 18.4; M = 64: 4001 x 8192 20.9 / 14.9, 4001 x 14336 18.5 / 21.5, 5803 x 14336 25.0 / 22.4
+//   8-bit (mixed), M = 16: 4096 x 1024 7.6 / 6.4 (6.8 / 6.5), 14336 x 4096 17.9 / 14.8 (16.4 / 13.5), 4096 x 8192 16.5 / 20.0 (15.3 / 19.8),
+//                    14336 x 8192 26.8 / 24.7 (22.2 / 21.1), 14336 x 14336 40.2 / 36.5 (30.3 / 32.3)
+//   8-bit (mixed), M = 64: 8192 x 1024 8.1 / 7.7 (7.5 / 7.3), 8192 x 4096 13.9 / 14.8 (13.2 / 14.1), 14336 x 4096 16.5 / 16.2 (15.3 / 14.7)
+//   8-bit, M = 128: 14336 x 8192 29.5 / 27.8 (24.4 / 26.0 mixed); unaligned 11001 x 4096 33.0 / 21.5 (31.4 / 19.9)
+bool one_round_pays(int M, int K, int h, DecodePair pair, bool c_aligned) {
+  const bool fp4 = pair == DecodePair::kFp4;
+  const int kb = fp4 ? (K + 255) / 256 : (K + 127) / 128;  // stages per tile
+  if (!c_aligned && M > (fp4 ? 16 : 32)) return h >= kb - (fp4 ? 20 : 32);
+  if (M <= 32) {
+    if (fp4) return h >= std::min(2 * (kb - 8), 72);
+    return h >= (pair == DecodePair::kFp8 ? std::min(2 * (kb - 16), 104) : 2 * (kb - 16));
+  }
+  if (M <= 64) return h >= (fp4 ? (kb <= 8 ? 40 : kb <= 32 ? 104 : 80) : kb <= 16 ? 56 : 104);
+  return (fp4 && kb >= 40 && h >= 112) || (pair == DecodePair::kFp8 && kb >= 64 && h >= 104);
+}
+
 // Whole N tiles taken from an atomic counter instead of a K split (skinny_whole_sm100.cuh), when there is at least one
 // tile per SM. For M > 16 always: the K-split kernel's partial tiles (M x 128 f32 each) cost more than any imbalance
 // (M = 128: 24.6 us against 29.4 us even at 150 tiles, where only two tiles are left for the second round). For M <= 16
 // only when the tiles left over after the full rounds are none, or at least half a round, or a small part of the whole:
 // a few stragglers alone run at one SM's bandwidth (150 tiles: 21.9 us whole against 19.2 us K-split; 185 tiles: 22.5
 // against 19.9; 224 tiles: 23.3 against 24.9; 148 tiles: 15.7 against 16.4).
-bool skinny_takes_whole_tiles(int sm_count, int M, int N, int elem_bits = 4) {
+bool skinny_takes_whole_tiles(int sm_count, int M, int N, int K, int elem_bits, bool mixed, bool c_aligned) {
   const int tiles = (N + 127) / 128, rest = tiles % sm_count;
-  if (tiles < sm_count) return false;
+  if (tiles < sm_count)
+    return balanced_tile_rows(sm_count, N) == 128 && one_round_pays(M, K, 128, elem_bits == 4 ? DecodePair::kFp4 : mixed ? DecodePair::kMixed : DecodePair::kFp8, c_aligned);
   if (M > 16) return true;
   // 8-bit operands stream twice the bytes per tile, so a partly empty last round costs twice as much: measured at
   // N = 28672, K = 8192, M = 16: 50.8 us with whole 128-row tiles against 42.5 us with the K split
@@ -859,12 +895,22 @@ bool skinny_takes_whole_tiles(int sm_count, int M, int N, int elem_bits = 4) {
 int decode_tile_rows(int sm_count, int N) {
   const int tiles = (N + 127) / 128;
   if (tiles < sm_count || tiles % sm_count == 0) return 128;
-  const long long slots = (long long)((tiles + sm_count - 1) / sm_count) * sm_count;
-  const int h = int(((N + slots - 1) / slots + 7) / 8 * 8);
+  const int h = balanced_tile_rows(sm_count, N);
   // Low tiles pay when the last round of 128-row tiles is thin, but there the K-split kernel (usual packing) is the
   // better answer for M <= 16, and one packing serves every M: N = 19072 / 20480 (h = 72) 19.0 / 19.4 us against
   // 16.4 / 16.9 us at M = 16, while M = 128 gains under 1 us; from h = 88 up (N = 24576) no M loses.
   return (h >= 88 && h < 128) ? h : 128;
+}
+// The height for a call whose M and K are known too, which may be one that decode_tile_rows does not give: one round of low tiles
+// (above), or several where K is short: there even thin tiles beat both the K split and a thin last round (us, 128 / h rows, N = 20480:
+// K = 1024 M = 16 8.8 / 6.1, M = 64 8.1 / 8.1; K = 4096 M = 16 14.7 / 13.9, M = 64 16.4 / 16.2, M = 128 17.5 / 18.1; K = 6144 M = 1 17.2 / 17.8;
+// 8-bit K = 1024 11.6 / 9.5, K = 2048 14.4 / 14.1, K = 4096 20.2 / 21.7; unaligned rows of C, N = 20483, M = 128: K = 1024 19.8 / 15.8).
+int decode_tile_rows_for(int sm_count, int M, int N, int K, DecodePair pair, bool c_aligned) {
+  const int tiles = (N + 127) / 128, usual = decode_tile_rows(sm_count, N);
+  if (usual != 128 || tiles % sm_count == 0) return usual;
+  const int h = balanced_tile_rows(sm_count, N);
+  if (tiles < sm_count) return one_round_pays(M, K, h, pair, c_aligned) ? h : 128;
+  return h >= 72 && K <= (pair == DecodePair::kFp4 ? 4096 : 1024) && (M <= 64 || !c_aligned) ? h : 128;
 }
 
 template <int NP, int STAGES, typename OutT, int EB, int WR, int SBUFS, typename Maps>
@@ -915,7 +961,7 @@ int launch_skinny_whole_maps(const DeviceInfo& dev, int M, int N, int K, const v
   rc = set_smem(kernel, Cfg::SMEM_BYTES, smem_set);
   if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(dev.sm_count, 1, 1);  // one CTA per SM; every CTA's first tile is its own index (tiles >= SMs)
+  cfg.gridDim = dim3(std::min(dev.sm_count, tiles_n), 1, 1);  // one CTA per SM; every CTA's first tile is its own index
   cfg.blockDim = dim3(Maps::kRowScales ? 224 : 192, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
@@ -1083,9 +1129,10 @@ int dispatch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, c
                     int elem_format = 0) {
   if (tl_b_tile_rows != 128) {
     // the weight scales are packed per tile of that height: only the whole-tile kernel reads them that way
-    if ((N + tl_b_tile_rows - 1) / tl_b_tile_rows < dev.sm_count)
-      return fail(WB200_ERR_UNSUPPORTED, "weight scales packed for %d-row tiles need at least one tile per SM (N = %d, %d SMs); "
-                  "pack them with wb200_repack_scales instead", tl_b_tile_rows, N, dev.sm_count);
+    if ((N + tl_b_tile_rows - 1) / tl_b_tile_rows < dev.sm_count && tl_b_tile_rows != balanced_tile_rows(dev.sm_count, N))
+      return fail(WB200_ERR_UNSUPPORTED, "weight scales packed for %d-row tiles need at least one tile per SM, or the height that gives every SM "
+                  "one (N = %d, %d SMs: %d); pack them with wb200_repack_scales instead", tl_b_tile_rows, N, dev.sm_count,
+                  balanced_tile_rows(dev.sm_count, N));
   }
   if (tl_b_tile_rows <= 104) {
     // tiles of at most 104 rows: stages with room for 104 weight rows, so that the ring holds more of them
@@ -1094,7 +1141,8 @@ int dispatch_skinny(const DeviceInfo& dev, int M, int N, int K, const void* a, c
     if (M <= 64) return launch_skinny_whole<64, 9, OutT, EB, 104>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
     return launch_skinny_whole<128, 7, OutT, EB, 104, 1>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
   }
-  if (tl_b_tile_rows != 128 || skinny_takes_whole_tiles(dev.sm_count, M, N, EB)) {
+  if (tl_b_tile_rows != 128 || skinny_takes_whole_tiles(dev.sm_count, M, N, K, EB, weights_are_fp4(EB, elem_format),
+                                                        rows_aligned(c, ldc, sizeof(OutT) == 4 ? WB200_F32 : WB200_BF16))) {
     if (M <= 16) return launch_skinny_whole<16, 10, OutT, EB>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
     if (M <= 32) return launch_skinny_whole<32, 9, OutT, EB>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
     if (M <= 64) return launch_skinny_whole<64, 8, OutT, EB>(dev, M, N, K, a, as, b, bs, c, ldc, ws, accumulate, stream, elem_format);
@@ -1128,7 +1176,7 @@ enum class DecodeRoute { kSkinny, kTile1, kTile2, kCluster };
 constexpr long long kRouteActivationBytes = 128 << 10;
 DecodeRoute decode_route(int sm_count, int M, int N, int K, bool c_aligned) {
   const int tiles = (N + 127) / 128, kb = (K + 255) / 256;
-  if (tiles >= sm_count) return DecodeRoute::kSkinny;
+  if (tiles >= sm_count || skinny_takes_whole_tiles(sm_count, M, N, K, 4, false, c_aligned)) return DecodeRoute::kSkinny;
   const long long units = (long long)tiles * kb, sms = sm_count;
   const bool few_activations = (long long)M * K / 2 < kRouteActivationBytes;
   const int slices = cluster_splitk_slices(M, N, K);
@@ -1153,7 +1201,7 @@ DecodeRoute decode_route(int sm_count, int M, int N, int K, bool c_aligned) {
 // Unaligned rows of C: 5803 x 5376, M = 17: 16.3 / 18.2, M = 128: 33.7 / 31.7; 11001 x 4096, M = 32: 17.9 / 18.6, M = 128: 30.9 / 34.0.
 DecodeRoute decode_route_8bit(int sm_count, int M, int N, int K, bool mixed, bool c_aligned) {
   const int tiles = (N + 127) / 128, kb = (K + 127) / 128;
-  if (tiles >= sm_count) return DecodeRoute::kSkinny;
+  if (tiles >= sm_count || skinny_takes_whole_tiles(sm_count, M, N, K, 8, mixed, c_aligned)) return DecodeRoute::kSkinny;
   const long long units = (long long)tiles * kb, sms = sm_count;
   const bool few_activations = (long long)M * K < kRouteActivationBytes;
   bool k_split;
@@ -1256,6 +1304,12 @@ int wb200_decode_tile_rows(int N) {
   return decode_tile_rows(dev->sm_count, N);
 }
 
+int wb200_decode_tile_rows_for(int M, int N, int K, int weight_bits, int activation_bits, int c_rows_aligned) {
+  DeviceInfo* dev;
+  if (M <= 0 || M > 128 || N <= 0 || K <= 0 || get_device(&dev)) return 128;
+  const DecodePair pair = activation_bits == 4 ? DecodePair::kFp4 : weight_bits == 4 ? DecodePair::kMixed : DecodePair::kFp8;
+  return decode_tile_rows_for(dev->sm_count, M, N, K, pair, c_rows_aligned != 0);
+}
 int wb200_mixed_decode_tile_rows(int N) {
   DeviceInfo* dev;
   if (N <= 0 || get_device(&dev)) return 128;

@@ -40,6 +40,7 @@ struct Abi {
   int (*gemm_quantize_a)(int, int, int, const void*, int, long long, void*, void*, const void*, const void*, void*, int, long long, void*, size_t,
                          unsigned, void*);
   size_t (*gemm_workspace_bytes)(int, int, int);
+  int (*decode_tile_rows_for)(int, int, int, int, int, int);
 } abi;
 
 // An ordinary CUDA tensor: no subclass, no wrapper of a functional transform, no inference tensor.
@@ -295,18 +296,19 @@ void object_free(PyObject* self) {
   Py_TYPE(self)->tp_free(self);
 }
 
-// linear(x, weight_codes, packed_scales, tile_rows, output dtype, workspaces) -> dequant(quantise(x)) @ dequant(W)^T, or None: left to
-// the Python code. packed_scales: of weight_codes, per tile_rows rows; the caller has chosen them for this number of rows.
+// linear(x, weight_codes, packed scales, those per tile of low_rows rows or None, low_rows, output dtype, workspaces)
+// -> dequant(quantise(x)) @ dequant(W)^T, or None: left to the Python code.
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 6) {
-    PyErr_SetString(PyExc_TypeError, "linear takes 6 arguments");
+  if (n != 7) {
+    PyErr_SetString(PyExc_TypeError, "linear takes 7 arguments");
     return nullptr;
   }
   try {
-    if (!plain(args[0]) || !plain(args[1]) || !plain(args[2]) || !THPDtype_Check(args[4])) Py_RETURN_NONE;
-    const at::Tensor &x = THPVariable_Unpack(args[0]), &w = THPVariable_Unpack(args[1]), &packed = THPVariable_Unpack(args[2]);
+    if (!plain(args[0]) || !plain(args[1]) || !plain(args[2]) || !THPDtype_Check(args[5])) Py_RETURN_NONE;
+    const at::Tensor &x = THPVariable_Unpack(args[0]), &w = THPVariable_Unpack(args[1]);
+    at::Tensor packed = THPVariable_Unpack(args[2]);
     const int device = x.device().index();
-    const at::ScalarType x_type = x.scalar_type(), out_type = reinterpret_cast<THPDtype*>(args[4])->scalar_type;
+    const at::ScalarType x_type = x.scalar_type(), out_type = reinterpret_cast<THPDtype*>(args[5])->scalar_type;
     const int64_t dims = x.dim();
     if (device != c10::cuda::current_device() || w.device().index() != device || packed.device().index() != device || dims < 1 || w.dim() != 2 ||
         !w.is_contiguous() || (x_type != at::kFloat && x_type != at::kBFloat16) || (out_type != at::kFloat && out_type != at::kBFloat16))
@@ -322,12 +324,21 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     size_t ws_bytes = 0;
     if (M <= 128) {
       ws_bytes = abi.gemm_workspace_bytes(int(M), int(N), int(K));
-      for (const auto& e : reinterpret_cast<PyWorkspaces*>(args[5])->table->entries)
+      for (const auto& e : reinterpret_cast<PyWorkspaces*>(args[6])->table->entries)
         if (e.device == device && e.stream == stream.stream()) ws = e.ws;
       if (!ws.defined() || size_t(ws.numel()) < ws_bytes) Py_RETURN_NONE;
     }
-    const long tile_rows = PyLong_AsLong(args[3]);
-    if (PyErr_Occurred()) return nullptr;
+    // (a fresh output starts on 16 bytes: its rows are aligned when N says so)
+    const bool aligned = M == 1 || N * (out_type == at::kFloat ? 4 : 2) % 16 == 0;
+    int tile_rows = 128;
+    if (M <= 128 && (tile_rows = abi.decode_tile_rows_for(int(M), int(N), int(K), 4, 4, aligned)) != 128) {
+      if (args[3] == Py_None || PyLong_AsLong(args[4]) != tile_rows || !plain(args[3])) {
+        if (PyErr_Occurred()) return nullptr;
+        Py_RETURN_NONE;
+      }
+      packed = THPVariable_Unpack(args[3]);
+      if (packed.device().index() != device) Py_RETURN_NONE;
+    }
     std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
     shape.back() = N;
     const at::Tensor out = at::detail::empty_cuda(shape, out_type, x.device(), c10::nullopt);
@@ -348,14 +359,15 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
 }
 
-// bind(gemm_repack_a, mxfp8_gemm_repack_a, gemm_quantize_a, gemm_workspace_bytes): addresses in the loaded library
+// bind(gemm_repack_a, mxfp8_gemm_repack_a, gemm_quantize_a, gemm_workspace_bytes, decode_tile_rows_for): addresses in the loaded library
 PyObject* bind(PyObject*, PyObject* args) {
-  unsigned long long p[4];
-  if (!PyArg_ParseTuple(args, "KKKK", &p[0], &p[1], &p[2], &p[3])) return nullptr;
+  unsigned long long p[5];
+  if (!PyArg_ParseTuple(args, "KKKKK", &p[0], &p[1], &p[2], &p[3], &p[4])) return nullptr;
   abi.gemm_repack_a = reinterpret_cast<decltype(abi.gemm_repack_a)>(p[0]);
   abi.mxfp8_gemm_repack_a = reinterpret_cast<decltype(abi.mxfp8_gemm_repack_a)>(p[1]);
   abi.gemm_quantize_a = reinterpret_cast<decltype(abi.gemm_quantize_a)>(p[2]);
   abi.gemm_workspace_bytes = reinterpret_cast<decltype(abi.gemm_workspace_bytes)>(p[3]);
+  abi.decode_tile_rows_for = reinterpret_cast<decltype(abi.decode_tile_rows_for)>(p[4]);
   Py_RETURN_NONE;
 }
 

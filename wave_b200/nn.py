@@ -25,9 +25,14 @@ class MXFP4Linear(torch.nn.Module):
         self.register_buffer("weight_codes", weight_codes.contiguous())
         self.register_buffer("weight_scales", weight_scales.contiguous())
         self._packed = ops.repack_scales(self.weight_scales)  # once
-        # decode calls (at most 128 rows) read a second packing, per tile of the height that gives every SM the same number
-        # of weight tiles; made on first use, and only where that height differs from 128
-        self._packed_decode = None
+
+    # Decode calls (at most 128 rows) may read a second packing, per tile of the height that gives every SM the same number of
+    # weight tiles (one height per layer: it follows from out_features); made when `ops.decode_tile_rows_for` first names it.
+    _packed_low = None
+
+    @property
+    def _packed_decode(self) -> ops.PackedScales:
+        return self._packed if self._packed_low is None else self._packed_low
 
     @classmethod
     def from_float(cls, weight: torch.Tensor, output_dtype=torch.bfloat16) -> "MXFP4Linear":
@@ -36,15 +41,14 @@ class MXFP4Linear(torch.nn.Module):
         return cls(q, s, output_dtype)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        rows = x.numel() // self.in_features
-        packed = self._packed if rows > 128 else self._packed_decode
-        if packed is not None:
-            # a call whose tensors need no preparation; anything else comes back unhandled
-            y = _lib.fast().linear(x, self._buffers.get("weight_codes"), packed.data, packed.tile_rows, self.output_dtype, ops._pool.fast)
-            if type(y) is int:
-                _lib.check(y)
-            elif y is not None:
-                return y
+        # a call whose tensors need no preparation; anything else comes back unhandled
+        low = self._packed_low
+        y = _lib.fast().linear(x, self._buffers.get("weight_codes"), self._packed.data, None if low is None else low.data,
+                               128 if low is None else low.tile_rows, self.output_dtype, ops._pool.fast)
+        if type(y) is int:
+            _lib.check(y)
+        elif y is not None:
+            return y
         return self._forward_checked(x)
 
     def _forward_checked(self, x: torch.Tensor) -> torch.Tensor:
@@ -53,9 +57,16 @@ class MXFP4Linear(torch.nn.Module):
         out = torch.empty(x2.shape[0], self.out_features, dtype=self.output_dtype, device=x.device)
         packed = self._packed
         if x2.shape[0] <= 128:
-            if self._packed_decode is None:
-                h = ops.decode_tile_rows(self.out_features, x.device)
-                self._packed_decode = self._packed if h == 128 else ops.repack_scales(self.weight_scales, tile_rows=h)
-            packed = self._packed_decode
+            packed = self._decode_packing(out)
         ops.quantized_gemm(x2, self.weight_codes, packed, out)
         return out.reshape(*lead, self.out_features)
+
+    def _decode_packing(self, out: torch.Tensor) -> ops.PackedScales:
+        h = ops.decode_tile_rows_for(out.shape[0], self.out_features, self.in_features, out.device, c_aligned=ops.rows_aligned(out))
+        if h == 128:
+            return self._packed
+        if self._packed_low is None:
+            if torch.cuda.is_current_stream_capturing():
+                return self._packed  # (a packing made by a captured call holds nothing before the first replay)
+            self._packed_low = ops.repack_scales(self.weight_scales, tile_rows=h)
+        return self._packed_low

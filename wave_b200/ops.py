@@ -61,6 +61,21 @@ def decode_tile_rows(N: int, device=None, mixed: bool = False) -> int:
         return int(fn(int(N)))
 
 
+def decode_tile_rows_for(M: int, N: int, K: int, device=None, weight_bits: int = 4, activation_bits: int = 4, c_aligned: bool = True) -> int:
+    """Tile height for calls of one M <= 128 and K: `decode_tile_rows(N)`, or a lower height where that is the faster one (one low tile
+    per SM when N has fewer than 128 rows per SM). c_aligned: every row of the output starts on 16 bytes."""
+    args = (int(M), int(N), int(K), weight_bits, activation_bits, int(c_aligned))
+    if device is None:
+        return int(_lib.load().wb200_decode_tile_rows_for(*args))
+    with torch.cuda.device(device):
+        return int(_lib.load().wb200_decode_tile_rows_for(*args))
+
+
+def rows_aligned(c: torch.Tensor) -> bool:
+    """Every row of the matrix starts on 16 bytes."""
+    return c.data_ptr() % 16 == 0 and (c.dim() != 2 or c.shape[0] == 1 or c.stride(0) * c.element_size() % 16 == 0)
+
+
 def repack_scales(scale: torch.Tensor, out: torch.Tensor | None = None, tile_rows: int = 128) -> PackedScales:
     """Row-major [rows, K/32] E8M0 scales -> PackedScales, on the current stream. tile_rows < 128: the weight packing
     of the decode kernel (one atom row per tile of that many rows, see `decode_tile_rows`)."""
