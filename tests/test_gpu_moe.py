@@ -446,3 +446,23 @@ def test_routed_gemm_with_a_row_count_inside_a_block(num_rows, out_dtype):
             check(c[lo:hi], a[lo:hi], a_s[lo:hi], b, b_s)
         else:
             assert bool((c[lo:] == -1.0).all())
+
+
+@pytest.mark.parametrize("T,E,k", [(127, 32, 32), (128, 9, 3), (129, 8, 8), (257, 32, 5), (8192, 8, 1), (8193, 17, 2), (20001, 32, 4)])
+def test_expert_mlp_routes_blocks_of_tokens(T, E, k):
+    """The routing of the single call at its edges: one launch and two, the last block of tokens partly filled, blocks of more than 128
+    tokens, every expert chosen, experts without tokens. Against the same steps one by one, whose rows are sorted by
+    moe_align_block_size; the outputs differ by the summation order of the last GEMM at most (one bf16 ulp of a term)."""
+    K = inter = 128
+    _, _, mlp = _small_expert_mlp(T + E, E=E, K=K, inter=inter, N=32, k=k)
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16).to(DEV)
+    logits = torch.randn(T, E, generator=g)
+    if E > k + 2:
+        logits[:, 1] = -50.0  # an expert without tokens
+    logits = logits.to(DEV)
+    assert mlp._takes_fused(x, logits)
+    y, ref = mlp(x, logits), mlp._forward_steps(x, logits)
+    assert y.shape == ref.shape and bool(torch.isfinite(y.float()).all())
+    assert float((y.float() - ref.float()).abs().max()) <= 2 ** -7 * float(ref.float().abs().max())
+    ops.check_device_status()

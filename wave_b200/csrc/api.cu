@@ -1478,11 +1478,11 @@ int wb200_moe_align_block_size(const void* topk_ids, int ids_are_int64, int num_
   if (ids_are_int64)
     wb::moe_align_block_size_kernel<long long><<<1, 1024, 0, s>>>(static_cast<const long long*>(topk_ids), num_ids, num_experts,
                                                                   block_size, sorted_capacity, sorted_ids, expert_ids,
-                                                                  num_tokens_post_pad, inverse, 0, nullptr);
+                                                                  num_tokens_post_pad, inverse);
   else
     wb::moe_align_block_size_kernel<int><<<1, 1024, 0, s>>>(static_cast<const int*>(topk_ids), num_ids, num_experts, block_size,
                                                             sorted_capacity, sorted_ids, expert_ids, num_tokens_post_pad,
-                                                            inverse, 0, nullptr);
+                                                            inverse);
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
 }
@@ -1639,11 +1639,11 @@ int wb200_moe_quantize_scatter(const void* x, int x_dtype, long long ldx, int to
   if (x_dtype == WB200_F32)
     wb::quantize_scatter_mxfp4_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), ldx, tokens, K, top_k, dst_rows,
                                                                     static_cast<uint8_t*>(q), q_vec,
-                                                                    static_cast<uint8_t*>(scale_rowmajor), nullptr, k_atoms, 0);
+                                                                    static_cast<uint8_t*>(scale_rowmajor), k_atoms);
   else
     wb::quantize_scatter_mxfp4_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), ldx, tokens, K,
                                                                             top_k, dst_rows, static_cast<uint8_t*>(q), q_vec,
-                                                                            static_cast<uint8_t*>(scale_rowmajor), nullptr, k_atoms, 0);
+                                                                            static_cast<uint8_t*>(scale_rowmajor), k_atoms);
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
 }
@@ -2007,7 +2007,7 @@ int wb200_mxfp4_moe_gemm(int num_experts, int max_rows, const int* expert_ids, c
 struct ExpertMlpPlan {
   bool decode;
   int block, cap;  // rows per routing block, rows of the routed matrices (the worst case of the routing)
-  size_t counters, weight, ids, inverse, expert_ids, num_rows, a, a_sf, q, q_sf, y, total;
+  size_t counters, weight, slots, route_counts, inverse, expert_ids, num_rows, a, a_sf, q, q_sf, y, total;
 };
 static ExpertMlpPlan plan_expert_mlp(int T, int E, int K, int inter, int N, int top_k) {
   ExpertMlpPlan p;
@@ -2022,7 +2022,8 @@ static ExpertMlpPlan plan_expert_mlp(int T, int E, int K, int inter, int N, int 
   auto take = [&](size_t bytes) { const size_t here = at; at += (bytes + 255) / 256 * 256; return here; };
   p.counters = take((wb::kWholeWorkCounter + 1) * 4);
   p.weight = take(n * 4);
-  p.ids = take(n * 4);
+  p.slots = take(n * 4);
+  p.route_counts = take(wb::kRouteMaxBlocks * wb::kRouteMaxExperts * 4);
   p.inverse = take(n * 4);
   p.expert_ids = take(blocks * 4);
   p.num_rows = take(4);
@@ -2034,6 +2035,31 @@ static ExpertMlpPlan plan_expert_mlp(int T, int E, int K, int inter, int N, int 
   p.total = at;
   return p;
 }
+
+static_assert(wb::kMaxGroups <= wb::kRouteMaxExperts, "the router holds every expert of a routed launch");
+extern "C++" {
+template <typename InT, typename T, int EM>
+static int launch_route_kernels(const void* x, long long ldx, int K, uint8_t* q, uint8_t* q_sf, const wb::RouteParams& route, cudaStream_t s) {
+  const int k_atoms = wb::sf_k_atoms(K);
+  const unsigned blocks = unsigned(((long long)route.tokens * ((k_atoms + 7) / 8) + 7) / 8);
+  const InT* in = static_cast<const InT*>(x);
+  if (route.tokens <= wb::kRouteTokens) {
+    WB_CUDA(launch_kernel(false, wb::moe_quantize_kernel<InT, T, EM, true>, blocks, 256, s, in, ldx, K, q, q_sf, k_atoms, route));
+    return WB200_OK;
+  }
+  const unsigned route_blocks = unsigned((route.tokens + route.tokens_per_block - 1) / route.tokens_per_block);
+  WB_CUDA(launch_kernel(false, wb::moe_route_kernel<T, EM>, route_blocks, wb::kRouteTokens, s, route));
+  WB_CUDA(launch_kernel(true, wb::moe_quantize_kernel<InT, T, EM, false>, blocks, 256, s, in, ldx, K, q, q_sf, k_atoms, route));
+  return WB200_OK;
+}
+template <typename InT>
+static int launch_route(const void* x, long long ldx, int K, uint8_t* q, uint8_t* q_sf, const wb::RouteParams& route, int logits_dtype, cudaStream_t s) {
+  if (logits_dtype == WB200_F32)
+    return route.E <= 8 ? launch_route_kernels<InT, float, 8>(x, ldx, K, q, q_sf, route, s) : launch_route_kernels<InT, float, 32>(x, ldx, K, q, q_sf, route, s);
+  return route.E <= 8 ? launch_route_kernels<InT, __nv_bfloat16, 8>(x, ldx, K, q, q_sf, route, s)
+                      : launch_route_kernels<InT, __nv_bfloat16, 32>(x, ldx, K, q, q_sf, route, s);
+}
+}  // extern "C++"
 
 static int check_expert_mlp(int T, int E, int K, int inter, int N, int top_k) {
   if (T <= 0 || E <= 0 || E > wb::kMaxGroups || top_k <= 0 || top_k > E)
@@ -2070,31 +2096,31 @@ int wb200_mxfp4_expert_mlp(int T, int E, int K, int inter, int N, int top_k, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   float* weight = reinterpret_cast<float*>(ws + plan.weight);
-  int *ids = reinterpret_cast<int*>(ws + plan.ids), *inverse = reinterpret_cast<int*>(ws + plan.inverse);
+  int* inverse = reinterpret_cast<int*>(ws + plan.inverse);
   int *expert_ids = reinterpret_cast<int*>(ws + plan.expert_ids), *num_rows = reinterpret_cast<int*>(ws + plan.num_rows);
   unsigned int* counters = reinterpret_cast<unsigned int*>(ws + plan.counters);
-  const int n = T * top_k;
   // Every launch after the first is the programmatic dependent of the one before it. The first one is an ordinary launch,
   // so what the kernels before this call wrote (x, the logits) is complete for all of them.
-  const unsigned topk_blocks = unsigned((T + 127) / 128);
-  if (logits_dtype == WB200_F32)
-    WB_CUDA(launch_kernel(false, wb::moe_topk_kernel<float>, topk_blocks, 128, s, static_cast<const float*>(logits), ld_logits, T, E, top_k, weight, ids));
-  else
-    WB_CUDA(launch_kernel(false, wb::moe_topk_kernel<__nv_bfloat16>, topk_blocks, 128, s, static_cast<const __nv_bfloat16*>(logits), ld_logits, T, E,
-                          top_k, weight, ids));
-  WB_CUDA(launch_kernel(true, wb::moe_align_block_size_kernel<int>, 1, 1024, s, ids, n, E, plan.block, 0, static_cast<int*>(nullptr), expert_ids,
-                        num_rows, inverse, 1, counters + wb::kWholeWorkCounter));
-  const int k_atoms = wb::sf_k_atoms(K);
-  const unsigned q_blocks = unsigned(((long long)T * ((k_atoms + 7) / 8) + 7) / 8);
+  wb::RouteParams route;
+  route.logits = logits;
+  route.ld = ld_logits;
+  route.tokens = T; route.E = E; route.top_k = top_k;
+  route.block_rows = plan.block;
+  const int chunks = (T + wb::kRouteTokens - 1) / wb::kRouteTokens;  // of tokens
+  route.tokens_per_block = (chunks + wb::kRouteMaxBlocks - 1) / wb::kRouteMaxBlocks * wb::kRouteTokens;
+  route.weight = weight;
+  route.slots = reinterpret_cast<int*>(ws + plan.slots);
+  route.counts = reinterpret_cast<int*>(ws + plan.route_counts);
+  route.inverse = inverse;
+  route.expert_ids = expert_ids;
+  route.num_rows = num_rows;
+  route.zero_word = counters + wb::kWholeWorkCounter;
   // Tokens are quantised once and written straight to their sorted rows, scales in the packed layout. Rows that pad an
   // expert to whole blocks are never written: an output row depends on its own input row only, and the combination
   // reads routed rows only.
-  if (x_dtype == WB200_F32)
-    WB_CUDA(launch_kernel(true, wb::quantize_scatter_mxfp4_kernel<float>, q_blocks, 256, s, static_cast<const float*>(x), ldx, T, K, top_k, inverse,
-                          ws + plan.a, 1, static_cast<uint8_t*>(nullptr), ws + plan.a_sf, k_atoms, 1));
-  else
-    WB_CUDA(launch_kernel(true, wb::quantize_scatter_mxfp4_kernel<__nv_bfloat16>, q_blocks, 256, s, static_cast<const __nv_bfloat16*>(x), ldx, T, K,
-                          top_k, inverse, ws + plan.a, 1, static_cast<uint8_t*>(nullptr), ws + plan.a_sf, k_atoms, 1));
+  if (x_dtype == WB200_F32) rc = launch_route<float>(x, ldx, K, ws + plan.a, ws + plan.a_sf, route, logits_dtype, s);
+  else rc = launch_route<__nv_bfloat16>(x, ldx, K, ws + plan.a, ws + plan.a_sf, route, logits_dtype, s);
+  if (rc) return rc;
   struct DependentScope {  // restores the previous value on every return path
     bool saved = tl_dependent_launch;
     DependentScope() { tl_dependent_launch = true; }

@@ -332,13 +332,12 @@ quantize_mxfp8_kernel(const InT* __restrict__ x, long long ldx, int rows, int K,
 
 // Quantise-and-scatter for routed tokens: row t of x is quantised once and written to the `copies` output rows
 // dst_rows[t * copies + j] (negative entries are skipped): the tokens of a mixture-of-experts layer go straight
-// to their expert-sorted rows without a separate gather pass. Scales are written row-major and / or packed.
+// to their expert-sorted rows without a separate gather pass. Scales are written row-major.
 template <typename InT>
 __global__ void __launch_bounds__(256)
 quantize_scatter_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int K, int copies,
                               const int* __restrict__ dst_rows, uint8_t* __restrict__ q, int q_vec, uint8_t* __restrict__ scale_rm,
-                              uint8_t* __restrict__ scale_packed, int k_atoms, int dependent) {
-  if (dependent) pdl_launch_dependents();  // (in a chain of the library's own; see quantize_mxfp4_kernel)
+                              int k_atoms) {
   const int lane = threadIdx.x & 31;
   const int kblocks = K >> 5;
   const unsigned chunks = unsigned(k_atoms + 7) >> 3;
@@ -349,7 +348,6 @@ quantize_scatter_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows
   uint4 codes;
   uint32_t scales;
   mxfp4_quantize_warp(x + (long long)r * ldx, kb0, kblocks, lane, codes, scales);
-  if (dependent) pdl_wait();  // the destination rows are the previous kernel's; the outputs may still be read before it
   const int g = lane >> 2, sub = lane & 3;
   for (int j = 0; j < copies; ++j) {
     const int dst = __ldcg(dst_rows + r * copies + j);
@@ -363,8 +361,7 @@ quantize_scatter_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows
         d4[0] = codes.x; d4[1] = codes.y; d4[2] = codes.z; d4[3] = codes.w;
       }
     }
-    if (sub == 0 && scale_packed && (kb0 >> 2) + g < k_atoms) *packed_scale_word(scale_packed, k_atoms, dst, (kb0 >> 2) + g) = scales;
-    if (sub == 1 && scale_rm) {
+    if (sub == 1) {
       uint8_t* d = scale_rm + (long long)dst * kblocks + kb0 + g * 4;
 #pragma unroll
       for (int u = 0; u < 4; ++u)
