@@ -259,9 +259,9 @@ moe_quantize_kernel(const InT* __restrict__ x, long long ldx, int K, uint8_t* __
   const int r = int(wid / chunks);
   const bool real = r < p.tokens;
   const int kb0 = int(wid - unsigned(r) * chunks) * 32;
-  uint4 codes;
-  uint32_t scales;
-  mxfp4_quantize_warp(real ? x + (long long)r * ldx : static_cast<const InT*>(nullptr), kb0, kblocks, lane, codes, scales);
+  using Quant = WarpQuant<InT>;
+  Quant w;
+  w.run(real ? x + (long long)r * ldx : static_cast<const InT*>(nullptr), rows_on_32(x, ldx), kb0, kblocks, lane);
   int slot = 0;  // of this row's pair `lane`
   if constexpr (HERE) {
     if (warp < kRouteTokens / 32) {
@@ -319,12 +319,17 @@ moe_quantize_kernel(const InT* __restrict__ x, long long ldx, int K, uint8_t* __
   }
   __syncthreads();
   if (!real) return;
-  const int g = lane >> 2, sub = lane & 3;
   for (int j = 0; j < p.top_k; ++j) {
     const int s = __shfl_sync(0xffffffffu, slot, j);
     const int dst = first[s & 255] + (s >> 8);
-    if (kb0 + lane < kblocks) *reinterpret_cast<uint4*>(q + (long long)dst * (K / 2) + (kb0 + lane) * 16) = codes;
-    if (sub == 0 && (kb0 >> 2) + g < k_atoms) *packed_scale_word(scale_packed, k_atoms, dst, (kb0 >> 2) + g) = scales;
+    w.store_codes(q + (long long)dst * (K / 2), true, kb0, kblocks, lane);
+    if (Quant::writes(lane)) {
+#pragma unroll
+      for (int i = 0; i < Quant::kWords; ++i) {
+        const int atom = (kb0 >> 2) + Quant::atom(i, lane);
+        if (atom < k_atoms) *packed_scale_word(scale_packed, k_atoms, dst, atom) = w.word[i];
+      }
+    }
     if (kb0 == 0 && lane == 0) p.inverse[(long long)r * p.top_k + j] = dst;
   }
 }

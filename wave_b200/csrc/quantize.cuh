@@ -13,16 +13,13 @@
 //   that row are NaN instead of plausible finite numbers.
 //
 // HBM-bound. What bounded the first form (one block per 4 lanes and thread, 8 values each) was instruction issue: index
-// arithmetic, two f32 maxima per pair and one scattered byte per scale. Here a warp takes 32 consecutive blocks (one
-// block group of 4 lanes = 4 consecutive K blocks = one scale word), so that
-//   * every lane has four (bf16) or eight (f32) 16-byte loads in flight before any arithmetic;
+// arithmetic, two f32 maxima per pair and one scattered byte per scale. Here a warp takes 32 consecutive blocks, so that
+//   * all of a lane's loads are in flight before any arithmetic, and a load covers whole lines;
 //   * the block maximum of bf16 input is taken on packed pairs, two values per instruction;
-//   * the four scale bytes of a group leave as one 32-bit word, row-major and in the packed layout alike (a word of an
-//     atom is the four K blocks of one row), and padding bytes are written by the same pass;
-//   * the codes of a block are gathered in one lane (4 x 4 transpose in the group): one 16-byte store per lane.
-// 28672 x 8192 bf16, codes and both scale layouts (602 MB): 160 us (3.8 TB/s) -> 123 us, and 119 us (5.1 TB/s) with the
-// words of a packed-scale sector written together; 3000 x 8192 with packed scales only: 23 us (with the padding kernel that
-// the pass absorbs) -> 14.8 us.
+//   * four scale bytes leave as one 32-bit word, row-major and in the packed layout alike (a word of an atom is four K blocks of one
+//     row), and padding bytes are written by the same pass.
+// 28672 x 8192 bf16, codes and both scale layouts (602 MB): 94.5 us (6.4 TB/s, the rate of a copy); 16384 x 8192 f32 (612 MB): 87 us;
+// 3000 x 8192 bf16 with packed scales only: 12.5 us.
 #pragma once
 #include "ptx.cuh"
 #include "scales.cuh"
@@ -128,40 +125,25 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
   v[6] = __uint_as_float(t.w << 16); v[7] = __uint_as_float(t.w & 0xffff0000u);
 }
 
-// Largest |v| of 8 values as bits of the input type's magnitude (f32: 31 bits, bf16: 15 bits in the low half). Unsigned
-// order of magnitudes is numeric order, infinity above every finite value and NaN above infinity.
-struct Raw8f { uint4 lo, hi; };  // 8 f32
-__device__ __forceinline__ void load_raw8(const float* p, Raw8f& v) {
-  v.lo = __ldg(reinterpret_cast<const uint4*>(p));
-  v.hi = __ldg(reinterpret_cast<const uint4*>(p) + 1);
-}
-__device__ __forceinline__ void load_raw8(const __nv_bfloat16* p, uint4& v) { v = __ldg(reinterpret_cast<const uint4*>(p)); }
-__device__ __forceinline__ void clear_raw8(Raw8f& v) { v.lo = v.hi = make_uint4(0u, 0u, 0u, 0u); }
-__device__ __forceinline__ void clear_raw8(uint4& v) { v = make_uint4(0u, 0u, 0u, 0u); }
-__device__ __forceinline__ uint32_t raw8_amax(const Raw8f& v) {
-  constexpr uint32_t m = 0x7fffffffu;
-  const uint32_t a = max(max(v.lo.x & m, v.lo.y & m), max(v.lo.z & m, v.lo.w & m));
-  const uint32_t b = max(max(v.hi.x & m, v.hi.y & m), max(v.hi.z & m, v.hi.w & m));
-  return max(a, b);
-}
-__device__ __forceinline__ uint32_t raw8_amax(const uint4& v) {
-  constexpr uint32_t m = 0x7fff7fffu;
-  const uint32_t p = __vmaxu2(__vmaxu2(v.x & m, v.y & m), __vmaxu2(v.z & m, v.w & m));
-  return max(p & 0xffffu, p >> 16) << 16;  // the f32 pattern of the largest magnitude
-}
-__device__ __forceinline__ void raw8_values(const Raw8f& r, float (&v)[8]) {
-  v[0] = __uint_as_float(r.lo.x); v[1] = __uint_as_float(r.lo.y); v[2] = __uint_as_float(r.lo.z); v[3] = __uint_as_float(r.lo.w);
-  v[4] = __uint_as_float(r.hi.x); v[5] = __uint_as_float(r.hi.y); v[6] = __uint_as_float(r.hi.z); v[7] = __uint_as_float(r.hi.w);
-}
 __device__ __forceinline__ void raw8_values(const uint4& t, float (&v)[8]) {
   v[0] = __uint_as_float(t.x << 16); v[1] = __uint_as_float(t.x & 0xffff0000u);
   v[2] = __uint_as_float(t.y << 16); v[3] = __uint_as_float(t.y & 0xffff0000u);
   v[4] = __uint_as_float(t.z << 16); v[5] = __uint_as_float(t.z & 0xffff0000u);
   v[6] = __uint_as_float(t.w << 16); v[7] = __uint_as_float(t.w & 0xffff0000u);
 }
-template <typename InT> struct Raw8;
-template <> struct Raw8<float> { using type = Raw8f; };
-template <> struct Raw8<__nv_bfloat16> { using type = uint4; };
+
+// 32 bytes. `wide`: the address is a multiple of 32 (otherwise of 16).
+struct Raw32 { uint32_t w[8]; };
+__device__ __forceinline__ void load_raw32(const void* p, bool wide, Raw32& v) {
+  if (wide) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p));
+  } else {
+    const uint4 lo = __ldg(static_cast<const uint4*>(p)), hi = __ldg(static_cast<const uint4*>(p) + 1);
+    v.w[0] = lo.x; v.w[1] = lo.y; v.w[2] = lo.z; v.w[3] = lo.w;
+    v.w[4] = hi.x; v.w[5] = hi.y; v.w[6] = hi.z; v.w[7] = hi.w;
+  }
+}
 
 // Scale byte of a block whose largest magnitude has the f32 pattern `amax_bits` (the rule at the head of this file) and
 // the factor that brings its values to codes: 2^(127 - byte). (Byte 255, a block with a NaN or an infinity, has none: the callers
@@ -176,46 +158,157 @@ __device__ __forceinline__ float mxfp4_code_factor(int sb) {
   return sb >= 254 ? __int_as_float(0x00400000) : __int_as_float((254 - sb) << 23);
 }
 
-// The 32 K blocks of one warp: blocks kb0 .. kb0 + 31 of the row at `row` (nullptr: all padding). Lane l belongs to group
-// g = l / 4, whose blocks are kb0 + 4 g .. + 3. On return `codes` is the 16 bytes of block kb0 + l (valid when that block
-// is below kblocks) and `scales` the group's scale word (padding bytes for blocks at or past kblocks).
+// The 32 K blocks of one warp: blocks kb0 .. kb0 + 31 of the row at `row` (nullptr: all padding); all loads are in flight before any
+// arithmetic. Maxima are taken on bit patterns: the unsigned order of magnitudes is numeric order, infinity above every
+// finite value and NaN above infinity. `word[i]` is the scale word of atom kb0 / 4 + atom(i, lane) (padding bytes for blocks at or past
+// kblocks), held by the lanes where writes(lane).
 template <typename InT>
-__device__ __forceinline__ void mxfp4_quantize_warp(const InT* __restrict__ row, int kb0, int kblocks, int lane, uint4& codes,
-                                                    uint32_t& scales) {
-  using Raw = typename Raw8<InT>::type;
-  const int g = lane >> 2, sub = lane & 3;
-  Raw raw[4];
+struct WarpQuant;
+
+// bf16: a block is 64 bytes, half a line. Two loads of 32 bytes per lane, each 1 KB of the row without a gap, two neighbouring lanes per
+// block (with four blocks per four lanes a load took half lines; 28672 x 8192: 102.7 -> 94.5 us).
+template <>
+struct WarpQuant<__nv_bfloat16> {
+  static constexpr int kWords = 2;
+  uint32_t codes[2][2];  // of load u: this lane's half of block kb0 + 16 u + lane / 2
+  uint32_t word[2];
+  static __device__ __forceinline__ int atom(int i, int lane) { return (i * 16 + lane / 2) >> 2; }
+  static __device__ __forceinline__ bool writes(int lane) { return lane % 8 == 0; }
+
+  // wide: rows start on 32 bytes (otherwise on 16)
+  __device__ __forceinline__ void run(const __nv_bfloat16* __restrict__ row, bool wide, int kb0, int kblocks, int lane) {
+    Raw32 raw[2];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int kb = kb0 + g * 4 + u;
-    if (row != nullptr && kb < kblocks) load_raw8(row + kb * 32 + sub * 8, raw[u]);
-    else clear_raw8(raw[u]);  // an all-zero block has the padding byte as its scale
-  }
-  uint32_t w[4];
-  scales = 0;
+    for (int u = 0; u < 2; ++u) {
+      if (row != nullptr && kb0 + u * 16 + (lane >> 1) < kblocks) {
+        load_raw32(reinterpret_cast<const uint8_t*>(row + (long long)(kb0 + u * 16) * 32) + lane * 32, wide, raw[u]);
+      } else {
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    uint32_t m = raw8_amax(raw[u]);
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
-    const int sb = mxfp4_scale_byte(m);
-    scales |= uint32_t(sb) << (8 * u);
-    const float f = mxfp4_code_factor(sb);
-    float v[8];
-    raw8_values(raw[u], v);
-    const uint32_t c = e2m1x2_code(v[0] * f, v[1] * f) | (e2m1x2_code(v[2] * f, v[3] * f) << 8) |
-                       (e2m1x2_code(v[4] * f, v[5] * f) << 16) | (e2m1x2_code(v[6] * f, v[7] * f) << 24);
-    w[u] = (sb == 255) ? 0u : c;
+        for (int i = 0; i < 8; ++i) raw[u].w[i] = 0u;  // an all-zero block has the padding byte as its scale
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      uint32_t p = raw[u].w[0] & 0x7fff7fffu;
+#pragma unroll
+      for (int i = 1; i < 8; ++i) p = __vmaxu2(p, raw[u].w[i] & 0x7fff7fffu);
+      uint32_t m = max(p & 0xffffu, p >> 16) << 16;  // the f32 pattern of the largest magnitude
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+      const int sb = mxfp4_scale_byte(m);
+      const float f = mxfp4_code_factor(sb);
+      uint32_t w = uint32_t(sb) << (8 * ((lane >> 1) & 3));
+      w |= __shfl_xor_sync(0xffffffffu, w, 2);
+      word[u] = w | __shfl_xor_sync(0xffffffffu, w, 4);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float lo = __uint_as_float(raw[u].w[4 * i + j] << 16), hi = __uint_as_float(raw[u].w[4 * i + j] & 0xffff0000u);
+          c |= e2m1x2_code(lo * f, hi * f) << (8 * j);
+        }
+        codes[u][i] = (sb == 255) ? 0u : c;
+      }
+    }
   }
-  // 4 x 4 transpose over the group: lane `sub` ends with the four words of block 4 g + sub
-  const bool b1 = sub & 1, b2 = sub & 2;
-  const uint32_t s0 = __shfl_xor_sync(0xffffffffu, b1 ? w[0] : w[1], 1), s1 = __shfl_xor_sync(0xffffffffu, b1 ? w[2] : w[3], 1);
-  const uint32_t x0 = b1 ? s0 : w[0], x1 = b1 ? w[1] : s0, x2 = b1 ? s1 : w[2], x3 = b1 ? w[3] : s1;
-  const uint32_t t0 = __shfl_xor_sync(0xffffffffu, b2 ? x0 : x2, 2), t1 = __shfl_xor_sync(0xffffffffu, b2 ? x1 : x3, 2);
-  codes.x = b2 ? t0 : x0;
-  codes.y = b2 ? t1 : x1;
-  codes.z = b2 ? x2 : t0;
-  codes.w = b2 ? x3 : t1;
+  // The codes to the row's code bytes; vec: they start on 16 bytes (otherwise on 4).
+  __device__ __forceinline__ void store_codes(uint8_t* __restrict__ q_row, bool vec, int kb0, int kblocks, int lane) const {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (kb0 + u * 16 + (lane >> 1) >= kblocks) continue;
+      uint8_t* d = q_row + (kb0 + u * 16) * 16 + lane * 8;
+      if (vec) {
+        *reinterpret_cast<uint2*>(d) = make_uint2(codes[u][0], codes[u][1]);
+      } else {
+        reinterpret_cast<uint32_t*>(d)[0] = codes[u][0];
+        reinterpret_cast<uint32_t*>(d)[1] = codes[u][1];
+      }
+    }
+  }
+};
+
+// f32: a block is a line. Lane l belongs to group g = l / 4, whose blocks are kb0 + 4 g .. + 3 = one scale word.
+template <>
+struct WarpQuant<float> {
+  static constexpr int kWords = 1;
+  uint4 codes;  // of block kb0 + lane
+  uint32_t word[1];
+  static __device__ __forceinline__ int atom(int, int lane) { return lane >> 2; }
+  static __device__ __forceinline__ bool writes(int lane) { return (lane & 3) == 0; }
+
+  __device__ __forceinline__ void run(const float* __restrict__ row, bool, int kb0, int kblocks, int lane) {
+    const int g = lane >> 2, sub = lane & 3;
+    Raw32 raw[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int kb = kb0 + g * 4 + u;
+      if (row != nullptr && kb < kblocks) {
+        load_raw32(row + kb * 32 + sub * 8, false, raw[u]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) raw[u].w[i] = 0u;
+      }
+    }
+    uint32_t w[4], scales = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      uint32_t m = 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m = max(m, raw[u].w[i] & 0x7fffffffu);
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+      const int sb = mxfp4_scale_byte(m);
+      scales |= uint32_t(sb) << (8 * u);
+      const float f = mxfp4_code_factor(sb);
+      w[u] = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        w[u] |= e2m1x2_code(__uint_as_float(raw[u].w[2 * j]) * f, __uint_as_float(raw[u].w[2 * j + 1]) * f) << (8 * j);
+      if (sb == 255) w[u] = 0u;
+    }
+    word[0] = scales;
+    // 4 x 4 transpose over the group: lane `sub` ends with the four words of block 4 g + sub
+    const bool b1 = sub & 1, b2 = sub & 2;
+    const uint32_t s0 = __shfl_xor_sync(0xffffffffu, b1 ? w[0] : w[1], 1), s1 = __shfl_xor_sync(0xffffffffu, b1 ? w[2] : w[3], 1);
+    const uint32_t x0 = b1 ? s0 : w[0], x1 = b1 ? w[1] : s0, x2 = b1 ? s1 : w[2], x3 = b1 ? w[3] : s1;
+    const uint32_t t0 = __shfl_xor_sync(0xffffffffu, b2 ? x0 : x2, 2), t1 = __shfl_xor_sync(0xffffffffu, b2 ? x1 : x3, 2);
+    codes.x = b2 ? t0 : x0;
+    codes.y = b2 ? t1 : x1;
+    codes.z = b2 ? x2 : t0;
+    codes.w = b2 ? x3 : t1;
+  }
+  __device__ __forceinline__ void store_codes(uint8_t* __restrict__ q_row, bool vec, int kb0, int kblocks, int lane) const {
+    if (kb0 + lane >= kblocks) return;
+    uint8_t* d = q_row + (kb0 + lane) * 16;
+    if (vec) {
+      *reinterpret_cast<uint4*>(d) = codes;
+    } else {
+      uint32_t* d4 = reinterpret_cast<uint32_t*>(d);
+      d4[0] = codes.x; d4[1] = codes.y; d4[2] = codes.z; d4[3] = codes.w;
+    }
+  }
+};
+
+// The scale bytes of a warp's blocks to the row's at `scale_row`; words: every row of them starts on 4 bytes.
+template <typename Quant>
+__device__ __forceinline__ void store_scale_row(const Quant& w, uint8_t* __restrict__ scale_row, bool words, int kb0, int kblocks, int lane) {
+  if (!Quant::writes(lane)) return;
+#pragma unroll
+  for (int i = 0; i < Quant::kWords; ++i) {
+    const int kb = kb0 + Quant::atom(i, lane) * 4;
+    if (words) {
+      if (kb < kblocks) *reinterpret_cast<uint32_t*>(scale_row + kb) = w.word[i];
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (kb + j < kblocks) scale_row[kb + j] = uint8_t(w.word[i] >> (8 * j));
+    }
+  }
+}
+// Rows of x start on 32 bytes.
+template <typename InT>
+__device__ __forceinline__ bool rows_on_32(const InT* x, long long ldx) {
+  return ((reinterpret_cast<uintptr_t>(x) | uintptr_t(ldx * (long long)sizeof(InT))) & 31) == 0;
 }
 
 // Word (row r, atom) of a packed scale array: the four K blocks of that atom.
@@ -231,6 +324,7 @@ __device__ __forceinline__ uint32_t* packed_scale_word(uint8_t* base, int k_atom
 // release: the library launches this kernel's programmatic dependent right behind it, which waits before it reads a scale
 // or a code. Otherwise it does not let dependents start early: what it writes may be the WEIGHTS of a GEMM two launches
 // on, which WB200_OVERLAP_PREVIOUS allows to be read before that GEMM's wait.
+// (bf16: 32 registers, so that an SM holds 2048 threads; a form that took 38 needed 100 us for 28672 x 8192.)
 template <typename InT>
 __global__ void __launch_bounds__(256)
 quantize_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int K, uint8_t* __restrict__ q, int q_vec,
@@ -244,31 +338,18 @@ quantize_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int K,
   const int kb0 = int(blockIdx.x - group * chunks) * 32;
   const int r = int(group >> 4) * 128 + (warp & 3) * 32 + int(group & 15) * 2 + (warp >> 2);
   const bool real = r < rows;
-  uint4 codes;
-  uint32_t scales;
-  mxfp4_quantize_warp(real ? x + (long long)r * ldx : static_cast<const InT*>(nullptr), kb0, kblocks, lane, codes, scales);
-  const int g = lane >> 2, sub = lane & 3;
-  if (real && kb0 + lane < kblocks) {
-    uint8_t* dst = q + (long long)r * (K / 2) + (kb0 + lane) * 16;
-    if (q_vec) {
-      *reinterpret_cast<uint4*>(dst) = codes;
-    } else {
-      uint32_t* d = reinterpret_cast<uint32_t*>(dst);
-      d[0] = codes.x; d[1] = codes.y; d[2] = codes.z; d[3] = codes.w;
-    }
-  }
-  if (sub == 1 && scale_rm && real) {
-    uint8_t* d = scale_rm + (long long)r * kblocks + kb0 + g * 4;
-    if ((kblocks & 3) == 0 && (reinterpret_cast<uintptr_t>(scale_rm) & 3) == 0) {
-      if (kb0 + g * 4 < kblocks) *reinterpret_cast<uint32_t*>(d) = scales;
-    } else {
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (kb0 + g * 4 + u < kblocks) d[u] = uint8_t(scales >> (8 * u));
-    }
+  using Quant = WarpQuant<InT>;
+  Quant w;
+  w.run(real ? x + (long long)r * ldx : static_cast<const InT*>(nullptr), rows_on_32(x, ldx), kb0, kblocks, lane);
+  if (real) {
+    w.store_codes(q + (long long)r * (K / 2), q_vec, kb0, kblocks, lane);
+    if (scale_rm) store_scale_row(w, scale_rm + (long long)r * kblocks, (kblocks & 3) == 0 && (reinterpret_cast<uintptr_t>(scale_rm) & 3) == 0, kb0, kblocks, lane);
   }
   if (scale_packed) {
-    if (sub == 0) words[g][warp] = scales;  // word (row of the pair, 32-row group) of the sector
+    if (Quant::writes(lane)) {
+#pragma unroll
+      for (int i = 0; i < Quant::kWords; ++i) words[Quant::atom(i, lane)][warp] = w.word[i];  // word (row of the pair, 32-row group) of the sector
+    }
     __syncthreads();
     const int atom = (kb0 >> 2) + (threadIdx.x >> 3);
     if (threadIdx.x < 64 && atom < k_atoms) {
@@ -345,28 +426,14 @@ quantize_scatter_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows
   const int r = int(wid / chunks);
   if (r >= rows) return;
   const int kb0 = int(wid - unsigned(r) * chunks) * 32;
-  uint4 codes;
-  uint32_t scales;
-  mxfp4_quantize_warp(x + (long long)r * ldx, kb0, kblocks, lane, codes, scales);
-  const int g = lane >> 2, sub = lane & 3;
+  WarpQuant<InT> w;
+  w.run(x + (long long)r * ldx, rows_on_32(x, ldx), kb0, kblocks, lane);
+  const bool words = (kblocks & 3) == 0 && (reinterpret_cast<uintptr_t>(scale_rm) & 3) == 0;
   for (int j = 0; j < copies; ++j) {
     const int dst = __ldcg(dst_rows + r * copies + j);
     if (dst < 0) continue;
-    if (kb0 + lane < kblocks) {
-      uint8_t* d = q + (long long)dst * (K / 2) + (kb0 + lane) * 16;
-      if (q_vec) {
-        *reinterpret_cast<uint4*>(d) = codes;
-      } else {
-        uint32_t* d4 = reinterpret_cast<uint32_t*>(d);
-        d4[0] = codes.x; d4[1] = codes.y; d4[2] = codes.z; d4[3] = codes.w;
-      }
-    }
-    if (sub == 1) {
-      uint8_t* d = scale_rm + (long long)dst * kblocks + kb0 + g * 4;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (kb0 + g * 4 + u < kblocks) d[u] = uint8_t(scales >> (8 * u));
-    }
+    w.store_codes(q + (long long)dst * (K / 2), q_vec, kb0, kblocks, lane);
+    store_scale_row(w, scale_rm + (long long)dst * kblocks, words, kb0, kblocks, lane);
   }
 }
 
