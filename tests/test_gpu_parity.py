@@ -1634,3 +1634,54 @@ def test_linear_layer_first_used_at_another_decode_batch():
         check_bf16(layer(x.to(DEV)), orc.scaled_gemm(xq, xs, wq, ws))
     assert layer._packed.tile_rows == 128
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_calls_see_what_the_kernel_before_them_wrote(captured):
+    """Every launch may become resident beside the kernel before it and waits for that kernel before it touches memory: operands,
+    scales, weights and outputs that an ordinary kernel, or another call of the library, has written just before are the ones that are read,
+    back to back and many times. Bits of the same calls with a synchronisation between all of them."""
+    g = torch.Generator(device=DEV)
+    cases = []
+    for M, N, K in ((8, 4096, 512), (200, 512, 768), (16, 19456, 256), (300, 1024, 512)):
+        b, b_s, b_sf = ops.quantize_mxfp4(torch.randn(N, K, device=DEV, generator=g) * 0.02)
+        cases.append((M, N, K, b, b_sf, torch.empty(M, K, device=DEV), torch.empty(M, N, dtype=torch.bfloat16, device=DEV), torch.empty(M, N, device=DEV),
+                      wb.MXFP4Linear(b, b_s)))
+
+    def step(i, sync):
+        outs = []
+        for M, N, K, b, b_sf, x, c, acc, layer in cases:
+            x.fill_(0.01 * (i + 1)).mul_(torch.arange(K, device=DEV) % 7 - 3.0)
+            sync()
+            q, s, sf = ops.quantize_mxfp4(x)
+            sync()
+            ops.scaled_gemm_packed(q, sf, b, b_sf, c)
+            sync()
+            acc.fill_(float(i))
+            sync()
+            ops.scaled_gemm_packed(q, ops.repack_scales(s), b, b_sf, acc, _lib.ACCUMULATE)
+            sync()
+            y = layer(x)
+            sync()
+            c.mul_(1.0)
+            outs += [c.clone(), acc.clone(), y]
+        return outs
+
+    for _ in range(2):
+        step(0, torch.cuda.synchronize)
+    refs = [step(i, torch.cuda.synchronize) for i in range(12)]
+    torch.cuda.synchronize()
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = [step(i, lambda: None) for i in range(12)]
+        for _ in range(3):
+            graph.replay()
+        torch.cuda.synchronize()
+    else:
+        got = [step(i, lambda: None) for i in range(12)]
+        torch.cuda.synchronize()
+    for a, b in zip(got, refs):
+        for u, v in zip(a, b):
+            assert torch.equal(u, v)
+    ops.check_device_status()

@@ -126,10 +126,9 @@ CUresult encode_2d(CUtensorMap* map, const MapKey& k) {
   return r;
 }
 
-// True while a launch is to be made a programmatic dependent of the kernel before it in the stream: the GEMM
-// behind the repack kernel of wb200_mxfp4_gemm_repack_a, and every launch of a call flagged
-// WB200_OVERLAP_PREVIOUS. A dependent kernel starts while its predecessor drains and executes
-// griddepcontrol.wait before touching anything but the weights.
+// True while launches are kDependent (ptx.cuh): the GEMM behind the repack kernel of wb200_mxfp4_gemm_repack_a, and every launch of
+// a call flagged WB200_OVERLAP_PREVIOUS. Such a kernel starts while its predecessor drains and executes
+// griddepcontrol.wait before touching anything but the weights; the others (kFirst) wait before they touch anything.
 static thread_local bool tl_dependent_launch = false;
 // N tiles per raster group of the tile kernels, from the WB200_GROUP_N bits of the call in progress
 static thread_local int tl_group_n = 16;
@@ -340,7 +339,7 @@ int launch_tile(const DeviceInfo& dev, int M, int N, int K, const void* a, const
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = tl_dependent_launch ? 2 : 1;
+  cfg.numAttrs = 2;
   WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   return WB200_OK;
 }
@@ -458,13 +457,13 @@ struct PairLaunch {
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = tl_dependent_launch ? 2 : 1;
+    cfg.numAttrs = 2;
   }
 };
 
-// An ordinary kernel, optionally a programmatic dependent of the one before it in the stream.
+// A kernel with the programmatic attribute (kFirst or kDependent of ptx.cuh), or without it.
 template <typename... P, typename... A>
-cudaError_t launch_kernel(bool dependent, void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t stream, A... args) {
+cudaError_t launch_kernel(bool programmatic, void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
   cfg.blockDim = dim3(threads, 1, 1);
@@ -473,7 +472,7 @@ cudaError_t launch_kernel(bool dependent, void (*kernel)(P...), unsigned grid, u
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = dependent ? 1 : 0;
+  cfg.numAttrs = programmatic ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
@@ -665,7 +664,7 @@ int launch_splitk(const DeviceInfo& dev, int slices, int M, int N, int K, const 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = tl_dependent_launch ? 2 : 1;
+  cfg.numAttrs = 2;
   WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   const long long vecs = (long long)M * ((N + 3) / 4);
   wb::splitk_reduce_kernel<OutT><<<unsigned((vecs + 255) / 256), 256, 0, stream>>>(slots, used, (long long)M * N, M, N,
@@ -694,7 +693,7 @@ int cluster_splitk_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, in
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = tl_dependent_launch ? 2 : 1;
+  cfg.numAttrs = 2;
   return WB200_OK;
 }
 
@@ -711,14 +710,13 @@ int clusters_in_flight(int slices) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     int count = 0;
-    const bool saved = tl_dependent_launch;
-    tl_dependent_launch = false;
-    if (cluster_splitk_config<128, float>(cfg, attr, slices, 1, nullptr) != WB200_OK ||
+    const int rc = cluster_splitk_config<128, float>(cfg, attr, slices, 1, nullptr);
+    cfg.numAttrs = 1;  // the cluster alone
+    if (rc != WB200_OK ||
         cudaOccupancyMaxActiveClusters(&count, wb::mxfp4_gemm_cluster_splitk_kernel<128, float>, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
       count = 0;
     }
-    tl_dependent_launch = saved;
     n = count > 0 ? count : -1;
   }
   return n > 0 ? n : 0;
@@ -802,7 +800,7 @@ int launch_skinny_scales(const DeviceInfo& dev, int M, int N, int K, const void*
   p.tiles_n = (N + 127) / 128;
   p.num_kb = (K + Cfg::BK - 1) / Cfg::BK;
   p.accumulate = accumulate;
-  p.dependent = tl_dependent_launch ? 1 : 0;
+  p.dependent = tl_dependent_launch ? wb::kDependent : wb::kFirst;
   p.elem_format = elem_format;
   p.status = dev.status_ptr;
   auto kernel = wb::mxfp4_skinny_kernel<NP, STAGES, OutT, EB, RS>;
@@ -820,7 +818,7 @@ int launch_skinny_scales(const DeviceInfo& dev, int M, int N, int K, const void*
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = tl_dependent_launch ? 1 : 0;
+  cfg.numAttrs = 1;
   WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, tmW, tmX, tmSFW, tmSFX, p));
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
@@ -945,7 +943,7 @@ int launch_skinny_whole_maps(const DeviceInfo& dev, int M, int N, int K, const v
   p.tile_rows = tile_rows;
   p.num_kb = (K + Base::BK - 1) / Base::BK;
   p.accumulate = accumulate;
-  p.dependent = tl_dependent_launch ? 1 : 0;
+  p.dependent = tl_dependent_launch ? wb::kDependent : wb::kFirst;
   p.elem_format = elem_format;
   p.c_vec = ((reinterpret_cast<uintptr_t>(c) & 15) == 0 && (ldc * (long long)sizeof(OutT)) % 16 == 0) ? 1 : 0;
   // TMA stores of the staged chunks: 16-byte aligned C, no accumulation, and two staging halves that each hold a chunk
@@ -969,7 +967,7 @@ int launch_skinny_whole_maps(const DeviceInfo& dev, int M, int N, int K, const v
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = tl_dependent_launch ? 1 : 0;
+  cfg.numAttrs = 1;
   WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   WB_CUDA(cudaGetLastError());
   return WB200_OK;
@@ -1032,7 +1030,7 @@ int launch_skinny_experts(const DeviceInfo& dev, const RoutedGemm& g, int T, voi
   p.tiles_n = tiles_n;
   p.tile_rows = 128;
   p.num_kb = (g.K + Base::BK - 1) / Base::BK;
-  p.dependent = tl_dependent_launch ? 1 : 0;
+  p.dependent = tl_dependent_launch ? wb::kDependent : wb::kFirst;
   p.c_vec = 1;
   p.status = dev.status_ptr;
   auto kernel = wb::mxfp4_skinny_whole_kernel<NP, STAGES, __nv_bfloat16, 4, 128, 2, Maps>;
@@ -1048,7 +1046,7 @@ int launch_skinny_experts(const DeviceInfo& dev, const RoutedGemm& g, int T, voi
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = tl_dependent_launch ? 1 : 0;
+  cfg.numAttrs = 1;
   WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   return WB200_OK;
 }
@@ -1093,7 +1091,7 @@ int launch_mixed_decode(const DeviceInfo& dev, int M, int N, int K, const void* 
   p.tile_rows = tile_rows;
   p.num_kb = K / 128;
   p.accumulate = accumulate;
-  p.dependent = tl_dependent_launch ? 1 : 0;
+  p.dependent = tl_dependent_launch ? wb::kDependent : wb::kFirst;
   p.elem_format = elem_format;
   p.vec_ok = ((reinterpret_cast<uintptr_t>(c) & 15) == 0 && (ldc * (long long)sizeof(OutT)) % 16 == 0) ? 1 : 0;
   p.status = dev.status_ptr;
@@ -1109,7 +1107,7 @@ int launch_mixed_decode(const DeviceInfo& dev, int M, int N, int K, const void* 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = tl_dependent_launch ? 1 : 0;
+  cfg.numAttrs = 1;
   WB_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   return WB200_OK;
 }
@@ -1354,7 +1352,7 @@ static int repack_scales_impl(const void* src, long long src_row_stride, int row
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = tl_dependent_launch ? 1 : 0;
+  cfg.numAttrs = 1;
   WB_CUDA(cudaLaunchKernelEx(&cfg, wb::repack_scales_kernel, static_cast<const uint8_t*>(src), src_row_stride, rows, K / 32,
                              k_atoms, static_cast<uint8_t*>(dst), broadcast, tl_dependent_launch, block_rows));
   return WB200_OK;
@@ -1439,15 +1437,23 @@ static int quantize_mxfp4_impl(const void* x, int x_dtype, long long ldx, int ro
   const int k_atoms = wb::sf_k_atoms(K);
   const int q_vec = (reinterpret_cast<uintptr_t>(q) & 15) == 0;
   const unsigned blocks = unsigned(wb::sf_row_blocks(rows)) * 16u * unsigned((k_atoms + 7) / 8);
+  // Started beside the tail of the kernel before it only where all its CTAs fit at one time; larger grids are slower for it
+  // in front of a GEMM (MXFP4Linear, ordinary / programmatic: 8 x 14336 x 4096 12.3 / 9.6 us, 300 x 8192 x 8192 20.5 / 19.1, 1000 x 4096 x
+  // 4096 18.3 / 17.0, 3000 x 8192 x 8192 93.7 / 94.9, 8000 x 4096 x 4096 73.2 / 75.9).
+  // In a graph, whose kernels follow one another without that gap, only up to one CTA per SM (1000 x 4096 x 4096 13.6 / 14.1, 8 x 14336 x 4096 9.4 / 9.0).
+  bool beside = blocks <= 8u * unsigned(dev->sm_count);
+  if (beside && blocks > unsigned(dev->sm_count)) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    WB_CUDA(cudaStreamIsCapturing(s, &status));
+    beside = status == cudaStreamCaptureStatusNone;
+  }
   if (x_dtype == WB200_F32)
-    wb::quantize_mxfp4_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), ldx, rows, K,
-                                                            static_cast<uint8_t*>(q), q_vec, static_cast<uint8_t*>(scale_rowmajor),
-                                                            static_cast<uint8_t*>(scale_packed), k_atoms, release);
+    WB_CUDA(launch_kernel(beside, wb::quantize_mxfp4_kernel<float>, blocks, 256, s, static_cast<const float*>(x), ldx, rows, K, static_cast<uint8_t*>(q),
+                          q_vec, static_cast<uint8_t*>(scale_rowmajor), static_cast<uint8_t*>(scale_packed), k_atoms, release));
   else
-    wb::quantize_mxfp4_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(x), ldx, rows, K, static_cast<uint8_t*>(q), q_vec,
-        static_cast<uint8_t*>(scale_rowmajor), static_cast<uint8_t*>(scale_packed), k_atoms, release);
-  WB_CUDA(cudaGetLastError());
+    WB_CUDA(launch_kernel(beside, wb::quantize_mxfp4_kernel<__nv_bfloat16>, blocks, 256, s, static_cast<const __nv_bfloat16*>(x), ldx, rows, K,
+                          static_cast<uint8_t*>(q), q_vec, static_cast<uint8_t*>(scale_rowmajor), static_cast<uint8_t*>(scale_packed), k_atoms,
+                          release));
   return WB200_OK;
 }
 
@@ -2044,11 +2050,11 @@ static int launch_route_kernels(const void* x, long long ldx, int K, uint8_t* q,
   const unsigned blocks = unsigned(((long long)route.tokens * ((k_atoms + 7) / 8) + 7) / 8);
   const InT* in = static_cast<const InT*>(x);
   if (route.tokens <= wb::kRouteTokens) {
-    WB_CUDA(launch_kernel(false, wb::moe_quantize_kernel<InT, T, EM, true>, blocks, 256, s, in, ldx, K, q, q_sf, k_atoms, route));
+    WB_CUDA(launch_kernel(true, wb::moe_quantize_kernel<InT, T, EM, true>, blocks, 256, s, in, ldx, K, q, q_sf, k_atoms, route));
     return WB200_OK;
   }
   const unsigned route_blocks = unsigned((route.tokens + route.tokens_per_block - 1) / route.tokens_per_block);
-  WB_CUDA(launch_kernel(false, wb::moe_route_kernel<T, EM>, route_blocks, wb::kRouteTokens, s, route));
+  WB_CUDA(launch_kernel(true, wb::moe_route_kernel<T, EM>, route_blocks, wb::kRouteTokens, s, route));
   WB_CUDA(launch_kernel(true, wb::moe_quantize_kernel<InT, T, EM, false>, blocks, 256, s, in, ldx, K, q, q_sf, k_atoms, route));
   return WB200_OK;
 }
@@ -2099,8 +2105,8 @@ int wb200_mxfp4_expert_mlp(int T, int E, int K, int inter, int N, int top_k, con
   int* inverse = reinterpret_cast<int*>(ws + plan.inverse);
   int *expert_ids = reinterpret_cast<int*>(ws + plan.expert_ids), *num_rows = reinterpret_cast<int*>(ws + plan.num_rows);
   unsigned int* counters = reinterpret_cast<unsigned int*>(ws + plan.counters);
-  // Every launch after the first is the programmatic dependent of the one before it. The first one is an ordinary launch,
-  // so what the kernels before this call wrote (x, the logits) is complete for all of them.
+  // Every launch after the first is kDependent. The first one waits before it releases the next, so what the kernels before this
+  // call wrote (x, the logits) is complete for all of them.
   wb::RouteParams route;
   route.logits = logits;
   route.ld = ld_logits;

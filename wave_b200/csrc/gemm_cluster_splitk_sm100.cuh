@@ -52,7 +52,6 @@ mxfp4_gemm_cluster_splitk_kernel(const __grid_constant__ PlainMaps maps, const G
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  pdl_launch_dependents();
   const uint32_t cluster_rank = cluster_ctarank();
   const int slice = int(cluster_rank >> 1);
   const uint32_t rank = cluster_rank & 1u;  // in the pair
@@ -115,6 +114,7 @@ mxfp4_gemm_cluster_splitk_kernel(const __grid_constant__ PlainMaps maps, const G
       __syncwarp();
       if (++stage == STAGES) { stage = 0; phase ^= 1u; }
     }
+    pdl_launch_dependents();  // (as in gemm_sm100.cuh)
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader of each pair)
     if (leader) {

@@ -260,7 +260,7 @@ __device__ __forceinline__ int decode_tile(const Maps& maps, const GemmParams& p
   }
 }
 
-// Adds the 32 values already in C (row pointer p) to r: the accumulate-into-C form the
+// Adds the 32 values already in C (row pointer p; read through L2) to r: the accumulate-into-C form the
 // reference's split-K template has (tagged_mxfp4_gemm.py:780-781, caller-initialised C).
 template <typename OutT>
 __device__ __forceinline__ void add_old_chunk32(const OutT* __restrict__ p, uint32_t (&r)[32], int ncols,
@@ -270,7 +270,7 @@ __device__ __forceinline__ void add_old_chunk32(const OutT* __restrict__ p, uint
       const uint4* q = reinterpret_cast<const uint4*>(p);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const uint4 v = q[j];
+        const uint4 v = __ldcg(q + j);
         r[4 * j + 0] = __float_as_uint(__uint_as_float(r[4 * j + 0]) + __uint_as_float(v.x));
         r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + __uint_as_float(v.y));
         r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + __uint_as_float(v.z));
@@ -279,12 +279,12 @@ __device__ __forceinline__ void add_old_chunk32(const OutT* __restrict__ p, uint
     } else {
 #pragma unroll
       for (int j = 0; j < 32; ++j)
-        if (j < ncols) r[j] = __float_as_uint(__uint_as_float(r[j]) + reinterpret_cast<const float*>(p)[j]);
+        if (j < ncols) r[j] = __float_as_uint(__uint_as_float(r[j]) + __ldcg(reinterpret_cast<const float*>(p) + j));
     }
   } else {
 #pragma unroll
     for (int j = 0; j < 32; ++j)
-      if (j < ncols) r[j] = __float_as_uint(__uint_as_float(r[j]) + __bfloat162float(p[j]));
+      if (j < ncols) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(uint32_t(__ldcg(reinterpret_cast<const unsigned short*>(p) + j)) << 16));
   }
 }
 
@@ -367,7 +367,6 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  pdl_launch_dependents();  // a kernel launched behind this one as a programmatic dependent may take SMs as they free up
   const uint32_t rank = (CG == 2) ? cluster_ctarank() : 0u;
   const bool leader = (rank == 0);
 
@@ -413,7 +412,10 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
   const uint32_t tmem_base = *tmem_slot;
 
   // The routing arrays of an aligned launch are written by the kernels before this one: every role waits for them.
-  if constexpr (Maps::kAligned) pdl_wait();
+  if constexpr (Maps::kAligned) {
+    pdl_wait();
+    pdl_launch_dependents();  // the next kernel of the expert MLP takes SMs as they free up
+  }
   RowSpan span;
   const int num_tiles = count_tiles(maps, p, span);
   const int first_tile = (CG == 2) ? (blockIdx.x >> 1) : blockIdx.x;
@@ -474,6 +476,9 @@ mxfp4_gemm_kernel(const __grid_constant__ Maps maps, const GemmParams p) {
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
     }
+    // Kernels behind this one may take SMs as they free up; not earlier: the waiting warps of a small kernel that became resident at the
+    // start cost a launch of 200 us 1 % under the board's power limit (8192^3 206.9 -> 209.8 us).
+    if constexpr (!Maps::kAligned) pdl_launch_dependents();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
     if (leader) {

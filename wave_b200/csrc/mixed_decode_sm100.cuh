@@ -54,7 +54,7 @@ struct MixedDecodeParams {
   int tile_rows;  // a multiple of 8, at most kMixedTileRowsMax
   int num_kb;     // K / 128
   int accumulate;
-  int dependent;  // launched as the programmatic dependent of the kernel that writes the activations' packed scales
+  int dependent;  // kFirst, or kDependent: behind the kernel that writes the activations' packed scales
   int elem_format;
   int vec_ok;
   int* status;
@@ -70,7 +70,7 @@ mixed_decode_kernel(const __grid_constant__ MixedDecodeMaps maps, const MixedDec
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  pdl_launch_dependents();
+  if (p.dependent) pdl_launch_dependents();
   if (warp == 0 && lane < 4)  // the copy engine fetches a descriptor on first use: start that now
     prefetch_tensormap(lane == 0 ? &maps.w : lane == 1 ? &maps.sfw : lane == 2 ? &maps.x : &maps.sfx);
   const uint32_t bar_base = smem_base + STAGES * Cfg::STAGE_BYTES;
@@ -112,6 +112,10 @@ mixed_decode_kernel(const __grid_constant__ MixedDecodeMaps maps, const MixedDec
     __syncwarp();
     stream_policy = l2_policy_evict_first();  // weights are read once
     keep_policy = l2_policy_evict_last();     // activations are re-read by every CTA
+    if (!p.dependent) {
+      pdl_wait();
+      pdl_launch_dependents();
+    }
     head = min(STAGES, p.num_kb);
     for (int i = 0; i < head; ++i) load_stage(int(blockIdx.x), i, uint32_t(i), p.dependent ? 1 : 0);
   }
@@ -177,7 +181,7 @@ mixed_decode_kernel(const __grid_constant__ MixedDecodeMaps maps, const MixedDec
     // ------------------------------------------------------------------ epilogue: warp quad q holds output rows 32 q ..
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
-    if (p.dependent) pdl_wait();  // C may still be read by the kernels before this one
+    pdl_wait();  // C may still be read by the kernels before this one
     int it = 0;
     for (int tile = blockIdx.x; tile < p.tiles_n; tile += gridDim.x, ++it) {
       const int as = it & 1;

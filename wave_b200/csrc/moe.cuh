@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(kRouteTokens)
 moe_route_kernel(const RouteParams p) {
   __shared__ RouteTable table;
   __shared__ int seen[kRouteMaxExperts];  // pairs of each expert in the tokens so far
+  pdl_wait();
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid < kRouteMaxExperts) seen[tid] = 0;
@@ -251,6 +252,7 @@ moe_quantize_kernel(const InT* __restrict__ x, long long ldx, int K, uint8_t* __
   __shared__ RouteTable table;
   __shared__ int totals[kRouteMaxExperts], before[kRouteMaxExperts];  // pairs per expert: in all, and in earlier blocks of tokens
   __shared__ int first[kRouteMaxExperts];                             // sorted row of rank 0 in this block of tokens
+  if constexpr (HERE) pdl_wait();  // (otherwise moe_route_kernel has released this one: what came before that is complete)
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kblocks = K >> 5;

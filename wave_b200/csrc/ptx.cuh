@@ -316,6 +316,16 @@ __device__ __forceinline__ uint32_t idesc_with_sf_id(uint32_t idesc, uint32_t sf
 // finished and its writes are visible (a no-op in a kernel launched without the attribute).
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// How a kernel of this library stands in its stream. Every launch carries the programmatic attribute: a kernel that is started the
+// ordinary way behind another one begins 1 to 2 us after that one's end (on the B200 the gap is rounded up to a 2.048 us
+// raster: 1024^3 alone 8.20 us a launch back to back, 5.36 with the attribute).
+//   kDependent: the kernel before it is the library's own, of the same call (or the caller says WB200_OVERLAP_PREVIOUS): it may touch what
+//     that kernel does not write before it waits, and release its own dependents at once.
+//   kFirst: anything may come before it. It waits before it touches memory, and releases its dependents after that: whoever starts
+//     then finds everything before this kernel complete.
+// What a kernel reads after its wait it reads with ordinary loads, not through the non-coherent path: the data may have been
+// written while the kernel was already resident.
+enum : int { kFirst = 0, kDependent = 1 };
 
 // Instruction descriptor of kind::mxf8f6f4 block-scaled: operand formats 0 = E4M3, 1 = E5M2, 5 = E2M1 (4-bit values in
 // the 8-bit container layout: 16 values in 8 bytes, then 8 bytes of padding), chosen per operand; K-major, UE8M0

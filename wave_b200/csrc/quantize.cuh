@@ -136,12 +136,13 @@ __device__ __forceinline__ void raw8_values(const uint4& t, float (&v)[8]) {
 struct Raw32 { uint32_t w[8]; };
 __device__ __forceinline__ void load_raw32(const void* p, bool wide, Raw32& v) {
   if (wide) {
-    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p));
   } else {
-    const uint4 lo = __ldg(static_cast<const uint4*>(p)), hi = __ldg(static_cast<const uint4*>(p) + 1);
-    v.w[0] = lo.x; v.w[1] = lo.y; v.w[2] = lo.z; v.w[3] = lo.w;
-    v.w[4] = hi.x; v.w[5] = hi.y; v.w[6] = hi.z; v.w[7] = hi.w;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(v.w[4 * i]), "=r"(v.w[4 * i + 1]), "=r"(v.w[4 * i + 2]), "=r"(v.w[4 * i + 3]) : "l"(static_cast<const uint4*>(p) + i));
   }
 }
 
@@ -330,6 +331,7 @@ __global__ void __launch_bounds__(256)
 quantize_mxfp4_kernel(const InT* __restrict__ x, long long ldx, int rows, int K, uint8_t* __restrict__ q, int q_vec,
                       uint8_t* __restrict__ scale_rm, uint8_t* __restrict__ scale_packed, int k_atoms, int release) {
   __shared__ uint32_t words[8][8];  // [atom of the chunk][word of the sector]
+  pdl_wait();
   if (release) pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kblocks = K >> 5;

@@ -25,6 +25,18 @@ __host__ __device__ inline size_t sf_packed_bytes(int rows, int K) {
   return size_t(sf_row_blocks(rows)) * sf_k_atoms(K) * 512;
 }
 
+// Ordinary loads (never through the non-coherent path): src may have been written while this kernel was already resident.
+__device__ __forceinline__ uint4 ld_global_v4(const uint8_t* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint8_t ld_global_u8(const uint8_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p));
+  return uint8_t(v);
+}
+
 // One thread block moves 128 rows x 32 K-blocks through shared memory: reads are 16 bytes per
 // thread along K, writes are 4 KiB contiguous. Rows [row_base, row_base + 128) of src, clipped at
 // row_limit, go to the 128-row block whose first atom is at dst_block. With `broadcast` src holds one
@@ -43,13 +55,13 @@ __device__ __forceinline__ void repack_tile(const uint8_t* __restrict__ src, lon
     const uint8_t* s = src + (long long)row * src_row_stride + (broadcast ? 0 : kb0);
     const bool row_ok = row < row_limit;
     if (!broadcast && row_ok && kb0 + 16 <= kblocks && ((reinterpret_cast<uintptr_t>(s) & 15) == 0)) {
-      const uint4 v = *reinterpret_cast<const uint4*>(s);
+      const uint4 v = ld_global_v4(s);
       uint32_t* d = reinterpret_cast<uint32_t*>(&tile[r][half * 16]);
       d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     } else {
 #pragma unroll
       for (int j = 0; j < 16; ++j)
-        tile[r][half * 16 + j] = (row_ok && kb0 + j < kblocks) ? s[broadcast ? 0 : j] : WB_SF_PAD;
+        tile[r][half * 16 + j] = (row_ok && kb0 + j < kblocks) ? ld_global_u8(s + (broadcast ? 0 : j)) : WB_SF_PAD;
     }
   }
   __syncthreads();
@@ -72,11 +84,11 @@ __device__ __forceinline__ void repack_tile(const uint8_t* __restrict__ src, lon
 __global__ void __launch_bounds__(256)
 repack_scales_kernel(const uint8_t* __restrict__ src, long long src_row_stride, int rows, int kblocks,
                      int k_atoms, uint8_t* __restrict__ dst, bool broadcast, bool dependent, int block_rows = 128) {
-  // a GEMM launched behind this kernel as a programmatic dependent may start its set-up now; it waits for
-  // this kernel's completion before it reads dst
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // launched as a programmatic dependent itself: the kernel before it may still be reading dst or writing src
-  if (dependent) asm volatile("griddepcontrol.wait;" ::: "memory");
+  // a GEMM launched behind this kernel may start its set-up once every CTA has come here; it waits for this kernel's
+  // completion before it reads dst (dependent: kDependent of ptx.cuh)
+  if (dependent) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the kernel before this one may still be reading dst or writing src
+  if (!dependent) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // block_rows != 128: a packing per tile of block_rows weight rows. Up to 128: one atom row per tile (the decode
   // kernel's tiles; rows block_rows..127 of every atom hold the padding byte). Above 128 (224: the tile kernel's
   // 224-column tiles): two atom rows per tile, rows 0..127 and 128..block_rows-1 of the tile.

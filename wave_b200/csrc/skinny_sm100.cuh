@@ -85,7 +85,7 @@ struct SkinnyParams {
   int tiles_n;   // ceil(N / 128)
   int num_kb;    // ceil(K / 256)
   int accumulate;  // add to the values already in C instead of overwriting them
-  int dependent;   // launched as the programmatic dependent of the kernel that writes the activations' packed scales
+  int dependent;   // kFirst, or kDependent: behind the kernel that writes the activations' packed scales
   int elem_format; // 8-bit operands only: 0 = E4M3, 1 = E5M2
   RowScales x_scales;
   int* status;
@@ -119,7 +119,7 @@ mxfp4_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  pdl_launch_dependents();  // a kernel launched behind this one as a programmatic dependent may take SMs as they free up
+  if (p.dependent) pdl_launch_dependents();  // kernels behind this one may take SMs as they free up
 #ifdef WB200_TRACE
   if (threadIdx.x == 0) WB_TRACE_SET(0, trace_now());
 #endif
@@ -208,8 +208,8 @@ mxfp4_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     __syncwarp();  // lane 0 initialised the barriers above
     stream_policy = l2_policy_evict_first();  // weights are read once
     keep_policy = l2_policy_evict_last();     // activations are re-read by every CTA
-    // The first pass over the ring needs no free-slot wait. When this kernel was launched as the programmatic
-    // dependent of the kernel that packs the activations' scales, the pass runs in two parts: the weight loads
+    // The first pass over the ring needs no free-slot wait. Behind the kernel that packs the activations' scales
+    // (kDependent) the pass runs in two parts: the weight loads
     // go out at once, the activation loads follow the dependency wait. Otherwise the four loads of a stage go
     // out together (the copy engine takes them in order: a stage completes sooner that way).
     if (p.dependent) {
@@ -220,6 +220,8 @@ mxfp4_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       pdl_wait();
       produce(STAGES, false, 2);
     } else {
+      pdl_wait();
+      pdl_launch_dependents();
       produce(STAGES, false, 0);
     }
 #ifdef WB200_TRACE
@@ -298,7 +300,7 @@ mxfp4_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     // ------------------------------------------------------------------ the activations' scales, row-major, into the stages
     if constexpr (RS) {
       static_assert(EB == 4 && NP <= kRowScaleRows, "a stage of 256 K, one row per lane");
-      if (p.dependent) pdl_wait();
+      pdl_wait();
       uint32_t stage = 0, phase = 0;
       feed_row_scales<STAGES>(
           p.x_scales, lane, head_kbs, nkb, u1 - u0, stage, phase,
@@ -310,7 +312,7 @@ mxfp4_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     // ------------------------------------------------------------------ epilogue warps 2..5
     const int quad = warp & 3;
     const int nl = quad * 32 + lane;  // weight row inside the tile
-    if (p.dependent) pdl_wait();  // C, the partial tiles and the counters may still be in use by the kernels before this one
+    pdl_wait();  // C, the partial tiles and the counters may still be in use by the kernels before this one
     OutT* __restrict__ C = reinterpret_cast<OutT*>(p.c);
     auto store_out = [&](int m, int n, float v) {
       if (!WB_CHECK(m >= 0 && m < p.M && n >= 0 && n < p.N, kCheckOutputIndex, (long long)m << 32 | unsigned(n))) return;

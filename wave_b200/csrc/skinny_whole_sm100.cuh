@@ -54,7 +54,7 @@ struct SkinnyWholeParams {
                  // that height (wb200_repack_scales_tiled) so that every SM gets the same number of tiles
   int num_kb;    // ceil(K / BK)
   int accumulate;
-  int dependent;
+  int dependent; // kFirst or kDependent
   int elem_format;
   int c_vec;     // C's base and row pitch allow 16-byte accesses
   int tma_store; // write C with TMA stores from the staged chunk (needs c_vec, no accumulate, a staging buffer pair that
@@ -114,7 +114,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  pdl_launch_dependents();  // a kernel launched behind this one as a programmatic dependent may take SMs as they free up
+  if (p.dependent) pdl_launch_dependents();  // kernels behind this one may take SMs as they free up
 #ifdef WB200_TRACE
   if (threadIdx.x == 0) WB_TRACE_SET(0, trace_now());  // timeline marks as in skinny_sm100.cuh; a "segment" is a tile here
 #endif
@@ -217,12 +217,16 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
   };
   // Warp 0 has just initialised the barriers: it starts the first ring of loads of this CTA's first tile (its own
   // index) right away, before the CTA-wide synchronisation that waits for the tensor-memory allocation. When the
-  // kernel was launched as a programmatic dependent, only the weight loads go out now; the activation loads follow
+  // kernel stands behind the one that writes the activations' scales, only the weight loads go out now; the activation loads follow
   // the dependency wait.
   int head = 0;
   if (warp == 0) {
     stream_policy = l2_policy_evict_first();  // weights are read once
     keep_policy = l2_policy_evict_last();     // activations are re-read by every CTA
+    if (!p.dependent) {
+      pdl_wait();
+      pdl_launch_dependents();
+    }
     if constexpr (!Maps::kExperts) {  // (which expert a tile belongs to is known after the dependency wait only)
       locate(int(blockIdx.x));
       head = min(STAGES, p.num_kb);
@@ -350,7 +354,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
   } else if (Maps::kScaleWarp && warp == 6) {
     // ------------------------------------------------------------------ scales that the copy engine cannot bring as the MMA reads them
     if constexpr (Maps::kSilu) {
-      if (p.dependent) pdl_wait();  // the routing arrays are the kernels' before this one
+      pdl_wait();  // the routing arrays are the kernels' before this one
       uint32_t stage = 0, phase = 0;
       for (int seq = 0;; ++seq) {
         const int item = next_tile(seq);
@@ -368,7 +372,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
     // the activations' scales, row-major, into the stages
     if constexpr (Maps::kRowScales) {
       static_assert(EB == 4 && NP <= kRowScaleRows, "a stage of 256 K, one row per lane");
-      if (p.dependent) pdl_wait();
+      pdl_wait();
       uint32_t stage = 0, phase = 0;
       for (int seq = 0;; ++seq) {
         if (next_tile(seq) < 0) break;
@@ -384,7 +388,7 @@ mxfp4_skinny_whole_kernel(const __grid_constant__ Maps maps, const SkinnyWholePa
     const int quad = warp & 3;
     const int nl = quad * 32 + lane;      // weight row inside the tile = tensor-memory lane
     const int t = int(threadIdx.x) - 64;  // 0..127
-    if (p.dependent) pdl_wait();  // C may still be read by the kernels before this one
+    pdl_wait();  // C may still be read by the kernels before this one
     OutT* __restrict__ C = reinterpret_cast<OutT*>(p.c);
     // Every thread owns two 32-byte pieces of a 16-row chunk: rows (t / 16) and (t / 16) + 8, columns 8 (t % 16) .. + 7.
     const int prow = t >> 4, pcol = (t & 15) * 8;
