@@ -27,6 +27,32 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+// 32 columns of one row of C as they are in memory (16-byte aligned, read through L2).
+template <typename OutT>
+struct OldChunk {
+  static constexpr int V = 32 * int(sizeof(OutT)) / 16;
+  uint4 v[V];
+  __device__ __forceinline__ void load(const OutT* p) {
+#pragma unroll
+    for (int j = 0; j < V; ++j) v[j] = __ldcg(reinterpret_cast<const uint4*>(p) + j);
+  }
+  __device__ __forceinline__ void add_to(uint32_t (&r)[32]) const {
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if constexpr (sizeof(OutT) == 4) {
+          r[4 * j + i] = __float_as_uint(__uint_as_float(r[4 * j + i]) + __uint_as_float(w[i]));
+        } else {
+          r[8 * j + 2 * i] = __float_as_uint(__uint_as_float(r[8 * j + 2 * i]) + __uint_as_float(w[i] << 16));
+          r[8 * j + 2 * i + 1] = __float_as_uint(__uint_as_float(r[8 * j + 2 * i + 1]) + __uint_as_float(w[i] & 0xffff0000u));
+        }
+      }
+    }
+  }
+};
+
 template <int BN, typename OutT>
 struct ClusterSplitCfg {
   using Base = GemmCfg<2, BN, int(sizeof(OutT))>;
@@ -34,6 +60,7 @@ struct ClusterSplitCfg {
   static constexpr int NUM_BARRIERS = 2 * STAGES + 1;
   static constexpr int SMEM_BYTES = 1024 + STAGES * Base::STAGE_BYTES + NUM_BARRIERS * 8 + 64;
   static constexpr int CHUNKS = BN / 32;
+  static constexpr int OWNED = (CHUNKS + 1) / 2;  // chunks that a pair owns at most: with two slices
   static constexpr int CHUNK_BYTES = 128 * 128;  // 128 rows x 32 columns of f32
   // what the other slices deposit here: at most (slices - 1) * ceil(CHUNKS / slices) chunks
   static_assert(3 * ((CHUNKS + 3) / 4) * CHUNK_BYTES <= STAGES * Base::STAGE_BYTES && 2 * ((CHUNKS + 2) / 3) * CHUNK_BYTES <= STAGES * Base::STAGE_BYTES &&
@@ -162,14 +189,27 @@ mxfp4_gemm_cluster_splitk_kernel(const __grid_constant__ PlainMaps maps, const G
   }
   __syncwarp();
   tc_fence_before_sync();
-  cluster_arrive();  // from here on the rings of all CTAs of the cluster are free
-  cluster_wait();
-  tc_fence_after_sync();
+  cluster_arrive();  // once all have come here the rings of all CTAs of the cluster are free
 
   const int quad = warp & 3;  // tensor-memory lane quadrant (warps 2 .. 5)
   const uint32_t t_acc = tmem_base + (uint32_t(quad * 32) << 16);
   const int lane_row = quad * 32 + lane;
+  const int row = (mt * 2 + int(rank)) * Cfg::BM + lane_row;
   const int per_owner = (Split::CHUNKS + slices - 1) / slices;  // chunks a pair can own
+  // What C holds under this pair's chunks is fetched while the slices are exchanged (whole chunks of 16-byte aligned rows).
+  OldChunk<OutT> old[Split::OWNED];
+  const bool early = p.accumulate && p.vec_ok && row < p.M;
+  if (warp >= 2) {
+    pdl_wait();  // C may still be used by the kernels before this one
+#pragma unroll
+    for (int i = 0; i < Split::OWNED; ++i) {
+      const int c = slice + i * slices, col = nt * BN + c * 32;
+      if (early && c < Split::CHUNKS && col + 32 <= p.N) old[i].load(reinterpret_cast<const OutT*>(p.c) + size_t(row) * p.ldc + col);
+    }
+  }
+  cluster_wait();
+  tc_fence_after_sync();
+
   if (warp >= 2) {
 #pragma unroll 1
     for (int c = 0; c < Split::CHUNKS; ++c) {
@@ -189,12 +229,10 @@ mxfp4_gemm_cluster_splitk_kernel(const __grid_constant__ PlainMaps maps, const G
   cluster_wait();
 
   if (warp >= 2) {
-    pdl_wait();  // C may still be read by the kernels before this one
-    const int row = (mt * 2 + int(rank)) * Cfg::BM + lane_row;
-#pragma unroll 1
-    for (int c = slice; c < Split::CHUNKS; c += slices) {
-      const int col = nt * BN + c * 32;
-      if (col >= p.N) break;
+#pragma unroll
+    for (int i = 0; i < Split::OWNED; ++i) {
+      const int c = slice + i * slices, col = nt * BN + c * 32;
+      if (c >= Split::CHUNKS || col >= p.N) break;
       uint32_t own[32];
       tmem_ld_32x32(t_acc + c * 32, own);
       tmem_ld_wait();
@@ -223,7 +261,8 @@ mxfp4_gemm_cluster_splitk_kernel(const __grid_constant__ PlainMaps maps, const G
       if (row < p.M && WB_CHECK(row >= 0 && col >= 0 && col < p.N, kCheckOutputIndex, (long long)row << 32 | unsigned(col))) {
         OutT* dst = reinterpret_cast<OutT*>(p.c) + size_t(row) * p.ldc + col;
         const int ncols = min(32, p.N - col);
-        if (p.accumulate) add_old_chunk32<OutT>(dst, r, ncols, p.vec_ok != 0);
+        if (early && ncols == 32) old[i].add_to(r);
+        else if (p.accumulate) add_old_chunk32<OutT>(dst, r, ncols, p.vec_ok != 0);
         store_chunk32<OutT>(dst, r, ncols, p.vec_ok != 0);
       }
     }
