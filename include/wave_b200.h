@@ -63,7 +63,11 @@ extern "C" {
                                      (barriers, tensor-memory allocation, descriptor prefetch) does, and every load
                                      waits for the preceding kernel. Everything else (a, scales of a, c, workspace) is
                                      touched only after the preceding kernel has completed. Back-to-back GEMMs of a
-                                     decode loop overlap their tails and heads this way. */
+                                     decode loop overlap their tails and heads this way. (Without the flag the first
+                                     kernel of a call may also become resident beside the kernel before it, but waits for
+                                     that kernel's completion before it touches memory: the order of the stream holds.
+                                     A preceding kernel that is a programmatic launch itself has to execute
+                                     griddepcontrol.wait for what it depends on.) */
 /* Tile order of the tile paths: output tiles are visited in groups of g N tiles (256 columns each, 128 / 192 with the
  * narrower tiles), each group swept down M with N fastest, so that the CTAs running at one time share few b tiles
  * and all of a group's a tiles in L2. This is the templates' `reorder_workgroups` / `group_size_n` pair
@@ -178,7 +182,7 @@ int wb200_quantize_mxfp4(const void* x, int x_dtype, long long ldx, int rows, in
 /* wb200_quantize_mxfp4 and wb200_mxfp4_gemm in one call, the GEMM launched as the programmatic dependent of the
  * quantiser: x [M, K] (f32 or bf16) is quantised to q_scratch [M, K/2] and scale_scratch
  * (wb200_packed_scale_bytes(M, K)), both 16-byte aligned, and the GEMM's set-up, and on the M <= 128 path its first ring of weight loads, run
- * while the quantiser does (an ordinary launch for M > 128 where rows of c are not 16-byte aligned). Other arguments as wb200_mxfp4_gemm; WB200_OVERLAP_PREVIOUS is refused. */
+ * while the quantiser does (after it for M > 128 where rows of c are not 16-byte aligned). Other arguments as wb200_mxfp4_gemm; WB200_OVERLAP_PREVIOUS is refused. */
 int wb200_mxfp4_gemm_quantize_a(int M, int N, int K, const void* x, int x_dtype, long long ldx, void* q_scratch, void* scale_scratch,
                                 const void* b, const void* b_scale_packed, void* c, int c_dtype, long long ldc, void* workspace,
                                 size_t workspace_bytes, unsigned flags, void* stream);
@@ -223,7 +227,7 @@ int wb200_silu_and_mul(const void* x1, const void* x2, long long ld1, long long 
                        long long ldo, void* q, void* scale_rowmajor, void* scale_packed, const int* num_rows, void* stream);
 
 /* The whole expert MLP on device-side routing: out[t] = sum_j w_j * down_e(silu(gate_e(x_t)) * up_e(x_t)) over the top_k
- * experts of token t, w = softmax(logits) in f32 (tests/kernel/moe_test.py:105-127). Six launches on `stream`, each the
+ * experts of token t, w = softmax(logits) in f32 (tests/kernel/moe_test.py:105-127). Five launches on `stream` (four up to 128 tokens), each the
  * programmatic dependent of the one before; nothing is read on the host. x [T, K] and logits [T, E] are f32 or bf16
  * (pitches in elements, x rows 16-byte aligned), out [T, N] bf16. w1[e]: packed E2M1 [2 inter, K/2], gate rows then up
  * rows; w2[e]: [N, inter/2]; w1_scale / w2_scale: their scales from wb200_repack_scales (HOST arrays of device
