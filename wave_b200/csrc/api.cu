@@ -1444,8 +1444,8 @@ static int quantize_mxfp4_impl(const void* x, int x_dtype, long long ldx, int ro
   bool beside = blocks <= 8u * unsigned(dev->sm_count);
   if (beside && blocks > unsigned(dev->sm_count)) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    WB_CUDA(cudaStreamIsCapturing(s, &status));
-    beside = status == cudaStreamCaptureStatusNone;
+    beside = cudaStreamIsCapturing(s, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
+    if (!beside) (void)cudaGetLastError();  // (the legacy stream beside another one's capture: the launch itself will say so)
   }
   if (x_dtype == WB200_F32)
     WB_CUDA(launch_kernel(beside, wb::quantize_mxfp4_kernel<float>, blocks, 256, s, static_cast<const float*>(x), ldx, rows, K, static_cast<uint8_t*>(q),
