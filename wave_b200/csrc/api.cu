@@ -1352,7 +1352,9 @@ static int repack_scales_impl(const void* src, long long src_row_stride, int row
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  // Beside the tail of the kernel before it up to one CTA per SM: the GEMM behind a larger one runs for 100 us and more under the power
+  // limit, where the gap costs nothing (8192^3 in a loop, ordinary / programmatic: 213.2 / 215.9 us).
+  cfg.numAttrs = tl_dependent_launch || grid.x * grid.y <= unsigned(dev->sm_count) ? 1 : 0;
   WB_CUDA(cudaLaunchKernelEx(&cfg, wb::repack_scales_kernel, static_cast<const uint8_t*>(src), src_row_stride, rows, K / 32,
                              k_atoms, static_cast<uint8_t*>(dst), broadcast, tl_dependent_launch, block_rows));
   return WB200_OK;
