@@ -1685,3 +1685,51 @@ def test_calls_see_what_the_kernel_before_them_wrote(captured):
         for u, v in zip(a, b):
             assert torch.equal(u, v)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("kind,M,N,K", [("linear", 8, 640, 512), ("fp4", 16, 1024, 512), ("fp4", 256, 512, 4096), ("fp8", 16, 1024, 512), ("mixed", 16, 1024, 512)])
+def test_a_capture_takes_the_memory_of_the_eager_call_before_it(kind, M, N, K, monkeypatch):
+    """A layer or kernel object called on S, then on T, then again on S, and captured: the graph holds the workspace and the scratch of S,
+    although the last call on S was recognised in native code. (At 256 rows the split-K workspace, which eager calls only ask for.)"""
+    monkeypatch.setattr(ops, "_pool", ops.WorkspacePool())
+    g = torch.Generator().manual_seed(1)
+    x, w = torch.randn(M, K, generator=g).to(DEV), (torch.randn(N, K, generator=g) * 0.02).to(DEV)
+    if kind == "linear":
+        layer = wb.MXFP4Linear.from_float(w)
+        call, pool = (lambda: layer(x)), ops._pool
+    else:
+        if kind == "fp4":
+            t, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+            args = [*ops.quantize_mxfp4(x)[:2], *ops.quantize_mxfp4(w)[:2]]
+        else:
+            t, subs = wb.get_scaled_gemm_mxfp8_kernel((M, N, K), wb.ScaledMMAType.F32_16x16x128_F8F6F4, "f8e4m3fn", wb.bf16,
+                                                      weight_format="f4e2m1fn" if kind == "mixed" else None)
+            options = wb.WaveCompileOptions(subs=subs)
+            args = [*ops.quantize_mxfp8(x, torch.float8_e4m3fn)[:2], *(ops.quantize_mxfp4(w) if kind == "mixed" else ops.quantize_mxfp8(w, torch.float8_e4m3fn))[:2]]
+        gemm = wb.wave_compile(wb.set_default_run_config(options), t)
+        c = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        call, pool = (lambda: (gemm(*args, c), c)[1]), gemm._workspaces if kind == "fp4" else ops._pool
+    S, T, C = (torch.cuda.Stream(DEV) for _ in range(3))
+    torch.cuda.synchronize()
+    for st in (S, S, T, T, S):
+        with torch.cuda.stream(st):
+            ref = call().clone()
+        torch.cuda.synchronize()
+    captured = []
+    get = ops.WorkspacePool.get
+    monkeypatch.setattr(ops.WorkspacePool, "get", lambda *a: (captured.append(get(*a)), captured[-1])[1])
+    if kind != "linear":
+        scratch = gemm._a_scale_buffer
+        monkeypatch.setattr(gemm, "_a_scale_buffer", lambda *a: (captured.append(scratch(*a)), captured[-1])[1])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=C):
+        out = call()
+    of_s = {pool._by_key[0, S.cuda_stream, "skinny" if M <= 128 else "splitk"].data_ptr()}
+    if kind != "linear":
+        of_s.add(gemm._a_scale_buf[0, S.cuda_stream][-1].data_ptr())
+    assert {t.data_ptr() for t in captured} == of_s
+    graph.replay()
+    torch.cuda.synchronize()
+    if M <= 128:  # (above, a captured call cuts K where an eager one does not)
+        assert torch.equal(out, ref)
+    ops.check_device_status()

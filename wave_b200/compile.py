@@ -120,7 +120,7 @@ class ScaledGemmKernel:
         self.asm = ""  # the reference exposes generated code here; nothing is generated at run time
         self._weight_scales = ops.WeightScaleCache()
         self._a_scale_buf: dict[tuple[int, int], list[torch.Tensor]] = {}  # (device, stream) -> scratches, the one in use last
-        self._a_scale_last: dict[int, tuple[int, int]] = {}  # device -> key of the scratch that was asked for last
+        self._a_scale_last: dict[int, list] = {}  # device -> [key] of the eager call before; native calls write the element too
         self._workspaces = ops.WorkspacePool()  # this object's own: calls through another object may overlap with these
         self._plans: dict = {}
         self._tile_rows: dict = {}
@@ -162,7 +162,7 @@ class ScaledGemmKernel:
         return self._invoke_checked(a, a_scale, b, b_scale, c)
 
     def _launch(self, plan, a, a_scale, b, b_scale, c) -> None:
-        M, N, K, a_buf, ws_ptr, ws_bytes, flags, dtype_code, dev_index, _ws_keepalive = plan
+        M, N, K, a_buf, ws_ptr, ws_bytes, flags, dtype_code, dev_index, _ws_keepalive, marks = plan
         if M > 128 and ws_bytes and not ops.split_k_pays() and (flags & _lib.PATH_MASK) != _lib.PATH_TILE_SPLITK:
             ws_ptr = ws_bytes = 0  # eager call: stay on the plain tile path (see ops.split_k_pays)
         tile_rows = self._weight_tile_rows(M, N, K, c, dev_index)
@@ -186,14 +186,21 @@ class ScaledGemmKernel:
         if rc:
             _lib.check(rc)
         flags = plan[6] | (_lib.B_TILE_ROWS(tile_rows) if tile_rows != 128 else 0)
-        self._remember(a, a_scale, b, b_scale, c, (M, N, K, -1, flags, tile_rows, ws_bytes), b_sf, a_buf, _ws_keepalive if ws_bytes else None)
+        self._remember(a, a_scale, b, b_scale, c, (M, N, K, -1, flags, tile_rows, ws_bytes), b_sf, a_buf, _ws_keepalive if ws_bytes else None, marks)
 
-    def _remember(self, a, a_scale, b, b_scale, c, sizes, b_sf, scratch, workspace) -> None:
-        """A call that went through: the next one with such tensors is recognised by the native module. Not under capture, where every
-        call takes the memory of its own warm-up."""
+    def _remember(self, a, a_scale, b, b_scale, c, sizes, b_sf, scratch, workspace, marks) -> None:
+        """A call that went through: the next one with such tensors is recognised by the native module, which notes whose scratch and
+        workspace it used as this one does (`marks`). Not under capture, where every call takes the memory of its own warm-up."""
         if not torch.cuda.is_current_stream_capturing():
+            for holder, value in marks:
+                holder[0] = value
             self._fast.add(a, a_scale, b, b_scale, c, self.options.decode_tiled_weight_scales, self.options.kernel_path, sizes, b_sf.data, scratch,
-                           workspace)
+                           workspace, marks)
+
+    def _marks(self, idx: int, pool=None, kind: str = "skinny") -> tuple:
+        """What notes that the eager call before used the scratch, and with a pool the workspace, that were asked for just now."""
+        holder = self._a_scale_last[idx]
+        return ((holder, holder[0]),) + ((pool.mark(idx, kind),) if pool is not None else ())
 
     def _invoke_mxfp8(self, a, a_scale, b, b_scale, c) -> None:
         t = self.template
@@ -231,13 +238,17 @@ class ScaledGemmKernel:
         flags = self.options.kernel_path | self._raster_flags() | (_lib.ACCUMULATE if t.accumulate else 0)
         ops.scaled_gemm_mxfp8_packed(a, a_sf, b, b_sf, c, fmt, flags, b_fp4=b_fp4, a_scale=rowmajor)
         if rowmajor is a_scale and given[0] is a and given[1] is b and not isinstance(b_scale, ops.PackedScales):
-            ws, ws_bytes = None, 0
+            if torch.cuda.is_current_stream_capturing():
+                return
+            ws, ws_bytes, pool = None, 0, None
             if M <= 128:
-                ws_bytes = int(self._lib.wb200_mxfp4_gemm_workspace_bytes(M, N, K))
+                ws_bytes, pool = int(self._lib.wb200_mxfp4_gemm_workspace_bytes(M, N, K)), ops._pool
                 ws = ops._workspace(a.device, ws_bytes, "skinny")
             if b_sf.tile_rows != 128:
                 flags |= _lib.B_TILE_ROWS(b_sf.tile_rows)
-            self._remember(a, a_scale, b, b_scale, c, (M, N, K, fmt | (_lib.B_FP4 if b_fp4 else 0), flags, b_sf.tile_rows, ws_bytes), b_sf, a_sf.data, ws)
+            idx = a.device.index if a.device.index is not None else torch.cuda.current_device()
+            self._remember(a, a_scale, b, b_scale, c, (M, N, K, fmt | (_lib.B_FP4 if b_fp4 else 0), flags, b_sf.tile_rows, ws_bytes), b_sf, a_sf.data, ws,
+                           self._marks(idx, pool))
 
     def _invoke_checked(self, a, a_scale, b, b_scale, c) -> None:
         t = self.template
@@ -288,15 +299,18 @@ class ScaledGemmKernel:
             ws_bytes = ws_ptr = 0
             ws = None  # the plan keeps the workspace tensor alive: it holds its address
             ws_bytes = int(self._lib.wb200_mxfp4_gemm_workspace_bytes(M, N, K))
+            kind = "skinny" if M <= 128 else "splitk"
             if ws_bytes:
-                ws = ops._workspace(a.device, ws_bytes, "skinny" if M <= 128 else "splitk", self._workspaces)
+                ws = ops._workspace(a.device, ws_bytes, kind, self._workspaces)
                 ws_ptr = ws.data_ptr()
             idx = a.device.index if a.device.index is not None else torch.cuda.current_device()
             a_buf = self._a_scale_buffer(a.device, M, K)
-            plan = (M, N, K, a_buf, ws_ptr, ws_bytes, flags, ops._DTYPE_CODE[c.dtype], idx, ws)
+            capturing = torch.cuda.is_current_stream_capturing()
+            marks = () if capturing else self._marks(idx, self._workspaces if ws_bytes else None, kind)
+            plan = (M, N, K, a_buf, ws_ptr, ws_bytes, flags, ops._DTYPE_CODE[c.dtype], idx, ws, marks)
             sig = (a.shape, a.stride(), a.dtype, a_scale.shape, a_scale.stride(), b.shape, b.stride(), b_scale.shape,
                    c.shape, c.stride(), c.dtype, a.device, torch.cuda.current_stream(a.device).cuda_stream)
-            if not torch.cuda.is_current_stream_capturing():  # (every capture takes the memory of its own warm-up)
+            if not capturing:  # (every capture takes the memory of its own warm-up)
                 self._plans[sig] = plan
             return self._launch(plan, a, a_scale, b, b_scale, c)
         a_sf = self._pack_activation_scales(a_scale, M, K)
@@ -395,14 +409,16 @@ class ScaledGemmKernel:
         need = ops.packed_scale_bytes(M, K)
         key = (idx, torch.cuda.current_stream(idx).cuda_stream)
         bufs = self._a_scale_buf.get(key)
+        capturing = torch.cuda.is_current_stream_capturing()
         if bufs is None or bufs[-1].numel() < need:
-            last = self._a_scale_buf.get(self._a_scale_last.get(idx))
-            if last is not None and last[-1].numel() >= need and torch.cuda.is_current_stream_capturing():
+            last = self._a_scale_buf.get(self._a_scale_last.get(idx, [None])[0])
+            if capturing and last is not None and last[-1].numel() >= need:
                 return last[-1]
             size = max(need, 2 * bufs[-1].numel()) if bufs else need
             bufs = self._a_scale_buf.setdefault(key, [])
             bufs.append(torch.empty(size, dtype=torch.uint8, device=device))
-        self._a_scale_last[idx] = key
+        if not capturing:
+            self._a_scale_last.setdefault(idx, [None])[0] = key
         return bufs[-1]
 
     def _pack_activation_scales(self, a_scale, M, K):

@@ -10,7 +10,8 @@
 // What is kept: per kernel object, the signatures (sizes, strides, types, device, stream, alignment of the output) of at most
 // kMaxPlans calls with their scratch, and at most kMaxWeights packings of weight scales, each found by the tensor it was made from
 // (a weak reference), its version counter and its address, as WeightScaleCache does. Nothing about activations or outputs
-// is kept but their shapes. Calls under stream capture, on another device than the current one, with tensor subclasses, under
+// is kept but their shapes. A call notes whose scratch and workspace it used where the Python code notes it (`marks`): a captured call takes the
+// memory of the eager call before it. Calls under stream capture, on another device than the current one, with tensor subclasses, under
 // functional transforms, or with inference tensors are left to the Python code.
 // us per call, calls back to back: 1024^3 f32 16.9 -> 8.2 (the GPU's time now), MXFP4Linear 8 x 14336 x 4096 26.8 -> 15.6.
 #define PY_SSIZE_T_CLEAN
@@ -42,6 +43,25 @@ struct Abi {
   size_t (*gemm_workspace_bytes)(int, int, int);
   int (*decode_tile_rows_for)(int, int, int, int, int, int);
 } abi;
+
+// A reference to a Python object; copied and dropped with the interpreter lock held.
+struct Ref {
+  PyObject* o = nullptr;
+  Ref() = default;
+  explicit Ref(PyObject* p) : o(p) { Py_XINCREF(o); }
+  Ref(const Ref& r) : Ref(r.o) {}
+  Ref(Ref&& r) noexcept : o(r.o) { r.o = nullptr; }
+  Ref& operator=(Ref r) noexcept {
+    std::swap(o, r.o);
+    return *this;
+  }
+  ~Ref() { Py_XDECREF(o); }
+};
+// A mark is a pair (list of one element, value): setting it makes the value the list's element.
+bool is_mark(PyObject* m) {
+  return PyTuple_Check(m) && PyTuple_GET_SIZE(m) == 2 && PyList_Check(PyTuple_GET_ITEM(m, 0)) && PyList_GET_SIZE(PyTuple_GET_ITEM(m, 0)) == 1;
+}
+void set_mark(PyObject* m) { PyList_SetItem(PyTuple_GET_ITEM(m, 0), 0, Py_NewRef(PyTuple_GET_ITEM(m, 1))); }
 
 // An ordinary CUDA tensor: no subclass, no wrapper of a functional transform, no inference tensor.
 bool plain(PyObject* o) {
@@ -93,6 +113,7 @@ struct Plan {
   at::Tensor scratch, workspace;  // packed activation scales; workspace (undefined: none)
   size_t workspace_bytes;
   int tile_rows;
+  Ref marks;  // a tuple of marks
 };
 struct Weight {
   c10::weak_intrusive_ptr<c10::TensorImpl> owner;
@@ -179,6 +200,7 @@ PyObject* calls_call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     const int c_type = key.sig[4].type == at::kFloat ? kF32 : kBF16;
     const long long a_scale_stride = M > 1 ? key.sig[1].stride[0] : K / 32, ldc = M > 1 ? key.sig[4].stride[0] : N;
     void* ws = workspace.defined() ? workspace.data_ptr() : nullptr;
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(found->marks.o); ++i) set_mark(PyTuple_GET_ITEM(found->marks.o, i));
     int rc;
     Py_BEGIN_ALLOW_THREADS
     if (elem_format < 0)
@@ -194,11 +216,13 @@ PyObject* calls_call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
   }
 }
 
-// add(a, a_scale, b, b_scale, c, tiled, path, (M, N, K, elem_format, flags, tile_rows, workspace_bytes), packed, scratch, workspace or None):
+// add(a, a_scale, b, b_scale, c, tiled, path, (M, N, K, elem_format, flags, tile_rows, workspace_bytes), packed, scratch, workspace or None, marks):
 // the Python code has just made this call with these arguments.
 PyObject* calls_add(PyObject* self, PyObject* const* args, Py_ssize_t n) {
-  if (n != 11) {
-    PyErr_SetString(PyExc_TypeError, "add takes 11 arguments");
+  bool marks_ok = n == 12 && PyTuple_Check(args[11]);
+  for (Py_ssize_t i = 0; marks_ok && i < PyTuple_GET_SIZE(args[11]); ++i) marks_ok = is_mark(PyTuple_GET_ITEM(args[11], i));
+  if (!marks_ok) {
+    PyErr_SetString(PyExc_TypeError, "add takes 12 arguments, the last one a tuple of (list of one element, value) pairs");
     return nullptr;
   }
   try {
@@ -215,6 +239,7 @@ PyObject* calls_add(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     p.scratch = THPVariable_Unpack(args[9]);
     if (args[10] != Py_None) p.workspace = THPVariable_Unpack(args[10]);
     p.workspace_bytes = size_t(ws_bytes);
+    p.marks = Ref(args[11]);
     if (const Plan* old = calls.find(p.key)) {
       const_cast<Plan&>(*old) = p;
     } else if (calls.plans.size() < kMaxPlans) {
@@ -254,6 +279,7 @@ struct Workspaces {
     int device;
     cudaStream_t stream;
     at::Tensor ws;
+    Ref mark;
   };
   std::vector<Entry> entries;
 };
@@ -261,10 +287,10 @@ struct PyWorkspaces {
   PyObject_HEAD
   Workspaces* table;
 };
-// put(device, stream, workspace)
+// put(device, stream, workspace, mark)
 PyObject* workspaces_put(PyObject* self, PyObject* const* args, Py_ssize_t n) {
-  if (n != 3 || !THPVariable_Check(args[2])) {
-    PyErr_SetString(PyExc_TypeError, "put takes a device index, a stream and a tensor");
+  if (n != 4 || !THPVariable_Check(args[2]) || !is_mark(args[3])) {
+    PyErr_SetString(PyExc_TypeError, "put takes a device index, a stream, a tensor and a (list of one element, value) pair");
     return nullptr;
   }
   const int device = int(PyLong_AsLong(args[0]));
@@ -274,9 +300,10 @@ PyObject* workspaces_put(PyObject* self, PyObject* const* args, Py_ssize_t n) {
   for (auto& e : entries)
     if (e.device == device && e.stream == stream) {
       e.ws = THPVariable_Unpack(args[2]);
+      e.mark = Ref(args[3]);
       Py_RETURN_NONE;
     }
-  entries.push_back({device, stream, THPVariable_Unpack(args[2])});
+  entries.push_back({device, stream, THPVariable_Unpack(args[2]), Ref(args[3])});
   Py_RETURN_NONE;
 }
 PyObject* workspaces_clear(PyObject* self, PyObject*) {
@@ -321,11 +348,15 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) Py_RETURN_NONE;
     const auto stream = c10::cuda::getCurrentCUDAStream(device);
     at::Tensor ws;
+    Ref mark;
     size_t ws_bytes = 0;
     if (M <= 128) {
       ws_bytes = abi.gemm_workspace_bytes(int(M), int(N), int(K));
       for (const auto& e : reinterpret_cast<PyWorkspaces*>(args[6])->table->entries)
-        if (e.device == device && e.stream == stream.stream()) ws = e.ws;
+        if (e.device == device && e.stream == stream.stream()) {
+          ws = e.ws;
+          mark = e.mark;
+        }
       if (!ws.defined() || size_t(ws.numel()) < ws_bytes) Py_RETURN_NONE;
     }
     // (a fresh output starts on 16 bytes: its rows are aligned when N says so)
@@ -345,6 +376,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const int64_t q_bytes = (M * K / 2 + 255) / 256 * 256;
     const at::Tensor scratch = at::detail::empty_cuda({q_bytes + (M + 127) / 128 * ((K + 255) / 256) * 1024}, at::kByte, x.device(), c10::nullopt);
     uint8_t* q = static_cast<uint8_t*>(scratch.data_ptr());
+    if (mark.o) set_mark(mark.o);
     const unsigned flags = tile_rows == 128 ? 0u : unsigned(tile_rows / 8) << 16;  // WB200_B_TILE_ROWS
     int rc;
     Py_BEGIN_ALLOW_THREADS

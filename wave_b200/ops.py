@@ -164,7 +164,7 @@ class WorkspacePool:
 
     def __init__(self):
         self._by_key: dict = {}
-        self._last: dict = {}  # (device, kind) -> key of the workspace that was asked for last
+        self._last: dict = {}  # (device, kind) -> [(key, workspace)] of the eager call before; native calls write the element too
         self._outgrown: list = []
         self._fast = None  # the "skinny" ones of eager calls, for the native linear call
 
@@ -180,14 +180,13 @@ class WorkspacePool:
         key = (idx, torch.cuda.current_stream(idx).cuda_stream, kind)
         ws = self._by_key.get(key)
         if ws is not None and ws.numel() >= nbytes:
-            self._last[idx, kind] = key
-            if kind == "skinny" and not capturing:
-                self.fast.put(idx, key[1], ws)
+            if not capturing:
+                self._note(key, ws)
             return ws
         if capturing:
-            last = self._by_key.get(self._last.get((idx, kind)))
-            for w in ([] if last is None else [last]) + [w for (d, _, k), w in self._by_key.items() if d == idx and k == kind]:
-                if w.numel() >= nbytes:
+            last_key, last = self._last.get((idx, kind), [None])[0] or (None, None)
+            for w in [self._by_key.get(last_key), last] + [w for (d, _, k), w in self._by_key.items() if d == idx and k == kind]:
+                if w is not None and w.numel() >= nbytes:
                     return w
             raise RuntimeError("this GEMM needs a workspace, which cannot be created while a CUDA graph is being captured: "
                                "call it once eagerly (with the same shapes) before the capture")
@@ -198,14 +197,24 @@ class WorkspacePool:
         with torch.cuda.device(idx):
             _lib.check(_lib.load().wb200_workspace_init(ws.data_ptr(), nbytes, _stream()))
         self._by_key[key] = ws
-        self._last[idx, kind] = key
-        if kind == "skinny":
-            self.fast.put(idx, key[1], ws)
+        self._note(key, ws)
         return ws
+
+    def _note(self, key, ws: torch.Tensor) -> None:
+        idx, stream, kind = key
+        self._last.setdefault((idx, kind), [None])[0] = (key, ws)
+        if kind == "skinny":
+            self.fast.put(idx, stream, ws, self.mark(idx, kind))
+
+    def mark(self, idx: int, kind: str) -> tuple:
+        """(list, value): storing the value as the list's element says that the eager call before used what it used just now."""
+        holder = self._last[idx, kind]
+        return holder, holder[0]
 
     def clear(self) -> None:
         self._by_key.clear()
-        self._last.clear()
+        for holder in self._last.values():
+            holder[0] = None
         self._outgrown.clear()
         if self._fast is not None:
             self._fast.clear()
