@@ -1733,3 +1733,43 @@ def test_a_capture_takes_the_memory_of_the_eager_call_before_it(kind, M, N, K, m
     if M <= 128:  # (above, a captured call cuts K where an eager one does not)
         assert torch.equal(out, ref)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("N,K", [(14336, 512), (4096, 1024), (28672, 256)])
+def test_first_decode_calls_of_a_linear_layer_on_two_streams(N, K):
+    """The first decode call of a layer stands behind queued work of its stream, the second one runs on another stream at once: both read
+    packings that were complete before. Bits of a layer that is alone."""
+    g = torch.Generator().manual_seed(N)
+    w, x = (torch.randn(N, K, generator=g) * 0.02).to(DEV), torch.randn(8, K, generator=g).to(DEV)
+    ref = wb.MXFP4Linear.from_float(w)(x)
+    layer = wb.MXFP4Linear.from_float(w)
+    blocks = [torch.full((ops.packed_scale_bytes(148 * 128, K),), 255, dtype=torch.uint8, device=DEV) for _ in range(4)]
+    S, T = torch.cuda.Stream(DEV), torch.cuda.Stream(DEV)
+    torch.cuda.synchronize()
+    del blocks
+    outs = []
+    with torch.cuda.stream(S):
+        torch.cuda._sleep(20_000_000)  # ~10 ms
+        outs.append(layer(x))
+    with torch.cuda.stream(T):
+        outs += [layer(x), layer(x)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, ref) for y in outs)
+    ops.check_device_status()
+
+
+def test_linear_layer_packs_its_scales_for_every_decode_batch_and_anew_from_a_state_dict():
+    from types import SimpleNamespace
+    for N in (8, 130, 1000, 4096, 4097, 5803, 11008, 14336, 17800, 18900, 18944, 19072, 20480, 20483, 28672, 37888):
+        for K in (32, 1024, 2080, 4096, 5376, 8192, 14336, 28672):
+            for dtype in (torch.bfloat16, torch.float32):
+                heights = {ops.decode_tile_rows_for(M, N, K, DEV, c_aligned=M == 1 or N * dtype.itemsize % 16 == 0) for M in range(1, 129)} - {128}
+                layer = SimpleNamespace(out_features=N, in_features=K, output_dtype=dtype, weight_scales=torch.empty(0, device=DEV))
+                assert len(heights) <= 1 and wb.MXFP4Linear._low_rows(layer) == min(heights, default=128)
+    g = torch.Generator().manual_seed(4)
+    one, two = (wb.MXFP4Linear.from_float((torch.randn(4096, 512, generator=g) * 0.02).to(DEV)) for _ in range(2))
+    xs = [torch.randn(m, 512, generator=g).to(DEV) for m in (4, 300)]
+    refs = [two(x) for x in xs]
+    assert two._packed_low is not None and not torch.equal(one(xs[0]), refs[0])
+    one.load_state_dict(two.state_dict())
+    assert all(torch.equal(one(x), r) for x, r in zip(xs, refs))

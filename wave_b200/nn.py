@@ -16,7 +16,8 @@ from .lang import as_output_dtype
 
 class MXFP4Linear(torch.nn.Module):
     def __init__(self, weight_codes: torch.Tensor, weight_scales: torch.Tensor, output_dtype=torch.bfloat16):
-        """weight_codes [N, K/2] uint8, weight_scales [N, K/32] uint8 (row-major E8M0), both on the GPU."""
+        """weight_codes [N, K/2] uint8, weight_scales [N, K/32] uint8 (row-major E8M0), both on the GPU. The GEMM reads the scales in
+        packings that are made here, on the current stream, and anew when a state dict is loaded."""
         super().__init__()
         ops._as_u8(weight_codes, "weight_codes")
         self.out_features, half_k = weight_codes.shape
@@ -24,11 +25,33 @@ class MXFP4Linear(torch.nn.Module):
         self.output_dtype = as_output_dtype(output_dtype).torch_dtype
         self.register_buffer("weight_codes", weight_codes.contiguous())
         self.register_buffer("weight_scales", weight_scales.contiguous())
-        self._packed = ops.repack_scales(self.weight_scales)  # once
+        self._pack()
 
-    # Decode calls (at most 128 rows) may read a second packing, per tile of the height that gives every SM the same number of
-    # weight tiles (one height per layer: it follows from out_features); made when `ops.decode_tile_rows_for` first names it.
+    # Decode calls (at most 128 rows) may read a second packing, per tile of the height h that gives every SM the same number of
+    # weight tiles: one height per layer, as it follows from out_features, and 128 / h times the bytes of the usual packing. Made with that one, not
+    # by the first call that reads it: other streams' calls would have to wait for that call's.
     _packed_low = None
+
+    def _pack(self) -> None:
+        self._packed = ops.repack_scales(self.weight_scales)
+        h = self._low_rows()
+        self._packed_low = None if h == 128 else ops.repack_scales(self.weight_scales, tile_rows=h)
+
+    def _low_rows(self) -> int:
+        """The height that decode calls of some number of rows read, 128 where none does. (One of each class that
+        `ops.decode_tile_rows_for` tells apart: by rows, and by whether rows of the output start on 16 bytes, as that of one row does.)"""
+        N, K, device = self.out_features, self.in_features, self.weight_scales.device
+        aligned = N * self.output_dtype.itemsize % 16 == 0
+        for rows, c_aligned in ((1, True), (2, aligned), (32, aligned), (64, aligned), (128, aligned)):
+            h = ops.decode_tile_rows_for(rows, N, K, device, c_aligned=c_aligned)
+            if h != 128:
+                return h
+        return 128
+
+    def _load_from_state_dict(self, *args, **kwargs) -> None:
+        super()._load_from_state_dict(*args, **kwargs)
+        if self.weight_scales is not None and self.weight_scales.is_cuda:
+            self._pack()
 
     @property
     def _packed_decode(self) -> ops.PackedScales:
@@ -62,11 +85,8 @@ class MXFP4Linear(torch.nn.Module):
         return out.reshape(*lead, self.out_features)
 
     def _decode_packing(self, out: torch.Tensor) -> ops.PackedScales:
-        h = ops.decode_tile_rows_for(out.shape[0], self.out_features, self.in_features, out.device, c_aligned=ops.rows_aligned(out))
-        if h == 128:
+        low = self._packed_low
+        if low is None:
             return self._packed
-        if self._packed_low is None:
-            if torch.cuda.is_current_stream_capturing():
-                return self._packed  # (a packing made by a captured call holds nothing before the first replay)
-            self._packed_low = ops.repack_scales(self.weight_scales, tile_rows=h)
-        return self._packed_low
+        h = ops.decode_tile_rows_for(out.shape[0], self.out_features, self.in_features, out.device, c_aligned=ops.rows_aligned(out))
+        return low if h == low.tile_rows else self._packed
