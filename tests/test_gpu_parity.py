@@ -1773,3 +1773,106 @@ def test_linear_layer_packs_its_scales_for_every_decode_batch_and_anew_from_a_st
     assert two._packed_low is not None and not torch.equal(one(xs[0]), refs[0])
     one.load_state_dict(two.state_dict())
     assert all(torch.equal(one(x), r) for x, r in zip(xs, refs))
+
+
+def _two_stream_problem(n, M=8, N=2048, K=1024):
+    """A kernel object, `n` weights (operands behind c), and the outputs of fresh kernel objects."""
+    t, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    compiled = lambda: wb.wave_compile(wb.set_default_run_config(options), t)  # noqa: E731
+    probs = [[x.to(DEV) for x in random_problem(M, N, K, seed=60 + i)] for i in range(n)]
+    refs = [torch.empty(M, N, dtype=torch.bfloat16, device=DEV) for _ in probs]
+    for p, c in zip(probs, refs):
+        compiled()(*p, c)
+    blocks = [torch.full((ops.packed_scale_bytes(148 * 128, K),), 255, dtype=torch.uint8, device=DEV) for _ in range(8)]
+    torch.cuda.synchronize()
+    del blocks  # what is allocated next holds no scales
+    return compiled(), probs, refs
+
+
+def test_weight_scales_packed_on_one_stream_are_waited_for_on_another():
+    """Both streams know the call. A weight's first call stands behind queued work of S; calls with that weight on T come at once, one of them while S's
+    call is already one that native code recognises."""
+    gemm, probs, refs = _two_stream_problem(3)
+    S, T = torch.cuda.Stream(DEV), torch.cuda.Stream(DEV)
+    outs = []
+
+    def run(i, stream):
+        with torch.cuda.stream(stream):
+            c = torch.full_like(refs[i], float("nan"))
+            gemm(*probs[i], c)
+        outs.append((c, refs[i]))
+
+    for stream in (S, T):
+        run(0, stream)
+        torch.cuda.synchronize()
+    for i in (1, 2):
+        with torch.cuda.stream(S):
+            torch.cuda._sleep(20_000_000)  # ~10 ms
+        for stream in (S, T, T) if i == 1 else (S, S, T, S, T):
+            run(i, stream)
+        torch.cuda.synchronize()
+    for i in (1, 2):
+        for _ in range(2):
+            run(i, T)
+    torch.cuda.synchronize()
+    assert all(torch.equal(c, ref) for c, ref in outs)
+    ops.check_device_status()
+
+
+def test_packed_weight_scales_outlive_calls_of_another_stream():
+    """A packing is dropped while a call of another stream that reads it is still queued: the memory goes to nobody on the stream it was made on."""
+    gemm, probs, refs = _two_stream_problem(1)
+    S, T = torch.cuda.Stream(DEV), torch.cuda.Stream(DEV)
+    for stream in (S, T, T):
+        with torch.cuda.stream(stream):
+            gemm(*probs[0], torch.empty_like(refs[0]))
+        torch.cuda.synchronize()
+    outs = [torch.empty_like(refs[0]) for _ in range(2)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(T):
+        torch.cuda._sleep(20_000_000)
+        for c in outs:
+            gemm(*probs[0], c)
+    sizes = {p.data.numel() for _, p in gemm._weight_scales._entries.values()}
+    gemm.drop_cached_weights()
+    with torch.cuda.stream(S):
+        blocks = [torch.full((n,), 255, dtype=torch.uint8, device=DEV) for n in sizes for _ in range(8)]
+    torch.cuda.synchronize()
+    assert len(blocks) and all(torch.equal(c, refs[0]) for c in outs)
+
+
+def test_a_capture_while_weight_scales_are_being_packed():
+    """Captured while the packing of its weight is still queued on another stream: the graph waits for nothing outside itself, so it packs
+    the scales itself. Once the packing is complete, a capture takes it."""
+    gemm, probs, refs = _two_stream_problem(2)
+    S, C = torch.cuda.Stream(DEV), torch.cuda.Stream(DEV)
+    with torch.cuda.stream(S):
+        gemm(*probs[0], torch.empty_like(refs[0]))
+    torch.cuda.synchronize()
+    packings = []
+    for complete in (False, True):
+        with torch.cuda.stream(S):
+            if not complete:
+                torch.cuda._sleep(200_000_000)  # ~0.1 s
+                gemm(*probs[1], torch.empty_like(refs[1]))
+                behind = torch.cuda.Event()
+                behind.record()
+        before, c = gemm._weight_scales.packings, torch.full_like(refs[1], float("nan"))
+        C.wait_stream(torch.cuda.current_stream())
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(C):
+            graph.capture_begin()
+            gemm(*probs[1], c)
+            graph.capture_end()
+            packings.append(gemm._weight_scales.packings - before)
+            if complete:
+                graph.replay()
+            else:
+                pending = not behind.query()  # (otherwise this machine took its time, and nothing was pending any more)
+        torch.cuda.synchronize()
+        if not complete:  # (its scratch is that of the call on S)
+            graph.replay()
+            torch.cuda.synchronize()
+        assert torch.equal(c, refs[1])
+    assert packings == [1, 0] or not pending
+    ops.check_device_status()

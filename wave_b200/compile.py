@@ -195,7 +195,7 @@ class ScaledGemmKernel:
             for holder, value in marks:
                 holder[0] = value
             self._fast.add(a, a_scale, b, b_scale, c, self.options.decode_tiled_weight_scales, self.options.kernel_path, sizes, b_sf.data, scratch,
-                           workspace, marks)
+                           workspace, marks, b_sf.made[0], b_sf.made[1] is None)
 
     def _marks(self, idx: int, pool=None, kind: str = "skinny") -> tuple:
         """What notes that the eager call before used the scratch, and with a pool the workspace, that were asked for just now."""

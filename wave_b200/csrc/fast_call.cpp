@@ -19,6 +19,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
@@ -122,6 +123,8 @@ struct Weight {
   uint32_t version;
   int tile_rows;
   at::Tensor packed;
+  cudaStream_t stream;  // the one that the packing was filled on,
+  bool complete;        // and whether that is known to be done: until then the Python code orders other streams behind it
 };
 
 struct Calls {
@@ -138,9 +141,9 @@ struct Calls {
       }
     return nullptr;
   }
-  const Weight* find(const at::Tensor& scale, int tile_rows) {
+  Weight* find(const at::Tensor& scale, int tile_rows) {
     const c10::TensorImpl* impl = scale.unsafeGetTensorImpl();
-    for (const Weight& w : weights)
+    for (Weight& w : weights)
       // (an address that another tensor has taken over belongs to a new object, and the reference to the old one has expired)
       if (w.impl == impl && w.tile_rows == tile_rows && !w.owner.expired() && w.ptr == scale.data_ptr() && w.version == scale._version()) return &w;
     return nullptr;
@@ -188,7 +191,7 @@ PyObject* calls_call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     }
     const Plan* found = calls.find(key);
     const Weight* weight = found ? calls.find(THPVariable_Unpack(args[3]), found->tile_rows) : nullptr;
-    if (!weight) Py_RETURN_NONE;
+    if (!weight || !(weight->complete || weight->stream == key.stream)) Py_RETURN_NONE;
     // another thread may change the tables while the lock is released: what the launch reads is held here
     const at::Tensor scratch = found->scratch, workspace = found->workspace, packed = weight->packed;
     const int M = found->M, N = found->N, K = found->K, elem_format = found->elem_format;
@@ -201,6 +204,8 @@ PyObject* calls_call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     const long long a_scale_stride = M > 1 ? key.sig[1].stride[0] : K / 32, ldc = M > 1 ? key.sig[4].stride[0] : N;
     void* ws = workspace.defined() ? workspace.data_ptr() : nullptr;
     for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(found->marks.o); ++i) set_mark(PyTuple_GET_ITEM(found->marks.o, i));
+    if (weight->stream != key.stream)  // its memory may be given back on the stream it was made on while this one reads it
+      c10::cuda::CUDACachingAllocator::recordStream(packed.storage().data_ptr(), c10::cuda::getCurrentCUDAStream(key.device));
     int rc;
     Py_BEGIN_ALLOW_THREADS
     if (elem_format < 0)
@@ -216,13 +221,14 @@ PyObject* calls_call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
   }
 }
 
-// add(a, a_scale, b, b_scale, c, tiled, path, (M, N, K, elem_format, flags, tile_rows, workspace_bytes), packed, scratch, workspace or None, marks):
+// add(a, a_scale, b, b_scale, c, tiled, path, (M, N, K, elem_format, flags, tile_rows, workspace_bytes), packed, scratch, workspace or None, marks,
+//     stream that the packing was filled on, whether it is complete):
 // the Python code has just made this call with these arguments.
 PyObject* calls_add(PyObject* self, PyObject* const* args, Py_ssize_t n) {
-  bool marks_ok = n == 12 && PyTuple_Check(args[11]);
+  bool marks_ok = n == 14 && PyTuple_Check(args[11]);
   for (Py_ssize_t i = 0; marks_ok && i < PyTuple_GET_SIZE(args[11]); ++i) marks_ok = is_mark(PyTuple_GET_ITEM(args[11], i));
   if (!marks_ok) {
-    PyErr_SetString(PyExc_TypeError, "add takes 12 arguments, the last one a tuple of (list of one element, value) pairs");
+    PyErr_SetString(PyExc_TypeError, "add takes 14 arguments, the twelfth a tuple of (list of one element, value) pairs");
     return nullptr;
   }
   try {
@@ -248,13 +254,19 @@ PyObject* calls_add(PyObject* self, PyObject* const* args, Py_ssize_t n) {
       calls.plans[calls.next_plan++ % kMaxPlans] = p;
     }
     const at::Tensor& scale = THPVariable_Unpack(args[3]);
-    if (!calls.find(scale, p.tile_rows)) {
+    const auto filled_on = reinterpret_cast<cudaStream_t>(PyLong_AsUnsignedLongLong(args[12]));
+    const bool complete = PyObject_IsTrue(args[13]) == 1;
+    if (PyErr_Occurred()) return nullptr;
+    Weight* known = calls.find(scale, p.tile_rows);
+    if (known && known->packed.is_same(THPVariable_Unpack(args[8]))) {
+      known->complete = known->complete || complete;
+    } else {
       const auto gone = std::remove_if(calls.weights.begin(), calls.weights.end(), [&](const Weight& w) {
         return w.owner.expired() || (w.impl == scale.unsafeGetTensorImpl() && w.tile_rows == p.tile_rows);
       });
       calls.weights.erase(gone, calls.weights.end());
       Weight w{c10::weak_intrusive_ptr<c10::TensorImpl>(scale.getIntrusivePtr()), scale.unsafeGetTensorImpl(), scale.data_ptr(),
-               uint32_t(scale._version()), p.tile_rows, THPVariable_Unpack(args[8])};
+               uint32_t(scale._version()), p.tile_rows, THPVariable_Unpack(args[8]), filled_on, complete};
       if (calls.weights.size() < kMaxWeights) calls.weights.push_back(std::move(w));
       else calls.weights[calls.next_weight++ % kMaxWeights] = std::move(w);
     }
@@ -391,6 +403,22 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
 }
 
+// event_done(event) -> whether the work in front of a recorded event is complete; may be asked while a stream is being captured (the event
+// is not part of the capture)
+PyObject* event_done(PyObject*, PyObject* arg) {
+  auto event = reinterpret_cast<cudaEvent_t>(PyLong_AsUnsignedLongLong(arg));
+  if (PyErr_Occurred()) return nullptr;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // of this thread: a query does not end a capture then
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
+    (void)cudaGetLastError();
+    Py_RETURN_FALSE;
+  }
+  const cudaError_t status = cudaEventQuery(event);
+  (void)cudaGetLastError();
+  (void)cudaThreadExchangeStreamCaptureMode(&mode);
+  return PyBool_FromLong(status == cudaSuccess);
+}
+
 // bind(gemm_repack_a, mxfp8_gemm_repack_a, gemm_quantize_a, gemm_workspace_bytes, decode_tile_rows_for): addresses in the loaded library
 PyObject* bind(PyObject*, PyObject* args) {
   unsigned long long p[5];
@@ -408,7 +436,8 @@ PyMethodDef calls_methods[] = {{"call", FASTCALL(calls_call), nullptr}, {"add", 
                                {"clear", calls_clear, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyMethodDef workspaces_methods[] = {{"put", FASTCALL(workspaces_put), nullptr}, {"clear", workspaces_clear, METH_NOARGS, nullptr},
                                     {nullptr, nullptr, 0, nullptr}};
-PyMethodDef module_methods[] = {{"bind", bind, METH_VARARGS, nullptr}, {"linear", FASTCALL(linear), nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyMethodDef module_methods[] = {{"bind", bind, METH_VARARGS, nullptr}, {"linear", FASTCALL(linear), nullptr},
+                                {"event_done", event_done, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_fast", nullptr, -1, module_methods, nullptr, nullptr, nullptr, nullptr};
 
 template <typename Object, typename Data, Data* Object::*Field>

@@ -36,10 +36,11 @@ class PackedScales:
     decode kernel's tile height (`repack_scales(..., tile_rows=decode_tile_rows(N))`), which only the M <= 128
     path reads."""
 
-    __slots__ = ("data", "rows", "K", "tile_rows")
+    __slots__ = ("data", "rows", "K", "tile_rows", "made")
 
     def __init__(self, data: torch.Tensor, rows: int, K: int, tile_rows: int = 128):
         self.data, self.rows, self.K, self.tile_rows = data, rows, K, tile_rows
+        self.made = None  # WeightScaleCache: (stream, event behind the kernel that fills it, None once that is known to be complete)
 
     @property
     def device(self):
@@ -406,7 +407,8 @@ class WeightScaleCache:
     that the allocator places at a freed tensor's address therefore never meets the old packing, and an in-place
     write (which bumps the version of every view) makes the next call repack. What the cache cannot see is a write
     through a raw pointer (a C extension, a CUDA graph replay that rewrites the scales): call `clear()` — or
-    `ScaledGemmKernel.drop_cached_weights()` — after such a write. A packing that a captured call was given stays in memory
+    `ScaledGemmKernel.drop_cached_weights()` — after such a write. A packing is filled on the stream of the call that made it: calls on
+    other streams wait for that, and its memory is not given to anything else before they are done. A packing that a captured call was given stays in memory
     as long as the cache, whatever is evicted or dropped: the graph holds its address. One that is made while a graph is
     captured is filled by the replays only and not given to any other call."""
 
@@ -422,18 +424,42 @@ class WeightScaleCache:
         if hit is not None:
             owner, packed = hit
             if owner() is scale:
-                self._entries.move_to_end(key)
-                self._keep_if_captured(packed)
-                return packed
-            del self._entries[key]  # same address, another (or a dead) tensor: the packing is not this tensor's
+                if self._usable(packed):
+                    self._entries.move_to_end(key)
+                    self._keep_if_captured(packed)
+                    return packed
+            else:
+                del self._entries[key]  # same address, another (or a dead) tensor: the packing is not this tensor's
         packed = repack_scales(scale, tile_rows=tile_rows)
         self.packings += 1
         if self._keep_if_captured(packed):
             return packed
+        stream, event = torch.cuda.current_stream(packed.device), torch.cuda.Event()
+        event.record(stream)
+        packed.made = (stream.cuda_stream, event)
         self._entries[key] = (weakref.ref(scale), packed)
         while len(self._entries) > self.capacity:
             self._entries.popitem(last=False)
         return packed
+
+    @staticmethod
+    def _usable(packed: PackedScales) -> bool:
+        """Whether what the current stream does next may read the packing, after a wait where one is needed. False while a graph is captured
+        and the packing is not known to be complete: a replay may come at any time and on any stream."""
+        stream, event = packed.made
+        capturing = torch.cuda.is_current_stream_capturing()
+        if event is not None:
+            if _lib.fast().event_done(event.cuda_event):
+                packed.made, event = (stream, None), None
+            elif capturing:
+                return False
+        if not capturing:
+            current = torch.cuda.current_stream(packed.device)
+            if current.cuda_stream != stream:
+                if event is not None:
+                    current.wait_event(event)
+                packed.data.record_stream(current)
+        return True
 
     def _keep_if_captured(self, packed: PackedScales) -> bool:
         if not torch.cuda.is_current_stream_capturing():
