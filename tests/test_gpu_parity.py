@@ -1876,3 +1876,32 @@ def test_a_capture_while_weight_scales_are_being_packed():
         assert torch.equal(c, refs[1])
     assert packings == [1, 0] or not pending
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("rows", [4, 300])
+def test_linear_refuses_codes_that_its_scales_were_not_packed_for(rows):
+    """weight_codes replaced by a matrix of another size is refused as before any call was recognised in native code, and nothing is launched; nor is
+    anything launched there on scales that are shorter than the matrix asks for."""
+    N, K = 1024, 512
+    g = torch.Generator().manual_seed(2)
+    layer = wb.MXFP4Linear.from_float((torch.randn(N, K, generator=g) * 0.02).to(DEV))
+    x = torch.randn(rows, K, generator=g).to(DEV)
+    ref, codes = layer(x), layer.weight_codes
+    for n, k in ((2 * N, K), (N // 2, K), (N + 8, K), (N, 2 * K)):
+        layer.weight_codes = torch.zeros(n, k // 2, dtype=torch.uint8, device=DEV)
+        with pytest.raises((ValueError, RuntimeError)):  # (another K: x does not fit)
+            layer(x)
+        if k == K:
+            with pytest.raises(ValueError, match="do not agree"):
+                layer(x)
+    layer.weight_codes = codes
+    packed, low = layer._packed, layer._packed_low
+    native = lambda p, q, r=N, c=codes: _lib.fast().linear(x, c, r, K, p, q, low.tile_rows, layer.output_dtype, ops._pool.fast)  # noqa: E731
+    assert torch.equal(native(packed.data, low.data), ref)
+    assert native(packed.data[:-512], low.data[:-512]) is None
+    assert native(packed.data, low.data, N + 8) is None
+    assert native(packed.data, low.data, N, codes.view(torch.int32).repeat(1, 4)) is None
+    with pytest.raises(TypeError):
+        _lib.fast().linear(x, codes, N, K, packed.data, low.data, low.tile_rows, layer.output_dtype, [])
+    assert torch.equal(layer(x), ref)
+    ops.check_device_status()

@@ -168,7 +168,7 @@ bool key_of(PyObject* const* args, CallKey* key) {
   key->aligned = rows_aligned(THPVariable_Unpack(args[4]));
   key->tiled = PyObject_IsTrue(args[5]) == 1;
   key->path = PyLong_AsLong(args[6]);
-  return true;
+  return !PyErr_Occurred();
 }
 
 PyObject* fail(const std::exception& e) {
@@ -335,24 +335,36 @@ void object_free(PyObject* self) {
   Py_TYPE(self)->tp_free(self);
 }
 
-// linear(x, weight_codes, packed scales, those per tile of low_rows rows or None, low_rows, output dtype, workspaces)
+bool is_workspaces(PyObject* o);
+
+// Packed scales of N rows and K values in tiles of tile_rows (at most 128) rows: a 512-byte atom per 128 K and tile, K padded to 256.
+// (The kernel's tensor map covers all of it, whatever the array holds.)
+bool holds_scales(const at::Tensor& packed, int64_t N, int64_t K, int64_t tile_rows) {
+  return packed.scalar_type() == at::kByte && packed.is_contiguous() && packed.numel() >= (N + tile_rows - 1) / tile_rows * ((K + 255) / 256) * 1024;
+}
+
+// linear(x, weight_codes, rows and K that the scales were packed for, packed scales, those per tile of low_rows rows or None, low_rows,
+//        output dtype, workspaces)
 // -> dequant(quantise(x)) @ dequant(W)^T, or None: left to the Python code.
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 7) {
-    PyErr_SetString(PyExc_TypeError, "linear takes 7 arguments");
+  if (n != 9 || !is_workspaces(args[8])) {
+    PyErr_SetString(PyExc_TypeError, "linear takes 9 arguments, the last one a Workspaces object");
     return nullptr;
   }
   try {
-    if (!plain(args[0]) || !plain(args[1]) || !plain(args[2]) || !THPDtype_Check(args[5])) Py_RETURN_NONE;
+    if (!plain(args[0]) || !plain(args[1]) || !plain(args[4]) || !THPDtype_Check(args[7])) Py_RETURN_NONE;
     const at::Tensor &x = THPVariable_Unpack(args[0]), &w = THPVariable_Unpack(args[1]);
-    at::Tensor packed = THPVariable_Unpack(args[2]);
+    at::Tensor packed = THPVariable_Unpack(args[4]);
+    const long long rows = PyLong_AsLongLong(args[2]), of_k = PyLong_AsLongLong(args[3]);
+    if (PyErr_Occurred()) return nullptr;
     const int device = x.device().index();
-    const at::ScalarType x_type = x.scalar_type(), out_type = reinterpret_cast<THPDtype*>(args[5])->scalar_type;
+    const at::ScalarType x_type = x.scalar_type(), out_type = reinterpret_cast<THPDtype*>(args[7])->scalar_type;
     const int64_t dims = x.dim();
     if (device != c10::cuda::current_device() || w.device().index() != device || packed.device().index() != device || dims < 1 || w.dim() != 2 ||
-        !w.is_contiguous() || (x_type != at::kFloat && x_type != at::kBFloat16) || (out_type != at::kFloat && out_type != at::kBFloat16))
+        !w.is_contiguous() || w.element_size() != 1 || (x_type != at::kFloat && x_type != at::kBFloat16) || (out_type != at::kFloat && out_type != at::kBFloat16))
       Py_RETURN_NONE;
     const int64_t K = w.size(1) * 2, N = w.size(0);
+    if (N != rows || K != of_k) Py_RETURN_NONE;  // refused there: the scales belong to another matrix
     if (x.size(dims - 1) != K || K == 0 || x.numel() == 0) Py_RETURN_NONE;
     const int64_t M = x.numel() / K;
     const bool strided = dims == 2 && x.stride(1) == 1 && x.stride(0) >= K;
@@ -364,7 +376,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     size_t ws_bytes = 0;
     if (M <= 128) {
       ws_bytes = abi.gemm_workspace_bytes(int(M), int(N), int(K));
-      for (const auto& e : reinterpret_cast<PyWorkspaces*>(args[6])->table->entries)
+      for (const auto& e : reinterpret_cast<PyWorkspaces*>(args[8])->table->entries)
         if (e.device == device && e.stream == stream.stream()) {
           ws = e.ws;
           mark = e.mark;
@@ -375,13 +387,14 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const bool aligned = M == 1 || N * (out_type == at::kFloat ? 4 : 2) % 16 == 0;
     int tile_rows = 128;
     if (M <= 128 && (tile_rows = abi.decode_tile_rows_for(int(M), int(N), int(K), 4, 4, aligned)) != 128) {
-      if (args[3] == Py_None || PyLong_AsLong(args[4]) != tile_rows || !plain(args[3])) {
+      if (args[5] == Py_None || PyLong_AsLong(args[6]) != tile_rows || !plain(args[5])) {
         if (PyErr_Occurred()) return nullptr;
         Py_RETURN_NONE;
       }
-      packed = THPVariable_Unpack(args[3]);
+      packed = THPVariable_Unpack(args[5]);
       if (packed.device().index() != device) Py_RETURN_NONE;
     }
+    if (!holds_scales(packed, N, K, tile_rows)) Py_RETURN_NONE;
     std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
     shape.back() = N;
     const at::Tensor out = at::detail::empty_cuda(shape, out_type, x.device(), c10::nullopt);
@@ -439,6 +452,10 @@ PyMethodDef workspaces_methods[] = {{"put", FASTCALL(workspaces_put), nullptr}, 
 PyMethodDef module_methods[] = {{"bind", bind, METH_VARARGS, nullptr}, {"linear", FASTCALL(linear), nullptr},
                                 {"event_done", event_done, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_fast", nullptr, -1, module_methods, nullptr, nullptr, nullptr, nullptr};
+
+bool is_workspaces(PyObject* o) {
+  return Py_TYPE(o)->tp_dealloc == object_free<PyWorkspaces, Workspaces, &PyWorkspaces::table>;
+}
 
 template <typename Object, typename Data, Data* Object::*Field>
 bool add_type(PyObject* module, const char* name, const char* qualified, PyMethodDef* methods) {
