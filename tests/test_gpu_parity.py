@@ -1905,3 +1905,25 @@ def test_linear_refuses_codes_that_its_scales_were_not_packed_for(rows):
         _lib.fast().linear(x, codes, N, K, packed.data, low.data, low.tile_rows, layer.output_dtype, [])
     assert torch.equal(layer(x), ref)
     ops.check_device_status()
+
+
+def test_a_repeated_call_follows_weight_scales_that_were_given_another_view():
+    """`scale.data = view` keeps the tensor, its address and its version. The packing belongs to the sizes and strides it was made with, also where
+    the new ones are of a form that another weight's calls have made known."""
+    M, N, K = 8, 512, 1024
+    a, a_s, b, wide = (t.to(DEV) for t in random_problem(M, 2 * N, K, seed=5))
+    b = b[:N].contiguous()
+    t, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    compiled = lambda: wb.wave_compile(wb.set_default_run_config(options), t)  # noqa: E731
+    gemm, views = compiled(), (wide[:N], wide[::2])
+    other, scale = wide.clone()[::2], torch.empty(0, dtype=torch.uint8, device=DEV)
+    for s in (other, other, *views, *views):
+        if s is not other:
+            scale.data = s
+            s = scale
+        for _ in range(2):
+            c, ref = (torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+            gemm(a, a_s, b, s, c)
+            compiled()(a, a_s, b, s.clone(), ref)
+            assert torch.equal(c, ref)
+    ops.check_device_status()

@@ -9,7 +9,7 @@
 //
 // What is kept: per kernel object, the signatures (sizes, strides, types, device, stream, alignment of the output) of at most
 // kMaxPlans calls with their scratch, and at most kMaxWeights packings of weight scales, each found by the tensor it was made from
-// (a weak reference), its version counter and its address, as WeightScaleCache does. Nothing about activations or outputs
+// (a weak reference), its version counter, address, sizes and strides, as WeightScaleCache does. Nothing about activations or outputs
 // is kept but their shapes. A call notes whose scratch and workspace it used where the Python code notes it (`marks`): a captured call takes the
 // memory of the eager call before it. Calls under stream capture, on another device than the current one, with tensor subclasses, under
 // functional transforms, or with inference tensors are left to the Python code.
@@ -119,6 +119,7 @@ struct Plan {
 struct Weight {
   c10::weak_intrusive_ptr<c10::TensorImpl> owner;
   const c10::TensorImpl* impl;
+  Signature sig;
   const void* ptr;
   uint32_t version;
   int tile_rows;
@@ -141,11 +142,11 @@ struct Calls {
       }
     return nullptr;
   }
-  Weight* find(const at::Tensor& scale, int tile_rows) {
+  Weight* find(const at::Tensor& scale, const Signature& sig, int tile_rows) {
     const c10::TensorImpl* impl = scale.unsafeGetTensorImpl();
     for (Weight& w : weights)
       // (an address that another tensor has taken over belongs to a new object, and the reference to the old one has expired)
-      if (w.impl == impl && w.tile_rows == tile_rows && !w.owner.expired() && w.ptr == scale.data_ptr() && w.version == scale._version()) return &w;
+      if (w.impl == impl && w.tile_rows == tile_rows && w.sig == sig && !w.owner.expired() && w.ptr == scale.data_ptr() && w.version == scale._version()) return &w;
     return nullptr;
   }
 };
@@ -190,7 +191,7 @@ PyObject* calls_call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
       Py_RETURN_NONE;
     }
     const Plan* found = calls.find(key);
-    const Weight* weight = found ? calls.find(THPVariable_Unpack(args[3]), found->tile_rows) : nullptr;
+    const Weight* weight = found ? calls.find(THPVariable_Unpack(args[3]), key.sig[3], found->tile_rows) : nullptr;
     if (!weight || !(weight->complete || weight->stream == key.stream)) Py_RETURN_NONE;
     // another thread may change the tables while the lock is released: what the launch reads is held here
     const at::Tensor scratch = found->scratch, workspace = found->workspace, packed = weight->packed;
@@ -257,7 +258,7 @@ PyObject* calls_add(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     const auto filled_on = reinterpret_cast<cudaStream_t>(PyLong_AsUnsignedLongLong(args[12]));
     const bool complete = PyObject_IsTrue(args[13]) == 1;
     if (PyErr_Occurred()) return nullptr;
-    Weight* known = calls.find(scale, p.tile_rows);
+    Weight* known = calls.find(scale, p.key.sig[3], p.tile_rows);
     if (known && known->packed.is_same(THPVariable_Unpack(args[8]))) {
       known->complete = known->complete || complete;
     } else {
@@ -265,7 +266,7 @@ PyObject* calls_add(PyObject* self, PyObject* const* args, Py_ssize_t n) {
         return w.owner.expired() || (w.impl == scale.unsafeGetTensorImpl() && w.tile_rows == p.tile_rows);
       });
       calls.weights.erase(gone, calls.weights.end());
-      Weight w{c10::weak_intrusive_ptr<c10::TensorImpl>(scale.getIntrusivePtr()), scale.unsafeGetTensorImpl(), scale.data_ptr(),
+      Weight w{c10::weak_intrusive_ptr<c10::TensorImpl>(scale.getIntrusivePtr()), scale.unsafeGetTensorImpl(), p.key.sig[3], scale.data_ptr(),
                uint32_t(scale._version()), p.tile_rows, THPVariable_Unpack(args[8]), filled_on, complete};
       if (calls.weights.size() < kMaxWeights) calls.weights.push_back(std::move(w));
       else calls.weights[calls.next_weight++ % kMaxWeights] = std::move(w);
