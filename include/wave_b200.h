@@ -57,7 +57,8 @@ extern "C" {
                                      caller-initialised c (tagged_mxfp4_gemm.py:780-781, 830-831) */
 
 #define WB200_OVERLAP_PREVIOUS 0x80u /* the caller asserts that b and b_scale_packed are NOT written by the kernel that
-                                     precedes this call in the stream: the GEMM is then launched as a programmatic
+                                     precedes this call in the stream (earlier ones may write them, if they are the quantisers or
+                                     the repack entries here, or kernels that do not release their dependents early): the GEMM is then launched as a programmatic
                                      dependent of that kernel. On the skinny path (M <= 128) its set-up AND the first
                                      ring of weight loads overlap that kernel's tail; on the tile paths only the set-up
                                      (barriers, tensor-memory allocation, descriptor prefetch) does, and every load

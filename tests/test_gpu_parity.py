@@ -1927,3 +1927,34 @@ def test_a_repeated_call_follows_weight_scales_that_were_given_another_view():
             compiled()(a, a_s, b, s.clone(), ref)
             assert torch.equal(c, ref)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("tiled", [False, True])
+def test_weight_scales_packed_two_launches_ahead_of_an_overlapping_gemm(tiled):
+    """The same chain with the scales of w packed by the repack entries: that kernel lets nothing start before it has ended, so the second
+    GEMM, which may read them before its wait, finds them written. The first GEMM leaves most SMs free."""
+    N, K, M = 16384, 8192, 16
+    g = torch.Generator(device=DEV).manual_seed(6)
+    lib, w = _lib.load(), torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, generator=g, device=DEV)
+    scales = [torch.randint(110 + 12 * i, 115 + 12 * i, (N, K // 32), dtype=torch.uint8, generator=g, device=DEV) for i in range(2)]
+    h = ops.decode_tile_rows_for(M, N, K) if tiled else 128
+    assert tiled == (h != 128)
+    pk = ops.repack_scales(scales[0], tile_rows=h)
+    a, _, a_sf = ops.quantize_mxfp4(torch.randn(M, K, generator=g, device=DEV))
+    q1, _, sf1 = ops.quantize_mxfp4(torch.randn(1024, K, generator=g, device=DEV))
+    c1 = torch.empty(M, 1024, dtype=torch.bfloat16, device=DEV)
+    refs = []
+    for s in scales:
+        ops.repack_scales(s, out=pk.data, tile_rows=h)
+        torch.cuda.synchronize()
+        refs.append(torch.empty(M, N, dtype=torch.bfloat16, device=DEV))
+        ops.scaled_gemm_packed(a, a_sf, w, pk, refs[-1])
+    outs = [torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(12)]
+    for i, c in enumerate(outs):  # no synchronisation in between
+        ops.repack_scales(scales[i & 1], out=pk.data, tile_rows=h)
+        ops.scaled_gemm_packed(a, a_sf, q1, sf1, c1, _lib.OVERLAP_PREVIOUS)
+        ops.scaled_gemm_packed(a, a_sf, w, pk, c, _lib.OVERLAP_PREVIOUS)
+    torch.cuda.synchronize()
+    for i, c in enumerate(outs):
+        assert torch.equal(c.view(torch.int16), refs[i & 1].view(torch.int16))
+    ops.check_device_status()

@@ -1336,7 +1336,7 @@ static int check_repack(const void* src, long long src_row_stride, int rows, int
 }
 
 static int repack_scales_impl(const void* src, long long src_row_stride, int rows, int K, void* dst, void* stream,
-                              bool broadcast, int block_rows = 128) {
+                              bool broadcast, bool release, int block_rows = 128) {
   int rc = check_repack(src, src_row_stride, rows, K, dst, broadcast);
   if (rc) return rc;
   DeviceInfo* dev;
@@ -1356,7 +1356,7 @@ static int repack_scales_impl(const void* src, long long src_row_stride, int row
   // limit, where the gap costs nothing (8192^3 in a loop, ordinary / programmatic: 213.2 / 215.9 us).
   cfg.numAttrs = tl_dependent_launch || grid.x * grid.y <= unsigned(dev->sm_count) ? 1 : 0;
   WB_CUDA(cudaLaunchKernelEx(&cfg, wb::repack_scales_kernel, static_cast<const uint8_t*>(src), src_row_stride, rows, K / 32,
-                             k_atoms, static_cast<uint8_t*>(dst), broadcast, tl_dependent_launch, block_rows));
+                             k_atoms, static_cast<uint8_t*>(dst), broadcast, tl_dependent_launch, release, block_rows));
   return WB200_OK;
 }
 
@@ -1368,7 +1368,7 @@ int pack_row_scales(int M, int K, cudaStream_t stream) {
   if (!tl_row_scales.src) return WB200_OK;
   const PendingRowScales s = tl_row_scales;
   tl_row_scales = {};
-  int rc = repack_scales_impl(s.src, s.stride, M, K, s.scratch, stream, false);
+  int rc = repack_scales_impl(s.src, s.stride, M, K, s.scratch, stream, false, true);
   if (rc == WB200_OK) tl_dependent_launch = true;
   return rc;
 }
@@ -1378,15 +1378,15 @@ int pack_row_scales(int M, int K, cudaStream_t stream) {
 int wb200_repack_scales_tiled(const void* src, long long src_row_stride, int rows, int K, int tile_rows, void* dst, void* stream) {
   if (!tile_rows_ok(tile_rows))
     return fail(WB200_ERR_INVALID_ARG, "repack_scales_tiled: %d rows per tile (8 .. 208 in steps of 8, or 224)", tile_rows);
-  return repack_scales_impl(src, src_row_stride, rows, K, dst, stream, false, tile_rows);
+  return repack_scales_impl(src, src_row_stride, rows, K, dst, stream, false, false, tile_rows);
 }
 
 int wb200_repack_scales(const void* src, long long src_row_stride, int rows, int K, void* dst, void* stream) {
-  return repack_scales_impl(src, src_row_stride, rows, K, dst, stream, false);
+  return repack_scales_impl(src, src_row_stride, rows, K, dst, stream, false, false);
 }
 
 int wb200_repack_scales_broadcast(const void* src, long long src_row_stride, int rows, int K, void* dst, void* stream) {
-  return repack_scales_impl(src, src_row_stride, rows, K, dst, stream, true);
+  return repack_scales_impl(src, src_row_stride, rows, K, dst, stream, true, false);
 }
 
 int wb200_repack_scales_grouped(const void* src, long long src_row_stride, int num_groups, const int* row_offsets,
@@ -1951,7 +1951,7 @@ int wb200_mxfp8_gemm_repack_a(int M, int N, int K, const void* a, const void* a_
                               void* workspace, size_t workspace_bytes, unsigned flags, void* stream) {
   if (!a_scale_scratch) return fail(WB200_ERR_INVALID_ARG, "mxfp8_gemm_repack_a: null scratch for the packed activation scales");
   tl_dependent_launch = (flags & WB200_OVERLAP_PREVIOUS) != 0;
-  int rc = wb200_repack_scales(a_scale, a_scale_stride, M, K, a_scale_scratch, stream);
+  int rc = repack_scales_impl(a_scale, a_scale_stride, M, K, a_scale_scratch, stream, false, true);
   tl_dependent_launch = false;
   if (rc) return rc;
   tl_dependent_launch = true;  // the GEMM is the repack kernel's programmatic dependent

@@ -81,14 +81,15 @@ __device__ __forceinline__ void repack_tile(const uint8_t* __restrict__ src, lon
 }
 
 // grid (ceil(k_atoms / 8), row_blocks), 256 threads.
+// release: the library launches a GEMM right behind this kernel that waits before it reads dst: dependents may start their set-up once every
+// CTA has come here (dependent: kDependent of ptx.cuh). Otherwise dst may be the scales of a WEIGHT, which a GEMM two launches on may
+// read before its wait (WB200_OVERLAP_PREVIOUS): as in the quantiser, nothing is released before the kernel ends.
 __global__ void __launch_bounds__(256)
 repack_scales_kernel(const uint8_t* __restrict__ src, long long src_row_stride, int rows, int kblocks,
-                     int k_atoms, uint8_t* __restrict__ dst, bool broadcast, bool dependent, int block_rows = 128) {
-  // a GEMM launched behind this kernel may start its set-up once every CTA has come here; it waits for this kernel's
-  // completion before it reads dst (dependent: kDependent of ptx.cuh)
-  if (dependent) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+                     int k_atoms, uint8_t* __restrict__ dst, bool broadcast, bool dependent, bool release, int block_rows = 128) {
+  if (release && dependent) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the kernel before this one may still be reading dst or writing src
-  if (!dependent) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (release && !dependent) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // block_rows != 128: a packing per tile of block_rows weight rows. Up to 128: one atom row per tile (the decode
   // kernel's tiles; rows block_rows..127 of every atom hold the padding byte). Above 128 (224: the tile kernel's
   // 224-column tiles): two atom rows per tile, rows 0..127 and 128..block_rows-1 of the tile.
