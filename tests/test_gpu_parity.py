@@ -1958,3 +1958,61 @@ def test_weight_scales_packed_two_launches_ahead_of_an_overlapping_gemm(tiled):
     for i, c in enumerate(outs):
         assert torch.equal(c.view(torch.int16), refs[i & 1].view(torch.int16))
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("kind,M", [("fp4", 64), ("fp4", 300), ("strided", 64), ("broadcast", 64), ("fp8", 64), ("mixed", 64)])
+def test_threads_share_a_kernel_object_and_a_stream(kind, M):
+    """Two threads call one kernel object on one stream, at sizes whose activation scales are packed into the object's scratch ahead of the GEMM: each
+    call's two launches stay together. The scales of the threads are powers of two apart, so that the other one's would show."""
+    import sys
+    import threading
+    N, K, calls = 1024, 2048, 400
+    g = torch.Generator().manual_seed(M)
+    bits = 8 if kind in ("fp8", "mixed") else 4
+    if bits == 8:
+        t, subs = wb.get_scaled_gemm_mxfp8_kernel((M, N, K), wb.ScaledMMAType.F32_16x16x128_F8F6F4, "f8e4m3fn", wb.bf16,
+                                                  weight_format="f4e2m1fn" if kind == "mixed" else None)
+        options = wb.WaveCompileOptions(subs=subs)
+    elif kind == "broadcast":
+        t, subs = wb.get_broadcasted_scale_gemm_mxfp4((M, N, K), wb.ScaledMMAType.F32_16x16x128_F8F6F4)
+        options = wb.WaveCompileOptions(subs=subs)
+    else:
+        t, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    gemm = wb.wave_compile(wb.set_default_run_config(options), t)
+
+    def operand(rows, bits):
+        x = torch.randint(0, 256, (rows, K * bits // 8), dtype=torch.uint8, generator=g)
+        return (x if bits == 4 else (x & 0xBF).view(torch.float8_e4m3fn)).to(DEV)
+
+    a = operand(M, bits)
+    if kind == "strided":
+        a = torch.cat([a, a], 1)[:, :K // 2]
+    b, b_s = operand(N, 8 if kind == "fp8" else 4), torch.randint(124, 131, (N, K // 32), dtype=torch.uint8, generator=g).to(DEV)
+    scales = [torch.randint(110 + 20 * i, 115 + 20 * i, (M,) if kind == "broadcast" else (M, K // 32), dtype=torch.uint8, generator=g).to(DEV) for i in range(2)]
+    dtype = t.output_dtype.torch_dtype
+    outs = [[torch.empty(M, N, dtype=dtype, device=DEV) for _ in range(8)] for _ in scales]
+    refs = [torch.empty(M, N, dtype=dtype, device=DEV) for _ in scales]
+    for s, c in zip(scales, refs):
+        gemm(a, s, b, b_s, c)
+        torch.cuda.synchronize()
+    wrong, start = [0, 0], threading.Barrier(2)
+
+    def work(i):
+        start.wait()
+        for n in range(calls):
+            gemm(a, scales[i], b, b_s, outs[i][n % 8])
+            if n % 8 == 7:
+                wrong[i] += sum(int(not torch.equal(c, refs[i])) for c in outs[i])
+
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+        for th in threads:
+            th.start()
+        for th in threads:
+            th.join()
+    finally:
+        sys.setswitchinterval(interval)
+    assert wrong == [0, 0]
+    ops.check_device_status()

@@ -8,6 +8,7 @@ are precompiled in libwave_b200.so, and "compiling" checks the options and picks
 
 from __future__ import annotations
 
+import threading
 from dataclasses import dataclass, field
 from typing import Any, Optional
 
@@ -121,6 +122,7 @@ class ScaledGemmKernel:
         self._weight_scales = ops.WeightScaleCache()
         self._a_scale_buf: dict[tuple[int, int], list[torch.Tensor]] = {}  # (device, stream) -> scratches, the one in use last
         self._a_scale_last: dict[int, list] = {}  # device -> [key] of the eager call before; native calls write the element too
+        self._broadcasting = threading.Lock()  # from the packing of broadcast scales into the scratch to the launch that reads it
         self._workspaces = ops.WorkspacePool()  # this object's own: calls through another object may overlap with these
         self._plans: dict = {}
         self._tile_rows: dict = {}
@@ -281,15 +283,14 @@ class ScaledGemmKernel:
             ops._as_u8(a_scale, "a_scale")
             if tuple(a_scale.shape) != (M,):
                 raise ValueError(f"a_scale must be [{M}] (one scale per row), got {tuple(a_scale.shape)}")
-            a_scale = ops.repack_scales_broadcast(a_scale, K, out=self._a_scale_buffer(a.device, M, K))
-        if t.preshuffled_scales and not (isinstance(a_scale, ops.PackedScales) and isinstance(b_scale, ops.PackedScales)):
+        elif t.preshuffled_scales and not (isinstance(a_scale, ops.PackedScales) and isinstance(b_scale, ops.PackedScales)):
             raise ValueError(f"{t.name} takes pre-shuffled scales: pass mxfp_utils.e8m0_shuffle(scale) for a_scale and b_scale")
         flags = self.options.kernel_path | self._raster_flags()
         if t.accumulate:
             flags |= _lib.ACCUMULATE
         if self.options.overlap_previous:
             flags |= _lib.OVERLAP_PREVIOUS
-        plain = type(a_scale) is torch.Tensor and type(b_scale) is torch.Tensor
+        plain = not t.broadcast_a_scale and type(a_scale) is torch.Tensor and type(b_scale) is torch.Tensor
         if plain:
             self._check_scale(a_scale, M, K, "a_scale")
             self._check_scale(b_scale, N, K, "b_scale")
@@ -313,7 +314,6 @@ class ScaledGemmKernel:
             if not capturing:  # (every capture takes the memory of its own warm-up)
                 self._plans[sig] = plan
             return self._launch(plan, a, a_scale, b, b_scale, c)
-        a_sf = self._pack_activation_scales(a_scale, M, K)
         if isinstance(b_scale, ops.PackedScales):
             b_sf = b_scale
         else:
@@ -322,7 +322,18 @@ class ScaledGemmKernel:
             b_sf = self._weight_scales.get(self._check_scale(b_scale, N, K, "b_scale"), self._weight_tile_rows(M, N, K, c, idx))
             if self._weight_scales.packings != packings:
                 flags &= ~_lib.OVERLAP_PREVIOUS  # as in _launch
-        ops.scaled_gemm_packed(a, a_sf, b, b_sf, c, flags)  # adds the tile-height bits a tiled packing needs
+        # (the GEMM calls add the tile-height bits a tiled packing needs)
+        if t.broadcast_a_scale:
+            with self._broadcasting:
+                a_sf = ops.repack_scales_broadcast(a_scale, K, out=self._a_scale_buffer(a.device, M, K))
+                ops.scaled_gemm_packed(a, a_sf, b, b_sf, c, flags)
+        elif isinstance(a_scale, ops.PackedScales):
+            ops.scaled_gemm_packed(a, a_scale, b, b_sf, c, flags)
+        else:  # packed by the call itself, ahead of the GEMM
+            a_scale = self._check_scale(a_scale, M, K, "a_scale")
+            if a_scale.stride(1) != 1:
+                a_scale = a_scale.contiguous()
+            ops.scaled_gemm_packed(a, ops.PackedScales(self._a_scale_buffer(a.device, M, K), M, K), b, b_sf, c, flags, a_scale=a_scale)
 
     @staticmethod
     def _check_scale(s, rows, K, name):
@@ -420,12 +431,6 @@ class ScaledGemmKernel:
         if not capturing:
             self._a_scale_last.setdefault(idx, [None])[0] = key
         return bufs[-1]
-
-    def _pack_activation_scales(self, a_scale, M, K):
-        if isinstance(a_scale, ops.PackedScales):
-            return a_scale
-        self._check_scale(a_scale, M, K, "a_scale")
-        return ops.repack_scales(a_scale, out=self._a_scale_buffer(a_scale.device, M, K))
 
 
 def invoke_with_profile(options: WaveCompileOptions, invoke, *args, **kwargs):

@@ -165,6 +165,19 @@ static wb::RowScales row_scales_param(int M, int K) {
   s.kblocks = K / 32;
   return s;
 }
+// A call that makes several launches over memory of the caller's (scratch for packed scales, the expert MLP's workspace) makes them in
+// one piece: another thread with the same memory and stream may not get in between. (launch_splitk has a lock of its own.)
+class LaunchSequence {
+ public:
+  explicit LaunchSequence(const void* memory) : lock_(mutexes_[(reinterpret_cast<uintptr_t>(memory) >> 8) % kLocks]) {}
+
+ private:
+  static constexpr int kLocks = 64;
+  static std::mutex mutexes_[kLocks];
+  std::lock_guard<std::mutex> lock_;
+};
+std::mutex LaunchSequence::mutexes_[LaunchSequence::kLocks];
+
 struct GroupNScope {  // restores the previous value on every return path
   int saved;
   explicit GroupNScope(unsigned flags) : saved(tl_group_n) { tl_group_n = group_n_from_flags(flags); }
@@ -1831,6 +1844,7 @@ int wb200_mxfp4_gemm_repack_a(int M, int N, int K, const void* a, const void* a_
     PendingScope(const void* src, long long stride, void* scratch) { tl_row_scales = {src, stride, scratch}; }
     ~PendingScope() { tl_row_scales = {}; tl_dependent_launch = false; }
   } pending(a_scale, a_scale_stride, a_scale_scratch);
+  LaunchSequence sequence(a_scale_scratch);
   return wb200_mxfp4_gemm(M, N, K, a, a_scale_scratch, b, b_scale_packed, c, c_dtype, ldc, workspace, workspace_bytes, flags, stream);
 }
 
@@ -1848,6 +1862,7 @@ int wb200_mxfp4_gemm_quantize_a(int M, int N, int K, const void* x, int x_dtype,
   // 512 x 4001 x 4096 33.5 / 31.9, 2000 x 5803 x 5344 163 / 156, 300 x 11001 x 4096 65.9 / 67.5; aligned: 512 x 5808 x 5344 16.4 / 16.6,
   // 300 x 11000 x 4096 16.0 / 17.2, 3000 x 8192 x 8192 83.7 / 84.5).
   const bool dependent = M <= 128 || rows_aligned(c, ldc, c_dtype);
+  LaunchSequence sequence(q_scratch);
   rc = quantize_mxfp4_impl(x, x_dtype, ldx, M, K, q_scratch, nullptr, scale_scratch, dependent, stream);
   if (rc) return rc;
   tl_dependent_launch = dependent;
@@ -1950,6 +1965,7 @@ int wb200_mxfp8_gemm_repack_a(int M, int N, int K, const void* a, const void* a_
                               const void* b, const void* b_scale_packed, void* c, int c_dtype, long long ldc, int elem_format,
                               void* workspace, size_t workspace_bytes, unsigned flags, void* stream) {
   if (!a_scale_scratch) return fail(WB200_ERR_INVALID_ARG, "mxfp8_gemm_repack_a: null scratch for the packed activation scales");
+  LaunchSequence sequence(a_scale_scratch);
   tl_dependent_launch = (flags & WB200_OVERLAP_PREVIOUS) != 0;
   int rc = repack_scales_impl(a_scale, a_scale_stride, M, K, a_scale_scratch, stream, false, true);
   tl_dependent_launch = false;
@@ -2107,6 +2123,7 @@ int wb200_mxfp4_expert_mlp(int T, int E, int K, int inter, int N, int top_k, con
   int* inverse = reinterpret_cast<int*>(ws + plan.inverse);
   int *expert_ids = reinterpret_cast<int*>(ws + plan.expert_ids), *num_rows = reinterpret_cast<int*>(ws + plan.num_rows);
   unsigned int* counters = reinterpret_cast<unsigned int*>(ws + plan.counters);
+  LaunchSequence sequence(workspace);
   // Every launch after the first is kDependent. The first one waits before it releases the next, so what the kernels before this
   // call wrote (x, the logits) is complete for all of them.
   wb::RouteParams route;

@@ -240,9 +240,10 @@ def split_k_pays() -> bool:
 
 
 def scaled_gemm_packed(a: torch.Tensor, a_sf: PackedScales, b: torch.Tensor, b_sf: PackedScales, c: torch.Tensor,
-                       flags: int = _lib.PATH_AUTO) -> None:
+                       flags: int = _lib.PATH_AUTO, a_scale: torch.Tensor | None = None) -> None:
     """c[M, N] = dequant(a) @ dequant(b).T with both scale sets already packed. c may be a column
-    block of a wider matrix (row stride >= N)."""
+    block of a wider matrix (row stride >= N). a_scale: row-major scales of a ([M, K/32], unit column stride), packed into a_sf's
+    memory first in the same native call."""
     lib = _lib.load()
     M, N, K = a.shape[0], b.shape[0], a.shape[1] * 2
     if c.dtype not in _DTYPE_CODE:
@@ -266,14 +267,20 @@ def scaled_gemm_packed(a: torch.Tensor, a_sf: PackedScales, b: torch.Tensor, b_s
         ws_bytes = int(lib.wb200_mxfp4_gemm_workspace_bytes(M, N, K))  # skinny shapes and split-K shapes use one
         if ws_bytes:
             ws_ptr = _workspace(a.device, ws_bytes, "skinny" if M <= 128 else "splitk").data_ptr()
-    dev_index = a.device.index
-    if dev_index is None or dev_index == torch.cuda.current_device():
-        rc = lib.wb200_mxfp4_gemm(M, N, K, a.data_ptr(), a_sf.data.data_ptr(), b.data_ptr(), b_sf.data.data_ptr(),
-                                  c.data_ptr(), _DTYPE_CODE[c.dtype], ldc, ws_ptr, ws_bytes, flags, _stream())
+
+    def run():
+        if a_scale is not None:
+            return lib.wb200_mxfp4_gemm_repack_a(M, N, K, a.data_ptr(), a_scale.data_ptr(), a_scale.stride(0) if M > 1 else K // 32,
+                                                 a_sf.data.data_ptr(), b.data_ptr(), b_sf.data.data_ptr(), c.data_ptr(), _DTYPE_CODE[c.dtype],
+                                                 ldc, ws_ptr, ws_bytes, flags, _stream())
+        return lib.wb200_mxfp4_gemm(M, N, K, a.data_ptr(), a_sf.data.data_ptr(), b.data_ptr(), b_sf.data.data_ptr(),
+                                    c.data_ptr(), _DTYPE_CODE[c.dtype], ldc, ws_ptr, ws_bytes, flags, _stream())
+
+    if a.device.index is None or a.device.index == torch.cuda.current_device():
+        rc = run()
     else:
         with torch.cuda.device(a.device):
-            rc = lib.wb200_mxfp4_gemm(M, N, K, a.data_ptr(), a_sf.data.data_ptr(), b.data_ptr(), b_sf.data.data_ptr(),
-                                      c.data_ptr(), _DTYPE_CODE[c.dtype], ldc, ws_ptr, ws_bytes, flags, _stream())
+            rc = run()
     if rc:
         _lib.check(rc)
 
