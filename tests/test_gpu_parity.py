@@ -2016,3 +2016,20 @@ def test_threads_share_a_kernel_object_and_a_stream(kind, M):
         sys.setswitchinterval(interval)
     assert wrong == [0, 0]
     ops.check_device_status()
+
+
+def test_a_workspace_that_is_not_aligned_is_no_obstacle_where_none_is_used():
+    """Fewer 128-row tiles than SMs, one tile per SM: the whole-tile kernel, or with a workspace it cannot use the tile kernel that ran there before."""
+    M, N, K = 16, 18800, 512
+    a, a_s, b, b_s = random_problem(M, N, K, seed=7)
+    ad, bd, a_sf, b_sf = a.to(DEV), b.to(DEV), ops.repack_scales(a_s.to(DEV)), ops.repack_scales(b_s.to(DEV))
+    lib, ref = _lib.load(), orc.scaled_gemm(a, a_s, b, b_s)
+    assert ops.decode_tile_rows_for(M, N, K) == 128
+    n = int(lib.wb200_mxfp4_gemm_workspace_bytes(M, N, K))
+    ws = torch.zeros(n + 16, dtype=torch.uint8, device=DEV)
+    for shift in (0, 8):
+        c = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+        _lib.check(lib.wb200_mxfp4_gemm(M, N, K, ad.data_ptr(), a_sf.data.data_ptr(), bd.data_ptr(), b_sf.data.data_ptr(), c.data_ptr(), _lib.WB200_BF16, N,
+                                        ws.data_ptr() + shift, n, 0, torch.cuda.current_stream().cuda_stream))
+        check(c, a, a_s, b, b_s, ref=ref)
+    ops.check_device_status()

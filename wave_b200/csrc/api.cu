@@ -1185,9 +1185,10 @@ enum class DecodeRoute { kSkinny, kTile1, kTile2, kCluster };
 // (14336 x 4096 15.1 / 13.2; unaligned 5803 x 5376, M = 32: 17.5 / 14.4). Where K is long enough and the tiles are few, a cluster
 // per tile: always ahead above 16 rows (M = 17: 4096 x 14336 16.3 / 18.2 for the K split, 2048 x 10240 14.5 / 19.7).
 constexpr long long kRouteActivationBytes = 128 << 10;
-DecodeRoute decode_route(int sm_count, int M, int N, int K, bool c_aligned) {
+// (ws_aligned: the whole-tile kernel can use the workspace. With fewer tiles than SMs a call may also run on a tile kernel, which needs none.)
+DecodeRoute decode_route(int sm_count, int M, int N, int K, bool c_aligned, bool ws_aligned) {
   const int tiles = (N + 127) / 128, kb = (K + 255) / 256;
-  if (tiles >= sm_count || skinny_takes_whole_tiles(sm_count, M, N, K, 4, false, c_aligned)) return DecodeRoute::kSkinny;
+  if (tiles >= sm_count || (ws_aligned && skinny_takes_whole_tiles(sm_count, M, N, K, 4, false, c_aligned))) return DecodeRoute::kSkinny;
   const long long units = (long long)tiles * kb, sms = sm_count;
   const bool few_activations = (long long)M * K / 2 < kRouteActivationBytes;
   const int slices = cluster_splitk_slices(M, N, K);
@@ -1763,7 +1764,7 @@ int wb200_mxfp4_gemm(int M, int N, int K, const void* a, const void* a_scale_pac
     if (M <= 128 && ws_ok) {
       path = WB200_PATH_SKINNY;
       if (tl_b_tile_rows == 128 && !(flags & (WB200_TILE_N128 | WB200_TILE_N192))) {
-        const DecodeRoute route = decode_route(dev->sm_count, M, N, K, rows_aligned(c, ldc, c_dtype));
+        const DecodeRoute route = decode_route(dev->sm_count, M, N, K, rows_aligned(c, ldc, c_dtype), (reinterpret_cast<uintptr_t>(workspace) & 15) == 0);
         if (route != DecodeRoute::kSkinny) {
           path = route == DecodeRoute::kTile1 ? WB200_PATH_TILE_1CTA : WB200_PATH_TILE_2CTA;
           if (route != DecodeRoute::kCluster) route_bn = 128;
