@@ -2033,3 +2033,31 @@ def test_a_workspace_that_is_not_aligned_is_no_obstacle_where_none_is_used():
                                         ws.data_ptr() + shift, n, 0, torch.cuda.current_stream().cuda_stream))
         check(c, a, a_s, b, b_s, ref=ref)
     ops.check_device_status()
+
+
+def test_calls_in_inference_mode_are_recognised():
+    """Tensors made in inference mode (every output of a layer there) take the native call as others do, with the bits of the ordinary ones. Weight scales
+    made there have no version counter and are refused as before."""
+    g = torch.Generator().manual_seed(8)
+    layers = [wb.MXFP4Linear.from_float((torch.randn(512, 512, generator=g) * 0.05).to(DEV)) for _ in range(3)]
+    x = torch.randn(8, 512, generator=g).to(torch.bfloat16).to(DEV)
+    ref = layers[2](layers[1](layers[0](x)))
+    M, N, K = 8, 640, 416
+    t, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    gemm = wb.wave_compile(wb.set_default_run_config(options), t)
+    args = [v.to(DEV) for v in random_problem(M, N, K, seed=1)]
+    c_ref = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    gemm(*args, c_ref)
+    with torch.inference_mode(), pytest.MonkeyPatch.context() as mp:
+        layers[0](x), gemm(*args, torch.empty_like(c_ref))
+        mp.setattr(wb.MXFP4Linear, "_forward_checked", lambda *a: pytest.fail("left to the Python code"))
+        y = layers[2](layers[1](layers[0](x)))
+        assert y.is_inference() and torch.equal(y, ref)
+        made = [v.clone() for v in args]
+        for operands in ([*made[:3], args[3]], [*made[:3], args[3]]):
+            c = torch.full_like(c_ref, float("nan"))
+            assert c.is_inference() and gemm._fast.call(*operands, c, options.decode_tiled_weight_scales, options.kernel_path) == 0
+            assert torch.equal(c, c_ref)
+        with pytest.raises(RuntimeError):
+            gemm(*made, c)
+    ops.check_device_status()

@@ -12,7 +12,7 @@
 // (a weak reference), its version counter, address, sizes and strides, as WeightScaleCache does. Nothing about activations or outputs
 // is kept but their shapes. A call notes whose scratch and workspace it used where the Python code notes it (`marks`): a captured call takes the
 // memory of the eager call before it. Calls under stream capture, on another device than the current one, with tensor subclasses, under
-// functional transforms, or with inference tensors are left to the Python code.
+// functional transforms, or with weight scales that are inference tensors (which have no version) are left to the Python code.
 // us per call, calls back to back: 1024^3 f32 16.9 -> 8.2 (the GPU's time now), MXFP4Linear 8 x 14336 x 4096 26.8 -> 15.6.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -64,14 +64,16 @@ bool is_mark(PyObject* m) {
 }
 void set_mark(PyObject* m) { PyList_SetItem(PyTuple_GET_ITEM(m, 0), 0, Py_NewRef(PyTuple_GET_ITEM(m, 1))); }
 
-// An ordinary CUDA tensor: no subclass, no wrapper of a functional transform, no inference tensor.
+// An ordinary CUDA tensor: no subclass, no wrapper of a functional transform. Tensors made in inference mode count (a layer's output there is the
+// next one's input): they only lack the autograd keys.
 bool plain(PyObject* o) {
   if (Py_TYPE(o) != reinterpret_cast<PyTypeObject*>(THPVariableClass)) return false;
   const at::Tensor& t = THPVariable_Unpack(o);
-  static const c10::DispatchKeySet keys = c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::ADInplaceOrView}) |
-                                          c10::getAutogradRelatedKeySetFromBackend(c10::BackendComponent::CUDABit) |
-                                          c10::getAutocastRelatedKeySetFromBackend(c10::BackendComponent::CUDABit);
-  return t.key_set() == keys && t.layout() == at::kStrided;
+  static const c10::DispatchKeySet inference = c10::DispatchKeySet(c10::DispatchKey::CUDA) |
+                                               c10::getAutocastRelatedKeySetFromBackend(c10::BackendComponent::CUDABit);
+  static const c10::DispatchKeySet ordinary = inference | c10::DispatchKeySet(c10::DispatchKey::ADInplaceOrView) |
+                                              c10::getAutogradRelatedKeySetFromBackend(c10::BackendComponent::CUDABit);
+  return (t.key_set() == ordinary || t.key_set() == inference) && t.layout() == at::kStrided;
 }
 
 struct Signature {
@@ -159,6 +161,7 @@ struct PyCalls {
 bool key_of(PyObject* const* args, CallKey* key) {
   for (int i = 0; i < 5; ++i)
     if (!plain(args[i])) return false;
+  if (THPVariable_Unpack(args[3]).is_inference()) return false;
   const at::Tensor& a = THPVariable_Unpack(args[0]);
   key->device = a.device().index();
   if (key->device != c10::cuda::current_device()) return false;
