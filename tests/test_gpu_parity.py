@@ -2061,3 +2061,47 @@ def test_calls_in_inference_mode_are_recognised():
         with pytest.raises(RuntimeError):
             gemm(*made, c)
     ops.check_device_status()
+
+
+def test_one_kernel_object_over_many_weights(monkeypatch):
+    """More layers than one object's tables held, each at a decode and a prefill size: packed once per size, recognised from the second walk on, given back when
+    their weights are gone. Where a packing has to go, it is not one that native calls have just read."""
+    N, K, n = 512, 256, 100
+    t, options = wb.get_tagged_mxfp4_gemm((8, N, K), output_dtype=wb.bf16)
+    options.dynamic_symbols = ["M"]
+    gemm = wb.wave_compile(wb.set_default_run_config(options), t)
+    weights = [[v.to(DEV) for v in random_problem(8, N, K, seed=i)[2:]] for i in range(n)]
+    acts = [[v.to(DEV) for v in random_problem(m, N, K, seed=m)[:2]] for m in (8, 200)]
+    heights = {ops.decode_tile_rows_for(8, N, K), 128}
+    assert len(heights) == 2
+
+    def walk():
+        outs = []
+        for b, b_s in weights:
+            for a, a_s in acts:
+                outs.append(torch.empty(a.shape[0], N, dtype=torch.bfloat16, device=DEV))
+                gemm(a, a_s, b, b_s, outs[-1])
+        return outs
+
+    first, packed = walk(), gemm._weight_scales.packings
+    assert packed == 2 * n
+    with monkeypatch.context() as mp:
+        mp.setattr(gemm, "_launch", lambda *a: pytest.fail("left to the Python code"))
+        again = walk()
+    assert all(torch.equal(x, y) for x, y in zip(first, again))
+    check(first[0], acts[0][0].cpu(), acts[0][1].cpu(), *(v.cpu() for v in weights[0]))
+    keep = weights[:2]
+    del weights[:]
+    weights += keep
+    weights.append([v.clone() for v in keep[0]])
+    walk()
+    assert gemm._weight_scales.packings == 2 * n + 2 and len(gemm._weight_scales._entries) == 6
+    gemm.drop_cached_weights()
+    gemm._weight_scales.capacity = 2
+    a, a_s = acts[0]
+    c = torch.empty(8, N, dtype=torch.bfloat16, device=DEV)
+    for i in (0, 1, 0, 0, 2):  # weight 0 is used through native calls only when room is made for weight 2
+        gemm(a, a_s, *weights[i], c)
+    owners = [owner() for owner, _ in gemm._weight_scales._entries.values()]
+    assert [any(o is weights[i][1] for o in owners) for i in range(3)] == [True, False, True]
+    ops.check_device_status()

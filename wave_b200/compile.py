@@ -119,7 +119,6 @@ class ScaledGemmKernel:
         self.template = template
         self.options = options
         self.asm = ""  # the reference exposes generated code here; nothing is generated at run time
-        self._weight_scales = ops.WeightScaleCache()
         self._a_scale_buf: dict[tuple[int, int], list[torch.Tensor]] = {}  # (device, stream) -> scratches, the one in use last
         self._a_scale_last: dict[int, list] = {}  # device -> [key] of the eager call before; native calls write the element too
         self._broadcasting = threading.Lock()  # from the packing of broadcast scales into the scratch to the launch that reads it
@@ -128,6 +127,7 @@ class ScaledGemmKernel:
         self._tile_rows: dict = {}
         self._lib = _lib.load()
         self._fast = _lib.fast().Calls()  # calls made before, recognised in native code
+        self._weight_scales = ops.WeightScaleCache(recent=self._fast.recent)
         self._bound_lib = self._lib  # the library that module calls: not used once `_lib` is another object
         self._static = None
         if template.shape is not None and not options.dynamic_symbols:

@@ -27,11 +27,15 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <iterator>
+#include <unordered_map>
 #include <vector>
 
 namespace {
 
-constexpr size_t kMaxPlans = 64, kMaxWeights = 64;
+// A model that walks all its layers through one kernel object uses one or two packings per layer, and one plan per distinct row count. Those of weights
+// that are gone are given back at the next registration.
+constexpr size_t kMaxPlans = 1024, kMaxWeights = 512;
 constexpr int kF32 = 0, kBF16 = 1;  // WB200_F32, WB200_BF16
 
 struct Abi {
@@ -108,8 +112,18 @@ struct CallKey {  // order: a, a_scale, b, b_scale, c
     return stream == o.stream && device == o.device && aligned == o.aligned && tiled == o.tiled && path == o.path && std::equal(sig, sig + 5, o.sig);
   }
 };
+struct CallKeyHash {
+  size_t operator()(const CallKey& k) const {
+    uint64_t h = reinterpret_cast<uintptr_t>(k.stream) + uint64_t(k.device) * 4 + k.aligned * 2 + k.tiled + uint64_t(k.path) * 64;
+    auto mix = [&h](uint64_t v) { h = (h ^ v) * 0x9e3779b97f4a7c15ull, h ^= h >> 29; };
+    for (const Signature& s : k.sig) {
+      for (int i = 0; i < 2; ++i) mix(uint64_t(s.size[i])), mix(uint64_t(s.stride[i]));
+      mix(uint64_t(s.type));
+    }
+    return size_t(h);
+  }
+};
 struct Plan {
-  CallKey key;
   int M, N, K;
   int elem_format;  // -1: MXFP4
   unsigned flags;
@@ -120,7 +134,6 @@ struct Plan {
 };
 struct Weight {
   c10::weak_intrusive_ptr<c10::TensorImpl> owner;
-  const c10::TensorImpl* impl;
   Signature sig;
   const void* ptr;
   uint32_t version;
@@ -128,28 +141,33 @@ struct Weight {
   at::Tensor packed;
   cudaStream_t stream;  // the one that the packing was filled on,
   bool complete;        // and whether that is known to be done: until then the Python code orders other streams behind it
+  uint64_t used;        // when the last call read it
 };
 
 struct Calls {
-  std::vector<Plan> plans;
-  std::vector<Weight> weights;
-  size_t next_plan = 0, next_weight = 0, last_plan = 0;
+  std::unordered_map<CallKey, Plan, CallKeyHash> plans;
+  std::unordered_multimap<const c10::TensorImpl*, Weight> weights;
+  uint64_t now = 0, asked = 0;  // calls so far, and when the Python code last asked which packings were used
 
-  const Plan* find(const CallKey& key) {
-    if (last_plan < plans.size() && plans[last_plan].key == key) return &plans[last_plan];
-    for (size_t i = 0; i < plans.size(); ++i)
-      if (plans[i].key == key) {
-        last_plan = i;
-        return &plans[i];
-      }
+  Weight* find(const at::Tensor& scale, const Signature& sig, int tile_rows) {
+    const auto [first, last] = weights.equal_range(scale.unsafeGetTensorImpl());
+    for (auto it = first; it != last; ++it) {
+      Weight& w = it->second;
+      // (an address that another tensor has taken over belongs to a new object, and the reference to the old one has expired)
+      if (w.tile_rows == tile_rows && w.sig == sig && !w.owner.expired() && w.ptr == scale.data_ptr() && w.version == scale._version()) return &w;
+    }
     return nullptr;
   }
-  Weight* find(const at::Tensor& scale, const Signature& sig, int tile_rows) {
-    const c10::TensorImpl* impl = scale.unsafeGetTensorImpl();
-    for (Weight& w : weights)
-      // (an address that another tensor has taken over belongs to a new object, and the reference to the old one has expired)
-      if (w.impl == impl && w.tile_rows == tile_rows && w.sig == sig && !w.owner.expired() && w.ptr == scale.data_ptr() && w.version == scale._version()) return &w;
-    return nullptr;
+  void insert(const c10::TensorImpl* impl, Weight w) {
+    for (auto it = weights.begin(); it != weights.end();)
+      it = it->second.owner.expired() || (it->first == impl && it->second.tile_rows == w.tile_rows) ? weights.erase(it) : std::next(it);
+    if (weights.size() >= kMaxWeights) {  // the one that was not used for longest
+      auto oldest = weights.begin();
+      for (auto it = weights.begin(); it != weights.end(); ++it)
+        if (it->second.used < oldest->second.used) oldest = it;
+      weights.erase(oldest);
+    }
+    weights.emplace(impl, std::move(w));
   }
 };
 
@@ -193,9 +211,11 @@ PyObject* calls_call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
       if (PyErr_Occurred()) return nullptr;
       Py_RETURN_NONE;
     }
-    const Plan* found = calls.find(key);
-    const Weight* weight = found ? calls.find(THPVariable_Unpack(args[3]), key.sig[3], found->tile_rows) : nullptr;
+    const auto plan = calls.plans.find(key);
+    const Plan* found = plan == calls.plans.end() ? nullptr : &plan->second;
+    Weight* weight = found ? calls.find(THPVariable_Unpack(args[3]), key.sig[3], found->tile_rows) : nullptr;
     if (!weight || !(weight->complete || weight->stream == key.stream)) Py_RETURN_NONE;
+    weight->used = ++calls.now;
     // another thread may change the tables while the lock is released: what the launch reads is held here
     const at::Tensor scratch = found->scratch, workspace = found->workspace, packed = weight->packed;
     const int M = found->M, N = found->N, K = found->K, elem_format = found->elem_format;
@@ -238,41 +258,33 @@ PyObject* calls_add(PyObject* self, PyObject* const* args, Py_ssize_t n) {
   try {
     Calls& calls = *reinterpret_cast<PyCalls*>(self)->calls;
     Plan p;
+    CallKey key;
     Py_ssize_t ws_bytes = 0;
     if (!PyArg_ParseTuple(args[7], "iiiiIin", &p.M, &p.N, &p.K, &p.elem_format, &p.flags, &p.tile_rows, &ws_bytes)) return nullptr;
-    if (!key_of(args, &p.key) || !THPVariable_Check(args[8]) || !THPVariable_Check(args[9])) {
+    if (!key_of(args, &key) || !THPVariable_Check(args[8]) || !THPVariable_Check(args[9])) {
       if (PyErr_Occurred()) return nullptr;
       Py_RETURN_NONE;
     }
-    const at::ScalarType c_type = p.key.sig[4].type;
-    if (p.key.sig[4].stride[1] != 1 || (c_type != at::kFloat && c_type != at::kBFloat16)) Py_RETURN_NONE;
+    const at::ScalarType c_type = key.sig[4].type;
+    if (key.sig[4].stride[1] != 1 || (c_type != at::kFloat && c_type != at::kBFloat16)) Py_RETURN_NONE;
     p.scratch = THPVariable_Unpack(args[9]);
     if (args[10] != Py_None) p.workspace = THPVariable_Unpack(args[10]);
     p.workspace_bytes = size_t(ws_bytes);
     p.marks = Ref(args[11]);
-    if (const Plan* old = calls.find(p.key)) {
-      const_cast<Plan&>(*old) = p;
-    } else if (calls.plans.size() < kMaxPlans) {
-      calls.plans.push_back(p);
-    } else {
-      calls.plans[calls.next_plan++ % kMaxPlans] = p;
-    }
+    if (calls.plans.size() >= kMaxPlans && !calls.plans.count(key)) calls.plans.erase(calls.plans.begin());
+    const int tile_rows = p.tile_rows;
+    calls.plans[key] = std::move(p);
     const at::Tensor& scale = THPVariable_Unpack(args[3]);
     const auto filled_on = reinterpret_cast<cudaStream_t>(PyLong_AsUnsignedLongLong(args[12]));
     const bool complete = PyObject_IsTrue(args[13]) == 1;
     if (PyErr_Occurred()) return nullptr;
-    Weight* known = calls.find(scale, p.key.sig[3], p.tile_rows);
+    Weight* known = calls.find(scale, key.sig[3], tile_rows);
     if (known && known->packed.is_same(THPVariable_Unpack(args[8]))) {
       known->complete = known->complete || complete;
     } else {
-      const auto gone = std::remove_if(calls.weights.begin(), calls.weights.end(), [&](const Weight& w) {
-        return w.owner.expired() || (w.impl == scale.unsafeGetTensorImpl() && w.tile_rows == p.tile_rows);
-      });
-      calls.weights.erase(gone, calls.weights.end());
-      Weight w{c10::weak_intrusive_ptr<c10::TensorImpl>(scale.getIntrusivePtr()), scale.unsafeGetTensorImpl(), p.key.sig[3], scale.data_ptr(),
-               uint32_t(scale._version()), p.tile_rows, THPVariable_Unpack(args[8]), filled_on, complete};
-      if (calls.weights.size() < kMaxWeights) calls.weights.push_back(std::move(w));
-      else calls.weights[calls.next_weight++ % kMaxWeights] = std::move(w);
+      calls.insert(scale.unsafeGetTensorImpl(),
+                   Weight{c10::weak_intrusive_ptr<c10::TensorImpl>(scale.getIntrusivePtr()), key.sig[3], scale.data_ptr(), uint32_t(scale._version()),
+                          tile_rows, THPVariable_Unpack(args[8]), filled_on, complete, ++calls.now});
     }
     Py_RETURN_NONE;
   } catch (const std::exception& e) {
@@ -285,6 +297,26 @@ PyObject* calls_clear(PyObject* self, PyObject*) {
   calls.plans.clear();
   calls.weights.clear();
   Py_RETURN_NONE;
+}
+
+// recent() -> addresses of the packings that calls have read since it was asked last, the one used last at the end
+PyObject* calls_recent(PyObject* self, PyObject*) {
+  Calls& calls = *reinterpret_cast<PyCalls*>(self)->calls;
+  std::vector<std::pair<uint64_t, const void*>> used;
+  for (const auto& [impl, w] : calls.weights)
+    if (w.used > calls.asked) used.emplace_back(w.used, w.packed.data_ptr());
+  calls.asked = calls.now;
+  std::sort(used.begin(), used.end());
+  PyObject* list = PyList_New(Py_ssize_t(used.size()));
+  for (size_t i = 0; list && i < used.size(); ++i) {
+    PyObject* address = PyLong_FromVoidPtr(const_cast<void*>(used[i].second));
+    if (!address) {
+      Py_DECREF(list);
+      return nullptr;
+    }
+    PyList_SET_ITEM(list, Py_ssize_t(i), address);
+  }
+  return list;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -450,7 +482,8 @@ PyObject* bind(PyObject*, PyObject* args) {
 
 #define FASTCALL(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL
 PyMethodDef calls_methods[] = {{"call", FASTCALL(calls_call), nullptr}, {"add", FASTCALL(calls_add), nullptr},
-                               {"clear", calls_clear, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
+                               {"clear", calls_clear, METH_NOARGS, nullptr}, {"recent", calls_recent, METH_NOARGS, nullptr},
+                               {nullptr, nullptr, 0, nullptr}};
 PyMethodDef workspaces_methods[] = {{"put", FASTCALL(workspaces_put), nullptr}, {"clear", workspaces_clear, METH_NOARGS, nullptr},
                                     {nullptr, nullptr, 0, nullptr}};
 PyMethodDef module_methods[] = {{"bind", bind, METH_VARARGS, nullptr}, {"linear", FASTCALL(linear), nullptr},

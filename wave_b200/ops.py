@@ -419,8 +419,10 @@ class WeightScaleCache:
     as long as the cache, whatever is evicted or dropped: the graph holds its address. One that is made while a graph is
     captured is filled by the replays only and not given to any other call."""
 
-    def __init__(self, capacity: int = 64):
-        self.capacity = capacity
+    def __init__(self, capacity: int = 512, recent=None):
+        """capacity: packings kept, of weights that are alive (one or two per weight). recent: called before a packing is evicted, gives the
+        addresses of those that calls have read past this cache, the last one at the end."""
+        self.capacity, self.recent = capacity, recent
         self.packings = 0  # launched so far: a call that moves it has put a repack kernel in front of its GEMM
         self._entries: OrderedDict = OrderedDict()
         self._captured: dict = {}
@@ -444,10 +446,21 @@ class WeightScaleCache:
         stream, event = torch.cuda.current_stream(packed.device), torch.cuda.Event()
         event.record(stream)
         packed.made = (stream.cuda_stream, event)
+        self._make_room()
         self._entries[key] = (weakref.ref(scale), packed)
         while len(self._entries) > self.capacity:
             self._entries.popitem(last=False)
         return packed
+
+    def _make_room(self) -> None:
+        """Drops the packings of weights that are gone; of the others the ones used last, here or past this cache, come last."""
+        for key in [k for k, (owner, _) in self._entries.items() if owner() is None]:
+            del self._entries[key]
+        if self.recent is not None and len(self._entries) >= self.capacity:
+            keys = {packed.data.data_ptr(): key for key, (_, packed) in self._entries.items()}
+            for address in self.recent():
+                if address in keys:
+                    self._entries.move_to_end(keys[address])
 
     @staticmethod
     def _usable(packed: PackedScales) -> bool:
