@@ -2105,3 +2105,23 @@ def test_one_kernel_object_over_many_weights(monkeypatch):
     owners = [owner() for owner, _ in gemm._weight_scales._entries.values()]
     assert [any(o is weights[i][1] for o in owners) for i in range(3)] == [True, False, True]
     ops.check_device_status()
+
+
+def test_calls_without_the_host_module(monkeypatch):
+    """Where the host module cannot be used every call takes the Python code, captured ones included, with the same bits."""
+    from wave_b200.graphs import GraphedScaledGemm
+    M, N, K = 16, 1024, 512
+    t, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    args = [v.to(DEV) for v in random_problem(M, N, K, seed=1)]
+    layer, x = wb.MXFP4Linear(*args[2:]), torch.randn(M, K, device=DEV)
+    c_ref, ref = torch.empty(M, N, dtype=torch.bfloat16, device=DEV), layer(x)
+    wb.wave_compile(options, t)(*args, c_ref)
+    monkeypatch.setattr(_lib, "_fast", False)
+    monkeypatch.setattr(ops, "_pool", ops.WorkspacePool())
+    gemm, c = wb.wave_compile(options, t), torch.empty_like(c_ref)
+    for run in (lambda: gemm(*args, c), lambda: gemm(*args, c), GraphedScaledGemm(gemm, *args, c).replay):
+        c.fill_(float("nan"))
+        run()
+        assert torch.equal(c, c_ref)
+    assert torch.equal(layer(x), ref) and gemm._fast is None
+    ops.check_device_status()

@@ -213,3 +213,31 @@ def test_profile_python_wrapper_times_the_host_side(capsys):
     kernel, options = wb.get_tagged_mxfp4_gemm((64, 64, 64))
     options.profile_python_wrapper = True
     assert isinstance(wb.wave_compile(options, kernel), wc.ScaledGemmKernelWithProfile)
+
+
+def test_a_missing_or_foreign_host_module_is_a_warning(built_library, monkeypatch):
+    """Without `_fast.so`, or with one that was built for another torch, kernel objects are made and calls take the Python code."""
+    import sys
+
+    import wave_b200
+    from wave_b200 import build
+    assert not build.fast_stale() and _lib.fast().target == build.fast_target()
+    module = _lib.fast()
+    kernel, options = wb.get_tagged_mxfp4_gemm((16, 16, 64))
+    for missing in (True, False):
+        with monkeypatch.context() as mp:
+            mp.setattr(_lib, "_fast", None)
+            if missing:
+                mp.setitem(sys.modules, "wave_b200._fast", None)
+                mp.delattr(wave_b200, "_fast")
+            else:
+                mp.setattr(build, "fast_target", lambda: "torch 0.0, python 3.0")
+                assert build.fast_stale()
+            with pytest.warns(RuntimeWarning, match="slower Python path"):
+                gemm = wb.wave_compile(options, kernel)
+            assert gemm._fast is None and _lib.fast() is None
+            with pytest.raises(ValueError, match="no CPU path"):
+                s = torch.zeros(16, 2, dtype=torch.uint8)
+                gemm(torch.zeros(16, 32, dtype=torch.uint8), s, torch.zeros(16, 32, dtype=torch.uint8), s, torch.zeros(16, 16))
+            gemm.drop_cached_weights()
+    assert _lib.fast() is module

@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import warnings
 from pathlib import Path
 
 WB200_OK = 0
@@ -281,23 +282,29 @@ def load() -> ctypes.CDLL:
     return lib
 
 
-_fast = None
+_fast = None  # the module, or False where it cannot be used
 
 
 def fast():
-    """The host module for repeated calls (csrc/fast_call.cpp), bound to the loaded library."""
+    """The host module for repeated calls (csrc/fast_call.cpp), bound to the loaded library. None, with one warning, where it was not built or was
+    built for another torch: every call then takes the Python code, which is complete and only slower in front of short kernels."""
     global _fast
     if _fast is None:
         lib = load()
         try:
-            from . import _fast as module
+            from . import _fast as module, build
+            if getattr(module, "target", None) != build.fast_target():
+                raise ImportError(f"built for {getattr(module, 'target', 'an unknown torch')}, running {build.fast_target()}")
         except ImportError as e:
-            raise RuntimeError(f"wave_b200._fast cannot be loaded ({e}): build it with `python -m wave_b200.build`") from e
+            _fast = False
+            warnings.warn(f"wave_b200._fast cannot be used ({e}): repeated calls take the slower Python path. Build it with "
+                          "`python -m wave_b200.build`", RuntimeWarning, stacklevel=2)
+            return None
         module.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.wb200_mxfp4_gemm_repack_a, lib.wb200_mxfp8_gemm_repack_a,
                                                                       lib.wb200_mxfp4_gemm_quantize_a, lib.wb200_mxfp4_gemm_workspace_bytes,
                                                                       lib.wb200_decode_tile_rows_for)))
         _fast = module
-    return _fast
+    return _fast or None
 
 
 def check(rc: int) -> None:

@@ -69,9 +69,20 @@ FAST_OUT = PKG / "_fast.so"
 FAST_SOURCE = CSRC / "fast_call.cpp"
 
 
+def fast_target() -> str:
+    """What `_fast.so` is compiled against; the module carries it."""
+    import torch
+    return f"torch {torch.__version__}, python {sys.version_info.major}.{sys.version_info.minor}"
+
+
+def fast_stale() -> bool:
+    """`_fast.so` is missing, older than its source, or was compiled against another torch or Python."""
+    return not FAST_OUT.exists() or FAST_SOURCE.stat().st_mtime > FAST_OUT.stat().st_mtime or fast_target().encode() not in FAST_OUT.read_bytes()
+
+
 def build_fast(force: bool = False) -> Path:
-    """Compile `wave_b200._fast` (csrc/fast_call.cpp, against the installed torch) if it is missing or older than its source."""
-    if not force and FAST_OUT.exists() and FAST_SOURCE.stat().st_mtime <= FAST_OUT.stat().st_mtime:
+    """Compile `wave_b200._fast` (csrc/fast_call.cpp, against the installed torch) if it is not there as it should be (`fast_stale`)."""
+    if not force and not fast_stale():
         return FAST_OUT
     import sysconfig
 
@@ -81,6 +92,7 @@ def build_fast(force: bool = False) -> Path:
     includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", nvcc.parent.parent / "include",
                 Path(sysconfig.get_paths()["include"])]
     cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f'-DWB200_FAST_TARGET="{fast_target()}"',
            *(f"-I{i}" for i in includes), str(FAST_SOURCE), "-o", str(FAST_OUT), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
            "-ltorch_cuda", "-ltorch_python"]
     res = subprocess.run(cmd, capture_output=True, text=True)

@@ -126,9 +126,10 @@ class ScaledGemmKernel:
         self._plans: dict = {}
         self._tile_rows: dict = {}
         self._lib = _lib.load()
-        self._fast = _lib.fast().Calls()  # calls made before, recognised in native code
-        self._weight_scales = ops.WeightScaleCache(recent=self._fast.recent)
-        self._bound_lib = self._lib  # the library that module calls: not used once `_lib` is another object
+        native = _lib.fast()
+        self._fast = native.Calls() if native is not None else None  # calls made before, recognised in native code
+        self._weight_scales = ops.WeightScaleCache(recent=self._fast.recent if self._fast is not None else None)
+        self._bound_lib = self._lib if native is not None else None  # the library that module calls: not used once `_lib` is another object
         self._static = None
         if template.shape is not None and not options.dynamic_symbols:
             self._static = tuple(template.shape)
@@ -196,8 +197,9 @@ class ScaledGemmKernel:
         if not torch.cuda.is_current_stream_capturing():
             for holder, value in marks:
                 holder[0] = value
-            self._fast.add(a, a_scale, b, b_scale, c, self.options.decode_tiled_weight_scales, self.options.kernel_path, sizes, b_sf.data, scratch,
-                           workspace, marks, b_sf.made[0], b_sf.made[1] is None)
+            if self._fast is not None:
+                self._fast.add(a, a_scale, b, b_scale, c, self.options.decode_tiled_weight_scales, self.options.kernel_path, sizes, b_sf.data, scratch,
+                               workspace, marks, b_sf.made[0], b_sf.made[1] is None)
 
     def _marks(self, idx: int, pool=None, kind: str = "skinny") -> tuple:
         """What notes that the eager call before used the scratch, and with a pool the workspace, that were asked for just now."""
@@ -396,7 +398,8 @@ class ScaledGemmKernel:
         else:
             self._weight_scales.drop(b_scale)
         self._plans.clear()
-        self._fast.clear()
+        if self._fast is not None:
+            self._fast.clear()
 
     def _raster_flags(self) -> int:
         """The template's reorder_workgroups / group_size_n as the tile kernels' raster-group bits. The reference

@@ -517,5 +517,9 @@ PyMODINIT_FUNC PyInit__fast() {
     Py_DECREF(m);
     return nullptr;
   }
+  if (PyModule_AddStringConstant(m, "target", WB200_FAST_TARGET) < 0) {  // what this was compiled against
+    Py_DECREF(m);
+    return nullptr;
+  }
   return m;
 }

@@ -65,9 +65,12 @@ class MXFP4Linear(torch.nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         # a call whose tensors need no preparation; anything else comes back unhandled
+        native = _lib.fast()
+        if native is None:
+            return self._forward_checked(x)
         packed, low = self._packed, self._packed_low
-        y = _lib.fast().linear(x, self._buffers.get("weight_codes"), packed.rows, packed.K, packed.data, None if low is None else low.data,
-                               128 if low is None else low.tile_rows, self.output_dtype, ops._pool.fast)
+        y = native.linear(x, self._buffers.get("weight_codes"), packed.rows, packed.K, packed.data, None if low is None else low.data,
+                          128 if low is None else low.tile_rows, self.output_dtype, ops._pool.fast)
         if type(y) is int:
             _lib.check(y)
         elif y is not None:

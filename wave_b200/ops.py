@@ -171,8 +171,9 @@ class WorkspacePool:
 
     @property
     def fast(self):
-        if self._fast is None:
-            self._fast = _lib.fast().Workspaces()
+        native = _lib.fast()
+        if self._fast is None and native is not None:
+            self._fast = native.Workspaces()
         return self._fast
 
     def get(self, device: torch.device, nbytes: int, kind: str) -> torch.Tensor:
@@ -204,8 +205,8 @@ class WorkspacePool:
     def _note(self, key, ws: torch.Tensor) -> None:
         idx, stream, kind = key
         self._last.setdefault((idx, kind), [None])[0] = (key, ws)
-        if kind == "skinny":
-            self.fast.put(idx, stream, ws, self.mark(idx, kind))
+        if kind == "skinny" and self.fast is not None:
+            self._fast.put(idx, stream, ws, self.mark(idx, kind))
 
     def mark(self, idx: int, kind: str) -> tuple:
         """(list, value): storing the value as the list's element says that the eager call before used what it used just now."""
@@ -469,7 +470,8 @@ class WeightScaleCache:
         stream, event = packed.made
         capturing = torch.cuda.is_current_stream_capturing()
         if event is not None:
-            if _lib.fast().event_done(event.cuda_event):
+            native = _lib.fast()  # (asks in a way that does not end another thread's capture, or this one)
+            if native.event_done(event.cuda_event) if native is not None else not capturing and event.query():
                 packed.made, event = (stream, None), None
             elif capturing:
                 return False
