@@ -2125,3 +2125,47 @@ def test_calls_without_the_host_module(monkeypatch):
         assert torch.equal(c, c_ref)
     assert torch.equal(layer(x), ref) and gemm._fast is None
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("where", ["handle", "function"])
+def test_calls_through_a_library_that_was_replaced_are_seen(where, monkeypatch):
+    """A caller that puts an object in the place of the library, or a function in the place of one of its functions, sees every call of the linear layer and of the
+    templates, also of forms that native code knows; and none of them once it has taken that back."""
+    M, N, K = 16, 1024, 512
+    t, options = wb.get_tagged_mxfp4_gemm((M, N, K), output_dtype=wb.bf16)
+    t8, subs = wb.get_scaled_gemm_mxfp8_kernel((M, N, K), wb.ScaledMMAType.F32_16x16x128_F8F6F4, "f8e4m3fn", wb.bf16)
+    gemm, gemm8 = wb.wave_compile(options, t), wb.wave_compile(wb.WaveCompileOptions(subs=subs), t8)
+    args = [v.to(DEV) for v in random_problem(M, N, K, seed=1)]
+    x, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    args8 = [*ops.quantize_mxfp8(x, torch.float8_e4m3fn)[:2], *ops.quantize_mxfp8(w, torch.float8_e4m3fn)[:2]]
+    layer, c = wb.MXFP4Linear(*args[2:]), torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    lib, seen = _lib.load(), []
+    entries = ["wb200_mxfp4_gemm_repack_a", "wb200_mxfp8_gemm_repack_a", "wb200_mxfp4_gemm_quantize_a"]
+
+    def calls():
+        gemm(*args, c), gemm8(*args8, c), layer(x)
+
+    def spy(name, fn):
+        return lambda *a: (seen.append(name), fn(*a))[1]
+
+    class Watched:
+        def __getattr__(self, name):
+            fn = getattr(lib, name)
+            return spy(name, fn) if name in entries else fn
+
+    for _ in range(2):
+        calls()
+    with monkeypatch.context() as mp:
+        if where == "handle":
+            for obj in (gemm, gemm8):
+                mp.setattr(obj, "_lib", Watched())
+            mp.setattr(_lib, "load", lambda: gemm._lib)
+        else:
+            for name in entries:
+                mp.setattr(lib, name, spy(name, getattr(lib, name)))
+        for _ in range(2):
+            calls()
+        assert seen == 2 * entries
+    calls()
+    assert len(seen) == 6
+    ops.check_device_status()

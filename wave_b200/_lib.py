@@ -283,14 +283,19 @@ def load() -> ctypes.CDLL:
 
 
 _fast = None  # the module, or False where it cannot be used
+_fast_bound: dict = {}  # the library and the functions that it calls
 
 
-def fast():
+def fast(lib=None, entry: str | None = None):
     """The host module for repeated calls (csrc/fast_call.cpp), bound to the loaded library. None, with one warning, where it was not built or was
-    built for another torch: every call then takes the Python code, which is complete and only slower in front of short kernels."""
+    built for another torch: every call then takes the Python code, which is complete and only slower in front of short kernels. None too where `lib` (default: the loaded library) or its function `entry` is not what the module
+    is bound to: a caller has put something in its place, to watch or to redirect calls."""
     global _fast
-    if _fast is None:
+    if lib is None:
         lib = load()
+    if _fast is None:
+        if not isinstance(lib, ctypes.CDLL):
+            return None
         try:
             from . import _fast as module, build
             if getattr(module, "target", None) != build.fast_target():
@@ -300,11 +305,14 @@ def fast():
             warnings.warn(f"wave_b200._fast cannot be used ({e}): repeated calls take the slower Python path. Build it with "
                           "`python -m wave_b200.build`", RuntimeWarning, stacklevel=2)
             return None
-        module.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (lib.wb200_mxfp4_gemm_repack_a, lib.wb200_mxfp8_gemm_repack_a,
-                                                                      lib.wb200_mxfp4_gemm_quantize_a, lib.wb200_mxfp4_gemm_workspace_bytes,
-                                                                      lib.wb200_decode_tile_rows_for)))
+        names = ("wb200_mxfp4_gemm_repack_a", "wb200_mxfp8_gemm_repack_a", "wb200_mxfp4_gemm_quantize_a", "wb200_mxfp4_gemm_workspace_bytes",
+                 "wb200_decode_tile_rows_for")
+        _fast_bound.update({name: getattr(lib, name) for name in names}, lib=lib)
+        module.bind(*(ctypes.cast(_fast_bound[name], ctypes.c_void_p).value for name in names))
         _fast = module
-    return _fast or None
+    if not _fast or lib is not _fast_bound["lib"] or (entry is not None and getattr(lib, entry) is not _fast_bound[entry]):
+        return None
+    return _fast
 
 
 def check(rc: int) -> None:

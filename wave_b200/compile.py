@@ -126,10 +126,10 @@ class ScaledGemmKernel:
         self._plans: dict = {}
         self._tile_rows: dict = {}
         self._lib = _lib.load()
-        native = _lib.fast()
+        self._entry = "wb200_mxfp8_gemm_repack_a" if template.element_bits == 8 else "wb200_mxfp4_gemm_repack_a"  # what a native call calls
+        native = _lib.fast(self._lib)
         self._fast = native.Calls() if native is not None else None  # calls made before, recognised in native code
         self._weight_scales = ops.WeightScaleCache(recent=self._fast.recent if self._fast is not None else None)
-        self._bound_lib = self._lib if native is not None else None  # the library that module calls: not used once `_lib` is another object
         self._static = None
         if template.shape is not None and not options.dynamic_symbols:
             self._static = tuple(template.shape)
@@ -147,7 +147,7 @@ class ScaledGemmKernel:
             finally:
                 self._in_bench = False
             return None
-        if self._lib is self._bound_lib:
+        if self._fast is not None and _lib.fast(self._lib, self._entry) is not None:
             options = self.options
             rc = self._fast.call(a, a_scale, b, b_scale, c, options.decode_tiled_weight_scales, options.kernel_path)
             if rc is not None:

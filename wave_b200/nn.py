@@ -65,7 +65,7 @@ class MXFP4Linear(torch.nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         # a call whose tensors need no preparation; anything else comes back unhandled
-        native = _lib.fast()
+        native = _lib.fast(None, "wb200_mxfp4_gemm_quantize_a")
         if native is None:
             return self._forward_checked(x)
         packed, low = self._packed, self._packed_low

@@ -171,9 +171,9 @@ class WorkspacePool:
 
     @property
     def fast(self):
-        native = _lib.fast()
-        if self._fast is None and native is not None:
-            self._fast = native.Workspaces()
+        if self._fast is None:
+            native = _lib.fast()
+            self._fast = native.Workspaces() if native is not None else None
         return self._fast
 
     def get(self, device: torch.device, nbytes: int, kind: str) -> torch.Tensor:
