@@ -158,7 +158,7 @@ class ScaledGemmKernel:
         if type(a_scale) is torch.Tensor and type(b_scale) is torch.Tensor and a.is_cuda:
             # (the stream is part of the signature: the plan holds a workspace, and calls on different streams may overlap)
             sig = (a.shape, a.stride(), a.dtype, a_scale.shape, a_scale.stride(), b.shape, b.stride(), b_scale.shape,
-                   c.shape, c.stride(), c.dtype, a.device, torch.cuda.current_stream(a.device).cuda_stream)
+                   c.shape, c.stride(), c.dtype, a.device, ops.raw_stream(a.device.index))
             plan = self._plans.get(sig)
             if plan is not None:
                 return self._launch(plan, a, a_scale, b, b_scale, c)
@@ -179,13 +179,13 @@ class ScaledGemmKernel:
         if dev_index == torch.cuda.current_device():
             rc = lib.wb200_mxfp4_gemm_repack_a(M, N, K, a.data_ptr(), a_scale.data_ptr(), a_scale.stride(0) if M > 1 else K // 32, a_buf.data_ptr(),
                                                b.data_ptr(), b_sf.data.data_ptr(), c.data_ptr(), dtype_code, c.stride(0) if M > 1 else N,
-                                               ws_ptr, ws_bytes, flags, torch.cuda.current_stream(dev_index).cuda_stream)
+                                               ws_ptr, ws_bytes, flags, ops.raw_stream(dev_index))
         else:
             with torch.cuda.device(dev_index):
                 rc = lib.wb200_mxfp4_gemm_repack_a(M, N, K, a.data_ptr(), a_scale.data_ptr(), a_scale.stride(0) if M > 1 else K // 32,
                                                    a_buf.data_ptr(), b.data_ptr(), b_sf.data.data_ptr(), c.data_ptr(),
                                                    dtype_code, c.stride(0) if M > 1 else N, ws_ptr, ws_bytes, flags,
-                                                   torch.cuda.current_stream(dev_index).cuda_stream)
+                                                   ops.raw_stream(dev_index))
         if rc:
             _lib.check(rc)
         flags = plan[6] | (_lib.B_TILE_ROWS(tile_rows) if tile_rows != 128 else 0)
@@ -312,7 +312,7 @@ class ScaledGemmKernel:
             marks = () if capturing else self._marks(idx, self._workspaces if ws_bytes else None, kind)
             plan = (M, N, K, a_buf, ws_ptr, ws_bytes, flags, ops._DTYPE_CODE[c.dtype], idx, ws, marks)
             sig = (a.shape, a.stride(), a.dtype, a_scale.shape, a_scale.stride(), b.shape, b.stride(), b_scale.shape,
-                   c.shape, c.stride(), c.dtype, a.device, torch.cuda.current_stream(a.device).cuda_stream)
+                   c.shape, c.stride(), c.dtype, a.device, ops.raw_stream(idx))
             if not capturing:  # (every capture takes the memory of its own warm-up)
                 self._plans[sig] = plan
             return self._launch(plan, a, a_scale, b, b_scale, c)
@@ -421,7 +421,7 @@ class ScaledGemmKernel:
         the stream that asked for one last, which is its warm-up's: allocating in a capture takes milliseconds."""
         idx = device.index if device.index is not None else torch.cuda.current_device()
         need = ops.packed_scale_bytes(M, K)
-        key = (idx, torch.cuda.current_stream(idx).cuda_stream)
+        key = (idx, ops.raw_stream(idx))
         bufs = self._a_scale_buf.get(key)
         capturing = torch.cuda.is_current_stream_capturing()
         if bufs is None or bufs[-1].numel() < need:

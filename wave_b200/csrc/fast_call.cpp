@@ -21,6 +21,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -320,6 +321,68 @@ PyObject* calls_recent(PyObject* self, PyObject*) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// What stands behind the work that the current stream of a device has been given so far: Fence(device)
+// ---------------------------------------------------------------------------------------------
+struct PyFence {
+  PyObject_HEAD
+  int device;
+  cudaStream_t stream;
+  cudaEvent_t event;
+};
+PyObject* fence_new(PyTypeObject* type, PyObject* args, PyObject*) {
+  int device;
+  if (!PyArg_ParseTuple(args, "i", &device)) return nullptr;
+  auto* self = reinterpret_cast<PyFence*>(type->tp_alloc(type, 0));
+  if (!self) return nullptr;
+  try {
+    const c10::cuda::CUDAGuard guard{c10::DeviceIndex(device)};
+    self->device = device;
+    self->stream = c10::cuda::getCurrentCUDAStream(device).stream();
+    cudaError_t rc = cudaEventCreateWithFlags(&self->event, cudaEventDisableTiming);
+    if (rc == cudaSuccess) rc = cudaEventRecord(self->event, self->stream);
+    if (rc == cudaSuccess) return reinterpret_cast<PyObject*>(self);
+    (void)cudaGetLastError();
+    PyErr_Format(PyExc_RuntimeError, "wave_b200: no event behind the work of stream %p: %s", self->stream, cudaGetErrorString(rc));
+  } catch (const std::exception& e) {
+    fail(e);
+  }
+  Py_DECREF(self);
+  return nullptr;
+}
+void fence_free(PyObject* o) {
+  auto* self = reinterpret_cast<PyFence*>(o);
+  if (self->event && cudaEventDestroy(self->event) != cudaSuccess) (void)cudaGetLastError();
+  Py_TYPE(o)->tp_free(o);
+}
+PyObject* fence_stream(PyObject* o, PyObject*) { return PyLong_FromVoidPtr(reinterpret_cast<PyFence*>(o)->stream); }
+// done() -> whether that work is complete; may be asked while a stream is being captured (the event is not part of the capture)
+PyObject* fence_done(PyObject* o, PyObject*) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // of this thread: a query does not end a capture then
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
+    (void)cudaGetLastError();
+    Py_RETURN_FALSE;
+  }
+  const cudaError_t status = cudaEventQuery(reinterpret_cast<PyFence*>(o)->event);
+  (void)cudaGetLastError();
+  (void)cudaThreadExchangeStreamCaptureMode(&mode);
+  return PyBool_FromLong(status == cudaSuccess);
+}
+// wait(): what the current stream of the device does next comes after that work
+PyObject* fence_wait(PyObject* o, PyObject*) {
+  auto* self = reinterpret_cast<PyFence*>(o);
+  try {
+    const c10::cuda::CUDAGuard guard{c10::DeviceIndex(self->device)};
+    const cudaError_t rc = cudaStreamWaitEvent(c10::cuda::getCurrentCUDAStream(self->device).stream(), self->event, 0);
+    if (rc == cudaSuccess) Py_RETURN_NONE;
+    (void)cudaGetLastError();
+    PyErr_SetString(PyExc_RuntimeError, cudaGetErrorString(rc));
+    return nullptr;
+  } catch (const std::exception& e) {
+    return fail(e);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // workspaces of the functional entry points, as WorkspacePool holds them
 // ---------------------------------------------------------------------------------------------
 struct Workspaces {
@@ -452,22 +515,6 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
 }
 
-// event_done(event) -> whether the work in front of a recorded event is complete; may be asked while a stream is being captured (the event
-// is not part of the capture)
-PyObject* event_done(PyObject*, PyObject* arg) {
-  auto event = reinterpret_cast<cudaEvent_t>(PyLong_AsUnsignedLongLong(arg));
-  if (PyErr_Occurred()) return nullptr;
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // of this thread: a query does not end a capture then
-  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
-    (void)cudaGetLastError();
-    Py_RETURN_FALSE;
-  }
-  const cudaError_t status = cudaEventQuery(event);
-  (void)cudaGetLastError();
-  (void)cudaThreadExchangeStreamCaptureMode(&mode);
-  return PyBool_FromLong(status == cudaSuccess);
-}
-
 // bind(gemm_repack_a, mxfp8_gemm_repack_a, gemm_quantize_a, gemm_workspace_bytes, decode_tile_rows_for): addresses in the loaded library
 PyObject* bind(PyObject*, PyObject* args) {
   unsigned long long p[5];
@@ -486,23 +533,24 @@ PyMethodDef calls_methods[] = {{"call", FASTCALL(calls_call), nullptr}, {"add", 
                                {nullptr, nullptr, 0, nullptr}};
 PyMethodDef workspaces_methods[] = {{"put", FASTCALL(workspaces_put), nullptr}, {"clear", workspaces_clear, METH_NOARGS, nullptr},
                                     {nullptr, nullptr, 0, nullptr}};
-PyMethodDef module_methods[] = {{"bind", bind, METH_VARARGS, nullptr}, {"linear", FASTCALL(linear), nullptr},
-                                {"event_done", event_done, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyMethodDef fence_methods[] = {{"stream", fence_stream, METH_NOARGS, nullptr}, {"done", fence_done, METH_NOARGS, nullptr},
+                               {"wait", fence_wait, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyMethodDef module_methods[] = {{"bind", bind, METH_VARARGS, nullptr}, {"linear", FASTCALL(linear), nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_fast", nullptr, -1, module_methods, nullptr, nullptr, nullptr, nullptr};
 
 bool is_workspaces(PyObject* o) {
   return Py_TYPE(o)->tp_dealloc == object_free<PyWorkspaces, Workspaces, &PyWorkspaces::table>;
 }
 
-template <typename Object, typename Data, Data* Object::*Field>
-bool add_type(PyObject* module, const char* name, const char* qualified, PyMethodDef* methods) {
+template <typename Object>
+bool add_type(PyObject* module, const char* name, const char* qualified, PyMethodDef* methods, newfunc make, destructor free) {
   static PyTypeObject type = {PyVarObject_HEAD_INIT(nullptr, 0)};
   type.tp_name = qualified;
   type.tp_basicsize = sizeof(Object);
   type.tp_flags = Py_TPFLAGS_DEFAULT;
   type.tp_methods = methods;
-  type.tp_new = object_new<Object, Data, Field>;
-  type.tp_dealloc = object_free<Object, Data, Field>;
+  type.tp_new = make;
+  type.tp_dealloc = free;
   if (PyType_Ready(&type) < 0) return false;
   return PyModule_AddObjectRef(module, name, reinterpret_cast<PyObject*>(&type)) == 0;
 }
@@ -512,8 +560,11 @@ bool add_type(PyObject* module, const char* name, const char* qualified, PyMetho
 PyMODINIT_FUNC PyInit__fast() {
   PyObject* m = PyModule_Create(&module_def);
   if (!m) return nullptr;
-  if (!add_type<PyCalls, Calls, &PyCalls::calls>(m, "Calls", "wave_b200._fast.Calls", calls_methods) ||
-      !add_type<PyWorkspaces, Workspaces, &PyWorkspaces::table>(m, "Workspaces", "wave_b200._fast.Workspaces", workspaces_methods)) {
+  if (!add_type<PyCalls>(m, "Calls", "wave_b200._fast.Calls", calls_methods, object_new<PyCalls, Calls, &PyCalls::calls>,
+                         object_free<PyCalls, Calls, &PyCalls::calls>) ||
+      !add_type<PyWorkspaces>(m, "Workspaces", "wave_b200._fast.Workspaces", workspaces_methods, object_new<PyWorkspaces, Workspaces, &PyWorkspaces::table>,
+                              object_free<PyWorkspaces, Workspaces, &PyWorkspaces::table>) ||
+      !add_type<PyFence>(m, "Fence", "wave_b200._fast.Fence", fence_methods, fence_new, fence_free)) {
     Py_DECREF(m);
     return nullptr;
   }

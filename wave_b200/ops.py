@@ -18,8 +18,13 @@ from . import _lib
 SCALE_GROUP_SIZE = 32
 
 
+# The handle of a device's current stream, without an object around it (torch.cuda.current_stream(i).cuda_stream is a microsecond, and a call that is not
+# recognised in native code asks five times)
+raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda idx: torch.cuda.current_stream(idx).cuda_stream)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream(torch.cuda.current_device()).cuda_stream  # (without the index it takes twice as long to find)
+    return raw_stream(torch.cuda.current_device())
 
 
 def _as_u8(t: torch.Tensor, what: str) -> torch.Tensor:
@@ -40,7 +45,7 @@ class PackedScales:
 
     def __init__(self, data: torch.Tensor, rows: int, K: int, tile_rows: int = 128):
         self.data, self.rows, self.K, self.tile_rows = data, rows, K, tile_rows
-        self.made = None  # WeightScaleCache: (stream, event behind the kernel that fills it, None once that is known to be complete)
+        self.made = None  # WeightScaleCache: (stream, fence behind the kernel that fills it, None once that is known to be complete)
 
     @property
     def device(self):
@@ -179,7 +184,7 @@ class WorkspacePool:
     def get(self, device: torch.device, nbytes: int, kind: str) -> torch.Tensor:
         idx = device.index if device.index is not None else torch.cuda.current_device()
         capturing = torch.cuda.is_current_stream_capturing()
-        key = (idx, torch.cuda.current_stream(idx).cuda_stream, kind)
+        key = (idx, raw_stream(idx), kind)
         ws = self._by_key.get(key)
         if ws is not None and ws.numel() >= nbytes:
             if not capturing:
@@ -196,8 +201,11 @@ class WorkspacePool:
             self._outgrown.append(ws)
             nbytes = max(nbytes, 2 * ws.numel())
         ws = torch.empty(nbytes, dtype=torch.uint8, device=torch.device("cuda", idx))
-        with torch.cuda.device(idx):
-            _lib.check(_lib.load().wb200_workspace_init(ws.data_ptr(), nbytes, _stream()))
+        if idx == torch.cuda.current_device():
+            _lib.check(_lib.load().wb200_workspace_init(ws.data_ptr(), nbytes, key[1]))
+        else:
+            with torch.cuda.device(idx):
+                _lib.check(_lib.load().wb200_workspace_init(ws.data_ptr(), nbytes, key[1]))
         self._by_key[key] = ws
         self._note(key, ws)
         return ws
@@ -407,6 +415,23 @@ def scaled_gemm_mxfp8_packed(a: torch.Tensor, a_sf: PackedScales, b: torch.Tenso
         _lib.check(rc)
 
 
+class _Fence:
+    """Fence of the host module (csrc/fast_call.cpp), where that cannot be used: whether a stream is through with its work is not asked in a capture."""
+
+    def __init__(self, idx: int):
+        self._idx, self._stream, self._event = idx, torch.cuda.current_stream(idx), torch.cuda.Event()
+        self._event.record(self._stream)
+
+    def stream(self) -> int:
+        return self._stream.cuda_stream
+
+    def done(self) -> bool:
+        return not torch.cuda.is_current_stream_capturing() and self._event.query()
+
+    def wait(self) -> None:
+        torch.cuda.current_stream(self._idx).wait_event(self._event)
+
+
 class WeightScaleCache:
     """Packed copies of weight scales, so that a weight's scales are repacked once and reused by later calls.
 
@@ -444,9 +469,9 @@ class WeightScaleCache:
         self.packings += 1
         if self._keep_if_captured(packed):
             return packed
-        stream, event = torch.cuda.current_stream(packed.device), torch.cuda.Event()
-        event.record(stream)
-        packed.made = (stream.cuda_stream, event)
+        native = _lib.fast()
+        fence = (_Fence if native is None else native.Fence)(packed.device.index)
+        packed.made = (fence.stream(), fence)
         self._make_room()
         self._entries[key] = (weakref.ref(scale), packed)
         while len(self._entries) > self.capacity:
@@ -467,19 +492,18 @@ class WeightScaleCache:
     def _usable(packed: PackedScales) -> bool:
         """Whether what the current stream does next may read the packing, after a wait where one is needed. False while a graph is captured
         and the packing is not known to be complete: a replay may come at any time and on any stream."""
-        stream, event = packed.made
+        stream, fence = packed.made
         capturing = torch.cuda.is_current_stream_capturing()
-        if event is not None:
-            native = _lib.fast()  # (asks in a way that does not end another thread's capture, or this one)
-            if native.event_done(event.cuda_event) if native is not None else not capturing and event.query():
-                packed.made, event = (stream, None), None
+        if fence is not None:
+            if fence.done():
+                packed.made, fence = (stream, None), None
             elif capturing:
                 return False
         if not capturing:
             current = torch.cuda.current_stream(packed.device)
             if current.cuda_stream != stream:
-                if event is not None:
-                    current.wait_event(event)
+                if fence is not None:
+                    fence.wait()
                 packed.data.record_stream(current)
         return True
 
