@@ -137,7 +137,8 @@ size_t wb200_packed_scale_bytes(int rows, int K);
 int wb200_decode_tile_rows(int N);
 /* The height for calls of one M and K (weight_bits / activation_bits: 4 or 8; c_rows_aligned: every row of c starts on 16 bytes),
  * 128 where the usual packing is the faster one: also with fewer 128-row tiles than SMs, where one low tile per SM is ahead of cutting K
- * as long as K is short for the height, and with a thin last round over a short K. A height for which N has fewer tiles than SMs is
+ * as long as K is short for the height, and with a thin last round over a short K. The packing for h rows has about 128 / h times the bytes of the
+ * usual one (wb200_packed_scale_bytes_tiled): as many as the weight itself at h = 8, which N <= 1184 gets on 148 SMs. A height for which N has fewer tiles than SMs is
  * read only if it is the lowest one with at most one tile per SM. */
 int wb200_decode_tile_rows_for(int M, int N, int K, int weight_bits, int activation_bits, int c_rows_aligned);
 /* wb200_decode_tile_rows for the mixed pair (8-bit activations, 4-bit weights, WB200_B_FP4): where it returns a height above 128 (up to

@@ -1366,8 +1366,9 @@ static int repack_scales_impl(const void* src, long long src_row_stride, int row
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  // Beside the tail of the kernel before it up to one CTA per SM: the GEMM behind a larger one runs for 100 us and more under the power
-  // limit, where the gap costs nothing (8192^3 in a loop, ordinary / programmatic: 213.2 / 215.9 us).
+  // Beside the tail of the kernel before it up to one CTA per SM. Behind a larger one there is mostly a GEMM that the power limit bounds, where the gap costs
+  // nothing (us in a loop, ordinary / programmatic: 8192^3 213.2 / 215.9, 4096^3 30.4 / 31.2, 2048 x 4096 x 8192 27.1 / 27.2). The line does not know N: in front
+  // of a short GEMM over a long K the gap shows (2048 x 512 x 16384 16.4 / 15.1, 2048 x 2048 x 16384 28.7 / 27.0, 3000 x 4096 x 8192 41 / 39).
   cfg.numAttrs = tl_dependent_launch || grid.x * grid.y <= unsigned(dev->sm_count) ? 1 : 0;
   WB_CUDA(cudaLaunchKernelEx(&cfg, wb::repack_scales_kernel, static_cast<const uint8_t*>(src), src_row_stride, rows, K / 32,
                              k_atoms, static_cast<uint8_t*>(dst), broadcast, tl_dependent_launch, release, block_rows));

@@ -316,13 +316,14 @@ __device__ __forceinline__ uint32_t idesc_with_sf_id(uint32_t idesc, uint32_t sf
 // finished and its writes are visible (a no-op in a kernel launched without the attribute).
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// How a kernel of this library stands in its stream. Every launch carries the programmatic attribute: a kernel that is started the
-// ordinary way behind another one begins 1 to 2 us after that one's end (on the B200 the gap is rounded up to a 2.048 us
-// raster: 1024^3 alone 8.20 us a launch back to back, 5.36 with the attribute).
+// How a kernel of this library stands in its stream. GEMMs, and the repack, MXFP4 quantiser and routing kernels in front of them up to the sizes that
+// api.cu states, are programmatic launches: a kernel that is started the ordinary way behind another one begins 1 to 2 us after that
+// one's end (on the B200 the gap is rounded up to a 2.048 us raster: 1024^3 alone 8.2 us a launch back to back, 5.4 with the attribute).
 //   kDependent: the kernel before it is the library's own, of the same call (or the caller says WB200_OVERLAP_PREVIOUS): it may touch what
 //     that kernel does not write before it waits, and release its own dependents at once.
 //   kFirst: anything may come before it. It waits before it touches memory, and releases its dependents after that: whoever starts
-//     then finds everything before this kernel complete.
+//     then finds everything before this kernel complete. (One that may write a weight, which a kDependent kernel two launches on
+//     reads before it waits, does not release them: quantize.cuh, scales.cuh.)
 // What a kernel reads after its wait it reads with ordinary loads, not through the non-coherent path: the data may have been
 // written while the kernel was already resident.
 enum : int { kFirst = 0, kDependent = 1 };

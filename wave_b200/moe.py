@@ -4,18 +4,18 @@ The reference's MoE is a Python loop over experts calling an f16/bf16 GEMM, `sil
 second GEMM per expert, followed by a weighted sum (tests/kernel/moe_test.py:183-260; kernels in
 wave_lang/kernel/wave/templates/moe.py). Its block-alignment step exists as a torch function
 (tests/kernel/moe/torch_kernels.py:10-97). Here every step is a CUDA kernel behind the C ABI and the
-two projections are grouped MXFP4 GEMMs over all experts at once. `MXFP4ExpertMLP` runs one native call of six launches:
+two projections are grouped MXFP4 GEMMs over all experts at once. `MXFP4ExpertMLP` runs one native call of five launches:
 
-    softmax and top-k -> block alignment -> quantise tokens into their sorted rows -> GEMM gate|up with silu(gate) * up
+    softmax, top-k and ranks per block of tokens -> quantise tokens into their sorted rows -> GEMM gate|up with silu(gate) * up
           and its MXFP4 quantisation in the epilogue -> GEMM down -> weighted combine
 
-with 256-row blocks on the CTA-pair tile kernel, and up to 128 tokens with 128-row blocks on the decode kernel. What that
+with 256-row blocks on the CTA-pair tile kernel, and up to 128 tokens of four, the first two in one, with 128-row blocks on the decode kernel. What that
 call is not built for (`_takes_fused`) runs the steps one by one, each of them a function of this module:
 
     route -> moe_align_block_size(256) -> quantize_scatter -> moe_scaled_gemm (gate|up) -> silu_and_mul with
           MXFP4 quantisation -> moe_scaled_gemm (down) -> combine
 
-Either way the GEMMs read the routing (expert of every block, padded row count) from the device arrays the alignment kernel
+Either way the GEMMs read the routing (expert of every block, padded row count) from the device arrays the kernels before them
 wrote, so a forward pass has no host synchronisation.
 """
 
