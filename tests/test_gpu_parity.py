@@ -2169,3 +2169,21 @@ def test_calls_through_a_library_that_was_replaced_are_seen(where, monkeypatch):
     calls()
     assert len(seen) == 6
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("rows", [4, 300])
+def test_a_captured_linear_call_follows_a_state_dict(rows):
+    """The graph holds the addresses of codes and packings: both stay where they are when a state dict is loaded, and a replay reads what it brought."""
+    g = torch.Generator().manual_seed(rows)
+    one, two = (wb.MXFP4Linear.from_float((torch.randn(4096, 512, generator=g) * 0.02).to(DEV)) for _ in range(2))
+    x = torch.randn(rows, 512, generator=g).to(DEV)
+    one(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = one(x)
+    at = one._packed.data.data_ptr(), one._packed_low.data.data_ptr()
+    one.load_state_dict(two.state_dict())
+    assert at == (one._packed.data.data_ptr(), one._packed_low.data.data_ptr())
+    graph.replay()
+    assert torch.equal(y, two(x)) and torch.equal(one(x), two(x))
+    ops.check_device_status()

@@ -30,12 +30,19 @@ class MXFP4Linear(torch.nn.Module):
     # Decode calls (at most 128 rows) may read a second packing, per tile of the height h that gives every SM the same number of
     # weight tiles: one height per layer, as it follows from out_features, and 128 / h times the bytes of the usual packing. Made with that one, not
     # by the first call that reads it: other streams' calls would have to wait for that call's.
-    _packed_low = None
+    _packed = _packed_low = None
 
     def _pack(self) -> None:
-        self._packed = ops.repack_scales(self.weight_scales)
+        self._packed = self._pack_as(self._packed, 128)
         h = self._low_rows()
-        self._packed_low = None if h == 128 else ops.repack_scales(self.weight_scales, tile_rows=h)
+        self._packed_low = None if h == 128 else self._pack_as(self._packed_low, h)
+
+    def _pack_as(self, old: ops.PackedScales | None, tile_rows: int) -> ops.PackedScales:
+        """In the memory of the packing that there is, if it is of that form: captured graphs hold its address, as they hold that of the codes,
+        which a state dict is copied into."""
+        s = self.weight_scales
+        same = old is not None and old.device == s.device and (old.rows, old.K, old.tile_rows) == (s.shape[0], s.shape[1] * ops.SCALE_GROUP_SIZE, tile_rows)
+        return ops.repack_scales(s, out=old.data if same else None, tile_rows=tile_rows)
 
     def _low_rows(self) -> int:
         """The height that decode calls of some number of rows read, 128 where none does. (One of each class that
