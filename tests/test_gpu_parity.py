@@ -1896,13 +1896,13 @@ def test_linear_refuses_codes_that_its_scales_were_not_packed_for(rows):
                 layer(x)
     layer.weight_codes = codes
     packed, low = layer._packed, layer._packed_low
-    native = lambda p, q, r=N, c=codes: _lib.fast().linear(x, c, r, K, p, q, low.tile_rows, layer.output_dtype, ops._pool.fast)  # noqa: E731
+    native = lambda p, q, r=N, c=codes: _lib.fast().linear(x, c, (r, K, p, q, low.tile_rows), layer.output_dtype, ops._pool.fast)  # noqa: E731
     assert torch.equal(native(packed.data, low.data), ref)
     assert native(packed.data[:-512], low.data[:-512]) is None
     assert native(packed.data, low.data, N + 8) is None
     assert native(packed.data, low.data, N, codes.view(torch.int32).repeat(1, 4)) is None
     with pytest.raises(TypeError):
-        _lib.fast().linear(x, codes, N, K, packed.data, low.data, low.tile_rows, layer.output_dtype, [])
+        _lib.fast().linear(x, codes, layer._native_scales, layer.output_dtype, [])
     assert torch.equal(layer(x), ref)
     ops.check_device_status()
 

@@ -283,18 +283,22 @@ def load() -> ctypes.CDLL:
 
 
 _fast = None  # the module, or False where it cannot be used
-_fast_bound: dict = {}  # the library and the functions that it calls
+_fast_lib = None  # the library that it calls,
+_fast_entries: dict = {}  # and the functions of it
+_loader = load  # (`load` may be something else while a caller watches calls)
 
 
-def fast(lib=None, entry: str | None = None):
+def fast(lib=None):
     """The host module for repeated calls (csrc/fast_call.cpp), bound to the loaded library. None, with one warning, where it was not built or was
-    built for another torch: every call then takes the Python code, which is complete and only slower in front of short kernels. None too where `lib` (default: the loaded library) or its function `entry` is not what the module
-    is bound to: a caller has put something in its place, to watch or to redirect calls."""
-    global _fast
+    built for another torch: every call then takes the Python code, which is complete and only slower in front of short kernels. None too where
+    `lib` (default: the loaded library) is not the one that the module is bound to."""
+    global _fast, _fast_lib
     if lib is None:
         lib = load()
     if _fast is None:
-        if not isinstance(lib, ctypes.CDLL):
+        names = ("wb200_mxfp4_gemm_repack_a", "wb200_mxfp8_gemm_repack_a", "wb200_mxfp4_gemm_quantize_a", "wb200_mxfp4_gemm_workspace_bytes",
+                 "wb200_decode_tile_rows_for")
+        if not isinstance(lib, ctypes.CDLL) or not all(isinstance(getattr(lib, name), lib._FuncPtr) for name in names):
             return None
         try:
             from . import _fast as module, build
@@ -305,14 +309,10 @@ def fast(lib=None, entry: str | None = None):
             warnings.warn(f"wave_b200._fast cannot be used ({e}): repeated calls take the slower Python path. Build it with "
                           "`python -m wave_b200.build`", RuntimeWarning, stacklevel=2)
             return None
-        names = ("wb200_mxfp4_gemm_repack_a", "wb200_mxfp8_gemm_repack_a", "wb200_mxfp4_gemm_quantize_a", "wb200_mxfp4_gemm_workspace_bytes",
-                 "wb200_decode_tile_rows_for")
-        _fast_bound.update({name: getattr(lib, name) for name in names}, lib=lib)
-        module.bind(*(ctypes.cast(_fast_bound[name], ctypes.c_void_p).value for name in names))
-        _fast = module
-    if not _fast or lib is not _fast_bound["lib"] or (entry is not None and getattr(lib, entry) is not _fast_bound[entry]):
-        return None
-    return _fast
+        _fast_entries.update({name: getattr(lib, name) for name in names})
+        module.bind(*(ctypes.cast(_fast_entries[name], ctypes.c_void_p).value for name in names))
+        _fast, _fast_lib = module, lib
+    return _fast if _fast and lib is _fast_lib else None
 
 
 def check(rc: int) -> None:

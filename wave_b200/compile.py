@@ -126,17 +126,19 @@ class ScaledGemmKernel:
         self._plans: dict = {}
         self._tile_rows: dict = {}
         self._lib = _lib.load()
-        self._entry = "wb200_mxfp8_gemm_repack_a" if template.element_bits == 8 else "wb200_mxfp4_gemm_repack_a"  # what a native call calls
         native = _lib.fast(self._lib)
         self._fast = native.Calls() if native is not None else None  # calls made before, recognised in native code
+        # what that module calls: not used where a caller has put something in the place of the library or of one of these functions
+        self._bound_lib = self._lib if native is not None else None
+        self._bound4, self._bound8 = (_lib._fast_entries.get(f"wb200_{kind}_gemm_repack_a") for kind in ("mxfp4", "mxfp8"))
         self._weight_scales = ops.WeightScaleCache(recent=self._fast.recent if self._fast is not None else None)
         self._static = None
         if template.shape is not None and not options.dynamic_symbols:
             self._static = tuple(template.shape)
 
     # the reference offers both spellings
-    def __call__(self, *args):
-        return self.invoke(*args)
+    def __call__(self, a, a_scale, b, b_scale, c):
+        return self.invoke(a, a_scale, b, b_scale, c)
 
     def invoke(self, a, a_scale, b, b_scale, c) -> None:
         if self.options.run_bench and not getattr(self, "_in_bench", False):
@@ -147,7 +149,8 @@ class ScaledGemmKernel:
             finally:
                 self._in_bench = False
             return None
-        if self._fast is not None and _lib.fast(self._lib, self._entry) is not None:
+        lib = self._lib
+        if lib is self._bound_lib and lib.wb200_mxfp4_gemm_repack_a is self._bound4 and lib.wb200_mxfp8_gemm_repack_a is self._bound8:
             options = self.options
             rc = self._fast.call(a, a_scale, b, b_scale, c, options.decode_tiled_weight_scales, options.kernel_path)
             if rc is not None:

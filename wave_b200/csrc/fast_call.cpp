@@ -150,7 +150,15 @@ struct Calls {
   std::unordered_map<CallKey, Plan, CallKeyHash> plans;
   std::unordered_multimap<const c10::TensorImpl*, Weight> weights;
   uint64_t now = 0, asked = 0;  // calls so far, and when the Python code last asked which packings were used
+  const std::pair<const CallKey, Plan>* last = nullptr;  // the plan of the last call (entries keep their place until they are erased)
 
+  const Plan* find(const CallKey& key) {
+    if (last && last->first == key) return &last->second;
+    const auto it = plans.find(key);
+    if (it == plans.end()) return nullptr;
+    last = &*it;
+    return &it->second;
+  }
   Weight* find(const at::Tensor& scale, const Signature& sig, int tile_rows) {
     const auto [first, last] = weights.equal_range(scale.unsafeGetTensorImpl());
     for (auto it = first; it != last; ++it) {
@@ -213,8 +221,7 @@ PyObject* calls_call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
       if (PyErr_Occurred()) return nullptr;
       Py_RETURN_NONE;
     }
-    const auto plan = calls.plans.find(key);
-    const Plan* found = plan == calls.plans.end() ? nullptr : &plan->second;
+    const Plan* found = calls.find(key);
     Weight* weight = found ? calls.find(THPVariable_Unpack(args[3]), key.sig[3], found->tile_rows) : nullptr;
     if (!weight || !(weight->complete || weight->stream == key.stream)) Py_RETURN_NONE;
     weight->used = ++calls.now;
@@ -273,7 +280,10 @@ PyObject* calls_add(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     if (args[10] != Py_None) p.workspace = THPVariable_Unpack(args[10]);
     p.workspace_bytes = size_t(ws_bytes);
     p.marks = Ref(args[11]);
-    if (calls.plans.size() >= kMaxPlans && !calls.plans.count(key)) calls.plans.erase(calls.plans.begin());
+    if (calls.plans.size() >= kMaxPlans && !calls.plans.count(key)) {
+      calls.last = nullptr;
+      calls.plans.erase(calls.plans.begin());
+    }
     const int tile_rows = p.tile_rows;
     calls.plans[key] = std::move(p);
     const at::Tensor& scale = THPVariable_Unpack(args[3]);
@@ -296,6 +306,7 @@ PyObject* calls_add(PyObject* self, PyObject* const* args, Py_ssize_t n) {
 
 PyObject* calls_clear(PyObject* self, PyObject*) {
   Calls& calls = *reinterpret_cast<PyCalls*>(self)->calls;
+  calls.last = nullptr;
   calls.plans.clear();
   calls.weights.clear();
   Py_RETURN_NONE;
@@ -443,22 +454,23 @@ bool holds_scales(const at::Tensor& packed, int64_t N, int64_t K, int64_t tile_r
   return packed.scalar_type() == at::kByte && packed.is_contiguous() && packed.numel() >= (N + tile_rows - 1) / tile_rows * ((K + 255) / 256) * 1024;
 }
 
-// linear(x, weight_codes, rows and K that the scales were packed for, packed scales, those per tile of low_rows rows or None, low_rows,
-//        output dtype, workspaces)
+// linear(x, weight_codes, (rows and K that the scales were packed for, packed scales, those per tile of low_rows rows, low_rows), output dtype,
+//        workspaces)
 // -> dequant(quantise(x)) @ dequant(W)^T, or None: left to the Python code.
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 9 || !is_workspaces(args[8])) {
-    PyErr_SetString(PyExc_TypeError, "linear takes 9 arguments, the last one a Workspaces object");
+  if (n != 5 || !PyTuple_Check(args[2]) || PyTuple_GET_SIZE(args[2]) != 5 || !is_workspaces(args[4])) {
+    PyErr_SetString(PyExc_TypeError, "linear takes 5 arguments, the third a tuple of 5 and the last one a Workspaces object");
     return nullptr;
   }
+  PyObject* const* scales = reinterpret_cast<PyTupleObject*>(args[2])->ob_item;
   try {
-    if (!plain(args[0]) || !plain(args[1]) || !plain(args[4]) || !THPDtype_Check(args[7])) Py_RETURN_NONE;
+    if (!plain(args[0]) || !plain(args[1]) || !plain(scales[2]) || !THPDtype_Check(args[3])) Py_RETURN_NONE;
     const at::Tensor &x = THPVariable_Unpack(args[0]), &w = THPVariable_Unpack(args[1]);
-    at::Tensor packed = THPVariable_Unpack(args[4]);
-    const long long rows = PyLong_AsLongLong(args[2]), of_k = PyLong_AsLongLong(args[3]);
+    at::Tensor packed = THPVariable_Unpack(scales[2]);
+    const long long rows = PyLong_AsLongLong(scales[0]), of_k = PyLong_AsLongLong(scales[1]);
     if (PyErr_Occurred()) return nullptr;
     const int device = x.device().index();
-    const at::ScalarType x_type = x.scalar_type(), out_type = reinterpret_cast<THPDtype*>(args[7])->scalar_type;
+    const at::ScalarType x_type = x.scalar_type(), out_type = reinterpret_cast<THPDtype*>(args[3])->scalar_type;
     const int64_t dims = x.dim();
     if (device != c10::cuda::current_device() || w.device().index() != device || packed.device().index() != device || dims < 1 || w.dim() != 2 ||
         !w.is_contiguous() || w.element_size() != 1 || (x_type != at::kFloat && x_type != at::kBFloat16) || (out_type != at::kFloat && out_type != at::kBFloat16))
@@ -476,7 +488,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     size_t ws_bytes = 0;
     if (M <= 128) {
       ws_bytes = abi.gemm_workspace_bytes(int(M), int(N), int(K));
-      for (const auto& e : reinterpret_cast<PyWorkspaces*>(args[8])->table->entries)
+      for (const auto& e : reinterpret_cast<PyWorkspaces*>(args[4])->table->entries)
         if (e.device == device && e.stream == stream.stream()) {
           ws = e.ws;
           mark = e.mark;
@@ -487,11 +499,11 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const bool aligned = M == 1 || N * (out_type == at::kFloat ? 4 : 2) % 16 == 0;
     int tile_rows = 128;
     if (M <= 128 && (tile_rows = abi.decode_tile_rows_for(int(M), int(N), int(K), 4, 4, aligned)) != 128) {
-      if (args[5] == Py_None || PyLong_AsLong(args[6]) != tile_rows || !plain(args[5])) {
+      if (PyLong_AsLong(scales[4]) != tile_rows || !plain(scales[3])) {
         if (PyErr_Occurred()) return nullptr;
         Py_RETURN_NONE;
       }
-      packed = THPVariable_Unpack(args[5]);
+      packed = THPVariable_Unpack(scales[3]);
       if (packed.device().index() != device) Py_RETURN_NONE;
     }
     if (!holds_scales(packed, N, K, tile_rows)) Py_RETURN_NONE;

@@ -14,6 +14,20 @@ from . import _lib, ops
 from .lang import as_output_dtype
 
 
+_entry = None  # the function that the host module calls
+
+
+def _native():
+    """The host module, unless it cannot be used or a caller has put something in the place of what it calls, to watch or to redirect calls."""
+    global _entry
+    if _entry is None and _lib.fast() is not None:
+        _entry = _lib._fast_entries["wb200_mxfp4_gemm_quantize_a"]
+    lib = _lib._lib
+    if not _lib._fast or _lib.load is not _lib._loader or lib is not _lib._fast_lib or lib.wb200_mxfp4_gemm_quantize_a is not _entry:
+        return None
+    return _lib._fast
+
+
 class MXFP4Linear(torch.nn.Module):
     def __init__(self, weight_codes: torch.Tensor, weight_scales: torch.Tensor, output_dtype=torch.bfloat16):
         """weight_codes [N, K/2] uint8, weight_scales [N, K/32] uint8 (row-major E8M0), both on the GPU. The GEMM reads the scales in
@@ -31,11 +45,14 @@ class MXFP4Linear(torch.nn.Module):
     # weight tiles: one height per layer, as it follows from out_features, and 128 / h times the bytes of the usual packing. Made with that one, not
     # by the first call that reads it: other streams' calls would have to wait for that call's.
     _packed = _packed_low = None
+    _native_scales = None  # of both, as the native call takes them
 
     def _pack(self) -> None:
         self._packed = self._pack_as(self._packed, 128)
         h = self._low_rows()
         self._packed_low = None if h == 128 else self._pack_as(self._packed_low, h)
+        low = self._packed_low or self._packed
+        self._native_scales = self._packed.rows, self._packed.K, self._packed.data, low.data, low.tile_rows
 
     def _pack_as(self, old: ops.PackedScales | None, tile_rows: int) -> ops.PackedScales:
         """In the memory of the packing that there is, if it is of that form: captured graphs hold its address, as they hold that of the codes,
@@ -72,12 +89,10 @@ class MXFP4Linear(torch.nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         # a call whose tensors need no preparation; anything else comes back unhandled
-        native = _lib.fast(None, "wb200_mxfp4_gemm_quantize_a")
-        if native is None:
+        native, scales = _native(), self._native_scales
+        if native is None or scales is None:
             return self._forward_checked(x)
-        packed, low = self._packed, self._packed_low
-        y = native.linear(x, self._buffers.get("weight_codes"), packed.rows, packed.K, packed.data, None if low is None else low.data,
-                          128 if low is None else low.tile_rows, self.output_dtype, ops._pool.fast)
+        y = native.linear(x, self._buffers.get("weight_codes"), scales, self.output_dtype, ops._pool._fast or ops._pool.fast)
         if type(y) is int:
             _lib.check(y)
         elif y is not None:
